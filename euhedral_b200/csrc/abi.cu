@@ -806,8 +806,8 @@ int euhedral_cuda_linear_nvfp4_bf16(const void* input, const void* weights, void
                        : nvfp4_decode<nvfp4::Format, false>(state, input, weights, output, rows, in_features, out_features);
 }
 
-// Process-wide: native calls of 512 rows and more run on CTA pairs (tcgen05 cta_group::2). Off unless selected.
-static std::atomic<bool> g_native_pairs{false};
+// Process-wide: native calls of 1024 rows and more run on CTA pairs (tcgen05 cta_group::2), unless switched off.
+static std::atomic<bool> g_native_pairs{true};
 
 void euhedral_b200_select_native_pairs(int enabled) { g_native_pairs.store(enabled != 0); }
 

@@ -47,8 +47,13 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
 // those of the plan's epilogue kernel), times 1/sqrt(128), times svh, BF16. No other thread is needed.
 __device__ __forceinline__ void store_rotated(uint32_t (&r)[4][32], uint16_t* __restrict__ out, const uint16_t* __restrict__ svh) {
     float* v = reinterpret_cast<float*>(&r[0][0]);
+    const bool wide = (reinterpret_cast<uintptr_t>(out) & 31u) == 0;
 #pragma unroll
-    for (int i = 0; i < 128; ++i) v[i] = eb::bf16_bits_to_float(eb::float_to_bf16_bits(v[i]));
+    for (int i = 0; i < 128; i += 2) {
+        const uint32_t pair = eb::bf16_pair(v[i], v[i + 1]);
+        v[i] = eb::bf16_bits_to_float(pair & 0xFFFFu);
+        v[i + 1] = __uint_as_float(pair & 0xFFFF0000u);
+    }
 #pragma unroll
     for (int h = 1; h < 128; h <<= 1) {
 #pragma unroll
@@ -60,21 +65,21 @@ __device__ __forceinline__ void store_rotated(uint32_t (&r)[4][32], uint16_t* __
         }
     }
 #pragma unroll
-    for (int c = 0; c < 16; ++c) {
-        const uint4 scales = *reinterpret_cast<const uint4*>(svh + 8 * c);
-        const uint32_t sw[4] = {scales.x, scales.y, scales.z, scales.w};
-        uint32_t packed[4];
+    for (int c = 0; c < 8; ++c) {
+        uint32_t packed[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            uint32_t bits[2];
+        for (int h = 0; h < 2; ++h) {
+            const uint4 scales = *reinterpret_cast<const uint4*>(svh + 16 * c + 8 * h);
+            const uint32_t sw[4] = {scales.x, scales.y, scales.z, scales.w};
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const float scale = __half2float(__ushort_as_half((unsigned short)(sw[i] >> (16 * e))));
-                bits[e] = eb::float_to_bf16_bits(__fmul_rn(scale, __fmul_rn(v[8 * c + 2 * i + e], trellis::kInvSqrt128)));
+            for (int i = 0; i < 4; ++i) {
+                const float2 scale = __half22float2(*reinterpret_cast<const __half2*>(&sw[i]));
+                const float* at = v + 16 * c + 8 * h + 2 * i;
+                packed[4 * h + i] = eb::bf16_pair(__fmul_rn(scale.x, __fmul_rn(at[0], trellis::kInvSqrt128)),
+                        __fmul_rn(scale.y, __fmul_rn(at[1], trellis::kInvSqrt128)));
             }
-            packed[i] = bits[0] | bits[1] << 16;
         }
-        *reinterpret_cast<uint4*>(out + 8 * c) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        nvfp4n::store_16(out + 16 * c, packed, wide);
     }
 }
 
@@ -228,15 +233,6 @@ constexpr uint32_t kPairShared = kPairStages * kPairStageBytes + 256u + 1024u;
 constexpr uint32_t kPairInstruction = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((256u >> 4) << 24);
 constexpr uint32_t kPairRows = 512;
 
-// A tiled TMA load of a CTA of a pair whose completion is counted on a barrier of either CTA of the pair (`bar`: a
-// shared::cluster address). No multicast: the box lands in the executing CTA's shared memory only.
-__device__ __forceinline__ void pair_tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                         eb::smem_u32(dst)),
-            "l"(map), "r"(c0), "r"(c1), "r"(bar)
-            : "memory");
-}
-
 __device__ __forceinline__ void pair_mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
     asm volatile(
             "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
@@ -312,8 +308,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_ge
                     // both CTAs' boxes are counted on the even CTA's barrier, where the thread that issues the MMAs waits
                     if (rank == 0u) eb::mbar_arrive_expect_tx(&full[s], 2u * kPairStageBytes);
                     const uint32_t bar = eb::map_to_rank(eb::smem_u32(&full[s]), 0u);
-                    pair_tma_load_2d(stage, &map_a, (int)((ks * kStepK) % a_period), (int)(row_tile * kTileM), bar);
-                    pair_tma_load_2d(stage + kATile, &map_b, (int)(ks * kStepK), (int)(weight_tile * 128u), bar);
+                    nvfp4n::pair_tma_load_2d(stage, &map_a, (int)((ks * kStepK) % a_period), (int)(row_tile * kTileM), bar);
+                    nvfp4n::pair_tma_load_2d(stage + kATile, &map_b, (int)(ks * kStepK), (int)(weight_tile * 128u), bar);
                 }
             }
         }
@@ -369,7 +365,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_ge
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             nvfp4n::tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0) nvfp4n::arrive_at_rank(&acc_empty[buffer], 0u);
+            if (lane == 0) nvfp4n::signal_rank(&acc_empty[buffer], 0u);   // what it orders are tensor-memory reads
             const uint32_t row = (2u * tm + rank) * kTileM + quarter * 32u + lane, col = paired ? tn * 128u + half * 64u : tn * kTileN + half * 128u;
             if (svh == nullptr) {
                 nvfp4n::store_block(r, out, row, rows, n, col, 1.0f, paired);   // row stride n

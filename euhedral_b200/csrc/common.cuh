@@ -25,6 +25,12 @@ __device__ __forceinline__ uint16_t float_to_bf16_bits(float value) {
     return (uint16_t)(bits >> 16);
 }
 __device__ __forceinline__ float bf16_bits_to_float(uint32_t bits) { return __uint_as_float(bits << 16); }
+// Two floats rounded to nearest even into one BF16 pair by the hardware conversion (low half from `low`); for finite values
+// the bits of float_to_bf16_bits.
+__device__ __forceinline__ uint32_t bf16_pair(float low, float high) {
+    const __nv_bfloat162 both = __floats2bfloat162_rn(low, high);
+    return *reinterpret_cast<const uint32_t*>(&both);
+}
 
 // ---- programmatic dependent launch -----------------------------------------------------------------------------
 // No-ops unless the launch carries the programmatic-stream-serialization attribute.

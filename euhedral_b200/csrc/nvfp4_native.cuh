@@ -8,20 +8,26 @@
 // run in increasing order with one MMA per term into the same FP32 accumulator; the result is
 // bf16(acc * row scale * tensor scale).
 //
-// Three launches per call, all on the selected stream, no allocation (everything lives in the caller's scratch):
+// Two launches per call, all on the selected stream, no allocation (everything lives in the caller's scratch):
 //   1. quantize_rows: BF16 rows -> code planes [term][row][K/2], block scales already in the layout tcgen05 wants
 //      (512-byte atoms of 128 rows x 4 scales, byte (r % 32) * 16 + (r / 32) * 4 + s), one FP32 scale per row. One warp
-//      per row; a lane's unit is a K block of 64 values, whose four scales are one 4-byte store into the atom.
-//   2. repack_weight_scales: the tensor's row-major E4M3 scale plane -> the same atom layout (the scales are 1/9 of
-//      the weight bytes; the codes are consumed in place through a tensor map).
-//   3. gemm: persistent CTAs, one per SM, 128 x 256 output tiles, K in steps of 256 through a 3-stage ring.
-//      warp 0 (one lane) issues the TMA loads (codes as 128-byte-swizzled tiles, scale atoms as bulk copies),
-//      warp 1 (one lane) copies the scale atoms to tensor memory (tcgen05.cp) and issues the MMAs
-//      (M 128, N 256, K 64; two terms x four K blocks per stage) and commits to the ring's and the accumulator's
-//      mbarriers, warps 2..9 drain the accumulator into registers (tcgen05.ld), hand it back at once, then scale, round
-//      and store BF16 while the next tile's MMAs already run.
+//      per row.
+//   2. gemm: persistent CTAs, one per SM, 128 x 256 output tiles, K in steps of 256 through a 3-stage ring.
+//      warp 0 (one lane) issues the TMA loads (codes as 128-byte-swizzled tiles, the weights' scale bytes as they lie in the
+//      tensor, the activations' scale atoms as bulk copies), warps 4..7 move the stage's scales from shared memory through
+//      registers into tensor memory (tcgen05.st), warp 1 (one lane) issues the MMAs (M 128, N 256, K 64; two terms x four K
+//      blocks per stage) and commits to the ring's and the accumulator's mbarriers, warps 8..15 drain the accumulator into
+//      registers (tcgen05.ld), hand it back at once, then scale, round and store BF16 while the next tile's MMAs already run.
+//      Calls of kPairRows rows and more run the same on CTA pairs (gemm_pair_kernel).
+// What bounds it: the tensor pipe under the power cap. Copying the scales with tcgen05.cp, as this kernel did before, queues in
+// order with the MMAs (16 copies of about 37 cycles beside 8 MMAs of 135 per stage) and wants the weights' scales re-laid-out by
+// a launch of its own; the registers' way runs beside the MMAs and reads the tensor's plane. What then limited the single-CTA
+// kernel was the epilogue's 16-byte stores (every sector written in halves) and shared-memory bandwidth (12 KB read per MMA
+// and 9 KB filled per 135 cycles at 128 bytes a cycle; the pairs read 8 and fill 7). 4096 x 17408 x 5120 under ncu, in SM
+// cycles: tcgen05.cp 478k; tcgen05.st 428k; with 32-byte stores 379k, on pairs 350k (tensor pipe 86 % active; the clock falls
+// to 1.4 GHz: the rest is power). Back to back: 300 us before, 262 to 277 us now.
 // Tiles are walked in panels of eight tile columns with the row index fastest, so that CTAs running together share
-// weight tiles and re-read activation tiles from L2. Every CTA issues its own loads; there is no cluster.
+// weight tiles and re-read activation tiles from L2. Every CTA issues its own loads.
 #pragma once
 
 #include <cuda.h>
@@ -46,8 +52,9 @@ constexpr uint32_t kStageBytes = kTerms * kATile + kBTile + kSfaStage + kSfbStag
 constexpr uint32_t kBarrierBytes = 128u;
 constexpr uint32_t kSharedBytes = kStages * kStageBytes + kBarrierBytes + 1024u;   // + slack to align to 1024
 constexpr uint32_t kThreads = 320u;                         // TMA warp, MMA warp, eight epilogue warps
+constexpr uint32_t kScaledThreads = 512u;                   // TMA and MMA warps (and two that idle), four scale warps, eight epilogue warps
 constexpr uint32_t kTmemColumns = 512u;
-constexpr uint32_t kTmemSfa = 256u, kTmemSfb = 288u;       // column offsets behind the 256 accumulator columns
+constexpr uint32_t kTmemScales = 256u, kScaleColumns = 64u; // behind the 256 accumulator columns: 64 columns of scales per ring stage
 constexpr uint32_t kPanel = 8u;                            // tile columns per panel of the tile walk
 
 __host__ __device__ inline uint64_t align256(uint64_t v) { return (v + 255ull) & ~255ull; }
@@ -169,26 +176,28 @@ __global__ void __launch_bounds__(32 * kQuantizeWarps, 5) quantize_rows(const __
     if (lane == 0) reinterpret_cast<float*>(scratch + layout.global_offset)[row] = global;
 }
 
-// ---- 2. weight scale repack ---------------------------------------------------------------------------------------------
-// scales[n][K/16] (row-major E4M3 bytes) -> atoms [n / 128][K / 64][512]. One thread per (row, K block): 4 bytes.
-// table != nullptr (layout row-split-k128-sd4-v1): `scales` holds 4-bit indices, two per byte with the even block in the
-// low nibble, into the tensor's 16 E4M3 codes at `table`; the atoms get the codes, so the GEMM is the same for both layouts.
-__global__ void __launch_bounds__(256) repack_weight_scales(const uint8_t* __restrict__ scales, const uint8_t* __restrict__ table,
-        uint8_t* __restrict__ atoms, uint32_t n, uint32_t k_blocks, uint32_t n_padded) {
-    const uint64_t index = (uint64_t)blockIdx.x * 256u + threadIdx.x;
+// ---- 2. table-indexed weight scales ---------------------------------------------------------------------------------------
+// Layout row-split-k128-sd4-v1 only: 4-bit indices, two per byte with the even block in the low nibble, into the tensor's 16
+// E4M3 codes at `table` -> the scale bytes [n][K/16] a plain tensor has, so that the GEMM is the same for both layouts. A
+// thread writes 16 bytes. grid ceil(n * K / 256 / 256).
+__global__ void __launch_bounds__(256) expand_table_scales(const uint8_t* __restrict__ indices, const uint8_t* __restrict__ table,
+        uint8_t* __restrict__ scales, uint32_t count) {
+    const uint32_t index = blockIdx.x * 256u + threadIdx.x;
     eb::pdl_launch_dependents();
-    eb::pdl_wait();   // the GEMM of the call before this one may still be reading these atoms
-    const uint32_t row = (uint32_t)(index / k_blocks), j = (uint32_t)(index % k_blocks);
-    if (row >= n_padded) return;
-    uint32_t word = 0u;
-    if (row < n && table == nullptr) {
-        word = *reinterpret_cast<const uint32_t*>(scales + (uint64_t)row * k_blocks * 4u + 4u * j);
-    } else if (row < n) {
-        const uint32_t pairs = *reinterpret_cast<const uint16_t*>(scales + (uint64_t)row * k_blocks * 2u + 2u * j);   // four indices
+    eb::pdl_wait();   // the GEMM of the call before this one may still be reading these bytes
+    if (index >= count) return;
+    const uint4 t = *reinterpret_cast<const uint4*>(table);
+    const uint2 pairs = reinterpret_cast<const uint2*>(indices)[index];
+    uint32_t words[4];
 #pragma unroll
-        for (uint32_t i = 0; i < 4u; ++i) word |= (uint32_t)table[(pairs >> (4u * i)) & 15u] << (8u * i);
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t four = ((i & 2) ? pairs.y : pairs.x) >> (16 * (i & 1));   // four indices; the upper half is ignored
+        const uint32_t within = four & 0x7777u;
+        const uint32_t low = __byte_perm(t.x, t.y, within), high = __byte_perm(t.z, t.w, within);
+        const uint32_t upper = __byte_perm(0u, 0xFFFFFFFFu, (four >> 1) & 0x4444u);   // a byte of ones where the index is 8 or more
+        words[i] = eb::lop3<eb::kLutSelect>(high, low, upper);
     }
-    *reinterpret_cast<uint32_t*>(atoms + ((uint64_t)(row >> 7) * k_blocks + j) * kAtom + atom_byte(row & 127u, 0)) = word;
+    reinterpret_cast<uint4*>(scales)[index] = make_uint4(words[0], words[1], words[2], words[3]);
 }
 
 // ---- 3. the GEMM ----------------------------------------------------------------------------------------------------------
@@ -211,20 +220,9 @@ __device__ __forceinline__ uint64_t tile_descriptor(const void* smem_tile) {
     d |= (uint64_t)2 << 61;
     return d;
 }
-// Descriptor of a 512-byte scale atom for tcgen05.cp: 32 rows of 16 bytes, no swizzle, 8-row groups 128 bytes apart.
-__device__ __forceinline__ uint64_t atom_descriptor(const void* smem_atom) {
-    uint64_t d = 0;
-    d |= (uint64_t)((eb::smem_u32(smem_atom) & 0x3FFFFu) >> 4);
-    d |= (uint64_t)(128u >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    return d;
-}
 // kind::mxf4nvf4 instruction descriptor: E2M1 x E2M1, UE4M3 scales, both operands K-major, M 128, N 256.
 constexpr uint32_t kInstruction = (1u << 7) | (1u << 10) | ((kTileN >> 3) << 17) | (0u << 23) | ((kTileM >> 4) << 24);
 
-__device__ __forceinline__ void tmem_copy_atom(uint32_t tmem_address, uint64_t descriptor) {
-    asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem_address), "l"(descriptor) : "memory");
-}
 __device__ __forceinline__ void mma_block_scaled(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t sfa_tmem, uint32_t sfb_tmem,
         uint32_t accumulate) {
     asm volatile(
@@ -251,13 +249,44 @@ __device__ __forceinline__ void tmem_load_32(uint32_t (&r)[32], uint32_t address
             : "r"(address));
 }
 
-// A thread's row of an epilogue block, scaled, rounded to BF16 and stored 16 bytes at a time from column col0.
+// 32 consecutive 32-bit columns of the calling warp's 32 lanes from registers into tensor memory.
+__device__ __forceinline__ void tmem_store_32(uint32_t address, const uint32_t (&r)[32]) {
+    asm volatile(
+            "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,"
+            "%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(address),
+            "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+            "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]),
+            "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+            : "memory");
+}
+// Register limit of the calling warpgroup (all of its four warps execute it). The kernels' splits stay within the launch's registers.
+template <int COUNT>
+__device__ __forceinline__ void registers_give_back() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(COUNT)); }
+template <int COUNT>
+__device__ __forceinline__ void registers_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(COUNT)); }
+
+// 16 BF16 values (eight registers) to global memory. A thread's 32 bytes lie in a row of their own, so one 32-byte store per
+// thread writes whole sectors where two of 16 bytes would write each sector in halves. `wide`: dst is 32-byte aligned.
+__device__ __forceinline__ void store_16(uint16_t* dst, const uint32_t (&v)[8], bool wide) {
+    if (wide) {
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]),
+                "r"(v[5]), "r"(v[6]), "r"(v[7])
+                : "memory");
+    } else {
+        reinterpret_cast<uint4*>(dst)[0] = make_uint4(v[0], v[1], v[2], v[3]);
+        reinterpret_cast<uint4*>(dst)[1] = make_uint4(v[4], v[5], v[6], v[7]);
+    }
+}
+
+// A thread's row of an epilogue block, scaled, rounded to BF16 and stored 32 bytes at a time from column col0 (n and col0 are
+// multiples of 64, out is 16-byte aligned).
 // plain: r holds 4 x 32 consecutive columns. paired (the gate/up region): r[0], r[1] are 64 gate columns, r[2], r[3] the 64
 // up columns that match them; out[row][col] = bf16(silu(gate) * up) with gate and up rounded to BF16 first (the reference's
 // region, native/src/nvfp4_native/native.cuh:390-413: the same expression, expf and division).
 __device__ __forceinline__ void store_block(const uint32_t (&r)[4][32], uint16_t* __restrict__ out, uint32_t row, uint32_t rows, uint32_t n,
         uint32_t col0, float scale, bool paired) {
     if (row >= rows) return;
+    const bool wide = (reinterpret_cast<uintptr_t>(out) & 31u) == 0;
 #pragma unroll
     for (uint32_t cb = 0; cb < 4u; ++cb) {
         if (paired && cb >= 2u) break;
@@ -265,14 +294,14 @@ __device__ __forceinline__ void store_block(const uint32_t (&r)[4][32], uint16_t
         if (col >= n) continue;
         uint16_t* dst = out + (uint64_t)row * n + col;
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            uint32_t packed[4];
+        for (int v = 0; v < 2; ++v) {
+            uint32_t packed[8];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < 8; ++i) {
                 float value[2];
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    const int c = 8 * v + 2 * i + e;
+                    const int c = 16 * v + 2 * i + e;
                     const float first = __fmul_rn(__uint_as_float(r[cb][c]), scale);
                     if (paired) {
                         const float gate = eb::bf16_bits_to_float(eb::float_to_bf16_bits(first));
@@ -282,11 +311,30 @@ __device__ __forceinline__ void store_block(const uint32_t (&r)[4][32], uint16_t
                         value[e] = first;
                     }
                 }
-                packed[i] = (uint32_t)eb::float_to_bf16_bits(value[0]) | (uint32_t)eb::float_to_bf16_bits(value[1]) << 16;
+                packed[i] = eb::bf16_pair(value[0], value[1]);
             }
-            if (col + 8u * v < n) *reinterpret_cast<uint4*>(dst + 8 * v) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            store_16(dst + 16 * v, packed, wide);
         }
     }
+}
+
+// One scale warp, one stage: the stage's scales from shared memory into the warp's quarter of tensor memory (every quarter
+// holds all of them). `sf`: this lane's 16 bytes of the first atom; `to`: the stage's columns in the warp's quarter.
+// Columns 8 j + 4 t + i: the four scales of K block j, term t, of activation row 32 i + lane (the atom's 16 bytes of this
+// lane). Columns 32 + 8 j + i: of weight row 32 i + lane of the tile's 256 (word j of that row's 16 scale bytes).
+__device__ __forceinline__ void scales_to_tmem(const uint4* sf, uint32_t to) {
+    uint32_t a[32], b[32];
+#pragma unroll
+    for (uint32_t i = 0; i < 8u; ++i) {
+        const uint4 v = sf[i * 32u], w = sf[kSfaStage / 16u + i * 32u];
+        a[4 * i] = v.x, a[4 * i + 1] = v.y, a[4 * i + 2] = v.z, a[4 * i + 3] = v.w;
+        b[i] = w.x, b[8 + i] = w.y, b[16 + i] = w.z, b[24 + i] = w.w;
+    }
+    tmem_store_32(to, a);
+    tmem_store_32(to + 32u, b);
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    tcgen05_fence_before();
+    __syncwarp();
 }
 
 struct TileWalk {
@@ -304,15 +352,16 @@ struct TileWalk {
     }
 };
 
-__global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-        const uint8_t* __restrict__ sfa, const uint8_t* __restrict__ sfb, const float* __restrict__ row_globals,
+__global__ void __launch_bounds__(kScaledThreads, 1) gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+        const __grid_constant__ CUtensorMap map_s, const uint8_t* __restrict__ sfa, const float* __restrict__ row_globals,
         const float* __restrict__ tensor_global, uint16_t* __restrict__ out, float* __restrict__ partials, uint32_t splits, uint32_t rows,
         uint32_t n, uint32_t k, uint32_t pair_tiles, uint32_t* __restrict__ error) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
     uint64_t* empty = full + kStages;
-    uint64_t* acc_full = empty + kStages;
+    uint64_t* scaled = empty + kStages;      // the stage's scales are in tensor memory
+    uint64_t* acc_full = scaled + kStages;
     uint64_t* acc_empty = acc_full + 1;
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_empty + 1);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -328,6 +377,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
         for (uint32_t s = 0; s < kStages; ++s) {
             eb::mbar_init(&full[s], 1);
             eb::mbar_init(&empty[s], 1);
+            eb::mbar_init(&scaled[s], 4);
         }
         eb::mbar_init(acc_full, 1);
         eb::mbar_init(acc_empty, 8);
@@ -342,9 +392,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
     tcgen05_fence_after();
     const uint32_t tmem = *tmem_holder;
     eb::pdl_launch_dependents();
-    eb::pdl_wait();   // the scratch comes from the two launches before this one
+    eb::pdl_wait();   // the scratch comes from the launches before this one
 
-    if (warp == 0) {
+    if (warp < 4u) {
+      registers_give_back<56>();
+      if (warp == 0) {
         if (lane == 0) {
             uint32_t step = 0;
             bool ok = true;
@@ -369,12 +421,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
                     tma_load_2d(stage + kTerms * kATile + kBTile / 2u, &map_b, (int)(ks * 128u), (int)(high * 128u), &full[s]);
                     uint8_t* sf = stage + kTerms * kATile + kBTile;
                     eb::bulk_g2s(sf, sfa + ((uint64_t)tm * k_blocks + ks * 4u) * kTerms * kAtom, kSfaStage, &full[s]);
-                    eb::bulk_g2s(sf + kSfaStage, sfb + ((uint64_t)low * k_blocks + ks * 4u) * kAtom, 4u * kAtom, &full[s]);
-                    eb::bulk_g2s(sf + kSfaStage + 4u * kAtom, sfb + ((uint64_t)high * k_blocks + ks * 4u) * kAtom, 4u * kAtom, &full[s]);
+                    tma_load_2d(sf + kSfaStage, &map_s, (int)(ks * 16u), (int)(low * 128u), &full[s]);
+                    tma_load_2d(sf + kSfaStage + kSfbStage / 2u, &map_s, (int)(ks * 16u), (int)(high * 128u), &full[s]);
                 }
             }
         }
-    } else if (warp == 1) {
+      } else if (warp == 1) {
         if (lane == 0) {
             uint32_t step = 0, local = 0;
             bool ok = true;
@@ -387,41 +439,50 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
                 const uint32_t split = item % splits, ks_begin = split * k_steps / splits, ks_end = (split + 1u) * k_steps / splits;
                 for (uint32_t ks = ks_begin; ks < ks_end; ++ks, ++step) {
                     const uint32_t s = step % kStages, round = step / kStages;
-                    if (!eb::mbar_wait(&full[s], round & 1u)) {
+                    if (!eb::mbar_wait(&full[s], round & 1u) || !eb::mbar_wait(&scaled[s], round & 1u)) {
                         atomicOr(error, 8u);
                         ok = false;
                         break;
                     }
                     tcgen05_fence_after();
                     const uint8_t* stage = smem + s * kStageBytes;
-                    const uint8_t* sf = stage + kTerms * kATile + kBTile;
                     const uint64_t a0 = tile_descriptor(stage), a1 = tile_descriptor(stage + kATile), b = tile_descriptor(stage + kTerms * kATile);
-                    auto cp_a = [&](uint32_t j, uint32_t t) { tmem_copy_atom(tmem + kTmemSfa + (j * 2u + t) * 4u, atom_descriptor(sf + (j * 2u + t) * kAtom)); };
-                    auto cp_b = [&](uint32_t j, uint32_t h) { tmem_copy_atom(tmem + kTmemSfb + j * 8u + h * 4u, atom_descriptor(sf + kSfaStage + (h * 4u + j) * kAtom)); };
-                    auto mma = [&](uint32_t j, uint32_t t) {
-                        mma_block_scaled(tmem, (t ? a1 : a0) + 2u * j, b + 2u * j, tmem + kTmemSfa + (j * 2u + t) * 4u, tmem + kTmemSfb + j * 8u,
-                                t ? 1u : (uint32_t)(((ks - ks_begin) | j) != 0u));
-                    };
-                    // K block by K block: its scale atoms, then its two MMAs (6 % faster than all sixteen copies of the stage first)
+                    const uint32_t scales = tmem + kTmemScales + s * kScaleColumns;
 #pragma unroll
                     for (uint32_t j = 0; j < 4u; ++j) {
-                        cp_a(j, 0);
-                        cp_b(j, 0);
-                        cp_b(j, 1);
-                        mma(j, 0);
-                        cp_a(j, 1);
-                        mma(j, 1);
+                        mma_block_scaled(tmem, a0 + 2u * j, b + 2u * j, scales + j * 8u, scales + 32u + j * 8u, (uint32_t)(((ks - ks_begin) | j) != 0u));
+                        mma_block_scaled(tmem, a1 + 2u * j, b + 2u * j, scales + j * 8u + 4u, scales + 32u + j * 8u, 1u);
                     }
                     mma_commit(&empty[s]);
                 }
                 if (ok) mma_commit(acc_full);
             }
         }
+      }
+    } else if (warp < 8u) {
+        registers_give_back<96>();
+        uint32_t step = 0;
+        bool ok = true;
+        for (uint32_t item = blockIdx.x; item < items && ok; item += gridDim.x) {
+            const uint32_t split = item % splits, ks_end = (split + 1u) * k_steps / splits;
+            for (uint32_t ks = split * k_steps / splits; ks < ks_end; ++ks, ++step) {
+                const uint32_t s = step % kStages, round = step / kStages;
+                if (!eb::mbar_wait(&full[s], round & 1u)) {
+                    if (lane == 0) atomicOr(error, 8u);
+                    ok = false;
+                    break;
+                }
+                scales_to_tmem(reinterpret_cast<const uint4*>(smem + s * kStageBytes + kTerms * kATile + kBTile) + lane,
+                        tmem + (((warp & 3u) * 32u) << 16) + kTmemScales + s * kScaleColumns);
+                if (lane == 0) eb::mbar_arrive(&scaled[s]);
+            }
+        }
     } else {
-        // Epilogue: warp w may read the 32 accumulator rows of lane quarter w % 4 only; warps 2..5 take columns 0..127 of
-        // their quarter, warps 6..9 columns 128..255. A warp first drains its 32 x 128 block into registers and hands the
+        // Epilogue: warp w may read the 32 accumulator rows of lane quarter w % 4 only; warps 8..11 take columns 0..127 of
+        // their quarter, warps 12..15 columns 128..255. A warp first drains its 32 x 128 block into registers and hands the
         // accumulator back (the MMA warp starts the next tile while this one is scaled, rounded and stored).
-        const uint32_t quarter = warp & 3u, half = (warp - 2u) >> 2;
+        registers_take<176>();
+        const uint32_t quarter = warp & 3u, half = (warp - 8u) >> 2;
         const float scale_w = *tensor_global;
         uint32_t local = 0;
         for (uint32_t item = blockIdx.x; item < items; item += gridDim.x, ++local) {
@@ -477,18 +538,29 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const __grid_constant
 // terms) and HALF of the weight tile (128 weight rows), and one thread of the even CTA issues tcgen05.mma.cta_group::2
 // (M 256, N 256, K 64), which reads both CTAs' shared memory and accumulates each CTA's 128 rows in its own tensor
 // memory. A stage is 56 KB per CTA instead of 72 KB for the same FLOP, so four stages fit and the ring carries 22 % fewer
-// bytes per MMA. Measured on B200 it is 6-9 % SLOWER than gemm_kernel (4.1 against 4.5 PFLOP/s issued on the gate shape,
-// three stages or four alike), so it runs only when the caller selects it. Every CTA issues its own plain TMA loads into its own shared memory (no load names another CTA); the odd
-// CTA's MMA warp only relays "my stage has landed" to a barrier of the even CTA; tcgen05.commit signals the ring's and the
-// accumulator's barriers of both CTAs. Weight scale atoms (all 256 columns) are loaded by both.
+// bytes per MMA. Every CTA issues its own loads into its own shared memory (no multicast); both CTAs' code tiles are counted
+// on the even CTA's stage barrier, where the thread that issues the MMAs waits, and each CTA's scale warps - its own 128
+// activation rows, all 256 weight rows of the tile - wait for their own CTA's scales and arrive on the even CTA's barrier.
 constexpr uint32_t kPairStages = 4;
 constexpr uint32_t kPairBTile = 128u * 128u;
-constexpr uint32_t kPairStageBytes = kTerms * kATile + kPairBTile + kSfaStage + kSfbStage;
+constexpr uint32_t kPairCodes = kTerms * kATile + kPairBTile;
+constexpr uint32_t kPairStageBytes = kPairCodes + kSfaStage + kSfbStage;
 constexpr uint32_t kPairShared = kPairStages * kPairStageBytes + 256u + 1024u;
 constexpr uint32_t kPairInstruction = (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | (0u << 23) | ((256u >> 4) << 24);
 
-__device__ __forceinline__ void pair_copy_atom(uint32_t tmem_address, uint64_t descriptor) {
-    asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem_address), "l"(descriptor) : "memory");
+// Tiled TMA loads of a CTA of a pair whose completion is counted on a barrier of either CTA of the pair (`bar`: a
+// shared::cluster address). No multicast: the box lands in the executing CTA's shared memory only.
+__device__ __forceinline__ void pair_tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                         eb::smem_u32(dst)),
+            "l"(map), "r"(c0), "r"(c1), "r"(bar)
+            : "memory");
+}
+__device__ __forceinline__ void pair_tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+                         eb::smem_u32(dst)),
+            "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+            : "memory");
 }
 __device__ __forceinline__ void pair_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate) {
     asm volatile(
@@ -503,20 +575,24 @@ __device__ __forceinline__ void pair_commit(uint64_t* bar) {
             "h"((uint16_t)3)
             : "memory");
 }
-__device__ __forceinline__ void arrive_at_rank(uint64_t* bar, uint32_t rank) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(eb::map_to_rank(eb::smem_u32(bar), rank)) : "memory");
+// Arrives on the barrier at this shared address in CTA `rank` without a release of ordinary memory: what it signals are completed
+// tensor-memory operations of the thread, which tcgen05.fence::before_thread_sync has ordered. (An arrive with release waits for
+// the thread's stores to be performed, about a microsecond: 420 us instead of 315 us for the GEMM of 4096 x 17408 x 5120.)
+__device__ __forceinline__ void signal_rank(uint64_t* bar, uint32_t rank) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(eb::map_to_rank(eb::smem_u32(bar), rank)) : "memory");
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
-        const __grid_constant__ CUtensorMap map_b, const uint8_t* __restrict__ sfa, const uint8_t* __restrict__ sfb,
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kScaledThreads, 1) gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
+        const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_s, const uint8_t* __restrict__ sfa,
         const float* __restrict__ row_globals, const float* __restrict__ tensor_global, uint16_t* __restrict__ out, uint32_t rows, uint32_t n,
         uint32_t k, uint32_t pair_tiles, uint32_t* __restrict__ error) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + kPairStages * kPairStageBytes);
-    uint64_t* empty = full + kPairStages;
-    uint64_t* peer_full = empty + kPairStages;   // even CTA: the odd CTA's stage has landed
-    uint64_t* acc_full = peer_full + kPairStages;
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + kPairStages * kPairStageBytes);   // even CTA: both CTAs' codes have landed
+    uint64_t* landed = full + kPairStages;       // this CTA's scales have landed
+    uint64_t* empty = landed + kPairStages;
+    uint64_t* scaled = empty + kPairStages;      // even CTA: both CTAs' scales are in tensor memory
+    uint64_t* acc_full = scaled + kPairStages;
     uint64_t* acc_empty = acc_full + 1;          // even CTA: both CTAs' epilogue warps have drained the accumulator
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_empty + 1);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -537,8 +613,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < kPairStages; ++s) {
             eb::mbar_init(&full[s], 1);
+            eb::mbar_init(&landed[s], 1);
             eb::mbar_init(&empty[s], 1);
-            eb::mbar_init(&peer_full[s], 1);
+            eb::mbar_init(&scaled[s], 8);
         }
         eb::mbar_init(acc_full, 1);
         eb::mbar_init(acc_empty, 16);
@@ -554,9 +631,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
     tcgen05_fence_after();
     const uint32_t tmem = *tmem_holder;
     eb::pdl_launch_dependents();
-    eb::pdl_wait();   // the scratch comes from the two launches before this one
+    eb::pdl_wait();   // the scratch comes from the launches before this one
 
-    if (warp == 0) {
+    if (warp < 4u) {
+      registers_give_back<56>();
+      if (warp == 0) {
         if (lane == 0) {
             uint32_t step = 0;
             bool ok = true;
@@ -564,8 +643,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
                 uint32_t tm, tn;
                 place(item, &tm, &tn);
                 const uint32_t row_tile = 2u * tm + rank;                      // this CTA's 128 rows
-                const uint32_t weight_tile = paired ? (rank == 0u ? tn : pair_tiles + tn) : 2u * tn + rank;   // its 128 weight rows
                 const uint32_t low = paired ? tn : 2u * tn, high = paired ? pair_tiles + tn : 2u * tn + 1u;
+                const uint32_t weight_tile = rank == 0u ? low : high;          // its 128 weight rows
                 const uint32_t scale_tile = min(row_tile, row_tiles - 1u);     // a CTA without rows multiplies zeros by some tile's scales
                 for (uint32_t ks = 0; ks < k_steps; ++ks, ++step) {
                     const uint32_t s = step % kPairStages, round = step / kPairStages;
@@ -575,33 +654,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
                         break;
                     }
                     uint8_t* stage = smem + s * kPairStageBytes;
-                    eb::mbar_arrive_expect_tx(&full[s], kPairStageBytes);
-                    tma_load_3d(stage, &map_a, (int)(ks * 128u), (int)(row_tile * kTileM), 0, &full[s]);
-                    tma_load_3d(stage + kATile, &map_a, (int)(ks * 128u), (int)(row_tile * kTileM), 1, &full[s]);
-                    tma_load_2d(stage + kTerms * kATile, &map_b, (int)(ks * 128u), (int)(weight_tile * 128u), &full[s]);
-                    uint8_t* sf = stage + kTerms * kATile + kPairBTile;
-                    eb::bulk_g2s(sf, sfa + ((uint64_t)scale_tile * k_blocks + ks * 4u) * kTerms * kAtom, kSfaStage, &full[s]);
-                    eb::bulk_g2s(sf + kSfaStage, sfb + ((uint64_t)low * k_blocks + ks * 4u) * kAtom, 4u * kAtom, &full[s]);
-                    eb::bulk_g2s(sf + kSfaStage + 4u * kAtom, sfb + ((uint64_t)high * k_blocks + ks * 4u) * kAtom, 4u * kAtom, &full[s]);
+                    if (rank == 0u) eb::mbar_arrive_expect_tx(&full[s], 2u * kPairCodes);
+                    const uint32_t bar = eb::map_to_rank(eb::smem_u32(&full[s]), 0u);
+                    eb::mbar_arrive_expect_tx(&landed[s], kSfaStage + kSfbStage);
+                    uint8_t* sf = stage + kPairCodes;
+                    eb::bulk_g2s(sf, sfa + ((uint64_t)scale_tile * k_blocks + ks * 4u) * kTerms * kAtom, kSfaStage, &landed[s]);
+                    tma_load_2d(sf + kSfaStage, &map_s, (int)(ks * 16u), (int)(low * 128u), &landed[s]);
+                    tma_load_2d(sf + kSfaStage + kSfbStage / 2u, &map_s, (int)(ks * 16u), (int)(high * 128u), &landed[s]);
+                    pair_tma_load_3d(stage, &map_a, (int)(ks * 128u), (int)(row_tile * kTileM), 0, bar);
+                    pair_tma_load_3d(stage + kATile, &map_a, (int)(ks * 128u), (int)(row_tile * kTileM), 1, bar);
+                    pair_tma_load_2d(stage + kTerms * kATile, &map_b, (int)(ks * 128u), (int)(weight_tile * 128u), bar);
                 }
             }
         }
-    } else if (warp == 1) {
-        if (lane == 0 && rank != 0u) {
-            // the odd CTA: tell the even one about every stage that has landed here
-            uint32_t step = 0;
-            bool ok = true;
-            for (uint32_t item = pair; item < items && ok; item += pairs)
-                for (uint32_t ks = 0; ks < k_steps; ++ks, ++step) {
-                    const uint32_t s = step % kPairStages, round = step / kPairStages;
-                    if (!eb::mbar_wait(&full[s], round & 1u)) {
-                        atomicOr(error, 8u);
-                        ok = false;
-                        break;
-                    }
-                    arrive_at_rank(&peer_full[s], 0u);
-                }
-        } else if (lane == 0) {
+      } else if (warp == 1) {
+        if (lane == 0 && rank == 0u) {   // the odd CTA issues nothing: its tiles are read by the even CTA's MMAs
             uint32_t step = 0, local = 0;
             bool ok = true;
             for (uint32_t item = pair; item < items && ok; item += pairs, ++local) {
@@ -612,32 +679,46 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
                 tcgen05_fence_after();
                 for (uint32_t ks = 0; ks < k_steps; ++ks, ++step) {
                     const uint32_t s = step % kPairStages, round = step / kPairStages;
-                    if (!eb::mbar_wait(&full[s], round & 1u) || !eb::mbar_wait(&peer_full[s], round & 1u)) {
+                    if (!eb::mbar_wait(&full[s], round & 1u) || !eb::mbar_wait(&scaled[s], round & 1u)) {
                         atomicOr(error, 8u);
                         ok = false;
                         break;
                     }
                     tcgen05_fence_after();
                     const uint8_t* stage = smem + s * kPairStageBytes;
-                    const uint8_t* sf = stage + kTerms * kATile + kPairBTile;
                     const uint64_t a0 = tile_descriptor(stage), a1 = tile_descriptor(stage + kATile), b = tile_descriptor(stage + kTerms * kATile);
+                    const uint32_t scales = tmem + kTmemScales + s * kScaleColumns;
 #pragma unroll
                     for (uint32_t j = 0; j < 4u; ++j) {
-                        pair_copy_atom(tmem + kTmemSfa + (j * 2u) * 4u, atom_descriptor(sf + (j * 2u) * kAtom));
-                        pair_copy_atom(tmem + kTmemSfb + j * 8u, atom_descriptor(sf + kSfaStage + j * kAtom));
-                        pair_copy_atom(tmem + kTmemSfb + j * 8u + 4u, atom_descriptor(sf + kSfaStage + (4u + j) * kAtom));
-                        pair_mma(tmem, a0 + 2u * j, b + 2u * j, tmem + kTmemSfa + (j * 2u) * 4u, tmem + kTmemSfb + j * 8u, (ks | j) != 0u);
-                        pair_copy_atom(tmem + kTmemSfa + (j * 2u + 1u) * 4u, atom_descriptor(sf + (j * 2u + 1u) * kAtom));
-                        pair_mma(tmem, a1 + 2u * j, b + 2u * j, tmem + kTmemSfa + (j * 2u + 1u) * 4u, tmem + kTmemSfb + j * 8u, 1u);
+                        pair_mma(tmem, a0 + 2u * j, b + 2u * j, scales + j * 8u, scales + 32u + j * 8u, (uint32_t)((ks | j) != 0u));
+                        pair_mma(tmem, a1 + 2u * j, b + 2u * j, scales + j * 8u + 4u, scales + 32u + j * 8u, 1u);
                     }
                     pair_commit(&empty[s]);
                 }
                 if (ok) pair_commit(acc_full);
             }
         }
+      }
+    } else if (warp < 8u) {
+        registers_give_back<96>();
+        uint32_t step = 0;
+        bool ok = true;
+        for (uint32_t item = pair; item < items && ok; item += pairs)
+            for (uint32_t ks = 0; ks < k_steps; ++ks, ++step) {
+                const uint32_t s = step % kPairStages, round = step / kPairStages;
+                if (!eb::mbar_wait(&landed[s], round & 1u)) {
+                    if (lane == 0) atomicOr(error, 8u);
+                    ok = false;
+                    break;
+                }
+                scales_to_tmem(reinterpret_cast<const uint4*>(smem + s * kPairStageBytes + kPairCodes) + lane,
+                        tmem + (((warp & 3u) * 32u) << 16) + kTmemScales + s * kScaleColumns);
+                if (lane == 0) signal_rank(&scaled[s], 0u);
+            }
     } else {
         // Epilogue, in both CTAs, each over its own 128 rows: as in gemm_kernel.
-        const uint32_t quarter = warp & 3u, half = (warp - 2u) >> 2;
+        registers_take<176>();
+        const uint32_t quarter = warp & 3u, half = (warp - 8u) >> 2;
         const float scale_w = *tensor_global;
         uint32_t local = 0;
         for (uint32_t item = pair; item < items; item += pairs, ++local) {
@@ -658,7 +739,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0) arrive_at_rank(acc_empty, 0u);
+            if (lane == 0) signal_rank(acc_empty, 0u);   // what it orders are tensor-memory reads
             const uint32_t row = (2u * tm + rank) * kTileM + quarter * 32u + lane;
             const float scale = row < rows ? __fmul_rn(row_globals[row], scale_w) : 0.0f;
             store_block(r, out, row, rows, n, paired ? tn * 128u + half * 64u : tn * kTileN + half * 128u, scale, paired);
@@ -705,7 +786,10 @@ inline cudaError_t initialize() {
     return e != cudaSuccess ? e : cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairShared);
 }
 
-constexpr uint32_t kPairRows = 512;   // fewer rows than this always run on single CTAs
+// Fewer rows than this run on single CTAs. The pairs are 2 to 6 % faster from 1024 rows on (1024 x 5120 x 17408: 171 against 176
+// us, 4096 x 17408 x 5120: 318 against 337 in turn) and equal or a little slower below, where their 256-row tiles leave more
+// of the last wave empty.
+constexpr uint32_t kPairRows = 1024;
 
 template <typename... Params, typename... Args>
 inline cudaError_t launch_on(cudaStream_t stream, bool pdl, void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared, Args... args) {
@@ -722,7 +806,7 @@ inline cudaError_t launch_on(cudaStream_t stream, bool pdl, void (*kernel)(Param
     return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
 }
 
-// The three launches of a native linear. Shapes are pre-checked by the caller: k % 256 == 0, out_features % 128 == 0,
+// The launches of a native linear. Shapes are pre-checked by the caller: k % 256 == 0, out_features % 128 == 0,
 // scratch aligned to 16 bytes and at least ActivationLayout(rows, k, out_features).bytes long.
 // quantize: BF16 rows -> the activation part of the scratch (code planes, scale atoms, row scales).
 inline cudaError_t quantize(const void* input, void* scratch, uint32_t rows, uint32_t k, cudaStream_t stream, bool pdl) {
@@ -730,7 +814,7 @@ inline cudaError_t quantize(const void* input, void* scratch, uint32_t rows, uin
             static_cast<const __nv_bfloat16*>(input), static_cast<uint8_t*>(scratch), rows, k);
 }
 
-// multiply: the weight scale plane -> scale atoms in the scratch, then the GEMM over the quantized activations found there.
+// multiply: the GEMM over the quantized activations found in the scratch (table-indexed weight scales are expanded there first).
 // paired: the weights are a gate/up object (gate rows first); the output is [rows][out_features / 2] SwiGLU values.
 // pairs: calls of kPairRows rows and more run on CTA pairs (gemm_pair_kernel).
 inline cudaError_t multiply(const void* weights, void* output, void* scratch, uint32_t rows, uint32_t k, uint32_t out_features, int sms,
@@ -745,7 +829,7 @@ inline cudaError_t multiply(const void* weights, void* output, void* scratch, ui
     const uint64_t scale_offset = align256((uint64_t)out_features * row_bytes);
     const uint64_t table_offset = align256(scale_offset + (uint64_t)out_features * (k / (table_scales ? 32u : 16u)));
     const uint64_t global_offset = table_scales ? table_offset + 16u : table_offset;
-    CUtensorMap map_a, map_b;
+    CUtensorMap map_a, map_b, map_s;
     const cuuint32_t ones[3] = {1u, 1u, 1u};
     const cuuint64_t a_dims[3] = {row_bytes, rows, kTerms}, a_strides[2] = {row_bytes, row_bytes * rows};
     const cuuint32_t a_box[3] = {128u, kTileM, 1u};
@@ -756,12 +840,21 @@ inline cudaError_t multiply(const void* weights, void* output, void* scratch, ui
     if (r == CUDA_SUCCESS)
         r = encode(&map_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(w), b_dims, b_strides, b_box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    // the scale bytes [n][K/16]: the tensor's own plane, or the plane a table-indexed tensor's indices are expanded to
+    const uint64_t scale_row = k / 16u;
+    uint8_t* scales = table_scales ? base + layout.sfb_offset : const_cast<uint8_t*>(w + scale_offset);
+    const cuuint64_t s_dims[2] = {scale_row, out_features}, s_strides[1] = {scale_row};
+    const cuuint32_t s_box[2] = {kStepK / 16u, 128u};
+    if (r == CUDA_SUCCESS)
+        r = encode(&map_s, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, scales, s_dims, s_strides, s_box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-    const uint32_t n_padded = (out_features + 255u) / 256u * 256u;
-    const uint64_t items = (uint64_t)n_padded * layout.k_blocks;
-    cudaError_t e = launch_on(stream, pdl, repack_weight_scales, dim3((unsigned)((items + 255u) / 256u)), dim3(256), 0, w + scale_offset,
-            table_scales ? w + table_offset : static_cast<const uint8_t*>(nullptr), base + layout.sfb_offset, out_features, layout.k_blocks, n_padded);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
+    if (table_scales) {
+        const uint32_t vectors = (uint32_t)((uint64_t)out_features * scale_row / 16u);
+        e = launch_on(stream, pdl, expand_table_scales, dim3((vectors + 255u) / 256u), dim3(256), 0, w + scale_offset, w + table_offset, scales, vectors);
+        if (e != cudaSuccess) return e;
+    }
     const uint32_t pair_tiles = paired ? out_features / 256u : 0u, width = paired ? out_features / 2u : out_features;
     const uint32_t tiles = ((rows + kTileM - 1u) / kTileM) * (paired ? pair_tiles : (out_features + kTileN - 1u) / kTileN);
     // The skinny route (the reference's 9..64-row kernel, native/src/nvfp4_native/native.cuh:435-585, cuts K the same way):
@@ -775,11 +868,11 @@ inline cudaError_t multiply(const void* weights, void* output, void* scratch, ui
     if (pairs && rows >= kPairRows) {
         const uint32_t pair_items = ((rows + 255u) / 256u) * (paired ? pair_tiles : (out_features + 255u) / 256u);
         const uint32_t ctas = 2u * std::max(1u, std::min((uint32_t)sms / 2u, pair_items));
-        return launch_on(stream, pdl, gemm_pair_kernel, dim3(ctas), dim3(kThreads), kPairShared, map_a, map_b, base + layout.sfa_offset,
-                base + layout.sfb_offset, row_globals, tensor_global, static_cast<uint16_t*>(output), rows, width, k, pair_tiles, error);
+        return launch_on(stream, pdl, gemm_pair_kernel, dim3(ctas), dim3(kScaledThreads), kPairShared, map_a, map_b, map_s,
+                base + layout.sfa_offset, row_globals, tensor_global, static_cast<uint16_t*>(output), rows, width, k, pair_tiles, error);
     }
-    e = launch_on(stream, pdl, gemm_kernel, dim3(grid), dim3(kThreads), kSharedBytes, map_a, map_b, base + layout.sfa_offset,
-            base + layout.sfb_offset, row_globals, tensor_global, static_cast<uint16_t*>(output), partials, splits, rows, width, k, pair_tiles, error);
+    e = launch_on(stream, pdl, gemm_kernel, dim3(grid), dim3(kScaledThreads), kSharedBytes, map_a, map_b, map_s,
+            base + layout.sfa_offset, row_globals, tensor_global, static_cast<uint16_t*>(output), partials, splits, rows, width, k, pair_tiles, error);
     if (e != cudaSuccess || splits == 1u) return e;
     const uint64_t quads = (uint64_t)rows * (out_features / 4u);
     return launch_on(stream, pdl, finish_splits, dim3((unsigned)((quads + 255u) / 256u)), dim3(256), 0, partials, row_globals, tensor_global,
