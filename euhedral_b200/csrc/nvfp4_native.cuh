@@ -10,7 +10,7 @@
 //
 // Two launches per call, all on the selected stream, no allocation (everything lives in the caller's scratch):
 //   1. quantize_rows: BF16 rows -> code planes [term][row][K/2], block scales already in the layout tcgen05 wants
-//      (512-byte atoms of 128 rows x 4 scales, byte (r % 32) * 16 + (r / 32) * 4 + s), one FP32 scale per row. One warp
+//      (512-byte atoms of 128 rows x 4 scales, byte (r % 32) * 16 + (r / 32) * 4 + s), one FP32 scale per row. One CTA
 //      per row.
 //   2. gemm: persistent CTAs, one per SM, 128 x 256 output tiles, K in steps of 256 through a 3-stage ring.
 //      warp 0 (one lane) issues the TMA loads (codes as 128-byte-swizzled tiles, the weights' scale bytes as they lie in the
@@ -89,11 +89,12 @@ __host__ __device__ inline uint32_t atom_byte(uint32_t row_in_tile, uint32_t sca
 // bit against that kernel compiled for this GPU): global = amax / (6 * 448) (1 for a zero row); per block of 16:
 // scale = e4m3_satfinite(amax * (1/6) * (1/global)); codes = e2m1_rn(v * ((1/global) / scale)), saturating; the next term
 // quantizes fma(-decoded, scale * global, v). All in FP32 with the hardware conversions.
-// The work split is this kernel's own: one warp per row, eight rows per CTA, no shared memory and no CTA barrier. Four
-// neighbouring lanes share a K block of 64 values, one 16-value block each; their four scale bytes meet by two shuffles
-// and leave as ONE 4-byte store, which is exactly one row's entry of the 512-byte atom tcgen05 reads; their codes leave
-// as 32 contiguous bytes per term.
-constexpr uint32_t kQuantizeWarps = 8;
+// The work split is this kernel's own: one CTA per row, a 16-value block per thread and turn, held in registers from the pass
+// that finds the row's largest magnitude to the pass that quantizes it (kHeld turns; what a longer row has beyond is read again). Four neighbouring lanes share a K block of 64 values; their four scale bytes meet by two shuffles
+// and leave as ONE 4-byte store, which is exactly one row's entry of the 512-byte atom tcgen05 reads; their codes leave as 32
+// contiguous bytes per term. A warp per row, which this replaces, read every row twice and left all but a few SMs idle on
+// calls of few rows.
+constexpr uint32_t kQuantizeThreads = 512;   // the most threads of a row
 
 // One block of 16 values: its scale code, its 8 code bytes, and v replaced by the residual.
 __device__ __forceinline__ uint32_t quantize_block(float (&v)[16], float global, float inverse_global, uint2* codes) {
@@ -119,42 +120,52 @@ __device__ __forceinline__ uint32_t quantize_block(float (&v)[16], float global,
     return (uint32_t)scale;
 }
 
-__global__ void __launch_bounds__(32 * kQuantizeWarps, 5) quantize_rows(const __nv_bfloat16* __restrict__ input, uint8_t* __restrict__ scratch,
+// Largest magnitude of 16 BF16 values (eight pairs).
+__device__ __forceinline__ float largest_of(const uint4& lo, const uint4& hi) {
+    const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    float most = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) most = fmaxf(most, fmaxf(fabsf(eb::bf16_bits_to_float(w[j] & 0xFFFFu)), fabsf(__uint_as_float(w[j] & 0xFFFF0000u))));
+    return most;
+}
+
+//   grid rows, block: the fewest whole warps that hold the row in kHeld turns, at most kQuantizeThreads. k a multiple of 64.
+template <uint32_t kHeld>
+__global__ void __launch_bounds__(kQuantizeThreads, 2) quantize_rows(const __nv_bfloat16* __restrict__ input, uint8_t* __restrict__ scratch,
         uint32_t rows, uint32_t k) {
-    const uint32_t lane = threadIdx.x & 31u, row = blockIdx.x * kQuantizeWarps + (threadIdx.x >> 5);
+    const uint32_t t = threadIdx.x, threads = blockDim.x, row = blockIdx.x;
+    __shared__ float warp_most[kQuantizeThreads / 32u];
     const ActivationLayout layout(rows, k);
     eb::pdl_launch_dependents();
     eb::pdl_wait();
-    if (row >= rows) return;
     const uint4* x = reinterpret_cast<const uint4*>(input + (uint64_t)row * k);   // 8 values per element
-    const uint32_t vectors = k / 8u, blocks64 = k / kBlockK;
-    float amax = 0.0f;
-#pragma unroll 4   // four loads in flight per lane: the pass is bound by load latency
-    for (uint32_t i = lane; i < vectors; i += 32u) {
-        const uint4 w = x[i];
-        const uint32_t words[4] = {w.x, w.y, w.z, w.w};
+    const uint32_t blocks = k / 16u;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    uint4 lo[kHeld], hi[kHeld];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            amax = fmaxf(amax, fmaxf(fabsf(eb::bf16_bits_to_float(words[j] & 0xFFFFu)), fabsf(__uint_as_float(words[j] & 0xFFFF0000u))));
+    for (uint32_t i = 0; i < kHeld; ++i) {
+        const uint32_t b = i * threads + t;
+        lo[i] = b < blocks ? x[2u * b] : zero;
+        hi[i] = b < blocks ? x[2u * b + 1u] : zero;
     }
+    float amax = 0.0f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    for (uint32_t i = 0; i < kHeld; ++i) amax = fmaxf(amax, largest_of(lo[i], hi[i]));
+    for (uint32_t b = kHeld * threads + t; b < blocks; b += threads) amax = fmaxf(amax, largest_of(x[2u * b], x[2u * b + 1u]));
+    // magnitudes are non-negative floats, whose bits order as integers
+    const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
+    if ((t & 31u) == 0u) warp_most[t >> 5] = __uint_as_float(most);
+    __syncthreads();
+    amax = 0.0f;
+    for (uint32_t w = 0; w < threads / 32u; ++w) amax = fmaxf(amax, warp_most[w]);
     const float global = amax > 0.0f ? __fdiv_rn(amax, 6.0f * 448.0f) : 1.0f;
     const float inverse_global = __fdiv_rn(1.0f, global);
     uint8_t* sfa = scratch + layout.sfa_offset + (uint64_t)(row / kTileM) * layout.k_blocks * kTerms * kAtom + atom_byte(row % kTileM, 0);
     const uint64_t plane = (uint64_t)rows * (k / 2u);
     uint8_t* codes_row = scratch + (uint64_t)row * (k / 2u);
-    // Four neighbouring lanes share a K block of 64 values, one 16-value block each; a warp covers eight K blocks per turn.
-    const uint32_t sub = lane & 3u;
-    for (uint32_t first = 0; first < blocks64; first += 8u) {   // the row was just read: these loads hit L1 / L2
-        const uint32_t b = first + (lane >> 2);
-        const bool live = b < blocks64;
-        uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;
-        if (live) {
-            lo = x[2u * (4u * b + sub)];
-            hi = x[2u * (4u * b + sub) + 1u];
-        }
-        const uint32_t words[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    auto quantize = [&](uint32_t b, const uint4& first, const uint4& second) {   // whole quartets of lanes come here together
+        const uint32_t words[8] = {first.x, first.y, first.z, first.w, second.x, second.y, second.z, second.w};
+        const uint32_t sub = b & 3u, members = 0xFu << (t & 28u);
         float v[16];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -162,18 +173,20 @@ __global__ void __launch_bounds__(32 * kQuantizeWarps, 5) quantize_rows(const __
             v[2 * i + 1] = __uint_as_float(words[i] & 0xFFFF0000u);
         }
 #pragma unroll
-        for (uint32_t t = 0; t < kTerms; ++t) {
+        for (uint32_t term = 0; term < kTerms; ++term) {
             uint2 codes;
             uint32_t scales = quantize_block(v, global, inverse_global, &codes) << (8u * sub);
-            scales |= __shfl_xor_sync(0xffffffffu, scales, 1);   // the K block's four scale bytes, in every one of the four lanes
-            scales |= __shfl_xor_sync(0xffffffffu, scales, 2);
-            if (live) {
-                *reinterpret_cast<uint2*>(codes_row + t * plane + 32u * b + 8u * sub) = codes;
-                if (sub == 0u) *reinterpret_cast<uint32_t*>(sfa + ((uint64_t)b * kTerms + t) * kAtom) = scales;
-            }
+            scales |= __shfl_xor_sync(members, scales, 1);   // the K block's four scale bytes, in every one of the four lanes
+            scales |= __shfl_xor_sync(members, scales, 2);
+            *reinterpret_cast<uint2*>(codes_row + term * plane + 8u * b) = codes;
+            if (sub == 0u) *reinterpret_cast<uint32_t*>(sfa + ((uint64_t)(b >> 2) * kTerms + term) * kAtom) = scales;
         }
-    }
-    if (lane == 0) reinterpret_cast<float*>(scratch + layout.global_offset)[row] = global;
+    };
+#pragma unroll
+    for (uint32_t i = 0; i < kHeld; ++i)
+        if (i * threads + t < blocks) quantize(i * threads + t, lo[i], hi[i]);
+    for (uint32_t b = kHeld * threads + t; b < blocks; b += threads) quantize(b, x[2u * b], x[2u * b + 1u]);
+    if (t == 0u) reinterpret_cast<float*>(scratch + layout.global_offset)[row] = global;
 }
 
 // ---- 2. table-indexed weight scales ---------------------------------------------------------------------------------------
@@ -810,8 +823,13 @@ inline cudaError_t launch_on(cudaStream_t stream, bool pdl, void (*kernel)(Param
 // scratch aligned to 16 bytes and at least ActivationLayout(rows, k, out_features).bytes long.
 // quantize: BF16 rows -> the activation part of the scratch (code planes, scale atoms, row scales).
 inline cudaError_t quantize(const void* input, void* scratch, uint32_t rows, uint32_t k, cudaStream_t stream, bool pdl) {
-    return launch_on(stream, pdl, quantize_rows, dim3((rows + kQuantizeWarps - 1u) / kQuantizeWarps), dim3(32u * kQuantizeWarps), 0,
-            static_cast<const __nv_bfloat16*>(input), static_cast<uint8_t*>(scratch), rows, k);
+    const uint32_t blocks = k / 16u;
+    auto run = [&](auto kernel, uint32_t held) {
+        const uint32_t threads = std::min(kQuantizeThreads, ((blocks + held - 1u) / held + 31u) / 32u * 32u);
+        return launch_on(stream, pdl, kernel, dim3(rows), dim3(threads), 0, static_cast<const __nv_bfloat16*>(input), static_cast<uint8_t*>(scratch), rows, k);
+    };
+    // two turns while they hold the row (rows of up to 16,384 values), else four
+    return blocks <= 2u * kQuantizeThreads ? run(quantize_rows<2>, 2u) : run(quantize_rows<4>, 4u);
 }
 
 // multiply: the GEMM over the quantized activations found in the scratch (table-indexed weight scales are expanded there first).
