@@ -12,8 +12,9 @@
 
 #include "common.cuh"
 #include "exact_kernels.cuh"
-#include "nvfp4_gemv.cuh"
+#include "nvfp4_geometry.cuh"
 #include "nvfp4_native.cuh"
+#include "nvfp4_decode.cuh"
 #include "bf16_gemm.cuh"
 #include "q3_gemv.cuh"
 #include "trellis.cuh"
@@ -80,8 +81,6 @@ void initialize_device(int device, DeviceState* state) {
     }
     // In host code the array's name is only a handle; the kernels need its device address on this device.
     if (e == cudaSuccess) e = cudaGetSymbolAddress(reinterpret_cast<void**>(&state->static_scratch), g_static_scratch);
-    if (e == cudaSuccess) e = allow_gemv<nvfp4::Format>();
-    if (e == cudaSuccess) e = allow_gemv<nvfp4::FormatSd4>();
     if (e == cudaSuccess) e = allow_gemv<q3::Format>();
     if (e == cudaSuccess) e = allow_big_smem(exact::trellis_linear);
 #define EB_ALLOW_ENCODER(KA, HALF) if (e == cudaSuccess) e = allow_big_smem(trellis_encode::viterbi_kernel<KA, HALF>);
@@ -92,6 +91,7 @@ void initialize_device(int device, DeviceState* state) {
     EB_TRELLIS_WIDTHS(EB_ALLOW)
 #undef EB_ALLOW
     if (e == cudaSuccess) e = nvfp4n::initialize();
+    if (e == cudaSuccess) e = nvfp4d::initialize();
     if (e == cudaSuccess) e = bf16n::initialize();
     state->status = (int)e;
 }
@@ -119,28 +119,7 @@ enum Overlap { kOrdered = 0, kOverlappable = 1 };
 
 template <typename... Params, typename... Args>
 cudaError_t launch(Overlap overlap, void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared, unsigned cluster, Args... args) {
-    cudaLaunchConfig_t config = {};
-    config.gridDim = grid;
-    config.blockDim = block;
-    config.dynamicSmemBytes = shared;
-    config.stream = t_stream;
-    cudaLaunchAttribute attributes[2];
-    unsigned count = 0;
-    if (cluster > 1) {
-        attributes[count].id = cudaLaunchAttributeClusterDimension;
-        attributes[count].val.clusterDim.x = cluster;
-        attributes[count].val.clusterDim.y = 1;
-        attributes[count].val.clusterDim.z = 1;
-        ++count;
-    }
-    if (t_pdl && overlap == kOverlappable && t_stream != nullptr) {
-        attributes[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attributes[count].val.programmaticStreamSerializationAllowed = 1;
-        ++count;
-    }
-    config.attrs = attributes;
-    config.numAttrs = count;
-    return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+    return eb::launch_on(t_stream, t_pdl && overlap == kOverlappable && t_stream != nullptr, cluster, kernel, grid, block, shared, args...);
 }
 
 // ---- decode GEMV planning ---------------------------------------------------------------------------------------------
@@ -176,45 +155,12 @@ cudaError_t allow_gemv() {
     return e;
 }
 
-// Clusters of `split` CTAs of this kernel that the current device holds at once (0: none fit), cached per (device, kernel,
-// shape of the CTA). Without a device: one CTA per SM.
+// Clusters of `split` CTAs of this kernel that the current device holds at once. Without a device: one CTA per SM.
 template <class F>
 uint32_t resident_clusters(GemvKernel<F> kernel, uint32_t warps, uint32_t shared, uint32_t split, int sms) {
-    struct Entry {
-        int device;
-        const void* kernel;
-        uint32_t warps, shared, split, clusters;
-    };
-    static std::mutex mutex;
-    static std::vector<Entry> cache;
-    int device = -1;
-    if (cudaGetDevice(&device) != cudaSuccess) {
-        (void)cudaGetLastError();
-        device = -1;
-    }
-    if (device >= 0) {
-        std::lock_guard<std::mutex> lock(mutex);
-        for (const Entry& e : cache)
-            if (e.device == device && e.kernel == (const void*)kernel && e.warps == warps && e.shared == shared && e.split == split) return e.clusters;
-        cudaLaunchConfig_t config = {};
-        config.gridDim = dim3(split * 1024u);
-        config.blockDim = dim3(32u * (warps + (F::kAddingWarp ? 1u : 0u)));   // the decoding warps and the adding warp
-        config.dynamicSmemBytes = shared;
-        cudaLaunchAttribute attribute;
-        attribute.id = cudaLaunchAttributeClusterDimension;
-        attribute.val.clusterDim.x = split;
-        attribute.val.clusterDim.y = 1;
-        attribute.val.clusterDim.z = 1;
-        config.attrs = &attribute;
-        config.numAttrs = 1;
-        int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) == cudaSuccess) {
-            cache.push_back({device, (const void*)kernel, warps, shared, split, (uint32_t)clusters});
-            return (uint32_t)clusters;
-        }
-        (void)cudaGetLastError();
-    }
-    return (uint32_t)sms / split;
+    const uint32_t threads = 32u * (warps + (F::kAddingWarp ? 1u : 0u));   // the decoding warps and the adding warp
+    const uint32_t now = eb::resident_clusters((const void*)kernel, threads, shared, split);
+    return now != 0u ? now : (uint32_t)sms / split;
 }
 
 // tiles: 16-row tiles of all tensors of the launch; widest: of the tallest tensor.
@@ -519,17 +465,25 @@ cudaError_t launch_trellis_finish(const void* partials, int splits, const void* 
 
 // Several decode linears that share K and the row count (the q, k and v projections of a layer, or gate and up) as ONE
 // launch per 8 tensors. Every output is bit for bit what the single-tensor entry point gives.
-template <class F>
+struct Nvfp4Cut {   // for euhedral_b200_decode_plan
+    static constexpr uint32_t kPieceChunks = 3, kMaxPiece = 4;
+};
+
+enum class DecodeFormat { kQ3, kNvfp4, kNvfp4Table };
+
+template <DecodeFormat kFormat>
 int linear_group(uint32_t count, const void* const* inputs, const void* const* weights, void* const* outputs, uint32_t rows,
         uint32_t in_features, const uint32_t* out_features, const uint64_t* weights_byte_sizes) {
+    constexpr bool kQ3 = kFormat == DecodeFormat::kQ3;
+    using Geometry = std::conditional_t<kQ3, q3::Geometry, std::conditional_t<kFormat == DecodeFormat::kNvfp4, nvfp4::Geometry, nvfp4::GeometrySd4>>;
     if (count == 0 || inputs == nullptr || weights == nullptr || outputs == nullptr || out_features == nullptr || weights_byte_sizes == nullptr
             || rows == 0 || in_features == 0)
         return EUHEDRAL_CUDA_INVALID_ARGUMENT;
     for (uint32_t i = 0; i < count; ++i) {
         if (inputs[i] == nullptr || weights[i] == nullptr || outputs[i] == nullptr || out_features[i] == 0) return EUHEDRAL_CUDA_INVALID_ARGUMENT;
-        if (typename F::Geometry(out_features[i], in_features).size != weights_byte_sizes[i]) return EUHEDRAL_CUDA_FORMAT_MISMATCH;
+        if (Geometry(out_features[i], in_features).size != weights_byte_sizes[i]) return EUHEDRAL_CUDA_FORMAT_MISMATCH;
         if (((uintptr_t)inputs[i] & 15u) != 0 || ((uintptr_t)weights[i] & 15u) != 0) return EUHEDRAL_CUDA_INVALID_ARGUMENT;
-        if (!decode_takes<F>(in_features, out_features[i])) return EUHEDRAL_CUDA_ROUTE_UNAVAILABLE;
+        if (!(kQ3 ? decode_takes<q3::Format>(in_features, out_features[i]) : nvfp4d::takes(in_features, out_features[i]))) return EUHEDRAL_CUDA_ROUTE_UNAVAILABLE;
     }
     if (rows > 32u || g_exact.load()) return EUHEDRAL_CUDA_ROUTE_UNAVAILABLE;
     DeviceState* state = nullptr;
@@ -537,9 +491,17 @@ int linear_group(uint32_t count, const void* const* inputs, const void* const* w
     if (status != EUHEDRAL_CUDA_SUCCESS) return status;
     for (uint32_t first = 0; first < count; first += gemv::kMaxGroup) {
         const uint32_t now = std::min<uint32_t>(gemv::kMaxGroup, count - first);
-        DecodeItem items[gemv::kMaxGroup];
-        for (uint32_t i = 0; i < now; ++i) items[i] = {inputs[first + i], weights[first + i], outputs[first + i], out_features[first + i]};
-        const cudaError_t e = run_decode<F>(items, now, rows, in_features, state->sms, state->error_word);
+        cudaError_t e;
+        if constexpr (kQ3) {
+            DecodeItem items[gemv::kMaxGroup];
+            for (uint32_t i = 0; i < now; ++i) items[i] = {inputs[first + i], weights[first + i], outputs[first + i], out_features[first + i]};
+            e = run_decode<q3::Format>(items, now, rows, in_features, state->sms, state->error_word);
+        } else {
+            nvfp4d::Item items[nvfp4d::kMaxGroup];
+            for (uint32_t i = 0; i < now; ++i) items[i] = {inputs[first + i], weights[first + i], outputs[first + i], out_features[first + i]};
+            e = nvfp4d::decode(items, now, rows, in_features, kFormat == DecodeFormat::kNvfp4Table, state->sms, t_stream, t_pdl != 0 && t_stream != nullptr,
+                    state->error_word);
+        }
         if (e == cudaErrorNotSupported || e == cudaErrorInvalidConfiguration) return first == 0 ? EUHEDRAL_CUDA_ROUTE_UNAVAILABLE : EUHEDRAL_CUDA_KERNEL_UNAVAILABLE;
         if (e != cudaSuccess) return (int)e;
     }
@@ -547,12 +509,12 @@ int linear_group(uint32_t count, const void* const* inputs, const void* const* w
 }
 
 // The decode kernel of the layout (plain or table-indexed scales) when it takes the shape, else the scalar kernel.
-template <class F, bool kTable>
+template <bool kTable>
 int nvfp4_decode(DeviceState* state, const void* input, const void* weights, void* output, uint32_t rows, uint32_t in_features,
         uint32_t out_features) {
-    if (!g_exact.load() && rows <= 32u && decode_takes<F>(in_features, out_features)) {
-        DecodeItem item = {input, weights, output, out_features};
-        const cudaError_t e = run_decode<F>(&item, 1, rows, in_features, state->sms, state->error_word);
+    if (!g_exact.load() && rows <= 32u && nvfp4d::takes(in_features, out_features)) {
+        const nvfp4d::Item item = {input, weights, output, out_features};
+        const cudaError_t e = nvfp4d::decode(&item, 1, rows, in_features, kTable, state->sms, t_stream, t_pdl != 0 && t_stream != nullptr, state->error_word);
         if (e != cudaErrorNotSupported && e != cudaErrorInvalidConfiguration) return finish(e);
     }
     return finish(launch(kOrdered, exact::nvfp4_linear<kTable>, dim3(capped_grid((uint64_t)rows * out_features)), dim3(128), 0, 1u,
@@ -802,11 +764,11 @@ int euhedral_cuda_linear_nvfp4_bf16(const void* input, const void* weights, void
     DeviceState* state = nullptr;
     const int status = bind(&state);
     if (status != EUHEDRAL_CUDA_SUCCESS) return status;
-    return layout == 1 ? nvfp4_decode<nvfp4::FormatSd4, true>(state, input, weights, output, rows, in_features, out_features)
-                       : nvfp4_decode<nvfp4::Format, false>(state, input, weights, output, rows, in_features, out_features);
+    return layout == 1 ? nvfp4_decode<true>(state, input, weights, output, rows, in_features, out_features)
+                       : nvfp4_decode<false>(state, input, weights, output, rows, in_features, out_features);
 }
 
-// Process-wide: native calls of 1024 rows and more run on CTA pairs (tcgen05 cta_group::2), unless switched off.
+// Process-wide: native calls of 512 rows and more run on CTA pairs (tcgen05 cta_group::2), unless switched off.
 static std::atomic<bool> g_native_pairs{true};
 
 void euhedral_b200_select_native_pairs(int enabled) { g_native_pairs.store(enabled != 0); }
@@ -1218,9 +1180,16 @@ int euhedral_b200_decode_plan(int format, uint32_t rows, uint32_t in_features, u
     if (out_features == 0 || out_features % 16u != 0 || in_features % 128u != 0) return EUHEDRAL_CUDA_INVALID_ARGUMENT;
     DecodePlan plan;
     const uint32_t tiles = out_features / 16u;
-    const bool ok = format == 0 ? plan_decode<nvfp4::Format>(rows, in_features, tiles, tiles, sms, &plan)
-                                : plan_decode<q3::Format>(rows, in_features, tiles, tiles, sms, &plan);
-    if (!ok) return EUHEDRAL_CUDA_INVALID_ARGUMENT;
+    if (format == 0) {
+        // The slices and pieces by which a register decode would cut K; the launch is nvfp4_decode.cuh's.
+        nvfp4d::Plan launch;
+        plan.order = gemv::order_of<Nvfp4Cut>(in_features);
+        if (!plan.order.ok || !nvfp4d::plan_rows(rows, in_features, &launch)) return EUHEDRAL_CUDA_INVALID_ARGUMENT;
+        plan.ctas = std::min((uint32_t)sms / plan.order.split, std::max(1u, out_features / nvfp4d::kTile)) * plan.order.split;
+        plan.shared = launch.shared;
+    } else if (!plan_decode<q3::Format>(rows, in_features, tiles, tiles, sms, &plan)) {
+        return EUHEDRAL_CUDA_INVALID_ARGUMENT;
+    }
     *k_slices = plan.order.split;
     *pieces = plan.order.team;
     *piece_chunks = plan.order.piece;
@@ -1231,7 +1200,7 @@ int euhedral_b200_decode_plan(int format, uint32_t rows, uint32_t in_features, u
 
 int euhedral_b200_linear_group_q3_bf16(uint32_t count, const void* const* inputs, const void* const* weights, void* const* outputs,
         uint32_t rows, uint32_t in_features, const uint32_t* out_features, const uint64_t* weights_byte_sizes) {
-    return linear_group<q3::Format>(count, inputs, weights, outputs, rows, in_features, out_features, weights_byte_sizes);
+    return linear_group<DecodeFormat::kQ3>(count, inputs, weights, outputs, rows, in_features, out_features, weights_byte_sizes);
 }
 
 int euhedral_b200_linear_group_nvfp4_bf16(uint32_t count, const void* const* inputs, const void* const* weights, void* const* outputs,
@@ -1239,8 +1208,8 @@ int euhedral_b200_linear_group_nvfp4_bf16(uint32_t count, const void* const* inp
     // plain or table-indexed scales, told apart by the first tensor's byte size; a group holds one layout
     if (count != 0 && out_features != nullptr && weights_byte_sizes != nullptr && out_features[0] != 0
             && nvfp4_layout(out_features[0], in_features, weights_byte_sizes[0]) == 1)
-        return linear_group<nvfp4::FormatSd4>(count, inputs, weights, outputs, rows, in_features, out_features, weights_byte_sizes);
-    return linear_group<nvfp4::Format>(count, inputs, weights, outputs, rows, in_features, out_features, weights_byte_sizes);
+        return linear_group<DecodeFormat::kNvfp4Table>(count, inputs, weights, outputs, rows, in_features, out_features, weights_byte_sizes);
+    return linear_group<DecodeFormat::kNvfp4>(count, inputs, weights, outputs, rows, in_features, out_features, weights_byte_sizes);
 }
 
 }  // extern "C"

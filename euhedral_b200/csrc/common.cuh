@@ -8,7 +8,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <type_traits>
+#include <vector>
 
 namespace eb {
 
@@ -94,6 +96,38 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
         if (mbar_try_wait(bar, parity)) return true;
     return false;
 }
+
+// Bounded wait of a role whose loops must not depend on its outcome: when the phase does not complete within kSpinLimit polls, or
+// another wait of the CTA has given up before, `failed` (a word of shared memory) is set and the wait is over. The kernel
+// runs to its end on whatever it has and reports the failure there.
+__device__ __forceinline__ void mbar_wait_or_fail(uint64_t* bar, uint32_t parity, uint32_t* failed) {
+    const uint32_t at = smem_u32(bar);
+    for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
+        if (mbar_try_wait_at(at, parity)) return;
+        if ((spin & 15u) == 15u && *reinterpret_cast<volatile uint32_t*>(failed) != 0u) return;
+    }
+    *reinterpret_cast<volatile uint32_t*>(failed) = 1u;
+}
+
+// True in one lane of the (converged) warp, the same one every time. A role that one thread plays is written as a loop of the whole
+// warp with the instructions that only one thread may issue under this predicate: control flow and addresses stay uniform, so
+// that they live in uniform registers. Under `if (lane == 0)` every tcgen05.mma cost about 190 cycles to issue.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t chosen;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xFFFFFFFF;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(chosen));
+    return chosen != 0;
+}
+
+// Where a role stands in a ring of `count` stages: the stage and the parity of its round.
+struct Ring {
+    uint32_t stage = 0, parity = 0;
+    __device__ __forceinline__ void advance(uint32_t count) {
+        if (++stage == count) {
+            stage = 0;
+            parity ^= 1u;
+        }
+    }
+};
 
 // ---- bulk asynchronous copy global -> shared (TMA engine, no tensor map) ----------------------------------------
 // Source, destination and size are multiples of 16 bytes. Completion is signalled on `bar` (complete_tx).
@@ -321,6 +355,68 @@ inline EncodeTiled encoder() {
         return reinterpret_cast<EncodeTiled>(entry);
     }();
     return cached;
+}
+
+// One launch on `stream` with a cluster dimension of `cluster` CTAs (1: none) and, when asked, programmatic dependent launch.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_on(cudaStream_t stream, bool pdl, unsigned cluster, void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared,
+        Args... args) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = shared;
+    config.stream = stream;
+    cudaLaunchAttribute attributes[2];
+    unsigned count = 0;
+    if (cluster > 1u) {
+        attributes[count].id = cudaLaunchAttributeClusterDimension;
+        attributes[count].val.clusterDim.x = cluster;
+        attributes[count].val.clusterDim.y = 1;
+        attributes[count].val.clusterDim.z = 1;
+        ++count;
+    }
+    if (pdl) {
+        attributes[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attributes[count].val.programmaticStreamSerializationAllowed = 1;
+        ++count;
+    }
+    config.attrs = attributes;
+    config.numAttrs = count;
+    return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
+// Clusters of `split` CTAs of a kernel that the current device holds at once (0: none fit), cached per device, kernel and shape.
+inline uint32_t resident_clusters(const void* kernel, uint32_t threads, uint32_t shared, uint32_t split) {
+    struct Entry {
+        int device;
+        const void* kernel;
+        uint32_t threads, shared, split, clusters;
+    };
+    static std::mutex mutex;
+    static std::vector<Entry> cache;
+    int device = -1;
+    if (cudaGetDevice(&device) != cudaSuccess) return 0u;
+    std::lock_guard<std::mutex> lock(mutex);
+    for (const Entry& e : cache)
+        if (e.device == device && e.kernel == kernel && e.threads == threads && e.shared == shared && e.split == split) return e.clusters;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(split * 1024u);
+    config.blockDim = dim3(threads);
+    config.dynamicSmemBytes = shared;
+    cudaLaunchAttribute attribute;
+    attribute.id = cudaLaunchAttributeClusterDimension;
+    attribute.val.clusterDim.x = split;
+    attribute.val.clusterDim.y = 1;
+    attribute.val.clusterDim.z = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0u;
+    }
+    cache.push_back({device, kernel, threads, shared, split, (uint32_t)clusters});
+    return (uint32_t)clusters;
 }
 
 }  // namespace eb

@@ -38,6 +38,13 @@
 
 #include "common.cuh"
 
+namespace nvfp4d {   // nvfp4_decode.cuh: the kernel that takes few rows
+inline cudaError_t quantized(const void* weights, void* output, const CUtensorMap& activations, const uint8_t* atoms, const float* row_globals, uint32_t rows,
+        uint32_t k, uint32_t out_features, bool paired, bool table, int sms, cudaStream_t stream, bool pdl, uint32_t* error);
+inline bool better_for(uint32_t rows, uint32_t k, uint32_t out_features, bool paired, uint32_t sms);
+inline uint32_t columns_of(uint32_t rows);
+}  // namespace nvfp4d
+
 namespace nvfp4n {
 
 constexpr uint32_t kTerms = 2;
@@ -60,8 +67,8 @@ constexpr uint32_t kPanel = 8u;                            // tile columns per p
 __host__ __device__ inline uint64_t align256(uint64_t v) { return (v + 255ull) & ~255ull; }
 
 // Caller scratch of one native linear.
-// Calls of at most kSkinnyRows rows (one row tile) may cut K over up to kMaxSplits CTAs per output tile, so that a call
-// with few output tiles still uses every SM; the FP32 partial tiles go to the end of the scratch.
+// Callers of at most kSkinnyRows rows are asked for room for kMaxSplits FP32 copies of the output behind it, which no kernel here
+// uses any more: the size is part of what callers were told.
 constexpr uint32_t kSkinnyRows = 64, kMaxSplits = 8;
 
 struct ActivationLayout {
@@ -367,8 +374,8 @@ struct TileWalk {
 
 __global__ void __launch_bounds__(kScaledThreads, 1) gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
         const __grid_constant__ CUtensorMap map_s, const uint8_t* __restrict__ sfa, const float* __restrict__ row_globals,
-        const float* __restrict__ tensor_global, uint16_t* __restrict__ out, float* __restrict__ partials, uint32_t splits, uint32_t rows,
-        uint32_t n, uint32_t k, uint32_t pair_tiles, uint32_t* __restrict__ error) {
+        const float* __restrict__ tensor_global, uint16_t* __restrict__ out, uint32_t rows, uint32_t n, uint32_t k,
+        uint32_t pair_tiles, uint32_t* __restrict__ error) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
@@ -383,8 +390,6 @@ __global__ void __launch_bounds__(kScaledThreads, 1) gemm_kernel(const __grid_co
     const bool paired = pair_tiles != 0u;
     const TileWalk walk(rows, n, paired ? 128u : kTileN);
     const uint32_t k_steps = k / kStepK, k_blocks = k / kBlockK;
-    // A work item is an output tile and one of `splits` ranges of its K steps (one range unless the call is skinny).
-    const uint32_t items = walk.total * splits;
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < kStages; ++s) {
@@ -413,11 +418,10 @@ __global__ void __launch_bounds__(kScaledThreads, 1) gemm_kernel(const __grid_co
         if (lane == 0) {
             uint32_t step = 0;
             bool ok = true;
-            for (uint32_t item = blockIdx.x; item < items && ok; item += gridDim.x) {
+            for (uint32_t item = blockIdx.x; item < walk.total && ok; item += gridDim.x) {
                 uint32_t tm, tn;
-                walk.at(item / splits, &tm, &tn);
-                const uint32_t split = item % splits, ks_end = (split + 1u) * k_steps / splits;
-                for (uint32_t ks = split * k_steps / splits; ks < ks_end; ++ks, ++step) {
+                walk.at(item, &tm, &tn);
+                for (uint32_t ks = 0; ks < k_steps; ++ks, ++step) {
                     const uint32_t s = step % kStages, round = step / kStages;
                     if (round > 0 && !eb::mbar_wait(&empty[s], (round - 1u) & 1u)) {
                         atomicOr(error, 8u);
@@ -443,14 +447,13 @@ __global__ void __launch_bounds__(kScaledThreads, 1) gemm_kernel(const __grid_co
         if (lane == 0) {
             uint32_t step = 0, local = 0;
             bool ok = true;
-            for (uint32_t item = blockIdx.x; item < items && ok; item += gridDim.x, ++local) {
+            for (uint32_t item = blockIdx.x; item < walk.total && ok; item += gridDim.x, ++local) {
                 if (local > 0 && !eb::mbar_wait(acc_empty, (local - 1u) & 1u)) {
                     atomicOr(error, 8u);
                     break;
                 }
                 tcgen05_fence_after();
-                const uint32_t split = item % splits, ks_begin = split * k_steps / splits, ks_end = (split + 1u) * k_steps / splits;
-                for (uint32_t ks = ks_begin; ks < ks_end; ++ks, ++step) {
+                for (uint32_t ks = 0; ks < k_steps; ++ks, ++step) {
                     const uint32_t s = step % kStages, round = step / kStages;
                     if (!eb::mbar_wait(&full[s], round & 1u) || !eb::mbar_wait(&scaled[s], round & 1u)) {
                         atomicOr(error, 8u);
@@ -463,7 +466,7 @@ __global__ void __launch_bounds__(kScaledThreads, 1) gemm_kernel(const __grid_co
                     const uint32_t scales = tmem + kTmemScales + s * kScaleColumns;
 #pragma unroll
                     for (uint32_t j = 0; j < 4u; ++j) {
-                        mma_block_scaled(tmem, a0 + 2u * j, b + 2u * j, scales + j * 8u, scales + 32u + j * 8u, (uint32_t)(((ks - ks_begin) | j) != 0u));
+                        mma_block_scaled(tmem, a0 + 2u * j, b + 2u * j, scales + j * 8u, scales + 32u + j * 8u, (uint32_t)((ks | j) != 0u));
                         mma_block_scaled(tmem, a1 + 2u * j, b + 2u * j, scales + j * 8u + 4u, scales + 32u + j * 8u, 1u);
                     }
                     mma_commit(&empty[s]);
@@ -476,9 +479,8 @@ __global__ void __launch_bounds__(kScaledThreads, 1) gemm_kernel(const __grid_co
         registers_give_back<96>();
         uint32_t step = 0;
         bool ok = true;
-        for (uint32_t item = blockIdx.x; item < items && ok; item += gridDim.x) {
-            const uint32_t split = item % splits, ks_end = (split + 1u) * k_steps / splits;
-            for (uint32_t ks = split * k_steps / splits; ks < ks_end; ++ks, ++step) {
+        for (uint32_t item = blockIdx.x; item < walk.total && ok; item += gridDim.x) {
+            for (uint32_t ks = 0; ks < k_steps; ++ks, ++step) {
                 const uint32_t s = step % kStages, round = step / kStages;
                 if (!eb::mbar_wait(&full[s], round & 1u)) {
                     if (lane == 0) atomicOr(error, 8u);
@@ -498,9 +500,9 @@ __global__ void __launch_bounds__(kScaledThreads, 1) gemm_kernel(const __grid_co
         const uint32_t quarter = warp & 3u, half = (warp - 8u) >> 2;
         const float scale_w = *tensor_global;
         uint32_t local = 0;
-        for (uint32_t item = blockIdx.x; item < items; item += gridDim.x, ++local) {
+        for (uint32_t item = blockIdx.x; item < walk.total; item += gridDim.x, ++local) {
             uint32_t tm, tn;
-            walk.at(item / splits, &tm, &tn);
+            walk.at(item, &tm, &tn);
             if (!eb::mbar_wait(acc_full, local & 1u)) {
                 if (lane == 0) atomicOr(error, 8u);
                 break;
@@ -520,23 +522,7 @@ __global__ void __launch_bounds__(kScaledThreads, 1) gemm_kernel(const __grid_co
             if (lane == 0) eb::mbar_arrive(acc_empty);
             const uint32_t row = tm * kTileM + quarter * 32u + lane;
             const float scale = row < rows ? __fmul_rn(row_globals[row], scale_w) : 0.0f;
-            if (splits > 1u) {
-                // the raw FP32 sums of this K range: partials[split][row][n]; finish_splits adds the ranges in order
-#pragma unroll
-                for (uint32_t cb = 0; cb < 4u; ++cb) {
-                    const uint32_t col = tn * kTileN + half * 128u + cb * 32u;
-                    if (row < rows && col < n) {
-                        float4* dst = reinterpret_cast<float4*>(partials + ((uint64_t)(item % splits) * rows + row) * n + col);
-#pragma unroll
-                        for (int v = 0; v < 8; ++v)
-                            if (col + 4u * v < n)
-                                dst[v] = make_float4(__uint_as_float(r[cb][4 * v]), __uint_as_float(r[cb][4 * v + 1]), __uint_as_float(r[cb][4 * v + 2]),
-                                        __uint_as_float(r[cb][4 * v + 3]));
-                    }
-                }
-            } else {
-                store_block(r, out, row, rows, n, paired ? tn * 128u + half * 64u : tn * kTileN + half * 128u, scale, paired);
-            }
+            store_block(r, out, row, rows, n, paired ? tn * 128u + half * 64u : tn * kTileN + half * 128u, scale, paired);
         }
     }
     tcgen05_fence_before();
@@ -766,29 +752,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kScaledThreads, 1) g
     }
 }
 
-// Skinny calls: out[row][col] = bf16((sum over the K ranges in order) * row scale * tensor scale). One thread per 4 columns.
-__global__ void __launch_bounds__(256) finish_splits(const float* __restrict__ partials, const float* __restrict__ row_globals,
-        const float* __restrict__ tensor_global, uint16_t* __restrict__ out, uint32_t splits, uint32_t rows, uint32_t n) {
-    const uint64_t index = (uint64_t)blockIdx.x * 256u + threadIdx.x;
-    eb::pdl_launch_dependents();
-    eb::pdl_wait();
-    const uint32_t quads = n / 4u;
-    if (index >= (uint64_t)rows * quads) return;
-    const uint32_t row = (uint32_t)(index / quads), col = (uint32_t)(index % quads) * 4u;
-    float4 sum = *reinterpret_cast<const float4*>(partials + (uint64_t)row * n + col);
-    for (uint32_t s = 1; s < splits; ++s) {
-        const float4 part = *reinterpret_cast<const float4*>(partials + ((uint64_t)s * rows + row) * n + col);
-        sum.x = __fadd_rn(sum.x, part.x);
-        sum.y = __fadd_rn(sum.y, part.y);
-        sum.z = __fadd_rn(sum.z, part.z);
-        sum.w = __fadd_rn(sum.w, part.w);
-    }
-    const float scale = __fmul_rn(row_globals[row], *tensor_global);
-    const uint32_t lo = (uint32_t)eb::float_to_bf16_bits(__fmul_rn(sum.x, scale)) | (uint32_t)eb::float_to_bf16_bits(__fmul_rn(sum.y, scale)) << 16;
-    const uint32_t hi = (uint32_t)eb::float_to_bf16_bits(__fmul_rn(sum.z, scale)) | (uint32_t)eb::float_to_bf16_bits(__fmul_rn(sum.w, scale)) << 16;
-    *reinterpret_cast<uint2*>(out + (uint64_t)row * n + col) = make_uint2(lo, hi);
-}
-
 // ---- host side ------------------------------------------------------------------------------------------------------------
 
 using eb::EncodeTiled;
@@ -800,23 +763,13 @@ inline cudaError_t initialize() {
 }
 
 // Fewer rows than this run on single CTAs. The pairs are 2 to 6 % faster from 1024 rows on (1024 x 5120 x 17408: 171 against 176
-// us, 4096 x 17408 x 5120: 318 against 337 in turn) and equal or a little slower below, where their 256-row tiles leave more
-// of the last wave empty.
-constexpr uint32_t kPairRows = 1024;
+// us, 4096 x 17408 x 5120: 318 against 337 in turn), equal within 1 % at 512 to 1024; with fewer rows their 256-row tiles
+// leave more of the last wave empty.
+constexpr uint32_t kPairRows = 512;
 
 template <typename... Params, typename... Args>
 inline cudaError_t launch_on(cudaStream_t stream, bool pdl, void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared, Args... args) {
-    cudaLaunchConfig_t config = {};
-    config.gridDim = grid;
-    config.blockDim = block;
-    config.dynamicSmemBytes = shared;
-    config.stream = stream;
-    cudaLaunchAttribute attribute;
-    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute.val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = &attribute;
-    config.numAttrs = pdl ? 1u : 0u;
-    return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+    return eb::launch_on(stream, pdl, 1u, kernel, grid, block, shared, args...);
 }
 
 // The launches of a native linear. Shapes are pre-checked by the caller: k % 256 == 0, out_features % 128 == 0,
@@ -850,11 +803,20 @@ inline cudaError_t multiply(const void* weights, void* output, void* scratch, ui
     CUtensorMap map_a, map_b, map_s;
     const cuuint32_t ones[3] = {1u, 1u, 1u};
     const cuuint64_t a_dims[3] = {row_bytes, rows, kTerms}, a_strides[2] = {row_bytes, row_bytes * rows};
-    const cuuint32_t a_box[3] = {128u, kTileM, 1u};
+    // few rows: one kernel with the weights as the 128-row operand (nvfp4_decode.cuh), the rows as columns of a narrower box
+    const bool few = nvfp4d::better_for(rows, k, out_features, paired, (uint32_t)sms);
+    const cuuint32_t a_box[3] = {128u, few ? nvfp4d::columns_of(rows) : kTileM, 1u};
     const cuuint64_t b_dims[2] = {row_bytes, out_features}, b_strides[1] = {row_bytes};
     const cuuint32_t b_box[2] = {128u, 128u};   // half a B tile: the kernel places the two halves itself
     CUresult r = encode(&map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, base, a_dims, a_strides, a_box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const float* row_globals = reinterpret_cast<const float*>(base + layout.global_offset);
+    if (few && r == CUDA_SUCCESS) {
+        const cudaError_t e = nvfp4d::quantized(weights, output, map_a, base + layout.sfa_offset, row_globals, rows, k, out_features, paired, table_scales, sms, stream,
+                pdl, error);
+        if (e != cudaErrorNotSupported) return e;
+        return cudaErrorInvalidValue;
+    }
     if (r == CUDA_SUCCESS)
         r = encode(&map_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(w), b_dims, b_strides, b_box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -875,13 +837,7 @@ inline cudaError_t multiply(const void* weights, void* output, void* scratch, ui
     }
     const uint32_t pair_tiles = paired ? out_features / 256u : 0u, width = paired ? out_features / 2u : out_features;
     const uint32_t tiles = ((rows + kTileM - 1u) / kTileM) * (paired ? pair_tiles : (out_features + kTileN - 1u) / kTileN);
-    // The skinny route (the reference's 9..64-row kernel, native/src/nvfp4_native/native.cuh:435-585, cuts K the same way):
-    // few rows make few output tiles; K is cut so that about every SM gets a work item.
-    uint32_t splits = 1;
-    if (!paired && rows <= kSkinnyRows && tiles * 2u <= (uint32_t)sms) splits = std::max(1u, std::min(std::min(kMaxSplits, k / kStepK), (uint32_t)sms / tiles));
-    const uint32_t work = tiles * splits, grid = work < (uint32_t)sms ? work : (uint32_t)sms;
-    float* partials = reinterpret_cast<float*>(base + layout.partial_offset);
-    const float* row_globals = reinterpret_cast<const float*>(base + layout.global_offset);
+    const uint32_t grid = tiles < (uint32_t)sms ? tiles : (uint32_t)sms;
     const float* tensor_global = reinterpret_cast<const float*>(w + global_offset);
     if (pairs && rows >= kPairRows) {
         const uint32_t pair_items = ((rows + 255u) / 256u) * (paired ? pair_tiles : (out_features + 255u) / 256u);
@@ -889,12 +845,8 @@ inline cudaError_t multiply(const void* weights, void* output, void* scratch, ui
         return launch_on(stream, pdl, gemm_pair_kernel, dim3(ctas), dim3(kScaledThreads), kPairShared, map_a, map_b, map_s,
                 base + layout.sfa_offset, row_globals, tensor_global, static_cast<uint16_t*>(output), rows, width, k, pair_tiles, error);
     }
-    e = launch_on(stream, pdl, gemm_kernel, dim3(grid), dim3(kScaledThreads), kSharedBytes, map_a, map_b, map_s,
-            base + layout.sfa_offset, row_globals, tensor_global, static_cast<uint16_t*>(output), partials, splits, rows, width, k, pair_tiles, error);
-    if (e != cudaSuccess || splits == 1u) return e;
-    const uint64_t quads = (uint64_t)rows * (out_features / 4u);
-    return launch_on(stream, pdl, finish_splits, dim3((unsigned)((quads + 255u) / 256u)), dim3(256), 0, partials, row_globals, tensor_global,
-            static_cast<uint16_t*>(output), splits, rows, out_features);
+    return launch_on(stream, pdl, gemm_kernel, dim3(grid), dim3(kScaledThreads), kSharedBytes, map_a, map_b, map_s, base + layout.sfa_offset, row_globals,
+            tensor_global, static_cast<uint16_t*>(output), rows, width, k, pair_tiles, error);
 }
 
 inline cudaError_t run(const void* input, const void* weights, void* output, void* scratch, uint32_t rows, uint32_t k, uint32_t out_features,

@@ -112,8 +112,9 @@ EUHEDRAL_CUDA_EXPORT int euhedral_cuda_linear_launch(int32_t kernel, uint32_t gr
 EUHEDRAL_CUDA_EXPORT int euhedral_b200_take_device_error(uint32_t* word);
 /* How a decode GEMV of this shape runs. k_slices (cluster size), pieces (warps that share a 16-row tile's slice) and
  * piece_chunks (128-value chunks of the widest piece) depend on the format and in_features only and fix the summation
- * order; ctas and shared_bytes are the launch for `rows` activation rows. format: 0 NVFP4, 1 Q3. Returns 0, or -1 for a
- * shape the decode kernels do not take. */
+ * order; ctas and shared_bytes are the launch for `rows` activation rows. format: 0 NVFP4, 1 Q3. For NVFP4, whose kernel lets
+ * the tensor core sum its slices, k_slices, pieces and piece_chunks are the cut of a decode through registers and say nothing
+ * about the launch. Returns 0, or -1 for a shape the decode kernels do not take. */
 EUHEDRAL_CUDA_EXPORT int euhedral_b200_decode_plan(int format, uint32_t rows, uint32_t in_features, uint32_t out_features,
         uint32_t* k_slices, uint32_t* pieces, uint32_t* piece_chunks, uint32_t* ctas, uint32_t* shared_bytes);
 
@@ -160,7 +161,7 @@ EUHEDRAL_CUDA_EXPORT int euhedral_b200_linear_nvfp4_native_prequantized_bf16(con
         void* scratch, uint32_t rows, uint32_t in_features, uint32_t out_features, uint64_t weights_byte_size,
         uint64_t scratch_byte_size);
 
-/* No counterpart in the reference. Process-wide switch of the native route: when enabled, calls of 1024 rows and more run
+/* No counterpart in the reference. Process-wide switch of the native route: when enabled, calls of 512 rows and more run
  * the GEMM on CTA pairs (tcgen05 cta_group::2: an output tile of 256 x 256 per pair, half of the weight tile per CTA);
  * the results are bit for bit those of the single-CTA kernel. On unless switched off: the pairs are 2-6 % faster. */
 EUHEDRAL_CUDA_EXPORT void euhedral_b200_select_native_pairs(int enabled);
