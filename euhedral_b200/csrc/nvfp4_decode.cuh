@@ -4,9 +4,11 @@
 // Two sources of activations (template parameter):
 //   * BF16 rows (euhedral_cuda_linear_nvfp4_bf16 and the grouped calls, up to kMaxRows). kind::mxf4nvf4 multiplies E2M1 by E2M1, so
 //     a CTA writes its K slice of every activation row as EIGHT E2M1 terms of three bits each - the octal digits, -4 to 3, of
-//     the value as an integer of 24 bits on the grid of the slice's largest value - and a row becomes eight columns. Products
-//     are exact; column t of a row counts 8^-t and the eight sums are added in FP32 once per K slice. A value is cut at 2^-22 of
-//     the slice's largest power of two: the size of one rounding of an FP32 sum that holds that value.
+//     the value as an integer of 24 bits, in units of 2^-21 of the power of two of the row's largest value of the slice - and a
+//     row becomes eight columns. Products are exact; column t of a row counts 8^-t and the eight sums are added in FP32 once per K
+//     slice. Where some eight neighbours of a row stay below 2^-4 of the slice's largest (outliers), four more columns hold the
+//     next four digits of what the eight cut off: nothing above 2^-33 of the largest value is lost then. The choice is a row's and
+//     slice's own and changes no bit of the rows beside it.
 //   * two NVFP4 terms per row, quantized into the scratch before (the native route): a row is one column, both terms accumulate
 //     into it, as in the large GEMM (nvfp4_native.cuh), and more than kMaxColumns rows take a tile of weights several times.
 //     With `pair_rows` a tile is 64 gate rows and the 64 up rows that match them, finished as SwiGLU (the paired region).
@@ -22,8 +24,7 @@
 // to 1.3 us at one row (1024 x 5120: 4.1 / 6.2 / 11.0 -> 5.4 / 7.5 / 8.5). The native route's few rows: a layer's four fused
 // linears at 40 rows 176 -> 98 us, quantizers included.
 // Instructions that one thread issues for the tensor core sit in a loop of the whole warp under an elected predicate (eb::elect_one):
-// 757 -> 453 cycles per unit of 256 values. Block scales of the digits would have to lie at multiples of four columns of tensor
-// memory; one grid per row and slice needs none.
+// 757 -> 453 cycles per unit of 256 values.
 //
 // Execution:
 //   * K is cut into units of 256 and these over the CTAs of a cluster. For BF16 rows the cut (split_of) is a function of K only, as is
@@ -45,7 +46,7 @@
 
 namespace nvfp4d {
 
-constexpr uint32_t kTile = 128, kUnit = 256, kDigits = 8;
+constexpr uint32_t kTile = 128, kUnit = 256, kDigits = 8, kMoreDigits = 4;
 constexpr uint32_t kMaxRows = 16;         // BF16 activation rows of a launch
 constexpr uint32_t kMaxColumns = 64;      // quantized activation rows of an item
 constexpr uint32_t kMaxGroup = 8;         // tensors of a launch
@@ -53,6 +54,7 @@ constexpr uint32_t kThreads = 512, kStagers = 320;   // staging warps: 2, 3 and 
 constexpr uint32_t kCodeBytes = kTile * kUnit / 2u, kScaleBytes = kTile * kUnit / 16u;
 constexpr uint32_t kMaxStages = 8;
 constexpr uint32_t kTmemColumns = 512;
+constexpr uint32_t kSpread = 4;           // powers of two that one grid covers (see above)
 constexpr uint32_t kLeastExponent = 48;   // of a row's slice: smaller values keep the grid of 2^-79
 
 __host__ __device__ inline uint32_t units_of(uint32_t k) { return (k + kUnit - 1u) / kUnit; }
@@ -88,10 +90,11 @@ struct alignas(64) Group {
 //   columns: of an item (resident: the digits of the rows; else the rows, to a multiple of 32). n: of the MMA - quantized rows
 //   bring their two terms as columns of their own.
 struct Layout {
-    uint32_t columns, n, width, pitch, stage_bytes, off_rows, off_gather, gather_bytes, off_bars, bytes;
+    uint32_t columns, n, plain_n, width, pitch, stage_bytes, off_rows, off_gather, gather_bytes, off_bars, bytes;
     __host__ __device__ Layout(bool resident, uint32_t rows, uint32_t units_cta, uint32_t stages, uint32_t split, bool paired) {
-        columns = resident ? (rows * kDigits + 15u) / 16u * 16u : rows >= kMaxColumns ? kMaxColumns : (rows + 7u) / 8u * 8u;
+        columns = resident ? (rows * (kDigits + kMoreDigits) + 15u) / 16u * 16u : rows >= kMaxColumns ? kMaxColumns : (rows + 7u) / 8u * 8u;
         n = resident ? columns : nvfp4n::kTerms * columns;
+        plain_n = resident ? (rows * kDigits + 15u) / 16u * 16u : n;   // of rows without outliers: the first eight digits come first
         width = resident ? rows : columns;                           // sums of a weight row and slice that travel together
         pitch = columns + 4u;                                        // quantized rows: floats from row to row of an exchange buffer
         gather_bytes = resident ? kTile * width * 4u : kTile * pitch * 4u;   // one of the two exchange buffers
@@ -132,6 +135,9 @@ __device__ __forceinline__ void tmem_store(uint32_t to, const uint32_t* r) {
             : "memory");
     if constexpr (N == 32) tmem_store<16>(to + 16u, r + 16);
 }
+__device__ __forceinline__ void tmem_load_4(uint32_t (&r)[4], uint32_t from) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(from));
+}
 __device__ __forceinline__ void tmem_load_8(uint32_t (&r)[8], uint32_t from) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
@@ -151,16 +157,18 @@ __device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t
             : "memory");
 }
 
-// Eight values of a block as eight octal digits each, transposed: word t holds digit t (the highest first) of the eight values as
-// E2M1 codes, value i in nibble i. `grid`: 2^21 over the block's power of two.
-__device__ __forceinline__ void octal_digits(const uint4& v, float grid, uint32_t (&word)[8]) {
+// Eight values as eight octal digits each, transposed: word t holds digit t (the highest first) of the eight values as E2M1 codes,
+// value i in nibble i. The values are counted in units of 1 / `per`; `more`: what that count cuts off, in units of 2^-22 / `per`.
+__device__ __forceinline__ void octal_digits(const uint4& v, float per, bool more, uint32_t (&word)[8]) {
     const uint32_t pairs[4] = {v.x, v.y, v.z, v.w};
+    const float unit = __uint_as_float(0x7F000000u - __float_as_uint(per)), count = more ? __uint_as_float(__float_as_uint(per) + (22u << 23)) : per;
     uint32_t a[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const float x = (i & 1) ? __uint_as_float(pairs[i >> 1] & 0xFFFF0000u) : __uint_as_float(pairs[i >> 1] << 16);
+        float x = (i & 1) ? __uint_as_float(pairs[i >> 1] & 0xFFFF0000u) : __uint_as_float(pairs[i >> 1] << 16);
+        if (more) x = __fmaf_rn(-__fsub_rn(__fmaf_rn(x, per, 12582912.0f), 12582912.0f), unit, x);   // exact
         // 1.5 * 2^23 + the integer, then + 4 in every octal digit: each digit less 4 is the signed digit
-        const uint32_t n = __float_as_uint(__fmaf_rn(x, grid, 12582912.0f)) - 0x4B400000u + 9586980u;
+        const uint32_t n = __float_as_uint(__fmaf_rn(x, count, 12582912.0f)) - 0x4B400000u + 9586980u;
         uint32_t s = (n & 0x00000FFFu) | ((n << 4) & 0x0FFF0000u);   // 24 bits of octal digits to eight nibbles
         s = (s & 0x003F003Fu) | ((s << 2) & 0x3F003F00u);
         s = (s & 0x07070707u) | ((s << 1) & 0x70707070u);
@@ -222,6 +230,8 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(gather_empty + 2);
     uint32_t* failed = tmem_holder + 1;
     uint32_t* exponents = failed + 1;        // per row: the largest exponent of the slice
+    uint32_t* least = exponents + kMaxRows;  // per row: the least of the largest exponents of eight neighbours
+    auto has_outliers = [&](uint32_t row) { return least[row] + kSpread < exponents[row]; };
     const uint32_t kBoxColumns = layout.columns;
 
     if (warp == 0) {
@@ -245,7 +255,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(eb::smem_u32(tmem_holder)), "r"(group.tmem_columns) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     } else if (warp == 2) {
-        if (lane < kMaxRows) exponents[lane] = kLeastExponent;
+        if (kResident && lane < kMaxRows) exponents[lane] = kLeastExponent, least[lane] = 255u;
     }
     nvfp4n::tcgen05_fence_before();
     __syncthreads();
@@ -345,7 +355,8 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
 
     if (warp == 1) {
         const bool leader = eb::elect_one();
-        const uint32_t instruction = (1u << 7) | (1u << 10) | ((layout.n >> 3) << 17) | ((kTile >> 4) << 24);
+        auto instruction_of = [](uint32_t n) { return (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((kTile >> 4) << 24); };
+        uint32_t instruction = instruction_of(layout.n);
         const uint64_t first_a = nvfp4n::tile_descriptor(smem), first_b = nvfp4n::tile_descriptor(smem + (kResident ? layout.off_rows : kCodeBytes));
         const uint16_t* held = nullptr;
         eb::Ring ring, accumulator;
@@ -355,6 +366,8 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
             if (kResident && t.x != held) {
                 held = t.x;
                 wait(staged, stagings++ & 1u);
+                const bool more = __any_sync(0xFFFFFFFFu, lane < rows && has_outliers(min(lane, rows - 1u)));
+                instruction = instruction_of(more ? layout.n : layout.plain_n);
             }
             const uint32_t buffer = accumulator.stage;
             if (used) wait(&acc_empty[buffer], accumulator.parity ^ 1u);
@@ -399,8 +412,8 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
         // The digits of every row of the slice, by the staging warps. Taken by all of them at the same points of the tile list; the
         // draining warps come when every MMA that reads the digits held before is done.
         auto stage_rows = [&](const uint16_t* x, bool again) {
-            // 8 values per lane. The first kHold loads of a warp are in flight together
-            // while it finds the rows' largest exponents; the pass that writes the digits finds the values in L1.
+            // 8 values per lane. The first kHold loads of a warp are in flight together while it finds the rows' exponents; the pass
+            // that writes the digits finds the values in L1.
             constexpr uint32_t kHold = 4;
             const uint32_t live = k / 8u - min(k / 8u, unit_begin * 32u);   // eighths of the slice
             Task at = first_task;
@@ -421,8 +434,12 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                 return max(most & 0xFFFFu, most >> 16) >> 7;
             };
             auto find = [&](uint32_t row, const uint4& v) {
-                const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, exponent(v));
-                if (row < rows && lane == 0) atomicMax(&exponents[row], most);
+                const uint32_t mine_most = exponent(v);   // 0: nothing but zeros (or subnormal values)
+                const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, mine_most), low = __reduce_min_sync(0xFFFFFFFFu, mine_most == 0u ? 255u : mine_most);
+                if (row < rows && lane == 0) {
+                    atomicMax(&exponents[row], most);
+                    atomicMin(&least[row], low);
+                }
             };
             if (mine != 0u) {
                 uint4 v[kHold];
@@ -434,7 +451,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                 }
                 if (again) {
                     stagers_sync();
-                    if (stager == 0u && lane < rows) exponents[lane] = kLeastExponent;
+                    if (stager == 0u && lane < rows) exponents[lane] = kLeastExponent, least[lane] = 255u;
                     stagers_sync();
                 }
 #pragma unroll
@@ -445,12 +462,21 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
 #pragma unroll 1
                 for (at = first_task; at.row < rows; next()) {
                     const uint4 values = load();
-                    const uint32_t m = at.row, unit = at.unit, top = exponents[m];
-                    uint32_t word[8];
-                    octal_digits(values, __uint_as_float((275u - top) << 23), word);
-                    uint8_t* tile = smem + layout.off_rows + unit * layout.columns * 128u + m * 1024u + (lane & 3u) * 4u;
+                    const uint32_t m = at.row, unit = at.unit;
+                    const float per = __uint_as_float((275u - exponents[m]) << 23);
+                    uint8_t* tile = smem + layout.off_rows + unit * layout.columns * 128u + (lane & 3u) * 4u;
+                    const uint32_t passes = has_outliers(m) ? 2u : 1u;
+#pragma unroll 1
+                    for (uint32_t pass = 0; pass < passes; ++pass) {
+                        uint32_t word[8];
+                        octal_digits(values, per, pass != 0u, word);
+                        const uint32_t column = pass == 0u ? m * kDigits : rows * kDigits + m * kMoreDigits;   // of digit 0; rows of 128 bytes, swizzled
+                        uint8_t* to = tile + (column >> 3) * 1024u;
+                        const uint32_t first = column & 7u;   // 0, or 4 for every other row's further digits
 #pragma unroll
-                    for (uint32_t t = 0; t < 8u; ++t) *reinterpret_cast<uint32_t*>(tile + t * 128u + (((lane >> 2) ^ t) << 4)) = word[t];
+                        for (uint32_t t = 0; t < 8u; ++t)
+                            if (t < kMoreDigits || pass == 0u) *reinterpret_cast<uint32_t*>(to + (first + t) * 128u + (((lane >> 2) ^ (first + t)) << 4)) = word[t];
+                    }
                 }
             }
             fence_async_proxy();
@@ -464,7 +490,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                 uint32_t ones[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) ones[i] = 0x38383838u;
-                tmem_store<16>(tm_rows + lanes, ones);
+                tmem_store<16>(tm_rows + lanes, ones);   // (of up to 192 columns: six words)
             }
             // ---- weight scales (and activation scales) of every stage to tensor memory ----
             eb::Ring ring;
@@ -581,6 +607,15 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                                 for (int i = 6; i >= 0; --i) sum = __fmaf_rn(sum, 0.125f, __uint_as_float(r[8 * h + i]));
                                 if (mine == 0u) sum = 0.0f;
                                 if (m + h < rows) {
+                                    if (has_outliers(m + h)) {
+                                        uint32_t q[4];
+                                        tmem_load_4(q, d + rows * kDigits + (m + h) * kMoreDigits);
+                                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                                        float rest = __uint_as_float(q[3]);
+#pragma unroll
+                                        for (int i = 2; i >= 0; --i) rest = __fmaf_rn(rest, 0.125f, __uint_as_float(q[i]));
+                                        if (mine != 0u) sum = __fmaf_rn(rest, 2.384185791015625e-07f, sum);   // 2^-22
+                                    }
                                     const uint32_t top = exponents[m + h];   // 255: a value of the slice is not finite
                                     send_f32(to + (m + h) * owned * 4u, __fmul_rn(__fadd_rn(sum, sum), top == 255u ? __uint_as_float(0x7FC00000u) : __uint_as_float(top << 23)), bar);
                                 }
@@ -653,7 +688,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                             const float* p = from + i * owned + row;
                             float sum = p[0];
                             for (uint32_t q = 1; q < split; ++q) sum = __fadd_rn(sum, p[q * width * owned]);
-                            if (at < before.t->n) before.t->y[(uint64_t)i * before.t->n + at] = eb::float_to_bf16_bits(__fmul_rn(sum, before.global));
+                            if (at < before.t->n) before.t->y[(uint64_t)i * before.t->n + at] = (uint16_t)eb::bf16_pair(__fmul_rn(sum, before.global), 0.0f);   // keeps a NaN one
                         }
                     } else {
                         const uint32_t quads = width / 4u;
@@ -826,7 +861,6 @@ inline cudaError_t launch(bool resident, bool table, Group* group, const Plan& p
     group->split = p.split;
     group->tmem_columns = p.tmem;
     group->buffers = p.buffers;
-
     group->scale_row_bytes = group->k / (table ? 32u : 16u);
     const Kernel kernel = kernel_of(resident, table);
     uint32_t most = (uint32_t)sms / p.split;

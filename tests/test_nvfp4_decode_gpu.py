@@ -1,0 +1,66 @@
+"""The tcgen05 kernel of few-row NVFP4 linears (csrc/nvfp4_decode.cuh) where it can go wrong: K below, at and past its unit of 256
+and past a cluster's share, output rows that end inside a tile, row counts at the edges of a launch, and activations whose
+magnitudes one grid cannot cover."""
+
+import numpy as np
+import pytest
+
+from oracle import oracle_c as OC
+from oracle import oracle_np as O
+from tests.gpu_util import Device, random_x
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    device = Device()
+    yield device
+    assert device.gpu.take_device_error() == 0
+    device.release()
+
+
+def run(dev, x_bits, d_w, n, k, size):
+    rows = x_bits.shape[0]
+    d_x, d_y = dev.put(x_bits), dev.empty(rows * n * 2)
+    with dev.submit(pdl=True, row_exact=True) as gpu:
+        gpu.linear_nvfp4_bf16(d_x.data_ptr(), d_w.data_ptr(), d_y.data_ptr(), rows, k, n, size)
+    return dev.get(d_y, np.uint16, (rows, n))
+
+
+@pytest.mark.parametrize("n,k", [(16, 128), (144, 256), (112, 384), (272, 1152), (1040, 4224), (128, 12416)])
+def test_edges_and_outliers(dev, n, k):
+    rng = np.random.default_rng(n + k)
+    weights = (rng.standard_normal((n, k)) * 0.02).astype(np.float32)
+    weights[:, 5::97] *= rng.integers(0, 2, (n, len(range(5, k, 97))))     # half of the outliers meet a zero weight
+    blob = OC.nvfp4_quantize(weights)
+    dense = OC.nvfp4_dense(blob, n, k)
+    d_w = dev.put(blob)
+    plain = rng.standard_normal((17, k)).astype(np.float32)
+    wide = plain.copy()
+    wide[:, 5::97] *= np.float32(2.0) ** rng.integers(4, 14, wide[:, 5::97].shape)   # up to 2^13 of their neighbours
+    wide[3] = plain[3]                                                             # rows of both kinds side by side
+    wide[4, : k // 2] = 0.0
+    wide[5] *= np.float32(2.0) ** -60
+    for values in (plain, wide):
+        x = O.bf16_bits(values)
+        single = np.concatenate([run(dev, x[r:r + 1], d_w, n, k, blob.size) for r in range(6)])
+        for rows in (2, 7, 16, 17):
+            got_bits = run(dev, x[:rows], d_w, n, k, blob.size)
+            assert np.array_equal(got_bits[:6], single[:min(rows, 6)]), rows          # a row's bits are its own
+            got, expect = O.bf16_to_f32(got_bits).astype(np.float64), O.linear_f64(x[:rows], dense)
+            # half a BF16 step of the value, and the rounding of FP32 sums of the terms that it is made of
+            terms = np.abs(O.bf16_to_f32(x[:rows]).astype(np.float64)) @ np.abs(dense.astype(np.float64)).T
+            assert np.all(np.abs(got - expect) <= np.abs(expect) * 2.0 ** -8 + terms * 2.0 ** -18), (rows, n, k)
+
+
+def test_values_that_are_not_finite(dev):
+    rng = np.random.default_rng(3)
+    n, k = 64, 512
+    blob = OC.nvfp4_quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32))
+    x = random_x(rng, 3, k)
+    clean = run(dev, x, dev.put(blob), n, k, blob.size)
+    x[1, 300] = 0x7F80                                                                 # infinity: the row is not a number, its neighbours stay
+    got = run(dev, x, dev.put(blob), n, k, blob.size)
+    assert np.array_equal(got[[0, 2]], clean[[0, 2]])
+    assert np.all((got[1] & 0x7FFF) > 0x7F80)
