@@ -438,13 +438,13 @@ cudaError_t launch_trellis_rotate(const void* x, const void* suh, void* act, int
             static_cast<const uint16_t*>(x), static_cast<const uint16_t*>(suh), static_cast<uint16_t*>(act), rows, k, s, layout);
 }
 
-cudaError_t launch_trellis_decode_bf16(const void* words, void* out, int k, int n, int w) {
+cudaError_t launch_trellis_decode_bf16(const void* words, void* out, int k, int n, int w, bool beside) {
     const uint64_t tiles = (uint64_t)(k / 16) * (uint64_t)(n / 16);
     switch (w) {
 #define EB_CASE(W) \
         case W: \
-            return launch(kOrdered, trellis::decode_bf16_kernel<W>, dim3((unsigned)((tiles + 8 * trellis::kBatch - 1) / (8 * trellis::kBatch))), dim3(256), 0, 1u, \
-                    static_cast<const uint16_t*>(words), static_cast<uint16_t*>(out), k, n);
+            return launch(kOverlappable, trellis::decode_bf16_kernel<W>, dim3((unsigned)((tiles + 8 * trellis::kBatch - 1) / (8 * trellis::kBatch))), dim3(256), 0, 1u, \
+                    static_cast<const uint16_t*>(words), static_cast<uint16_t*>(out), k, n, beside ? 1 : 0);
         EB_TRELLIS_WIDTHS(EB_CASE)
 #undef EB_CASE
         default: return cudaErrorInvalidValue;
@@ -917,7 +917,7 @@ int euhedral_cuda_linear_launch(int32_t kernel, uint32_t grid_x, uint32_t grid_y
                 return EUHEDRAL_CUDA_INVALID_ARGUMENT;   // 4-byte loads of the ring words, 16-byte stores of eight values
             const uint64_t tiles = (uint64_t)(k / 16) * (uint64_t)(n / 16);
             if (tiles > 2147483647ull) return EUHEDRAL_CUDA_SIZE_OVERFLOW;
-            return finish(launch_trellis_decode_bf16(reinterpret_cast<const void*>(a[0]), reinterpret_cast<void*>(a[1]), k, n, w));
+            return finish(launch_trellis_decode_bf16(reinterpret_cast<const void*>(a[0]), reinterpret_cast<void*>(a[1]), k, n, w, false));
         }
         case 6: {   // epilogue_bf16(rotated, ends, s, svh, out, rows, n)
             const int s = (int)a[2], rows = (int)a[5], n = (int)a[6];
@@ -1104,13 +1104,17 @@ int euhedral_b200_prefill_trellis_bf16(const void* input, const void* words, con
     uint8_t* activations = static_cast<uint8_t*>(scratch);
     uint8_t* decoded = activations + align_scratch((uint64_t)segments * rows * k * 2u);
     cudaError_t e = launch_trellis_rotate(input, suh, activations, (int)rows, (int)k, (int)segments, 1);
-    if (e == cudaSuccess) e = launch_trellis_decode_bf16(words, decoded, (int)k, (int)n, (int)tile_words);
+    if (e == cudaSuccess) e = launch_trellis_decode_bf16(words, decoded, (int)k, (int)n, (int)tile_words, true);
+    const bool pdl = t_pdl != 0 && t_stream != nullptr;
+    // the GEMM takes up to kMaxSegments segments a launch
     start = 0;
-    for (uint32_t g = 0; g < segments && e == cudaSuccess; ++g) {
-        const uint32_t width = (uint32_t)(host_segment_ends[g] - start);
+    for (uint32_t g = 0; g < segments && e == cudaSuccess; g += bf16n::kMaxSegments) {
+        const uint32_t count = std::min(bf16n::kMaxSegments, segments - g);
+        int32_t ends[bf16n::kMaxSegments];
+        for (uint32_t i = 0; i < count; ++i) ends[i] = host_segment_ends[g + i] - start;
         e = bf16n::linear(activations + (uint64_t)g * rows * k * 2u, decoded + (uint64_t)start * k * 2u, static_cast<uint16_t*>(output) + start,
-                static_cast<const uint16_t*>(svh) + start, n, rows, k, width, state->sms, t_stream, false, state->error_word);
-        start = host_segment_ends[g];
+                static_cast<const uint16_t*>(svh) + start, n, rows, k, (uint32_t)ends[count - 1u], state->sms, t_stream, pdl, state->error_word, 0, false, ends, count);
+        start = host_segment_ends[g + count - 1u];
     }
     return finish(e);
 }

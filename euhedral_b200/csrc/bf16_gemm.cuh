@@ -18,11 +18,11 @@
 
 namespace bf16n {
 
-using nvfp4n::kThreads;
 using nvfp4n::kTileM;
 using nvfp4n::kTileN;
 using nvfp4n::kTmemColumns;
 
+constexpr uint32_t kThreads = 384;                                // TMA warp, MMA warp, two that idle, eight epilogue warps
 constexpr uint32_t kStepK = 64;                                   // BF16 values of K per stage: 128 bytes a row
 constexpr uint32_t kATile = kTileM * 128u, kBTile = kTileN * 128u;
 constexpr uint32_t kStageBytes = kATile + kBTile;
@@ -30,6 +30,7 @@ constexpr uint32_t kStages = 4;
 constexpr uint32_t kSharedBytes = kStages * kStageBytes + 128u + 1024u;   // + barriers + slack to align to 1024
 constexpr uint32_t kWaitFailed = 16u;                             // error bit: a bounded wait of this kernel gave up
 
+// Registers: the launch's 168 a thread are shared out as 64 for the control warps and 208 for the epilogue, which holds 128 sums.
 // kind::f16 instruction descriptor: FP32 accumulator, BF16 x BF16, both operands K-major, M 128, N 256.
 constexpr uint32_t kInstruction = (1u << 4) | (1u << 7) | (1u << 10) | ((kTileN >> 3) << 17) | ((kTileM >> 4) << 24);
 
@@ -83,13 +84,27 @@ __device__ __forceinline__ void store_rotated(uint32_t (&r)[4][32], uint16_t* __
     }
 }
 
-//   grid: min(tiles, SMs), block nvfp4n::kThreads, dynamic shared kSharedBytes. map_a: [rows][k] BF16, box 64 x 128;
+// The columns of a call as segments that each have activations of their own (a fused trellis object rotates its input once per
+// segment): segment g is columns [begin[g], begin[g + 1]) and multiplies rows [g * rows, (g + 1) * rows) of map_a. An output tile
+// lies in one segment; tile_begin[g] is the number of tile columns before it.
+constexpr uint32_t kMaxSegments = 8;
+struct Segments {
+    uint32_t count, begin[kMaxSegments + 1], tile_begin[kMaxSegments + 1];
+    // Segment of tile column tn.
+    __device__ __forceinline__ uint32_t of(uint32_t tn) const {
+        uint32_t g = 0;
+        while (g + 1u < count && tn >= tile_begin[g + 1u]) ++g;
+        return g;
+    }
+};
+
+//   grid: min(tiles, SMs), block kThreads, dynamic shared kSharedBytes. map_a: [rows][k] BF16, box 64 x 128;
 //   map_b: [n][k] BF16, box 64 x 128 (a B tile is two boxes). n a multiple of 128. out: row stride `stride` elements.
 //   svh null: out[r][j] = bf16(sum); else out[r][j] = the trellis output of the 128-column block j belongs to (svh [n]).
-//   a_period: K of map_a (k is a multiple of it). pair_tiles: see below (svh must be null then).
+//   a_period: K of map_a (k is a multiple of it). pair_tiles: see below (svh must be null then; one segment).
 __global__ void __launch_bounds__(kThreads, 1) bf16_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
         uint16_t* __restrict__ out, const uint16_t* __restrict__ svh, uint32_t stride, uint32_t rows, uint32_t n, uint32_t k,
-        uint32_t a_period, uint32_t pair_tiles, uint32_t* __restrict__ error) {
+        uint32_t a_period, uint32_t pair_tiles, const __grid_constant__ Segments segments, uint32_t* __restrict__ error) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
@@ -101,7 +116,7 @@ __global__ void __launch_bounds__(kThreads, 1) bf16_gemm_kernel(const __grid_con
     // pair_tiles != 0: the gate/up region. `n` is the output width (half of the weight rows); an output tile of 128 columns
     // takes the 128 gate rows at its own place and the 128 up rows pair_tiles * 128 further down as the halves of its B tile.
     const bool paired = pair_tiles != 0u;
-    const nvfp4n::TileWalk walk(rows, n, paired ? 128u : kTileN);
+    const nvfp4n::TileWalk walk(rows, paired ? n / 128u : segments.tile_begin[segments.count]);
     const uint32_t k_steps = k / kStepK;
 
     if (threadIdx.x == 0) {
@@ -126,13 +141,17 @@ __global__ void __launch_bounds__(kThreads, 1) bf16_gemm_kernel(const __grid_con
     eb::pdl_launch_dependents();
     eb::pdl_wait();   // both operands come from the launches before this one
 
-    if (warp == 0) {
+    if (warp < 4u) {
+      nvfp4n::registers_give_back<64>();
+      if (warp == 0) {
         if (lane == 0) {
             uint32_t step = 0;
             bool ok = true;
             for (uint32_t tile = blockIdx.x; tile < walk.total && ok; tile += gridDim.x) {
                 uint32_t tm, tn;
                 walk.at(tile, &tm, &tn);
+                const uint32_t g = segments.of(tn), column = segments.begin[g] + (tn - segments.tile_begin[g]) * kTileN;
+                const uint32_t low = paired ? tn * 128u : column, high = paired ? (pair_tiles + tn) * 128u : column + 128u;
                 for (uint32_t ks = 0; ks < k_steps; ++ks, ++step) {
                     const uint32_t s = step % kStages, round = step / kStages;
                     if (round > 0 && !eb::mbar_wait(&empty[s], (round - 1u) & 1u)) {
@@ -144,14 +163,13 @@ __global__ void __launch_bounds__(kThreads, 1) bf16_gemm_kernel(const __grid_con
                     eb::mbar_arrive_expect_tx(&full[s], kStageBytes);
                     // rows past the end of a matrix read as zeros (and the transaction still counts the whole box)
                     // the activations' K index wraps at a_period (the weight's K holds several terms of the same activations)
-                    eb::tma_load_2d(stage, &map_a, (int)((ks * kStepK) % a_period), (int)(tm * kTileM), &full[s]);
-                    const uint32_t low = paired ? tn : 2u * tn, high = paired ? pair_tiles + tn : 2u * tn + 1u;
-                    eb::tma_load_2d(stage + kATile, &map_b, (int)(ks * kStepK), (int)(low * 128u), &full[s]);
-                    eb::tma_load_2d(stage + kATile + kBTile / 2u, &map_b, (int)(ks * kStepK), (int)(high * 128u), &full[s]);
+                    eb::tma_load_2d(stage, &map_a, (int)((ks * kStepK) % a_period), (int)(g * rows + tm * kTileM), &full[s]);
+                    eb::tma_load_2d(stage + kATile, &map_b, (int)(ks * kStepK), (int)low, &full[s]);
+                    eb::tma_load_2d(stage + kATile + kBTile / 2u, &map_b, (int)(ks * kStepK), (int)high, &full[s]);
                 }
             }
         }
-    } else if (warp == 1) {
+      } else if (warp == 1) {
         if (lane == 0) {
             uint32_t step = 0, local = 0;
             bool ok = true;
@@ -180,9 +198,11 @@ __global__ void __launch_bounds__(kThreads, 1) bf16_gemm_kernel(const __grid_con
                 if (ok) nvfp4n::mma_commit(&acc_full[buffer]);
             }
         }
+      }
     } else {
-        // warp w reads the 32 accumulator rows of lane quarter w % 4; warps 2..5 take columns 0..127, warps 6..9 128..255
-        const uint32_t quarter = warp & 3u, half = (warp - 2u) >> 2;
+        // warp w reads the 32 accumulator rows of lane quarter w % 4; warps 4..7 take columns 0..127, warps 8..11 128..255
+        nvfp4n::registers_take<208>();
+        const uint32_t quarter = warp & 3u, half = (warp - 4u) >> 2;
         uint32_t local = 0;
         for (uint32_t tile = blockIdx.x; tile < walk.total; tile += gridDim.x, ++local) {
             uint32_t tm, tn;
@@ -205,10 +225,12 @@ __global__ void __launch_bounds__(kThreads, 1) bf16_gemm_kernel(const __grid_con
             nvfp4n::tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) eb::mbar_arrive(&acc_empty[buffer]);
-            const uint32_t row = tm * kTileM + quarter * 32u + lane, col = paired ? tn * 128u + half * 64u : tn * kTileN + half * 128u;
+            const uint32_t g = segments.of(tn), end = segments.begin[g + 1u];
+            const uint32_t row = tm * kTileM + quarter * 32u + lane;
+            const uint32_t col = paired ? tn * 128u + half * 64u : segments.begin[g] + (tn - segments.tile_begin[g]) * kTileN + half * 128u;
             if (svh == nullptr) {
                 nvfp4n::store_block(r, out, row, rows, n, col, 1.0f, paired);   // row stride n
-            } else if (row < rows && col < n) {
+            } else if (row < rows && col < end) {
                 store_rotated(r, out + (uint64_t)row * stride + col, svh + col);
             }
         }
@@ -227,23 +249,28 @@ __global__ void __launch_bounds__(kThreads, 1) bf16_gemm_kernel(const __grid_con
 // instead of 48 KB for the same FLOP: a third fewer operand bytes from L2 per FLOP and six stages in flight instead of four.
 // No multicast loads: each CTA requests its own tiles, and both CTAs' loads are counted on the even CTA's stage barrier
 // (the pair form of the TMA load may signal a barrier of the peer), so no thread relays arrivals between the CTAs. Used for calls of kPairRows rows and more.
+// A last wave with fewer tiles than half of the pairs runs them as halves of 128 columns: 5120 columns at 2048 rows are 160 tiles on
+// 74 pairs, 2 waves and 12 tiles, which took a third whole wave. The segments of a trellis object share one launch for the same
+// reason (query_key_value at 2048 rows: 160 + 32 + 32 tiles were 3 + 1 + 1 waves). A trellis layer of 512 / 1024 / 2048 rows, with
+// its rotate and decode side by side: 702 / 975 / 1630 -> 598 / 892 / 1568 us.
 constexpr uint32_t kPairStages = 6;
 constexpr uint32_t kPairStageBytes = kATile + 128u * 128u;
 constexpr uint32_t kPairShared = kPairStages * kPairStageBytes + 256u + 1024u;
 constexpr uint32_t kPairInstruction = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((256u >> 4) << 24);
+constexpr uint32_t kPairInstructionHalf = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((256u >> 4) << 24);   // N 128
 constexpr uint32_t kPairRows = 512;
 
-__device__ __forceinline__ void pair_mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
+__device__ __forceinline__ void pair_mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t instruction, uint32_t accumulate) {
     asm volatile(
             "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
             "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
-            "l"(a_desc), "l"(b_desc), "r"(kPairInstruction), "r"(accumulate)
+            "l"(a_desc), "l"(b_desc), "r"(instruction), "r"(accumulate)
             : "memory");
 }
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
-        const __grid_constant__ CUtensorMap map_b, uint16_t* __restrict__ out, const uint16_t* __restrict__ svh, uint32_t stride, uint32_t rows,
-        uint32_t n, uint32_t k, uint32_t a_period, uint32_t pair_tiles, uint32_t* __restrict__ error) {
+        const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_half, uint16_t* __restrict__ out, const uint16_t* __restrict__ svh,
+        uint32_t stride, uint32_t rows, uint32_t n, uint32_t k, uint32_t a_period, uint32_t pair_tiles, const __grid_constant__ Segments segments, uint32_t* __restrict__ error) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + kPairStages * kPairStageBytes);
@@ -255,14 +282,37 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_ge
     const uint32_t rank = eb::cluster_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     // pair_tiles != 0: the gate/up region; the even CTA's half of the weight tile is the gate rows, the odd CTA's the up rows.
     const bool paired = pair_tiles != 0u;
-    const uint32_t tiles_m = (rows + 255u) / 256u, tiles_n = paired ? pair_tiles : (n + 255u) / 256u, items = tiles_m * tiles_n;
+    const uint32_t tiles_m = (rows + 255u) / 256u, tiles_n = paired ? pair_tiles : segments.tile_begin[segments.count], tiles = tiles_m * tiles_n;
     const uint32_t k_steps = k / kStepK;
+    // The tiles of a last wave that would leave more than half of the pairs idle are cut into two items of 128 columns each.
+    const uint32_t rest = tiles % pairs, whole = 2u * rest <= pairs ? tiles - rest : tiles, items = whole + 2u * (tiles - whole);
+    struct Place {
+        uint32_t tm, segment;
+        uint32_t low, high;              // first weight row of the item's lower and upper half
+        uint32_t out, end;               // first output column, end of the output columns that may be written
+    };
     // Panels of kPanel tile columns; inside a panel the row index runs fastest across the panel's columns.
-    auto place = [&](uint32_t item, uint32_t* tm, uint32_t* tn) {
-        const uint32_t per_panel = tiles_m * nvfp4n::kPanel, panel = item / per_panel, rest = item - panel * per_panel;
-        const uint32_t width = min(nvfp4n::kPanel, tiles_n - panel * nvfp4n::kPanel);
-        *tm = rest / width;
-        *tn = panel * nvfp4n::kPanel + rest % width;
+    auto place = [&](uint32_t item) {
+        const bool cut = item >= whole;
+        const uint32_t tile = cut ? whole + ((item - whole) >> 1) : item, part = cut ? (item - whole) & 1u : 0u;
+        const uint32_t per_panel = tiles_m * nvfp4n::kPanel, panel = tile / per_panel, in_panel = tile - panel * per_panel;
+        const uint32_t width = min(nvfp4n::kPanel, tiles_n - panel * nvfp4n::kPanel), tn = panel * nvfp4n::kPanel + in_panel % width;
+        Place at;
+        at.tm = in_panel / width;
+        if (paired) {
+            at.segment = 0u;
+            at.out = tn * 128u + part * 64u;
+            at.low = at.out;
+            at.high = pair_tiles * 128u + at.out;
+            at.end = n;
+        } else {
+            at.segment = segments.of(tn);
+            at.out = segments.begin[at.segment] + (tn - segments.tile_begin[at.segment]) * 256u + part * 128u;
+            at.low = at.out;
+            at.high = at.out + (cut ? 64u : 128u);
+            at.end = segments.begin[at.segment + 1u];
+        }
+        return at;
     };
 
     if (threadIdx.x == 0) {
@@ -288,15 +338,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_ge
     eb::pdl_launch_dependents();
     eb::pdl_wait();   // both operands come from the launches before this one
 
-    if (warp == 0) {
+    if (warp < 4u) {
+      nvfp4n::registers_give_back<64>();
+      if (warp == 0) {
         if (lane == 0) {
             uint32_t step = 0;
             bool ok = true;
             for (uint32_t item = pair; item < items && ok; item += pairs) {
-                uint32_t tm, tn;
-                place(item, &tm, &tn);
-                const uint32_t row_tile = 2u * tm + rank;                      // this CTA's 128 rows
-                const uint32_t weight_tile = paired ? (rank == 0u ? tn : pair_tiles + tn) : 2u * tn + rank;   // its 128 weight rows
+                const Place at = place(item);
+                const uint32_t row = at.segment * rows + (2u * at.tm + rank) * kTileM;   // this CTA's 128 rows
+                const uint32_t weight = rank == 0u ? at.low : at.high;                   // its half of the weight rows
+                const CUtensorMap* map_weights = item < whole ? &map_b : &map_half;
+                const uint32_t bytes = kATile + (item < whole ? 128u : 64u) * 128u;
                 for (uint32_t ks = 0; ks < k_steps; ++ks, ++step) {
                     const uint32_t s = step % kPairStages, round = step / kPairStages;
                     if (round > 0 && !eb::mbar_wait(&empty[s], (round - 1u) & 1u)) {
@@ -306,14 +359,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_ge
                     }
                     uint8_t* stage = smem + s * kPairStageBytes;
                     // both CTAs' boxes are counted on the even CTA's barrier, where the thread that issues the MMAs waits
-                    if (rank == 0u) eb::mbar_arrive_expect_tx(&full[s], 2u * kPairStageBytes);
+                    if (rank == 0u) eb::mbar_arrive_expect_tx(&full[s], 2u * bytes);
                     const uint32_t bar = eb::map_to_rank(eb::smem_u32(&full[s]), 0u);
-                    nvfp4n::pair_tma_load_2d(stage, &map_a, (int)((ks * kStepK) % a_period), (int)(row_tile * kTileM), bar);
-                    nvfp4n::pair_tma_load_2d(stage + kATile, &map_b, (int)(ks * kStepK), (int)(weight_tile * 128u), bar);
+                    nvfp4n::pair_tma_load_2d(stage, &map_a, (int)((ks * kStepK) % a_period), (int)row, bar);
+                    nvfp4n::pair_tma_load_2d(stage + kATile, map_weights, (int)(ks * kStepK), (int)weight, bar);
                 }
             }
         }
-    } else if (warp == 1) {
+      } else if (warp == 1) {
         if (lane == 0 && rank == 0u) {   // the odd CTA issues nothing: its tiles are read by the even CTA's MMAs
             uint32_t step = 0, local = 0;
             bool ok = true;
@@ -325,6 +378,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_ge
                 }
                 nvfp4n::tcgen05_fence_after();
                 const uint32_t accumulator = tmem + buffer * kTileN;
+                const uint32_t instruction = item < whole ? kPairInstruction : kPairInstructionHalf;
                 for (uint32_t ks = 0; ks < k_steps; ++ks, ++step) {
                     const uint32_t s = step % kPairStages, round = step / kPairStages;
                     if (!eb::mbar_wait(&full[s], round & 1u)) {
@@ -336,19 +390,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_ge
                     const uint8_t* stage = smem + s * kPairStageBytes;
                     const uint64_t a = nvfp4n::tile_descriptor(stage), b = nvfp4n::tile_descriptor(stage + kATile);
 #pragma unroll
-                    for (uint32_t j = 0; j < 4u; ++j) pair_mma_bf16(accumulator, a + 2u * j, b + 2u * j, (uint32_t)((ks | j) != 0u));
+                    for (uint32_t j = 0; j < 4u; ++j) pair_mma_bf16(accumulator, a + 2u * j, b + 2u * j, instruction, (uint32_t)((ks | j) != 0u));
                     nvfp4n::pair_commit(&empty[s]);
                 }
                 if (ok) nvfp4n::pair_commit(&acc_full[buffer]);
             }
         }
+      }
     } else {
         // Epilogue, in both CTAs, each over its own 128 rows: as in bf16_gemm_kernel.
-        const uint32_t quarter = warp & 3u, half = (warp - 2u) >> 2;
+        nvfp4n::registers_take<208>();
+        const uint32_t quarter = warp & 3u, half = (warp - 4u) >> 2;
         uint32_t local = 0;
         for (uint32_t item = pair; item < items; item += pairs, ++local) {
-            uint32_t tm, tn;
-            place(item, &tm, &tn);
+            const bool cut = item >= whole, works = !cut || half == 0u;   // a cut item's 128 accumulator columns are one warp's
             const uint32_t buffer = local & 1u;
             if (!eb::mbar_wait(&acc_full[buffer], (local >> 1) & 1u)) {
                 if (lane == 0) atomicOr(error, kWaitFailed);
@@ -357,19 +412,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_ge
             nvfp4n::tcgen05_fence_after();
             uint32_t r[4][32];
             const uint32_t from = tmem + ((quarter * 32u) << 16) + buffer * kTileN + (paired ? half * 64u : half * 128u);
-            const uint32_t other = paired ? from + 128u : from + 64u;
-            nvfp4n::tmem_load_32(r[0], from);
-            nvfp4n::tmem_load_32(r[1], from + 32u);
-            nvfp4n::tmem_load_32(r[2], other);
-            nvfp4n::tmem_load_32(r[3], other + 32u);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            const uint32_t other = paired ? from + (cut ? 64u : 128u) : from + 64u;
+            if (works) {
+                nvfp4n::tmem_load_32(r[0], from);
+                nvfp4n::tmem_load_32(r[1], from + 32u);
+                nvfp4n::tmem_load_32(r[2], other);
+                nvfp4n::tmem_load_32(r[3], other + 32u);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            }
             nvfp4n::tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) nvfp4n::signal_rank(&acc_empty[buffer], 0u);   // what it orders are tensor-memory reads
-            const uint32_t row = (2u * tm + rank) * kTileM + quarter * 32u + lane, col = paired ? tn * 128u + half * 64u : tn * kTileN + half * 128u;
+            if (!works) continue;
+            const Place at = place(item);
+            const uint32_t row = (2u * at.tm + rank) * kTileM + quarter * 32u + lane, col = at.out + (paired ? half * 64u : half * 128u);
             if (svh == nullptr) {
                 nvfp4n::store_block(r, out, row, rows, n, col, 1.0f, paired);   // row stride n
-            } else if (row < rows && col < n) {
+            } else if (row < rows && col < at.end) {
                 store_rotated(r, out + (uint64_t)row * stride + col, svh + col);
             }
         }
@@ -431,31 +490,41 @@ inline std::atomic<bool> g_pairs{true};
 // a [rows][k], b [n][k] -> out [rows][n] at row stride `stride`, all BF16 in device memory, 16-byte aligned; k % 64 == 0,
 // n % 128 == 0. svh (FP16 [n], may be null): finish the trellis output in the epilogue instead of storing the sums.
 // a_k: K of a (k = terms x a_k: b's K holds `terms` planes that all multiply the same activations). paired: b is a gate/up
-// object of n rows (gate first) and out is [rows][n / 2] SwiGLU values.
+// object of n rows (gate first) and out is [rows][n / 2] SwiGLU values. ends: the exclusive column ends of `count` (at most
+// kMaxSegments) segments, for which a is [count][rows][k]; null: one segment.
 inline cudaError_t linear(const void* a, const void* b, void* out, const void* svh, uint32_t stride, uint32_t rows, uint32_t k, uint32_t n, int sms,
-        cudaStream_t stream, bool pdl, uint32_t* error, uint32_t a_k = 0, bool paired = false) {
+        cudaStream_t stream, bool pdl, uint32_t* error, uint32_t a_k = 0, bool paired = false, const int32_t* ends = nullptr, uint32_t count = 1) {
     if (a_k == 0) a_k = k;
     const eb::EncodeTiled encode = eb::encoder();
     if (encode == nullptr) return cudaErrorNotSupported;
-    CUtensorMap map_a, map_b;
-    const cuuint32_t ones[2] = {1u, 1u}, box[2] = {kStepK, 128u};
-    const cuuint64_t a_dims[2] = {a_k, rows}, b_dims[2] = {k, n}, strides[1] = {(cuuint64_t)k * 2u}, a_strides[1] = {(cuuint64_t)a_k * 2u};
-    CUresult r = encode(&map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(a), a_dims, a_strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r == CUDA_SUCCESS)
-        r = encode(&map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(b), b_dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-    const uint32_t pair_tiles = paired ? n / 256u : 0u, width = paired ? n / 2u : n;
-    if (rows >= kPairRows && g_pairs.load()) {
-        const uint32_t items = ((rows + 255u) / 256u) * (paired ? pair_tiles : (n + 255u) / 256u);
-        const uint32_t ctas = 2u * std::max(1u, std::min((uint32_t)sms / 2u, items));
-        return nvfp4n::launch_on(stream, pdl, bf16_gemm_pair_kernel, dim3(ctas), dim3(kThreads), kPairShared, map_a, map_b, static_cast<uint16_t*>(out),
-                static_cast<const uint16_t*>(svh), stride, rows, width, k, a_k, pair_tiles, error);
+    const bool pairs = rows >= kPairRows && g_pairs.load();
+    CUtensorMap map_a, map_b, map_half;   // boxes of 128 rows, and of 64 for the cut tiles of the pair kernel
+    const cuuint32_t ones[2] = {1u, 1u}, box[2] = {kStepK, 128u}, half_box[2] = {kStepK, 64u};
+    const cuuint64_t a_dims[2] = {a_k, (cuuint64_t)rows * count}, b_dims[2] = {k, n}, strides[1] = {(cuuint64_t)k * 2u}, a_strides[1] = {(cuuint64_t)a_k * 2u};
+    auto encode_bf16 = [&](CUtensorMap* map, const void* at, const cuuint64_t* dims, const cuuint64_t* pitch, const cuuint32_t* of) {
+        return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(at), dims, pitch, of, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                       CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
+                == CUDA_SUCCESS;
+    };
+    if (!encode_bf16(&map_a, a, a_dims, a_strides, box) || !encode_bf16(&map_b, b, b_dims, strides, box)
+            || (pairs && !encode_bf16(&map_half, b, b_dims, strides, half_box)))
+        return cudaErrorInvalidValue;
+    Segments segments = {};
+    segments.count = count;
+    for (uint32_t g = 0; g < count; ++g) {
+        segments.begin[g + 1u] = ends != nullptr ? (uint32_t)ends[g] : n;
+        segments.tile_begin[g + 1u] = segments.tile_begin[g] + (segments.begin[g + 1u] - segments.begin[g] + kTileN - 1u) / kTileN;
     }
-    const uint32_t tiles = ((rows + kTileM - 1u) / kTileM) * (paired ? pair_tiles : (n + kTileN - 1u) / kTileN);
+    const uint32_t pair_tiles = paired ? n / 256u : 0u, width = paired ? n / 2u : n, tiles_n = paired ? pair_tiles : segments.tile_begin[count];
+    if (pairs) {
+        const uint32_t most = (uint32_t)sms / 2u, tiles = ((rows + 255u) / 256u) * tiles_n;   // a short call's tiles are cut in two (see the kernel)
+        const uint32_t ctas = 2u * std::max(1u, 2u * tiles <= most ? 2u * tiles : std::min(most, tiles));
+        return nvfp4n::launch_on(stream, pdl, bf16_gemm_pair_kernel, dim3(ctas), dim3(kThreads), kPairShared, map_a, map_b, map_half,
+                static_cast<uint16_t*>(out), static_cast<const uint16_t*>(svh), stride, rows, width, k, a_k, pair_tiles, segments, error);
+    }
+    const uint32_t tiles = ((rows + kTileM - 1u) / kTileM) * tiles_n;
     return nvfp4n::launch_on(stream, pdl, bf16_gemm_kernel, dim3(tiles < (uint32_t)sms ? tiles : (uint32_t)sms), dim3(kThreads), kSharedBytes, map_a, map_b,
-            static_cast<uint16_t*>(out), static_cast<const uint16_t*>(svh), stride, rows, width, k, a_k, pair_tiles, error);
+            static_cast<uint16_t*>(out), static_cast<const uint16_t*>(svh), stride, rows, width, k, a_k, pair_tiles, segments, error);
 }
 
 }  // namespace bf16n

@@ -58,7 +58,6 @@ constexpr uint32_t kSfbStage = (kStepK / kBlockK) * (kTileN / 128u) * kAtom;
 constexpr uint32_t kStageBytes = kTerms * kATile + kBTile + kSfaStage + kSfbStage;
 constexpr uint32_t kBarrierBytes = 128u;
 constexpr uint32_t kSharedBytes = kStages * kStageBytes + kBarrierBytes + 1024u;   // + slack to align to 1024
-constexpr uint32_t kThreads = 320u;                         // TMA warp, MMA warp, eight epilogue warps
 constexpr uint32_t kScaledThreads = 512u;                   // TMA and MMA warps (and two that idle), four scale warps, eight epilogue warps
 constexpr uint32_t kTmemColumns = 512u;
 constexpr uint32_t kTmemScales = 256u, kScaleColumns = 64u; // behind the 256 accumulator columns: 64 columns of scales per ring stage
@@ -359,9 +358,7 @@ __device__ __forceinline__ void scales_to_tmem(const uint4* sf, uint32_t to) {
 
 struct TileWalk {
     uint32_t tiles_m, tiles_n, total;
-    __device__ TileWalk(uint32_t rows, uint32_t n, uint32_t tile_columns) : tiles_m((rows + kTileM - 1u) / kTileM), tiles_n((n + tile_columns - 1u) / tile_columns) {
-        total = tiles_m * tiles_n;
-    }
+    __device__ TileWalk(uint32_t rows, uint32_t tile_columns) : tiles_m((rows + kTileM - 1u) / kTileM), tiles_n(tile_columns) { total = tiles_m * tiles_n; }
     // Panels of kPanel tile columns; inside a panel the row index runs fastest across the panel's columns.
     __device__ void at(uint32_t tile, uint32_t* tm, uint32_t* tn) const {
         const uint32_t per_panel = tiles_m * kPanel;
@@ -388,7 +385,7 @@ __global__ void __launch_bounds__(kScaledThreads, 1) gemm_kernel(const __grid_co
     // pair_tiles != 0: the gate/up region. `n` is the output width (half of the weight rows); an output tile of 128 columns
     // takes the 128 gate rows at its own place and the 128 up rows pair_tiles * 128 further down as the halves of its B tile.
     const bool paired = pair_tiles != 0u;
-    const TileWalk walk(rows, n, paired ? 128u : kTileN);
+    const TileWalk walk(rows, paired ? n / 128u : (n + kTileN - 1u) / kTileN);
     const uint32_t k_steps = k / kStepK, k_blocks = k / kBlockK;
 
     if (threadIdx.x == 0) {

@@ -110,8 +110,8 @@ __global__ void __launch_bounds__(256) rotate_kernel(const uint16_t* __restrict_
         uint16_t* __restrict__ out, int rows, int k, int s, int layout) {
     const int lane = threadIdx.x & 31;
     const uint32_t blocks = (uint32_t)k >> 7, task = blockIdx.x * 8u + (threadIdx.x >> 5);   // the launch holds fewer than 2^31 tasks
-    eb::pdl_launch_dependents();
     eb::pdl_wait();
+    eb::pdl_launch_dependents();   // not before: the launch behind may write what the launch in front still reads
     if (task >= (uint32_t)s * (uint32_t)rows * blocks) return;
     const uint32_t block = task % blocks, above = task / blocks, row = above % (uint32_t)rows, seg = above / (uint32_t)rows;
     float v[4];
@@ -142,8 +142,8 @@ __global__ void __launch_bounds__(kRotateRowsThreads) rotate_rows_kernel(const u
     const uint32_t t = threadIdx.x, blocks = k >> 7, seg = blockIdx.y;
     const uint32_t total = rows * blocks, first = blockIdx.x * (uint32_t)kRotateRowsThreads;   // < 2^31 blocks per segment
     const uint32_t count = min((uint32_t)kRotateRowsThreads, total - first);
-    eb::pdl_launch_dependents();
     eb::pdl_wait();
+    eb::pdl_launch_dependents();   // not before: the launch behind may write what the launch in front still reads
     const uint4* from = reinterpret_cast<const uint4*>(x + (size_t)first * 128);
 #pragma unroll
     for (uint32_t i = 0; i < 16u; ++i) {
@@ -303,16 +303,24 @@ struct Lane {
 // Payload -> BF16 rotated weight [n][k] (row-major weights of a BF16 linear). A warp takes kBatch tiles side by side: a lane
 // reads its ring words of all of them from global memory first, then takes its eight states of each as the linear does and
 // stores 16 contiguous bytes of one weight row (the quad's pairs regrouped through shared memory).
+// `beside`: the launch in front of this one neither writes what this one reads nor reads what it writes (the prefill's rotate), so
+// both may run at a time.
 //   grid ceil((k / 16) * (n / 16) / (8 kBatch)), block 256.
 template <int W>
-__global__ void __launch_bounds__(256) decode_bf16_kernel(const uint16_t* __restrict__ words, uint16_t* __restrict__ out, int k, int n) {
+__global__ void __launch_bounds__(256) decode_bf16_kernel(const uint16_t* __restrict__ words, uint16_t* __restrict__ out, int k, int n,
+        int beside) {
     using L = Lane<W>;
     const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
     constexpr int kExchangePitch = 40;   // words of an exchange row: 32 lanes + 8, so that a quarter warp's 16-byte loads tile the banks
     __shared__ __align__(16) uint32_t exchange_rows[8][4 * kExchangePitch];
     uint32_t* exchange = exchange_rows[threadIdx.x >> 5];
     const uint32_t first = (blockIdx.x * 8u + (threadIdx.x >> 5)) * (uint32_t)kBatch, tiles = (uint32_t)(k >> 4) * (uint32_t)(n >> 4);   // < 2^31
-    if (first >= tiles) return;
+    eb::pdl_launch_dependents();
+    if (beside == 0) eb::pdl_wait();
+    if (first >= tiles) {
+        eb::pdl_wait();
+        return;
+    }
     L me;
     me.init(lane);
     uint32_t u[kBatch][L::kWords + 1];
@@ -350,6 +358,7 @@ __global__ void __launch_bounds__(256) decode_bf16_kernel(const uint16_t* __rest
         const uint4 mine = *reinterpret_cast<const uint4*>(exchange + q * kExchangePitch + 4 * g);
         *reinterpret_cast<uint4*>(out + (size_t)(tj * 16 + g + 8 * (q >> 1)) * k + ti * 16 + 8 * (q & 1)) = mine;
     }
+    eb::pdl_wait();   // the launch behind waits for this one: when it runs, the one in front has ended too
 }
 
 // What a launch of the linear works on. `activations` (the scratch's fragment-order FP16 [s][rows][k], written by a
