@@ -17,6 +17,7 @@
 #include "nvfp4_decode.cuh"
 #include "bf16_gemm.cuh"
 #include "q3_gemv.cuh"
+#include "q3_prefill.cuh"
 #include "trellis.cuh"
 #include "trellis_encode.cuh"
 
@@ -93,6 +94,7 @@ void initialize_device(int device, DeviceState* state) {
     if (e == cudaSuccess) e = nvfp4n::initialize();
     if (e == cudaSuccess) e = nvfp4d::initialize();
     if (e == cudaSuccess) e = bf16n::initialize();
+    if (e == cudaSuccess) e = q3p::initialize();
     state->status = (int)e;
 }
 
@@ -729,14 +731,8 @@ static int q3_prefill(const void* input, const void* weights, void* output, void
     DeviceState* state = nullptr;
     status = bind(&state);
     if (status != EUHEDRAL_CUDA_SUCCESS) return status;
-    const q3::Geometry geo(weight_rows, in_features);
-    const uint64_t groups = (uint64_t)weight_rows * (in_features / 64u);
-    cudaError_t e = launch(kOrdered, bf16n::q3_terms_kernel, dim3((unsigned)((groups * 8u + 255u) / 256u)), dim3(256), 0, 1u,
-            static_cast<const uint8_t*>(weights), geo.scale_offset, static_cast<uint16_t*>(scratch), weight_rows, in_features);
-    if (e == cudaSuccess)
-        e = bf16n::linear(input, scratch, output, nullptr, 0, rows, 2u * in_features, weight_rows, state->sms, t_stream, false, state->error_word,
-                in_features, paired);
-    return finish(e);
+    return finish(q3p::linear(input, weights, output, rows, in_features, weight_rows, paired, state->sms, t_stream, t_pdl != 0 && t_stream != nullptr,
+            state->error_word));
 }
 
 int euhedral_cuda_linear_q3_mx_bf16(const void* input, const void* weights, void* output, void* scratch, uint32_t rows, uint32_t in_features,
