@@ -97,13 +97,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     return false;
 }
 
-// Bounded wait of a role whose loops must not depend on its outcome: when the phase does not complete within 4 kParkLimit polls, or
+// Bounded wait of a role whose loops must not depend on its outcome: when the phase does not complete within kSpinLimit polls, or
 // another wait of the CTA has given up before, `failed` (a word of shared memory) is set and the wait is over. The kernel
 // runs to its end on whatever it has and reports the failure there.
 __device__ __forceinline__ void mbar_wait_or_fail(uint64_t* bar, uint32_t parity, uint32_t* failed) {
-    const uint32_t at = smem_u32(bar);
-    for (uint32_t spin = 0; spin < 4u * kParkLimit; ++spin) {
-        if (mbar_try_wait_at(at, parity)) return;
+    for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
+        if (mbar_try_wait(bar, parity)) return;
         if ((spin & 15u) == 15u && *reinterpret_cast<volatile uint32_t*>(failed) != 0u) return;
     }
     *reinterpret_cast<volatile uint32_t*>(failed) = 1u;
