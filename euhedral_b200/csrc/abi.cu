@@ -697,10 +697,10 @@ int euhedral_cuda_linear_q3_reference_bf16(const void* input, const void* weight
 
 // ---- Q3 prefill --------------------------------------------------------------------------------------------------------------
 // The reference's entry points for Q3 linears of 9 rows and more (native/include/euhedral_cuda.h:173-197; its kernels run
-// block-scaled FP8 MMAs of sm_12x on two-term E4M3 activations). Here the operands are exact the other way round: every
-// weight code * f32(scale) is written to the scratch as two BF16 terms whose sum is the weight exactly
-// (bf16n::q3_terms_kernel), and one tcgen05 BF16 GEMM over K' = 2 K multiplies both planes with the unchanged BF16
-// activations, FP32 sums in tensor memory: sums of exact products, rounded once to BF16, as the reference's route gives.
+// block-scaled FP8 MMAs of sm_12x on two-term E4M3 activations). Here the operands are exact the other way round: every weight
+// code * f32(scale) is two BF16 terms whose sum is the weight exactly, made on their way into the tensor core's tiles (q3_prefill.cuh);
+// both multiply the unchanged BF16 activations: sums of exact products, rounded once to BF16, as the reference's route gives. The
+// scratch, which an earlier form of this route filled with the terms, is asked for and checked as before and not used.
 constexpr uint32_t kQ3PrefillMinRows = 33;
 
 int euhedral_cuda_q3_mx_available(void) {
@@ -1109,7 +1109,7 @@ int euhedral_b200_prefill_trellis_bf16(const void* input, const void* words, con
         int32_t ends[bf16n::kMaxSegments];
         for (uint32_t i = 0; i < count; ++i) ends[i] = host_segment_ends[g + i] - start;
         e = bf16n::linear(activations + (uint64_t)g * rows * k * 2u, decoded + (uint64_t)start * k * 2u, static_cast<uint16_t*>(output) + start,
-                static_cast<const uint16_t*>(svh) + start, n, rows, k, (uint32_t)ends[count - 1u], state->sms, t_stream, pdl, state->error_word, 0, false, ends, count);
+                static_cast<const uint16_t*>(svh) + start, n, rows, k, (uint32_t)ends[count - 1u], state->sms, t_stream, pdl, state->error_word, ends, count);
         start = host_segment_ends[g + count - 1u];
     }
     return finish(e);

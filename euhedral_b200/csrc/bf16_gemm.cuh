@@ -101,10 +101,9 @@ struct Segments {
 //   grid: min(tiles, SMs), block kThreads, dynamic shared kSharedBytes. map_a: [rows][k] BF16, box 64 x 128;
 //   map_b: [n][k] BF16, box 64 x 128 (a B tile is two boxes). n a multiple of 128. out: row stride `stride` elements.
 //   svh null: out[r][j] = bf16(sum); else out[r][j] = the trellis output of the 128-column block j belongs to (svh [n]).
-//   a_period: K of map_a (k is a multiple of it). pair_tiles: see below (svh must be null then; one segment).
 __global__ void __launch_bounds__(kThreads, 1) bf16_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
         uint16_t* __restrict__ out, const uint16_t* __restrict__ svh, uint32_t stride, uint32_t rows, uint32_t n, uint32_t k,
-        uint32_t a_period, uint32_t pair_tiles, const __grid_constant__ Segments segments, uint32_t* __restrict__ error) {
+        const __grid_constant__ Segments segments, uint32_t* __restrict__ error) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
@@ -113,10 +112,7 @@ __global__ void __launch_bounds__(kThreads, 1) bf16_gemm_kernel(const __grid_con
     uint64_t* acc_empty = acc_full + 2;
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_empty + 2);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    // pair_tiles != 0: the gate/up region. `n` is the output width (half of the weight rows); an output tile of 128 columns
-    // takes the 128 gate rows at its own place and the 128 up rows pair_tiles * 128 further down as the halves of its B tile.
-    const bool paired = pair_tiles != 0u;
-    const nvfp4n::TileWalk walk(rows, paired ? n / 128u : segments.tile_begin[segments.count]);
+    const nvfp4n::TileWalk walk(rows, segments.tile_begin[segments.count]);
     const uint32_t k_steps = k / kStepK;
 
     if (threadIdx.x == 0) {
@@ -151,7 +147,6 @@ __global__ void __launch_bounds__(kThreads, 1) bf16_gemm_kernel(const __grid_con
                 uint32_t tm, tn;
                 walk.at(tile, &tm, &tn);
                 const uint32_t g = segments.of(tn), column = segments.begin[g] + (tn - segments.tile_begin[g]) * kTileN;
-                const uint32_t low = paired ? tn * 128u : column, high = paired ? (pair_tiles + tn) * 128u : column + 128u;
                 for (uint32_t ks = 0; ks < k_steps; ++ks, ++step) {
                     const uint32_t s = step % kStages, round = step / kStages;
                     if (round > 0 && !eb::mbar_wait(&empty[s], (round - 1u) & 1u)) {
@@ -162,10 +157,9 @@ __global__ void __launch_bounds__(kThreads, 1) bf16_gemm_kernel(const __grid_con
                     uint8_t* stage = smem + s * kStageBytes;
                     eb::mbar_arrive_expect_tx(&full[s], kStageBytes);
                     // rows past the end of a matrix read as zeros (and the transaction still counts the whole box)
-                    // the activations' K index wraps at a_period (the weight's K holds several terms of the same activations)
-                    eb::tma_load_2d(stage, &map_a, (int)((ks * kStepK) % a_period), (int)(g * rows + tm * kTileM), &full[s]);
-                    eb::tma_load_2d(stage + kATile, &map_b, (int)(ks * kStepK), (int)low, &full[s]);
-                    eb::tma_load_2d(stage + kATile + kBTile / 2u, &map_b, (int)(ks * kStepK), (int)high, &full[s]);
+                    eb::tma_load_2d(stage, &map_a, (int)(ks * kStepK), (int)(g * rows + tm * kTileM), &full[s]);
+                    eb::tma_load_2d(stage + kATile, &map_b, (int)(ks * kStepK), (int)column, &full[s]);
+                    eb::tma_load_2d(stage + kATile + kBTile / 2u, &map_b, (int)(ks * kStepK), (int)column + 128, &full[s]);
                 }
             }
         }
@@ -214,22 +208,18 @@ __global__ void __launch_bounds__(kThreads, 1) bf16_gemm_kernel(const __grid_con
             }
             nvfp4n::tcgen05_fence_after();
             uint32_t r[4][32];
-            // plain: 128 consecutive columns; paired: 64 gate columns (r[0], r[1]) and the 64 up columns that match them (r[2], r[3])
-            const uint32_t from = tmem + ((quarter * 32u) << 16) + buffer * kTileN + (paired ? half * 64u : half * 128u);
-            const uint32_t other = paired ? from + 128u : from + 64u;
-            nvfp4n::tmem_load_32(r[0], from);
-            nvfp4n::tmem_load_32(r[1], from + 32u);
-            nvfp4n::tmem_load_32(r[2], other);
-            nvfp4n::tmem_load_32(r[3], other + 32u);
+            const uint32_t from = tmem + ((quarter * 32u) << 16) + buffer * kTileN + half * 128u;
+#pragma unroll
+            for (uint32_t i = 0; i < 4u; ++i) nvfp4n::tmem_load_32(r[i], from + 32u * i);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             nvfp4n::tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) eb::mbar_arrive(&acc_empty[buffer]);
             const uint32_t g = segments.of(tn), end = segments.begin[g + 1u];
             const uint32_t row = tm * kTileM + quarter * 32u + lane;
-            const uint32_t col = paired ? tn * 128u + half * 64u : segments.begin[g] + (tn - segments.tile_begin[g]) * kTileN + half * 128u;
+            const uint32_t col = segments.begin[g] + (tn - segments.tile_begin[g]) * kTileN + half * 128u;
             if (svh == nullptr) {
-                nvfp4n::store_block(r, out, row, rows, n, col, 1.0f, paired);   // row stride n
+                nvfp4n::store_block(r, out, row, rows, n, col, 1.0f, false);   // row stride n
             } else if (row < rows && col < end) {
                 store_rotated(r, out + (uint64_t)row * stride + col, svh + col);
             }
@@ -270,7 +260,7 @@ __device__ __forceinline__ void pair_mma_bf16(uint32_t d_tmem, uint64_t a_desc, 
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
         const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_half, uint16_t* __restrict__ out, const uint16_t* __restrict__ svh,
-        uint32_t stride, uint32_t rows, uint32_t n, uint32_t k, uint32_t a_period, uint32_t pair_tiles, const __grid_constant__ Segments segments, uint32_t* __restrict__ error) {
+        uint32_t stride, uint32_t rows, uint32_t n, uint32_t k, const __grid_constant__ Segments segments, uint32_t* __restrict__ error) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + kPairStages * kPairStageBytes);
@@ -280,15 +270,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_ge
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_empty + 2);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t rank = eb::cluster_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-    // pair_tiles != 0: the gate/up region; the even CTA's half of the weight tile is the gate rows, the odd CTA's the up rows.
-    const bool paired = pair_tiles != 0u;
-    const uint32_t tiles_m = (rows + 255u) / 256u, tiles_n = paired ? pair_tiles : segments.tile_begin[segments.count], tiles = tiles_m * tiles_n;
+    const uint32_t tiles_m = (rows + 255u) / 256u, tiles_n = segments.tile_begin[segments.count], tiles = tiles_m * tiles_n;
     const uint32_t k_steps = k / kStepK;
     // The tiles of a last wave that would leave more than half of the pairs idle are cut into two items of 128 columns each.
     const uint32_t rest = tiles % pairs, whole = 2u * rest <= pairs ? tiles - rest : tiles, items = whole + 2u * (tiles - whole);
     struct Place {
         uint32_t tm, segment;
-        uint32_t low, high;              // first weight row of the item's lower and upper half
         uint32_t out, end;               // first output column, end of the output columns that may be written
     };
     // Panels of kPanel tile columns; inside a panel the row index runs fastest across the panel's columns.
@@ -299,19 +286,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_ge
         const uint32_t width = min(nvfp4n::kPanel, tiles_n - panel * nvfp4n::kPanel), tn = panel * nvfp4n::kPanel + in_panel % width;
         Place at;
         at.tm = in_panel / width;
-        if (paired) {
-            at.segment = 0u;
-            at.out = tn * 128u + part * 64u;
-            at.low = at.out;
-            at.high = pair_tiles * 128u + at.out;
-            at.end = n;
-        } else {
-            at.segment = segments.of(tn);
-            at.out = segments.begin[at.segment] + (tn - segments.tile_begin[at.segment]) * 256u + part * 128u;
-            at.low = at.out;
-            at.high = at.out + (cut ? 64u : 128u);
-            at.end = segments.begin[at.segment + 1u];
-        }
+        at.segment = segments.of(tn);
+        at.out = segments.begin[at.segment] + (tn - segments.tile_begin[at.segment]) * 256u + part * 128u;
+        at.end = segments.begin[at.segment + 1u];
         return at;
     };
 
@@ -347,7 +324,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_ge
             for (uint32_t item = pair; item < items && ok; item += pairs) {
                 const Place at = place(item);
                 const uint32_t row = at.segment * rows + (2u * at.tm + rank) * kTileM;   // this CTA's 128 rows
-                const uint32_t weight = rank == 0u ? at.low : at.high;                   // its half of the weight rows
+                const uint32_t weight = at.out + rank * (item < whole ? 128u : 64u);     // its half of the weight rows
                 const CUtensorMap* map_weights = item < whole ? &map_b : &map_half;
                 const uint32_t bytes = kATile + (item < whole ? 128u : 64u) * 128u;
                 for (uint32_t ks = 0; ks < k_steps; ++ks, ++step) {
@@ -361,7 +338,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_ge
                     // both CTAs' boxes are counted on the even CTA's barrier, where the thread that issues the MMAs waits
                     if (rank == 0u) eb::mbar_arrive_expect_tx(&full[s], 2u * bytes);
                     const uint32_t bar = eb::map_to_rank(eb::smem_u32(&full[s]), 0u);
-                    nvfp4n::pair_tma_load_2d(stage, &map_a, (int)((ks * kStepK) % a_period), (int)row, bar);
+                    nvfp4n::pair_tma_load_2d(stage, &map_a, (int)(ks * kStepK), (int)row, bar);
                     nvfp4n::pair_tma_load_2d(stage + kATile, map_weights, (int)(ks * kStepK), (int)weight, bar);
                 }
             }
@@ -411,13 +388,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_ge
             }
             nvfp4n::tcgen05_fence_after();
             uint32_t r[4][32];
-            const uint32_t from = tmem + ((quarter * 32u) << 16) + buffer * kTileN + (paired ? half * 64u : half * 128u);
-            const uint32_t other = paired ? from + (cut ? 64u : 128u) : from + 64u;
+            const uint32_t from = tmem + ((quarter * 32u) << 16) + buffer * kTileN + half * 128u;
             if (works) {
-                nvfp4n::tmem_load_32(r[0], from);
-                nvfp4n::tmem_load_32(r[1], from + 32u);
-                nvfp4n::tmem_load_32(r[2], other);
-                nvfp4n::tmem_load_32(r[3], other + 32u);
+#pragma unroll
+                for (uint32_t i = 0; i < 4u; ++i) nvfp4n::tmem_load_32(r[i], from + 32u * i);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             }
             nvfp4n::tcgen05_fence_before();
@@ -425,9 +399,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_ge
             if (lane == 0) nvfp4n::signal_rank(&acc_empty[buffer], 0u);   // what it orders are tensor-memory reads
             if (!works) continue;
             const Place at = place(item);
-            const uint32_t row = (2u * at.tm + rank) * kTileM + quarter * 32u + lane, col = at.out + (paired ? half * 64u : half * 128u);
+            const uint32_t row = (2u * at.tm + rank) * kTileM + quarter * 32u + lane, col = at.out + half * 128u;
             if (svh == nullptr) {
-                nvfp4n::store_block(r, out, row, rows, n, col, 1.0f, paired);   // row stride n
+                nvfp4n::store_block(r, out, row, rows, n, col, 1.0f, false);   // row stride n
             } else if (row < rows && col < at.end) {
                 store_rotated(r, out + (uint64_t)row * stride + col, svh + col);
             }
@@ -441,44 +415,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_ge
     }
 }
 
-// Q3G64_F16S tensor -> two BF16 planes side by side along K, [n][2 k]: columns [0, k) hold hi = bf16(code * scale), columns
-// [k, 2 k) lo = code * scale - hi. code * f32(scale) has at most 14 significant bits, hi keeps 8 and the rest fits BF16:
-// hi + lo is the weight exactly, and both products with a BF16 activation are exact in FP32. Eight threads per group of 64:
-// a thread takes 8 codes (24 bits) and writes 16 bytes of each plane, so a warp's stores are whole 128-byte lines.
-//   grid ceil(n * (k / 64) * 8 / 256), block 256. k a multiple of 128.
-__global__ void __launch_bounds__(256) q3_terms_kernel(const uint8_t* __restrict__ w, uint64_t scale_offset, uint16_t* __restrict__ out,
-        uint32_t n, uint32_t k) {
-    const uint32_t groups = k / 64u;
-    const uint64_t index = (uint64_t)blockIdx.x * 256u + threadIdx.x, group_index = index >> 3;
-    if (group_index >= (uint64_t)n * groups) return;
-    const uint32_t sub = (uint32_t)index & 7u, row = (uint32_t)(group_index / groups), group = (uint32_t)(group_index % groups);
-    const uint32_t* words = reinterpret_cast<const uint32_t*>(w + group_index * 24u);
-    const uint32_t byte = 3u * sub, word = byte >> 2;              // the thread's 24 bits start at this byte of the group's 24
-    const uint32_t bits = __funnelshift_r(__ldg(words + word), __ldg(words + min(word + 1u, 5u)), 8u * (byte & 3u));
-    const float scale = __half2float(__ushort_as_half(__ldg(reinterpret_cast<const uint16_t*>(w + scale_offset) + group_index)));
-    uint32_t high[4], low[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        float value[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            // the 3-bit two's complement code as a float without an integer conversion: code + 4 = field ^ 4 sits in the
-            // mantissa of 2^23, and 2^23 + 4 is subtracted (exact)
-            const uint32_t field = (bits >> (3 * (2 * i + e))) & 7u;
-            value[e] = __fmul_rn(__fsub_rn(__uint_as_float(0x4B000000u | (field ^ 4u)), 8388612.0f), scale);
-        }
-        // round to nearest even in one conversion per pair; the values are finite
-        const __nv_bfloat162 top = __floats2bfloat162_rn(value[0], value[1]);
-        const float2 back = __bfloat1622float2(top);
-        const __nv_bfloat162 rest = __floats2bfloat162_rn(__fsub_rn(value[0], back.x), __fsub_rn(value[1], back.y));
-        high[i] = *reinterpret_cast<const uint32_t*>(&top);
-        low[i] = *reinterpret_cast<const uint32_t*>(&rest);
-    }
-    uint16_t* hi = out + (uint64_t)row * 2u * k + (uint64_t)group * 64u + 8u * sub;
-    *reinterpret_cast<uint4*>(hi) = make_uint4(high[0], high[1], high[2], high[3]);
-    *reinterpret_cast<uint4*>(hi + k) = make_uint4(low[0], low[1], low[2], low[3]);
-}
-
 inline cudaError_t initialize() {
     const cudaError_t e = cudaFuncSetAttribute(bf16_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSharedBytes);
     return e != cudaSuccess ? e : cudaFuncSetAttribute(bf16_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairShared);
@@ -489,24 +425,22 @@ inline std::atomic<bool> g_pairs{true};
 
 // a [rows][k], b [n][k] -> out [rows][n] at row stride `stride`, all BF16 in device memory, 16-byte aligned; k % 64 == 0,
 // n % 128 == 0. svh (FP16 [n], may be null): finish the trellis output in the epilogue instead of storing the sums.
-// a_k: K of a (k = terms x a_k: b's K holds `terms` planes that all multiply the same activations). paired: b is a gate/up
-// object of n rows (gate first) and out is [rows][n / 2] SwiGLU values. ends: the exclusive column ends of `count` (at most
+// ends: the exclusive column ends of `count` (at most
 // kMaxSegments) segments, for which a is [count][rows][k]; null: one segment.
 inline cudaError_t linear(const void* a, const void* b, void* out, const void* svh, uint32_t stride, uint32_t rows, uint32_t k, uint32_t n, int sms,
-        cudaStream_t stream, bool pdl, uint32_t* error, uint32_t a_k = 0, bool paired = false, const int32_t* ends = nullptr, uint32_t count = 1) {
-    if (a_k == 0) a_k = k;
+        cudaStream_t stream, bool pdl, uint32_t* error, const int32_t* ends = nullptr, uint32_t count = 1) {
     const eb::EncodeTiled encode = eb::encoder();
     if (encode == nullptr) return cudaErrorNotSupported;
     const bool pairs = rows >= kPairRows && g_pairs.load();
     CUtensorMap map_a, map_b, map_half;   // boxes of 128 rows, and of 64 for the cut tiles of the pair kernel
     const cuuint32_t ones[2] = {1u, 1u}, box[2] = {kStepK, 128u}, half_box[2] = {kStepK, 64u};
-    const cuuint64_t a_dims[2] = {a_k, (cuuint64_t)rows * count}, b_dims[2] = {k, n}, strides[1] = {(cuuint64_t)k * 2u}, a_strides[1] = {(cuuint64_t)a_k * 2u};
+    const cuuint64_t a_dims[2] = {k, (cuuint64_t)rows * count}, b_dims[2] = {k, n}, strides[1] = {(cuuint64_t)k * 2u};
     auto encode_bf16 = [&](CUtensorMap* map, const void* at, const cuuint64_t* dims, const cuuint64_t* pitch, const cuuint32_t* of) {
         return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(at), dims, pitch, of, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
                 == CUDA_SUCCESS;
     };
-    if (!encode_bf16(&map_a, a, a_dims, a_strides, box) || !encode_bf16(&map_b, b, b_dims, strides, box)
+    if (!encode_bf16(&map_a, a, a_dims, strides, box) || !encode_bf16(&map_b, b, b_dims, strides, box)
             || (pairs && !encode_bf16(&map_half, b, b_dims, strides, half_box)))
         return cudaErrorInvalidValue;
     Segments segments = {};
@@ -515,16 +449,16 @@ inline cudaError_t linear(const void* a, const void* b, void* out, const void* s
         segments.begin[g + 1u] = ends != nullptr ? (uint32_t)ends[g] : n;
         segments.tile_begin[g + 1u] = segments.tile_begin[g] + (segments.begin[g + 1u] - segments.begin[g] + kTileN - 1u) / kTileN;
     }
-    const uint32_t pair_tiles = paired ? n / 256u : 0u, width = paired ? n / 2u : n, tiles_n = paired ? pair_tiles : segments.tile_begin[count];
+    const uint32_t tiles_n = segments.tile_begin[count];
     if (pairs) {
         const uint32_t most = (uint32_t)sms / 2u, tiles = ((rows + 255u) / 256u) * tiles_n;   // a short call's tiles are cut in two (see the kernel)
         const uint32_t ctas = 2u * std::max(1u, 2u * tiles <= most ? 2u * tiles : std::min(most, tiles));
         return nvfp4n::launch_on(stream, pdl, bf16_gemm_pair_kernel, dim3(ctas), dim3(kThreads), kPairShared, map_a, map_b, map_half,
-                static_cast<uint16_t*>(out), static_cast<const uint16_t*>(svh), stride, rows, width, k, a_k, pair_tiles, segments, error);
+                static_cast<uint16_t*>(out), static_cast<const uint16_t*>(svh), stride, rows, n, k, segments, error);
     }
     const uint32_t tiles = ((rows + kTileM - 1u) / kTileM) * tiles_n;
     return nvfp4n::launch_on(stream, pdl, bf16_gemm_kernel, dim3(tiles < (uint32_t)sms ? tiles : (uint32_t)sms), dim3(kThreads), kSharedBytes, map_a, map_b,
-            static_cast<uint16_t*>(out), static_cast<const uint16_t*>(svh), stride, rows, width, k, a_k, pair_tiles, segments, error);
+            static_cast<uint16_t*>(out), static_cast<const uint16_t*>(svh), stride, rows, n, k, segments, error);
 }
 
 }  // namespace bf16n
