@@ -18,10 +18,10 @@
 // Bound: HBM, with about 5 us of launch, staging and exchange around the stream. Per 128 rows x 64 values the weights are 4.6 KB =
 // 200 cycles of an SM's share of the bandwidth; an MMA takes about 110 of them, whatever its columns up to 64. The decode
 // through registers and mma.sync that this replaces was bound by its instruction issue at 0.4 of the bandwidth. Measured, NVFP4,
-// back to back with programmatic dependent launch, before -> now (us at 1 / 5 / 8 rows): 34816 x 5120 34.0 / 35.8 / 68.2 -> 21.1 /
-// 24.8 / 27.7 (4.7 TB/s at one row); 17408 x 5120 19.6 / 21.4 / 40.8 -> 13.3 / 16.6 / 17.6; 5120 x 17408 22.4 / 25.6 / 46.4 -> 13.7
-// / 16.8 / 19.3; 5120 x 5120 9.5 / 11.4 / 21.6 -> 8.4 / 10.6 / 11.5; tensors of a few MB, where only the fixed part counts, lose up
-// to 1.3 us at one row (1024 x 5120: 4.1 / 6.2 / 11.0 -> 5.4 / 7.5 / 8.5). The native route's few rows: a layer's four fused
+// back to back with programmatic dependent launch, before -> now (us at 1 / 5 rows): 34816 x 5120 32.8 / 34.7 -> 20.6 / 24.4 (4.87
+// TB/s at one row); 17408 x 5120 19.2 / 21.1 -> 13.4 / 16.8; 5120 x 17408 22.1 / 25.1 -> 13.4 / 17.1; 5120 x 5120 10.0 / 11.6 -> 8.8 /
+// 11.1. Tensors of a few MB, where the fixed part is not hidden, lose 1.4 to 1.7 us (1024 x 5120: 4.7 / 6.7 -> 6.1 / 8.5): a
+// choice by the number of rows of the weights would give shards and group members other bits than the whole. The native route's few rows: a layer's four fused
 // linears at 40 rows 176 -> 98 us, quantizers included.
 // Instructions that one thread issues for the tensor core sit in a loop of the whole warp under an elected predicate (eb::elect_one):
 // 757 -> 453 cycles per unit of 256 values.
