@@ -96,17 +96,18 @@ __host__ __device__ inline uint32_t atom_byte(uint32_t row_in_tile, uint32_t sca
 // scale = e4m3_satfinite(amax * (1/6) * (1/global)); codes = e2m1_rn(v * ((1/global) / scale)), saturating; the next term
 // quantizes fma(-decoded, scale * global, v). All in FP32 with the hardware conversions.
 // The work split is this kernel's own: one CTA per row, a 16-value block per thread and turn, held in registers from the pass
-// that finds the row's largest magnitude to the pass that quantizes it (kHeld turns; what a longer row has beyond is read again). Four neighbouring lanes share a K block of 64 values; their four scale bytes meet by two shuffles
+// that finds the row's largest magnitude to the pass that quantizes it (kHeld turns; what a longer row has beyond is read again).
+// Four neighbouring lanes share a K block of 64 values; their four scale bytes meet by two shuffles
 // and leave as ONE 4-byte store, which is exactly one row's entry of the 512-byte atom tcgen05 reads; their codes leave as 32
 // contiguous bytes per term. A warp per row, which this replaces, read every row twice and left all but a few SMs idle on
 // calls of few rows.
-constexpr uint32_t kQuantizeThreads = 512;   // the most threads of a row
+// Bound: no single pipe was profiled; fewer instructions and more rows resident on an SM both measured faster; spilled registers, a CTA that walks several rows and
+// loads a row ahead all measured slower. Alone, us at 512 / 4096 / 32768 rows, warp per row -> now: 5120 values 8.2 / 20.6 / 113 -> 4.6 /
+// 15.7 / 119; 17,408 values 25.2 / 86.3 / 473 -> 8.8 / 57.7 / 429; 25,600 values (partly read twice) 36.2 / 123 / 698 -> 13.2 / 97.9 / 731.
+__host__ __device__ constexpr uint32_t quantize_threads(uint32_t held) { return held == 2u ? 512u : 384u; }   // the most of a row: two CTAs per SM without spills
 
-// One block of 16 values: its scale code, its 8 code bytes, and v replaced by the residual.
-__device__ __forceinline__ uint32_t quantize_block(float (&v)[16], float global, float inverse_global, uint2* codes) {
-    float block_max = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) block_max = fmaxf(block_max, fabsf(v[i]));
+// One block of 16 values with its largest magnitude: its scale code, its 8 code bytes, and v replaced by the residual.
+__device__ __forceinline__ uint32_t quantize_block(float (&v)[16], float block_max, float global, float inverse_global, uint2* codes) {
     const __nv_fp8_storage_t scale = __nv_cvt_float_to_fp8(__fmul_rn(__fmul_rn(block_max, 1.0f / 6.0f), inverse_global), __NV_SATFINITE, __NV_E4M3);
     const float decoded = __half2float(__half(__nv_cvt_fp8_to_halfraw(scale, __NV_E4M3)));
     const float inverse = decoded > 0.0f ? __fdiv_rn(inverse_global, decoded) : 0.0f;
@@ -126,21 +127,21 @@ __device__ __forceinline__ uint32_t quantize_block(float (&v)[16], float global,
     return (uint32_t)scale;
 }
 
-// Largest magnitude of 16 BF16 values (eight pairs).
+// Largest magnitude of 16 BF16 values, two at a time (a NaN loses against any number, as with fmaxf).
 __device__ __forceinline__ float largest_of(const uint4& lo, const uint4& hi) {
     const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-    float most = 0.0f;
+    __nv_bfloat162 most = __float2bfloat162_rn(0.0f);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) most = fmaxf(most, fmaxf(fabsf(eb::bf16_bits_to_float(w[j] & 0xFFFFu)), fabsf(__uint_as_float(w[j] & 0xFFFF0000u))));
-    return most;
+    for (int j = 0; j < 8; ++j) most = __hmax2(most, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[j])));
+    return fmaxf(__low2float(most), __high2float(most));
 }
 
-//   grid rows, block: the fewest whole warps that hold the row in kHeld turns, at most kQuantizeThreads. k a multiple of 64.
+//   grid rows, block: the fewest whole warps that hold the row in kHeld turns, at most quantize_threads. k a multiple of 64.
 template <uint32_t kHeld>
-__global__ void __launch_bounds__(kQuantizeThreads, 2) quantize_rows(const __nv_bfloat16* __restrict__ input, uint8_t* __restrict__ scratch,
+__global__ void __launch_bounds__(quantize_threads(kHeld), 2) quantize_rows(const __nv_bfloat16* __restrict__ input, uint8_t* __restrict__ scratch,
         uint32_t rows, uint32_t k) {
     const uint32_t t = threadIdx.x, threads = blockDim.x, row = blockIdx.x;
-    __shared__ float warp_most[kQuantizeThreads / 32u];
+    __shared__ float warp_most[quantize_threads(kHeld) / 32u];
     const ActivationLayout layout(rows, k);
     eb::pdl_launch_dependents();
     eb::pdl_wait();
@@ -154,9 +155,9 @@ __global__ void __launch_bounds__(kQuantizeThreads, 2) quantize_rows(const __nv_
         lo[i] = b < blocks ? x[2u * b] : zero;
         hi[i] = b < blocks ? x[2u * b + 1u] : zero;
     }
-    float amax = 0.0f;
+    float amax = 0.0f, block_max[kHeld];
 #pragma unroll
-    for (uint32_t i = 0; i < kHeld; ++i) amax = fmaxf(amax, largest_of(lo[i], hi[i]));
+    for (uint32_t i = 0; i < kHeld; ++i) amax = fmaxf(amax, block_max[i] = largest_of(lo[i], hi[i]));
     for (uint32_t b = kHeld * threads + t; b < blocks; b += threads) amax = fmaxf(amax, largest_of(x[2u * b], x[2u * b + 1u]));
     // magnitudes are non-negative floats, whose bits order as integers
     const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
@@ -169,7 +170,7 @@ __global__ void __launch_bounds__(kQuantizeThreads, 2) quantize_rows(const __nv_
     uint8_t* sfa = scratch + layout.sfa_offset + (uint64_t)(row / kTileM) * layout.k_blocks * kTerms * kAtom + atom_byte(row % kTileM, 0);
     const uint64_t plane = (uint64_t)rows * (k / 2u);
     uint8_t* codes_row = scratch + (uint64_t)row * (k / 2u);
-    auto quantize = [&](uint32_t b, const uint4& first, const uint4& second) {   // whole quartets of lanes come here together
+    auto quantize = [&](uint32_t b, const uint4& first, const uint4& second, float most_of_block) {   // whole quartets of lanes come here together
         const uint32_t words[8] = {first.x, first.y, first.z, first.w, second.x, second.y, second.z, second.w};
         const uint32_t sub = b & 3u, members = 0xFu << (t & 28u);
         float v[16];
@@ -181,7 +182,12 @@ __global__ void __launch_bounds__(kQuantizeThreads, 2) quantize_rows(const __nv_
 #pragma unroll
         for (uint32_t term = 0; term < kTerms; ++term) {
             uint2 codes;
-            uint32_t scales = quantize_block(v, global, inverse_global, &codes) << (8u * sub);
+            if (term != 0u) {
+                most_of_block = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) most_of_block = fmaxf(most_of_block, fabsf(v[i]));
+            }
+            uint32_t scales = quantize_block(v, most_of_block, global, inverse_global, &codes) << (8u * sub);
             scales |= __shfl_xor_sync(members, scales, 1);   // the K block's four scale bytes, in every one of the four lanes
             scales |= __shfl_xor_sync(members, scales, 2);
             *reinterpret_cast<uint2*>(codes_row + term * plane + 8u * b) = codes;
@@ -190,8 +196,11 @@ __global__ void __launch_bounds__(kQuantizeThreads, 2) quantize_rows(const __nv_
     };
 #pragma unroll
     for (uint32_t i = 0; i < kHeld; ++i)
-        if (i * threads + t < blocks) quantize(i * threads + t, lo[i], hi[i]);
-    for (uint32_t b = kHeld * threads + t; b < blocks; b += threads) quantize(b, x[2u * b], x[2u * b + 1u]);
+        if (i * threads + t < blocks) quantize(i * threads + t, lo[i], hi[i], block_max[i]);
+    for (uint32_t b = kHeld * threads + t; b < blocks; b += threads) {
+        const uint4 first = x[2u * b], second = x[2u * b + 1u];
+        quantize(b, first, second, largest_of(first, second));
+    }
     if (t == 0u) reinterpret_cast<float*>(scratch + layout.global_offset)[row] = global;
 }
 
@@ -774,12 +783,13 @@ inline cudaError_t launch_on(cudaStream_t stream, bool pdl, void (*kernel)(Param
 // quantize: BF16 rows -> the activation part of the scratch (code planes, scale atoms, row scales).
 inline cudaError_t quantize(const void* input, void* scratch, uint32_t rows, uint32_t k, cudaStream_t stream, bool pdl) {
     const uint32_t blocks = k / 16u;
+    auto threads_of = [&](uint32_t held) { return std::min(quantize_threads(held), ((blocks + held - 1u) / held + 31u) / 32u * 32u); };
     auto run = [&](auto kernel, uint32_t held) {
-        const uint32_t threads = std::min(kQuantizeThreads, ((blocks + held - 1u) / held + 31u) / 32u * 32u);
-        return launch_on(stream, pdl, kernel, dim3(rows), dim3(threads), 0, static_cast<const __nv_bfloat16*>(input), static_cast<uint8_t*>(scratch), rows, k);
+        return launch_on(stream, pdl, kernel, dim3(rows), dim3(threads_of(held)), 0, static_cast<const __nv_bfloat16*>(input), static_cast<uint8_t*>(scratch), rows, k);
     };
-    // two turns while they hold the row (rows of up to 16,384 values), else four
-    return blocks <= 2u * kQuantizeThreads ? run(quantize_rows<2>, 2u) : run(quantize_rows<4>, 4u);
+    // rows an SM holds at once, by registers; three turns measured no better where they hold no more (rows of 8192 and 16,384 values)
+    auto resident = [&](uint32_t held, uint32_t registers) { return 65536u / (threads_of(held) * registers); };
+    return resident(3u, 80u) > resident(2u, 64u) || blocks > 2u * quantize_threads(2u) ? run(quantize_rows<3>, 3u) : run(quantize_rows<2>, 2u);
 }
 
 // multiply: the GEMM over the quantized activations found in the scratch (table-indexed weight scales are expanded there first).
