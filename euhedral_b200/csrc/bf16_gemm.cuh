@@ -344,33 +344,39 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_ge
             }
         }
       } else if (warp == 1) {
-        if (lane == 0 && rank == 0u) {   // the odd CTA issues nothing: its tiles are read by the even CTA's MMAs
-            uint32_t step = 0, local = 0;
+        if (rank == 0u) {   // the odd CTA issues nothing: its tiles are read by the even CTA's MMAs
+            const bool leader = eb::elect_one();   // in a loop of the whole warp: see eb::elect_one
+            eb::Ring ring;
+            uint32_t local = 0;
             bool ok = true;
             for (uint32_t item = pair; item < items && ok; item += pairs, ++local) {
                 const uint32_t buffer = local & 1u, use = local >> 1;
-                if (use > 0 && !eb::mbar_wait(&acc_empty[buffer], (use - 1u) & 1u)) {
-                    atomicOr(error, kWaitFailed);
+                if (use > 0 && !__all_sync(0xFFFFFFFFu, eb::mbar_wait(&acc_empty[buffer], (use - 1u) & 1u))) {
+                    if (lane == 0) atomicOr(error, kWaitFailed);
                     break;
                 }
                 nvfp4n::tcgen05_fence_after();
                 const uint32_t accumulator = tmem + buffer * kTileN;
                 const uint32_t instruction = item < whole ? kPairInstruction : kPairInstructionHalf;
-                for (uint32_t ks = 0; ks < k_steps; ++ks, ++step) {
-                    const uint32_t s = step % kPairStages, round = step / kPairStages;
-                    if (!eb::mbar_wait(&full[s], round & 1u)) {
-                        atomicOr(error, kWaitFailed);
+                for (uint32_t ks = 0; ks < k_steps; ++ks) {
+                    if (!__all_sync(0xFFFFFFFFu, eb::mbar_wait(&full[ring.stage], ring.parity))) {
+                        if (lane == 0) atomicOr(error, kWaitFailed);
                         ok = false;
                         break;
                     }
                     nvfp4n::tcgen05_fence_after();
-                    const uint8_t* stage = smem + s * kPairStageBytes;
+                    const uint8_t* stage = smem + ring.stage * kPairStageBytes;
                     const uint64_t a = nvfp4n::tile_descriptor(stage), b = nvfp4n::tile_descriptor(stage + kATile);
+                    if (leader) {
 #pragma unroll
-                    for (uint32_t j = 0; j < 4u; ++j) pair_mma_bf16(accumulator, a + 2u * j, b + 2u * j, instruction, (uint32_t)((ks | j) != 0u));
-                    nvfp4n::pair_commit(&empty[s]);
+                        for (uint32_t j = 0; j < 4u; ++j) pair_mma_bf16(accumulator, a + 2u * j, b + 2u * j, instruction, (uint32_t)((ks | j) != 0u));
+                        nvfp4n::pair_commit(&empty[ring.stage]);
+                    }
+                    __syncwarp();
+                    ring.advance(kPairStages);
                 }
-                if (ok) nvfp4n::pair_commit(&acc_full[buffer]);
+                if (ok && leader) nvfp4n::pair_commit(&acc_full[buffer]);
+                __syncwarp();
             }
         }
       }
