@@ -450,19 +450,21 @@ __global__ void __launch_bounds__(kScaledThreads, 1) gemm_kernel(const __grid_co
             }
         }
       } else if (warp == 1) {
-        if (lane == 0) {
-            uint32_t step = 0, local = 0;
+        {
+            const bool leader = eb::elect_one();   // in a loop of the whole warp: see eb::elect_one
+            eb::Ring ring;
+            uint32_t local = 0;
             bool ok = true;
             for (uint32_t item = blockIdx.x; item < walk.total && ok; item += gridDim.x, ++local) {
-                if (local > 0 && !eb::mbar_wait(acc_empty, (local - 1u) & 1u)) {
-                    atomicOr(error, 8u);
+                if (local > 0 && !__all_sync(0xFFFFFFFFu, eb::mbar_wait(acc_empty, (local - 1u) & 1u))) {
+                    if (lane == 0) atomicOr(error, 8u);
                     break;
                 }
                 tcgen05_fence_after();
-                for (uint32_t ks = 0; ks < k_steps; ++ks, ++step) {
-                    const uint32_t s = step % kStages, round = step / kStages;
-                    if (!eb::mbar_wait(&full[s], round & 1u) || !eb::mbar_wait(&scaled[s], round & 1u)) {
-                        atomicOr(error, 8u);
+                for (uint32_t ks = 0; ks < k_steps; ++ks) {
+                    const uint32_t s = ring.stage;
+                    if (!__all_sync(0xFFFFFFFFu, eb::mbar_wait(&full[s], ring.parity) && eb::mbar_wait(&scaled[s], ring.parity))) {
+                        if (lane == 0) atomicOr(error, 8u);
                         ok = false;
                         break;
                     }
@@ -470,14 +472,19 @@ __global__ void __launch_bounds__(kScaledThreads, 1) gemm_kernel(const __grid_co
                     const uint8_t* stage = smem + s * kStageBytes;
                     const uint64_t a0 = tile_descriptor(stage), a1 = tile_descriptor(stage + kATile), b = tile_descriptor(stage + kTerms * kATile);
                     const uint32_t scales = tmem + kTmemScales + s * kScaleColumns;
+                    if (leader) {
 #pragma unroll
-                    for (uint32_t j = 0; j < 4u; ++j) {
-                        mma_block_scaled(tmem, a0 + 2u * j, b + 2u * j, scales + j * 8u, scales + 32u + j * 8u, (uint32_t)((ks | j) != 0u));
-                        mma_block_scaled(tmem, a1 + 2u * j, b + 2u * j, scales + j * 8u + 4u, scales + 32u + j * 8u, 1u);
+                        for (uint32_t j = 0; j < 4u; ++j) {
+                            mma_block_scaled(tmem, a0 + 2u * j, b + 2u * j, scales + j * 8u, scales + 32u + j * 8u, (uint32_t)((ks | j) != 0u));
+                            mma_block_scaled(tmem, a1 + 2u * j, b + 2u * j, scales + j * 8u + 4u, scales + 32u + j * 8u, 1u);
+                        }
+                        mma_commit(&empty[s]);
                     }
-                    mma_commit(&empty[s]);
+                    __syncwarp();
+                    ring.advance(kStages);
                 }
-                if (ok) mma_commit(acc_full);
+                if (ok && leader) mma_commit(acc_full);
+                __syncwarp();
             }
         }
       }
@@ -673,19 +680,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kScaledThreads, 1) g
             }
         }
       } else if (warp == 1) {
-        if (lane == 0 && rank == 0u) {   // the odd CTA issues nothing: its tiles are read by the even CTA's MMAs
-            uint32_t step = 0, local = 0;
+        if (rank == 0u) {   // the odd CTA issues nothing: its tiles are read by the even CTA's MMAs
+            const bool leader = eb::elect_one();   // in a loop of the whole warp: see eb::elect_one
+            eb::Ring ring;
+            uint32_t local = 0;
             bool ok = true;
             for (uint32_t item = pair; item < items && ok; item += pairs, ++local) {
-                if (local > 0 && !eb::mbar_wait(acc_empty, (local - 1u) & 1u)) {
-                    atomicOr(error, 8u);
+                if (local > 0 && !__all_sync(0xFFFFFFFFu, eb::mbar_wait(acc_empty, (local - 1u) & 1u))) {
+                    if (lane == 0) atomicOr(error, 8u);
                     break;
                 }
                 tcgen05_fence_after();
-                for (uint32_t ks = 0; ks < k_steps; ++ks, ++step) {
-                    const uint32_t s = step % kPairStages, round = step / kPairStages;
-                    if (!eb::mbar_wait(&full[s], round & 1u) || !eb::mbar_wait(&scaled[s], round & 1u)) {
-                        atomicOr(error, 8u);
+                for (uint32_t ks = 0; ks < k_steps; ++ks) {
+                    const uint32_t s = ring.stage;
+                    if (!__all_sync(0xFFFFFFFFu, eb::mbar_wait(&full[s], ring.parity) && eb::mbar_wait(&scaled[s], ring.parity))) {
+                        if (lane == 0) atomicOr(error, 8u);
                         ok = false;
                         break;
                     }
@@ -693,14 +702,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kScaledThreads, 1) g
                     const uint8_t* stage = smem + s * kPairStageBytes;
                     const uint64_t a0 = tile_descriptor(stage), a1 = tile_descriptor(stage + kATile), b = tile_descriptor(stage + kTerms * kATile);
                     const uint32_t scales = tmem + kTmemScales + s * kScaleColumns;
+                    if (leader) {
 #pragma unroll
-                    for (uint32_t j = 0; j < 4u; ++j) {
-                        pair_mma(tmem, a0 + 2u * j, b + 2u * j, scales + j * 8u, scales + 32u + j * 8u, (uint32_t)((ks | j) != 0u));
-                        pair_mma(tmem, a1 + 2u * j, b + 2u * j, scales + j * 8u + 4u, scales + 32u + j * 8u, 1u);
+                        for (uint32_t j = 0; j < 4u; ++j) {
+                            pair_mma(tmem, a0 + 2u * j, b + 2u * j, scales + j * 8u, scales + 32u + j * 8u, (uint32_t)((ks | j) != 0u));
+                            pair_mma(tmem, a1 + 2u * j, b + 2u * j, scales + j * 8u + 4u, scales + 32u + j * 8u, 1u);
+                        }
+                        pair_commit(&empty[s]);
                     }
-                    pair_commit(&empty[s]);
+                    __syncwarp();
+                    ring.advance(kPairStages);
                 }
-                if (ok) pair_commit(acc_full);
+                if (ok && leader) pair_commit(acc_full);
+                __syncwarp();
             }
         }
       }
