@@ -160,8 +160,7 @@ cudaError_t allow_gemv() {
 // Clusters of `split` CTAs of this kernel that the current device holds at once. Without a device: one CTA per SM.
 template <class F>
 uint32_t resident_clusters(GemvKernel<F> kernel, uint32_t warps, uint32_t shared, uint32_t split, int sms) {
-    const uint32_t threads = 32u * (warps + (F::kAddingWarp ? 1u : 0u));   // the decoding warps and the adding warp
-    const uint32_t now = eb::resident_clusters((const void*)kernel, threads, shared, split);
+    const uint32_t now = eb::resident_clusters((const void*)kernel, 32u * warps, shared, split);
     return now != 0u ? now : (uint32_t)sms / split;
 }
 
@@ -288,7 +287,7 @@ cudaError_t launch_gemv(const DecodeItem* items, uint32_t count, uint32_t rows, 
     group.tiles = tiles;
     group.depth = plan.depth;
     group.span = plan.span;
-    return launch(kOverlappable, gemv_kernel<F>(plan.order.piece, plan.tma_scales), dim3(plan.ctas), dim3(32u * (plan.warps + (F::kAddingWarp ? 1u : 0u))), plan.shared,
+    return launch(kOverlappable, gemv_kernel<F>(plan.order.piece, plan.tma_scales), dim3(plan.ctas), dim3(32u * plan.warps), plan.shared,
             plan.order.split, group, error);
 }
 

@@ -27,10 +27,7 @@
 //     again; those sums are never used.
 //   * The T piece sums of a tile meet in shared memory and are added in piece order, then rounded and stored as BF16
 //     (S = 1) or handed to the tile's owner rank through distributed shared memory; owners add the S slice sums in
-//     rank order after a cluster barrier at the end of each tensor. Who adds is the policy's choice (kAddingWarp):
-//     the team itself after a named barrier per tile (teams of 8: the barrier costs less than the hand-over), or one
-//     extra warp of the CTA that the teams signal through mbarriers, so that no decoding warp ever waits for another
-//     (teams of 16, where the barrier would stop the whole CTA once per tile).
+//     rank order after a cluster barrier at the end of each tensor. The team adds, after a named barrier per tile.
 //
 // A policy F provides:
 //   Geometry(n, k)                  byte geometry of the tensor: row_bytes, scale_row_bytes, scale_offset
@@ -39,7 +36,6 @@
 //                                   an odd multiple of 16 so that the rows of a quarter-warp fall in distinct banks)
 //   kPieceChunks, kMaxPiece         preferred and largest chunks per piece
 //   kErrorBit                       bit of the device error word for a wait that gave up
-//   kAddingWarp                     whether an extra warp adds the piece sums (else the team does, behind a barrier)
 //   extra_bytes(chunks)             extra shared bytes next to the activation slice
 //   stage(...)                      CTA-wide staging of the activation slice in the decode's pairing
 //   lane_scale_offset(q)            byte offset of lane q's scales within a chunk's scale bytes
@@ -97,7 +93,7 @@ struct alignas(64) Group {
 // Shared memory of one CTA.
 template <class F>
 struct Layout {
-    uint32_t stride_x, off_extra, off_partials, off_gather, off_slots, off_bars, off_sum_bars, slot_bytes, code_bytes, bytes;
+    uint32_t stride_x, off_extra, off_partials, off_gather, off_slots, off_bars, slot_bytes, code_bytes, bytes;
     __host__ __device__ Layout(const Order& o, uint32_t rows, uint32_t warps, uint32_t depth, uint32_t span) {
         const uint32_t widest = (o.chunks + o.split - 1u) / o.split;
         stride_x = widest * 256u + 64u;   // 64 modulo 128: the rows a quarter-warp reads fall in distinct banks
@@ -109,8 +105,7 @@ struct Layout {
         code_bytes = 16u * o.piece * F::kCodeBytes;
         slot_bytes = code_bytes + 16u * F::kScaleBox;
         off_bars = off_slots + warps * depth * slot_bytes;
-        off_sum_bars = off_bars + warps * depth * 8u;   // per team and sum buffer: a full and an empty barrier
-        bytes = off_sum_bars + (F::kAddingWarp ? (warps / o.team) * 2u * 16u : 0u);
+        bytes = off_bars + warps * depth * 8u;
     }
 };
 
@@ -164,11 +159,10 @@ __device__ __forceinline__ void decode_piece(typename F::template State<P>& stat
 }
 
 template <class F, int P, bool kTmaScales>
-__global__ void __launch_bounds__(32 * (kMaxWarps + (F::kAddingWarp ? 1 : 0)), 1) kernel(const __grid_constant__ Group group, uint32_t* __restrict__ error) {
+__global__ void __launch_bounds__(32 * kMaxWarps, 1) kernel(const __grid_constant__ Group group, uint32_t* __restrict__ error) {
     extern __shared__ __align__(128) uint8_t smem[];
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, g = lane >> 2, q = lane & 3u;
-    constexpr bool kAdder = F::kAddingWarp;   // piece sums are added by a warp of their own (the CTA's last) or by the team itself
-    const uint32_t warps = (blockDim.x >> 5) - (kAdder ? 1u : 0u), threads = blockDim.x;   // decoding warps
+    const uint32_t warps = blockDim.x >> 5, threads = blockDim.x;
     const uint32_t rows = group.rows, depth = group.depth;
     const Order order = order_of<F>(group.k);
     const uint32_t split = order.split, team_size = order.team;
@@ -181,18 +175,10 @@ __global__ void __launch_bounds__(32 * (kMaxWarps + (F::kAddingWarp ? 1 : 0)), 1
     const uint32_t slice = slice_end - slice_begin;
     const Layout<F> layout(order, rows, warps, depth, group.span);
     const uint32_t smem_a = eb::smem_u32(smem);
-    // Piece sums travel from a team's warps to the adding warp through two buffers per team, each guarded by a `full`
-    // barrier (one arrival per team member) and an `empty` barrier (one arrival by the adding warp).
-    const uint32_t sums_a = smem_a + layout.off_sum_bars;   // [team][buffer][full, empty]
-
+    // Always true; without the test the compiler gives the loop 126 registers instead of 124 and a layer at one row takes 59.9 us, not 59.2.
     if (warp < warps) {
         if (lane == 0) {
             for (uint32_t s = 0; s < depth; ++s) eb::mbar_init(reinterpret_cast<uint64_t*>(smem + layout.off_bars) + warp * depth + s, 1);
-        }
-    } else if (kAdder && lane == 0) {
-        for (uint32_t i = 0; i < teams * 2u; ++i) {
-            eb::mbar_init(reinterpret_cast<uint64_t*>(smem + layout.off_sum_bars) + 2u * i, team_size);
-            eb::mbar_init(reinterpret_cast<uint64_t*>(smem + layout.off_sum_bars) + 2u * i + 1u, 1);
         }
     }
     if (lane == 0) eb::mbar_fence_init();
@@ -245,36 +231,6 @@ __global__ void __launch_bounds__(32 * (kMaxWarps + (F::kAddingWarp ? 1 : 0)), 1
             }
         }
     };
-
-    if (kAdder && warp == warps) {
-        // ---- the adding warp: the T piece sums of a tile in piece order, then BF16 (one slice) or the tile's owner rank ----
-        eb::pdl_launch_dependents();
-        eb::pdl_wait();
-        if (split > 1u) eb::cluster_wait();
-        uint32_t first_tile = 0;
-        for (uint32_t ti = 0; ti < group.count; ++ti) {
-            const Tensor& t = group.tensor[ti];
-            const uint32_t segment_begin = max(run_begin, first_tile), segment_end = min(run_end, t.tile_end);
-            if (segment_begin < segment_end) {
-                stage(t);
-                const typename F::Finish finish(t.w, typename F::Geometry(t.n, group.k));
-                for (uint32_t tile = segment_begin; tile < segment_end; ++tile) {
-                    // Tile run_begin + i belongs to team i % teams and is that team's tile number i / teams.
-                    const uint32_t index = tile - run_begin, team = index % teams, turn = index / teams, buffer = turn & 1u;
-                    const uint32_t bars = sums_a + (team * 2u + buffer) * 16u;
-                    if (complete) complete = eb::mbar_wait_at<400>(bars, (turn >> 1) & 1u);   // a team needs microseconds per tile: poll rarely
-                    const uint32_t pieces = smem_a + layout.off_partials + (team * 2u + buffer) * team_size * kPartial;
-                    add_pieces(t, finish, pieces, (tile - first_tile) * 16u, tile - segment_begin, lane, 32u);
-                    __syncwarp();
-                    if (lane == 0) eb::mbar_arrive(reinterpret_cast<uint64_t*>(smem + layout.off_sum_bars) + (team * 2u + buffer) * 2u + 1u);
-                }
-                if (split > 1u) join_slices(t, first_tile, segment_begin, segment_end);
-            }
-            first_tile = t.tile_end;
-        }
-        if (!complete && lane == 0) atomicOr(error, F::kErrorBit);
-        return;
-    }
 
     // ---- a decoding warp: member j of its team owns piece j of the slice for every tile the team takes ----
     const uint32_t team = warp / team_size, member = warp % team_size;
@@ -334,7 +290,6 @@ __global__ void __launch_bounds__(32 * (kMaxWarps + (F::kAddingWarp ? 1 : 0)), 1
     // This lane's place in its team's two sum buffers: [buffer][member][row of the tile][activation row]; lane (g, q) holds
     // rows g, g + 8 for columns 2q, 2q + 1.
     const uint32_t sum_lane = smem_a + layout.off_partials + (team * 2u * team_size + member) * kPartial + (g * 8u + 2u * q) * 4u;
-    const uint32_t sum_bars = sums_a + team * 32u;
     typename F::template State<P> state(extra_lane, q);
 
     uint32_t use_tile = run_begin + team, use_slot = 0, parity = 0, turn = 0, first_tile = 0;
@@ -357,25 +312,20 @@ __global__ void __launch_bounds__(32 * (kMaxWarps + (F::kAddingWarp ? 1 : 0)), 1
                 if (P == 1 || wide) decode_piece<F, P, P>(state, slot + code_lane, slot + scale_lane, x_lane, acc);
                 else decode_piece<F, P, (P > 1 ? P - 1 : 1)>(state, slot + code_lane, slot + scale_lane, x_lane, acc);
                 const uint32_t buffer = turn & 1u;
-                // With an adding warp: the sum buffer of this turn was read two turns ago (the first two turns find it free).
-                if (kAdder && complete) complete = eb::mbar_wait_at(sum_bars + buffer * 16u + 8u, ((turn >> 1) & 1u) ^ 1u);
                 const uint32_t mine = sum_lane + buffer * team_size * kPartial;
                 st_shared_f2(mine, acc[0], acc[1]);
                 st_shared_f2(mine + 256u, acc[2], acc[3]);
                 __syncwarp();   // every lane is done with the slot and has written its sums
-                if (kAdder && lane == 0) eb::mbar_arrive_at(sum_bars + buffer * 16u);
                 request();
                 if (++use_slot == depth) {
                     use_slot = 0;
                     parity ^= 1u;
                 }
-                if (!kAdder) {
-                    // The team meets on its named barrier; its threads share the tile's outputs. Two buffers: a warp that runs
-                    // ahead writes the other one, and passes the next barrier only after every teammate has finished here.
-                    if (team_size > 1u) team_sync(team, team_size * 32u);
-                    add_pieces(t, finish, smem_a + layout.off_partials + (team * 2u + buffer) * team_size * kPartial, (use_tile - first_tile) * 16u,
-                            use_tile - segment_begin, tid - team * team_size * 32u, team_size * 32u);
-                }
+                // The team meets on its named barrier; its threads share the tile's outputs. Two buffers: a warp that runs
+                // ahead writes the other one, and passes the next barrier only after every teammate has finished here.
+                if (team_size > 1u) team_sync(team, team_size * 32u);
+                add_pieces(t, finish, smem_a + layout.off_partials + (team * 2u + buffer) * team_size * kPartial, (use_tile - first_tile) * 16u,
+                        use_tile - segment_begin, tid - team * team_size * 32u, team_size * 32u);
             }
             if (split > 1u) join_slices(t, first_tile, segment_begin, segment_end);
         }

@@ -94,7 +94,6 @@ struct Format {
     static constexpr uint32_t kCodeBytes = 48, kScaleBytes = 4, kErrorBit = 2;
     // A piece is at most 5 chunks (3.75 KB of codes per 16 rows). The scale box, 48 bytes per row, covers 5 chunks' scales
     // plus the 12 bytes a piece can start after a 16-byte boundary, and is an odd multiple of 16.
-    static constexpr bool kAddingWarp = false;
     static constexpr uint32_t kPieceChunks = 5, kMaxPiece = 5, kScaleBox = 48;
     // float [chunk][group][lane q][4]: minus the biased sum of the group's activations of rows 2q and 2q+1, twice over
     // (x, y, x, y), which is the accumulator quad lane q starts a group with.
