@@ -8,7 +8,8 @@
 //     row becomes eight columns. Products are exact; column t of a row counts 8^-t and the eight sums are added in FP32 once per K
 //     slice. Where some eight neighbours of a row stay below 2^-4 of the slice's largest (outliers), four more columns hold the
 //     next four digits of what the eight cut off: nothing above 2^-33 of the largest value is lost then. The choice is a row's and
-//     slice's own and changes no bit of the rows beside it.
+//     slice's own and changes no bit of the rows beside it. Values that are not finite have no digits: the draining warps add their products
+//     in FP32 from the weights in memory, so that an infinity gives every output what IEEE arithmetic gives it.
 //   * two NVFP4 terms per row, quantized into the scratch before (the native route): a row is one column, both terms accumulate
 //     into it, as in the large GEMM (nvfp4_native.cuh), and more than kMaxColumns rows take a tile of weights several times.
 //     With `pair_rows` a tile is 64 gate rows and the 64 up rows that match them, finished as SwiGLU (the paired region).
@@ -42,6 +43,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "exact_kernels.cuh"
 #include "nvfp4_native.cuh"
 
 namespace nvfp4d {
@@ -55,6 +57,7 @@ constexpr uint32_t kCodeBytes = kTile * kUnit / 2u, kScaleBytes = kTile * kUnit 
 constexpr uint32_t kMaxStages = 8;
 constexpr uint32_t kTmemColumns = 512;
 constexpr uint32_t kSpread = 4;           // powers of two that one grid covers (see above)
+constexpr uint32_t kLeftWords = 128;      // rows times units of a CTA: more than its shared memory has room for digits of
 constexpr uint32_t kLeastExponent = 48;   // of a row's slice: smaller values keep the grid of 2^-79
 
 __host__ __device__ inline uint32_t units_of(uint32_t k) { return (k + kUnit - 1u) / kUnit; }
@@ -66,6 +69,7 @@ __host__ __device__ inline uint32_t split_of(uint32_t units) { return units < 4u
 struct alignas(64) Tensor {
     CUtensorMap codes;         // bytes [n][K/2], box 128 x 64 rows (half a tile)
     const uint16_t* x;         // BF16 [rows][K] (decode)
+    const uint8_t* weights;    // the code plane
     const uint8_t* scales;     // the scale (or index) plane
     const uint8_t* table;      // the 16 E4M3 codes of a table-indexed tensor, else null
     const float* global;
@@ -103,7 +107,7 @@ struct Layout {
         off_rows = stages * stage_bytes;                             // resident digits: a tile of `columns` x 128 bytes per unit
         off_gather = off_rows + (resident ? units_cta * columns * 128u : 0u);
         off_bars = off_gather + (split > 1u ? 2u * gather_bytes : paired ? gather_bytes / 2u : 0u);
-        bytes = off_bars + 1024u + 1024u;                            // barriers, the rows' exponents or scales; slack to align to 1024
+        bytes = off_bars + 1024u + 1024u;                            // barriers, the rows' exponents and left-out values or scales; slack to align to 1024
     }
 };
 
@@ -194,6 +198,106 @@ __device__ __forceinline__ void octal_digits(const uint4& v, float per, bool mor
     finish(high, 4);
 }
 
+// The largest exponent of eight BF16 values. 0: nothing but zeros (or subnormal values); 255: not all of them are finite.
+__device__ __forceinline__ uint32_t largest_exponent(const uint4& v) {
+    const uint32_t most = __vmaxu2(__vmaxu2(v.x & 0x7FFF7FFFu, v.y & 0x7FFF7FFFu), __vmaxu2(v.z & 0x7FFF7FFFu, v.w & 0x7FFF7FFFu));
+    return max(most & 0xFFFFu, most >> 16) >> 7;
+}
+// Eight BF16 values with zeros in the place of those that are not finite.
+__device__ __forceinline__ uint4 finite_only(const uint4& v) {
+    auto word = [](uint32_t w) {
+        return w & (((w & 0x7F80u) == 0x7F80u ? 0u : 0xFFFFu) | ((w & 0x7F800000u) == 0x7F800000u ? 0u : 0xFFFF0000u));
+    };
+    return make_uint4(word(v.x), word(v.y), word(v.z), word(v.w));
+}
+
+// What the staging warps of a CTA share about its slice of the rows.
+struct Slice {
+    const uint16_t* x;
+    uint32_t rows, k, unit_begin, units;
+    uint32_t stager, lane;                  // the staging warp among them
+    uint32_t *exponents, *least, *left;
+    uint8_t* digits;
+    uint32_t columns;
+    __device__ __forceinline__ uint4 load(uint32_t row, uint32_t unit) const {   // this lane's eight values of a unit
+        const uint32_t at = (unit_begin + unit) * kUnit + lane * 8u;
+        return row < rows && at < k ? *reinterpret_cast<const uint4*>(x + (uint64_t)row * k + at) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    __device__ __forceinline__ bool has_outliers(uint32_t row) const { return least[row] + kSpread < exponents[row]; }
+    __device__ __forceinline__ void find(uint32_t row, const uint4& v) const {
+        const uint32_t mine = largest_exponent(v);
+        const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, mine), low = __reduce_min_sync(0xFFFFFFFFu, mine == 0u ? 255u : mine);
+        if (row < rows && lane == 0) {
+            atomicMax(&exponents[row], most);
+            atomicMin(&least[row], low);
+        }
+    }
+    __device__ __forceinline__ void write(uint32_t row, uint32_t unit, const uint4& values) const {
+        const float per = __uint_as_float((275u - exponents[row]) << 23);
+        uint8_t* tile = digits + unit * columns * 128u + (lane & 3u) * 4u;
+        const uint32_t passes = has_outliers(row) ? 2u : 1u;
+#pragma unroll 1
+        for (uint32_t pass = 0; pass < passes; ++pass) {
+            uint32_t word[8];
+            octal_digits(values, per, pass != 0u, word);
+            const uint32_t column = pass == 0u ? row * kDigits : rows * kDigits + row * kMoreDigits;   // of digit 0; rows of 128 bytes, swizzled
+            uint8_t* to = tile + (column >> 3) * 1024u;
+            const uint32_t first = column & 7u;   // 0, or 4 for every other row's further digits
+#pragma unroll
+            for (uint32_t t = 0; t < 8u; ++t)
+                if (t < kMoreDigits || pass == 0u) *reinterpret_cast<uint32_t*>(to + (first + t) * 128u + (((lane >> 2) ^ (first + t)) << 4)) = word[t];
+        }
+    }
+};
+
+// The rows of a mask, whose digits leave values out, once more: their exponents over the other values, their digits, and the words that
+// say where the values left out are. Taken by every staging warp when all digits have been written.
+__device__ __forceinline__ void stage_again(const Slice& slice, const uint32_t odd_rows) {
+    auto for_units = [&](auto&& body) {
+#pragma unroll 1
+        for (uint32_t odd = odd_rows; odd != 0u; odd &= odd - 1u)
+#pragma unroll 1
+            for (uint32_t u = slice.stager; u < slice.units; u += kStagers / 32u) body((uint32_t)__ffs((int)odd) - 1u, u);
+    };
+    stagers_sync();   // nobody needs the exponents that led here any more
+    if (slice.stager == 0u && ((odd_rows >> slice.lane) & 1u)) slice.exponents[slice.lane] = kLeastExponent, slice.least[slice.lane] = 255u;
+    stagers_sync();
+    for_units([&](uint32_t row, uint32_t u) { slice.find(row, finite_only(slice.load(row, u))); });
+    stagers_sync();
+    for_units([&](uint32_t row, uint32_t u) {
+        const uint4 values = slice.load(row, u);
+        const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, largest_exponent(values) == 255u);
+        if (slice.lane == 0u) slice.left[row * slice.units + u] = lanes;
+        slice.write(row, u, finite_only(values));
+    });
+    stagers_sync();   // the words are there for the draining warps
+}
+
+// What the digits of activation row m leave out of a slice (`left`: its words, one per unit), summed against one weight row in FP32 in
+// K order. The weights are read where they lie: the ring has moved on.
+template <bool kTable>
+__device__ __forceinline__ float left_out(const Tensor& t, uint32_t row, uint32_t m, uint32_t k, uint32_t unit_begin, uint32_t units, const uint32_t* left) {
+    float sum = 0.0f;
+    if (row >= t.n) return sum;
+    const uint32_t* codes = reinterpret_cast<const uint32_t*>(t.weights) + (uint64_t)row * (k / 8u);
+    const uint8_t* scale_codes = t.scales + (uint64_t)row * (k / (kTable ? 32u : 16u));
+#pragma unroll 1
+    for (uint32_t u = 0; u < units; ++u)
+#pragma unroll 1
+        for (uint32_t lanes = left[u]; lanes != 0u; lanes &= lanes - 1u) {
+            const uint32_t eighth = (unit_begin + u) * 32u + (uint32_t)__ffs((int)lanes) - 1u;   // of K
+            const uint4 values = *reinterpret_cast<const uint4*>(t.x + (uint64_t)m * k + eighth * 8u);
+            const uint32_t pairs[4] = {values.x, values.y, values.z, values.w}, word = codes[eighth];
+            const float scale = exact::e4m3(kTable ? t.table[(scale_codes[eighth >> 2] >> ((eighth & 2u) * 2u)) & 15u] : scale_codes[eighth >> 1]);
+#pragma unroll
+            for (uint32_t i = 0; i < 8u; ++i) {
+                const uint32_t bits = (pairs[i >> 1] >> (16u * (i & 1u))) & 0xFFFFu;
+                if ((bits & 0x7F80u) == 0x7F80u) sum = __fmaf_rn(eb::bf16_bits_to_float(bits), __fmul_rn(exact::e2m1((word >> (4u * i)) & 15u), scale), sum);
+            }
+        }
+    return sum;
+}
+
 // One lane's four words of scales (K blocks 0..3 of a unit) of a row, from its bytes in the stage.
 template <bool kTable>
 __device__ __forceinline__ uint4 row_scales(const uint8_t* at, const uint4& table) {
@@ -231,6 +335,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
     uint32_t* failed = tmem_holder + 1;
     uint32_t* exponents = failed + 1;        // per row: the largest exponent of the slice
     uint32_t* least = exponents + kMaxRows;  // per row: the least of the largest exponents of eight neighbours
+    uint32_t* left = least + kMaxRows;       // of a row whose digits leave values out, [row][unit of the slice]: bit i: of values 8 i .. 8 i + 7 of the unit
     auto has_outliers = [&](uint32_t row) { return least[row] + kSpread < exponents[row]; };
     const uint32_t kBoxColumns = layout.columns;
 
@@ -409,13 +514,15 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
         const uint32_t divisor = max(mine, 1u), step_rows = kStagers / 32u / divisor, step_units = kStagers / 32u % divisor;
         const Task first_task = {stager / divisor, stager % divisor};
 
+        uint32_t odd_rows = 0u;   // bit m: the digits of row m leave values of the slice out
+
         // The digits of every row of the slice, by the staging warps. Taken by all of them at the same points of the tile list; the
         // draining warps come when every MMA that reads the digits held before is done.
         auto stage_rows = [&](const uint16_t* x, bool again) {
             // 8 values per lane. The first kHold loads of a warp are in flight together while it finds the rows' exponents; the pass
             // that writes the digits finds the values in L1.
             constexpr uint32_t kHold = 4;
-            const uint32_t live = k / 8u - min(k / 8u, unit_begin * 32u);   // eighths of the slice
+            const Slice slice = {x, rows, k, unit_begin, mine, stager, lane, exponents, least, left, smem + layout.off_rows, layout.columns};
             Task at = first_task;
             auto next = [&]() {
                 at.row += step_rows;
@@ -425,28 +532,12 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                     ++at.row;
                 }
             };
-            auto load = [&]() {
-                const uint32_t e = at.unit * 32u + lane;
-                return at.row < rows && e < live ? *reinterpret_cast<const uint4*>(x + (uint64_t)at.row * k + unit_begin * kUnit + e * 8u) : make_uint4(0u, 0u, 0u, 0u);
-            };
-            auto exponent = [](const uint4& v) {
-                const uint32_t most = __vmaxu2(__vmaxu2(v.x & 0x7FFF7FFFu, v.y & 0x7FFF7FFFu), __vmaxu2(v.z & 0x7FFF7FFFu, v.w & 0x7FFF7FFFu));
-                return max(most & 0xFFFFu, most >> 16) >> 7;
-            };
-            auto find = [&](uint32_t row, const uint4& v) {
-                const uint32_t mine_most = exponent(v);   // 0: nothing but zeros (or subnormal values)
-                const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, mine_most), low = __reduce_min_sync(0xFFFFFFFFu, mine_most == 0u ? 255u : mine_most);
-                if (row < rows && lane == 0) {
-                    atomicMax(&exponents[row], most);
-                    atomicMin(&least[row], low);
-                }
-            };
             if (mine != 0u) {
                 uint4 v[kHold];
                 uint32_t row[kHold];
 #pragma unroll
                 for (uint32_t i = 0; i < kHold; ++i, next()) {
-                    v[i] = load();
+                    v[i] = slice.load(at.row, at.unit);
                     row[i] = at.row;
                 }
                 if (again) {
@@ -455,29 +546,14 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                     stagers_sync();
                 }
 #pragma unroll
-                for (uint32_t i = 0; i < kHold; ++i) find(row[i], v[i]);
+                for (uint32_t i = 0; i < kHold; ++i) slice.find(row[i], v[i]);
 #pragma unroll 1
-                for (; at.row < rows; next()) find(at.row, load());
+                for (; at.row < rows; next()) slice.find(at.row, slice.load(at.row, at.unit));
                 stagers_sync();
+                odd_rows = __ballot_sync(0xFFFFFFFFu, lane < rows && exponents[lane & (kMaxRows - 1u)] == 255u);
 #pragma unroll 1
-                for (at = first_task; at.row < rows; next()) {
-                    const uint4 values = load();
-                    const uint32_t m = at.row, unit = at.unit;
-                    const float per = __uint_as_float((275u - exponents[m]) << 23);
-                    uint8_t* tile = smem + layout.off_rows + unit * layout.columns * 128u + (lane & 3u) * 4u;
-                    const uint32_t passes = has_outliers(m) ? 2u : 1u;
-#pragma unroll 1
-                    for (uint32_t pass = 0; pass < passes; ++pass) {
-                        uint32_t word[8];
-                        octal_digits(values, per, pass != 0u, word);
-                        const uint32_t column = pass == 0u ? m * kDigits : rows * kDigits + m * kMoreDigits;   // of digit 0; rows of 128 bytes, swizzled
-                        uint8_t* to = tile + (column >> 3) * 1024u;
-                        const uint32_t first = column & 7u;   // 0, or 4 for every other row's further digits
-#pragma unroll
-                        for (uint32_t t = 0; t < 8u; ++t)
-                            if (t < kMoreDigits || pass == 0u) *reinterpret_cast<uint32_t*>(to + (first + t) * 128u + (((lane >> 2) ^ (first + t)) << 4)) = word[t];
-                    }
-                }
+                for (at = first_task; at.row < rows; next()) slice.write(at.row, at.unit, slice.load(at.row, at.unit));
+                if (odd_rows != 0u) stage_again(slice, odd_rows);
             }
             fence_async_proxy();
             __syncwarp();
@@ -595,31 +671,44 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                     if (exchange && e >= 2u) wait(&gather_empty[slot], ((e >> 1) - 1u) & 1u);
                     const uint32_t to = peer_gather + slot * slot_bytes, bar = peer_full + slot * 8u;
                     if constexpr (kResident) {
+                        // This thread's sum of row m of the slice, from its eight digits' sums.
+                        auto joined = [&](uint32_t m, const uint32_t* r) {
+                            float sum = __uint_as_float(r[7]);
+#pragma unroll
+                            for (int i = 6; i >= 0; --i) sum = __fmaf_rn(sum, 0.125f, __uint_as_float(r[i]));
+                            if (mine == 0u) sum = 0.0f;
+                            if (has_outliers(m)) {
+                                uint32_t q[4];
+                                tmem_load_4(q, d + rows * kDigits + m * kMoreDigits);
+                                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                                float rest = __uint_as_float(q[3]);
+#pragma unroll
+                                for (int i = 2; i >= 0; --i) rest = __fmaf_rn(rest, 0.125f, __uint_as_float(q[i]));
+                                if (mine != 0u) sum = __fmaf_rn(rest, 2.384185791015625e-07f, sum);   // 2^-22
+                            }
+                            return __fmul_rn(__fadd_rn(sum, sum), __uint_as_float(exponents[m] << 23));
+                        };
 #pragma unroll 1
                         for (uint32_t m = 0; m < rows; m += 2u) {   // two rows at a time (the columns of an odd last one's neighbour exist)
                             uint32_t r[16];
                             tmem_load_16(r, d + m * 8u);
                             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                            for (uint32_t h = 0; h < 2u; ++h) {
-                                float sum = __uint_as_float(r[8 * h + 7]);
-#pragma unroll
-                                for (int i = 6; i >= 0; --i) sum = __fmaf_rn(sum, 0.125f, __uint_as_float(r[8 * h + i]));
-                                if (mine == 0u) sum = 0.0f;
+                            for (uint32_t h = 0; h < 2u; ++h)
                                 if (m + h < rows) {
-                                    if (has_outliers(m + h)) {
-                                        uint32_t q[4];
-                                        tmem_load_4(q, d + rows * kDigits + (m + h) * kMoreDigits);
-                                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                                        float rest = __uint_as_float(q[3]);
-#pragma unroll
-                                        for (int i = 2; i >= 0; --i) rest = __fmaf_rn(rest, 0.125f, __uint_as_float(q[i]));
-                                        if (mine != 0u) sum = __fmaf_rn(rest, 2.384185791015625e-07f, sum);   // 2^-22
-                                    }
-                                    const uint32_t top = exponents[m + h];   // 255: a value of the slice is not finite
-                                    send_f32(to + (m + h) * owned * 4u, __fmul_rn(__fadd_rn(sum, sum), top == 255u ? __uint_as_float(0x7FC00000u) : __uint_as_float(top << 23)), bar);
+                                    const float value = joined(m + h, r + 8u * h);
+                                    if (((odd_rows >> (m + h)) & 1u) == 0u) send_f32(to + (m + h) * owned * 4u, value, bar);
                                 }
-                            }
+                        }
+#pragma unroll 1
+                        for (uint32_t odd = odd_rows; odd != 0u; odd &= odd - 1u) {   // with what their digits leave out
+                            const uint32_t m = (uint32_t)__ffs((int)odd) - 1u;
+                            uint32_t r[8];
+                            tmem_load_8(r, d + m * 8u);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                            const float rest = left_out<kTable>(t, now.tile * kTile + local, m, k, unit_begin, mine, left + m * mine);
+                            __syncwarp();
+                            send_f32(to + m * owned * 4u, __fadd_rn(joined(m, r), rest), bar);
                         }
                     } else {
                         // eight columns of this thread's weight row: both terms' sums added
@@ -769,7 +858,7 @@ struct Plan {
 // smallest (34816 x 5120, 1 row: 24.7 us against 22.6).
 inline bool plan(bool resident, uint32_t rows, uint32_t k, uint32_t split, bool paired, Plan* out) {
     const uint32_t units = units_of(k), units_cta = (units + split - 1u) / split;
-    if (rows == 0u || (resident && rows > kMaxRows)) return false;
+    if (rows == 0u || (resident && (rows > kMaxRows || rows * units_cta > kLeftWords))) return false;
     for (uint32_t stages = kMaxStages; stages >= 3u; --stages)
         for (uint32_t buffers = 2; buffers >= 1u; --buffers) {
             const Layout layout(resident, rows, units_cta, stages, split, paired);
@@ -848,6 +937,7 @@ inline cudaError_t fill_tensor(Tensor* t, const Item& item, uint32_t k, bool tab
     const uint64_t plane = nvfp4n::align256((uint64_t)item.n * (k / 2u)), after = nvfp4n::align256(plane + (uint64_t)item.n * (k / (table ? 32u : 16u)));
     t->codes = *map;
     t->x = static_cast<const uint16_t*>(item.x);
+    t->weights = w;
     t->scales = w + plane;
     t->table = table ? w + after : nullptr;
     t->global = reinterpret_cast<const float*>(w + after + (table ? 16u : 0u));

@@ -54,13 +54,31 @@ def test_edges_and_outliers(dev, n, k):
             assert np.all(np.abs(got - expect) <= np.abs(expect) * 2.0 ** -8 + terms * 2.0 ** -18), (rows, n, k)
 
 
-def test_values_that_are_not_finite(dev):
-    rng = np.random.default_rng(3)
-    n, k = 64, 512
-    blob = OC.nvfp4_quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32))
-    x = random_x(rng, 3, k)
-    clean = run(dev, x, dev.put(blob), n, k, blob.size)
-    x[1, 300] = 0x7F80                                                                 # infinity: the row is not a number, its neighbours stay
-    got = run(dev, x, dev.put(blob), n, k, blob.size)
-    assert np.array_equal(got[[0, 2]], clean[[0, 2]])
-    assert np.all((got[1] & 0x7FFF) > 0x7F80)
+@pytest.mark.parametrize("n,k", [(64, 512), (144, 1152), (272, 5120)])
+@pytest.mark.parametrize("sd4", [False, True])
+def test_values_that_are_not_finite(dev, n, k, sd4):
+    """An infinity gives every output of its row an infinity of the product's sign, NaN where it meets a zero weight or an infinity of
+    the other sign; a NaN makes its row NaN. Rows without such values keep their bits."""
+    rng = np.random.default_rng(n + k)
+    weights = (rng.standard_normal((n, k)) * 0.02).astype(np.float32)
+    weights[::3, 300] = weights[1::5, 17] = 0.0
+    blob = OC.nvfp4_quantize(weights).tobytes()
+    if sd4:
+        blob = O.nvfp4_sd4_from_plain(blob, n, k, rng)
+    dense = O.nvfp4_dense(O.nvfp4_sd4_to_plain(blob, n, k) if sd4 else blob, n, k)
+    d_w = dev.put(np.frombuffer(blob, dtype=np.uint8))
+    x = random_x(rng, 7, k)
+    clean = run(dev, x, d_w, n, k, len(blob))
+    x[1, 300] = 0x7F80
+    x[2, [300, 17]] = 0x7F80, 0xFF80
+    x[3, 17] = 0x7FC0
+    x[4, [0, k - 1]] = 0xFF80
+    x[6, 64:72] = 0x7F80
+    got = run(dev, x, d_w, n, k, len(blob))
+    assert np.array_equal(got[[0, 5]], clean[[0, 5]])
+    with np.errstate(invalid="ignore"):
+        expect = np.stack([(O.bf16_to_f32(row).astype(np.float64) * dense).sum(axis=1) for row in x])
+    special = [1, 2, 3, 4, 6]
+    assert np.isinf(expect[special]).any() and np.isnan(expect[special]).any() and not np.isfinite(expect[special]).any()
+    assert np.array_equal(O.bf16_to_f32(got[special]).astype(np.float64), expect[special], equal_nan=True)
+    assert np.array_equal(run(dev, x[1:2], d_w, n, k, len(blob)), got[1:2])             # and alone
