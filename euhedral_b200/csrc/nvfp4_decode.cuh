@@ -6,10 +6,12 @@
 //     a CTA writes its K slice of every activation row as EIGHT E2M1 terms of three bits each - the octal digits, -4 to 3, of
 //     the value as an integer of 24 bits, in units of 2^-21 of the power of two of the row's largest value of the slice - and a
 //     row becomes eight columns. Products are exact; column t of a row counts 8^-t and the eight sums are added in FP32 once per K
-//     slice. Where some eight neighbours of a row stay below 2^-4 of the slice's largest (outliers), four more columns hold the
-//     next four digits of what the eight cut off: nothing above 2^-33 of the largest value is lost then. The choice is a row's and
-//     slice's own and changes no bit of the rows beside it. Values that are not finite have no digits: the draining warps add their products
-//     in FP32 from the weights in memory, so that an infinity gives every output what IEEE arithmetic gives it.
+//     slice. Every value counts in full. Eight digits hold a BF16 value exactly down to 2^-14 of the power of two of the slice's largest;
+//     where a row has smaller ones, four more columns hold the next four digits, down to 2^-24; what is smaller still (or is below
+//     2^-103 whatever the largest, or not finite) is left out of the digits, and the draining warps add its products in FP32 from the
+//     weights in memory. So an infinity gives every output what IEEE arithmetic gives it. The choice is a row's and slice's own and
+//     changes no bit of the rows beside it. Of 1280 normally distributed values, one slice in eight takes more digits, one in ten
+//     thousand leaves a value out.
 //   * two NVFP4 terms per row, quantized into the scratch before (the native route): a row is one column, both terms accumulate
 //     into it, as in the large GEMM (nvfp4_native.cuh), and more than kMaxColumns rows take a tile of weights several times.
 //     With `pair_rows` a tile is 64 gate rows and the 64 up rows that match them, finished as SwiGLU (the paired region).
@@ -56,9 +58,9 @@ constexpr uint32_t kThreads = 512, kStagers = 320;   // staging warps: 2, 3 and 
 constexpr uint32_t kCodeBytes = kTile * kUnit / 2u, kScaleBytes = kTile * kUnit / 16u;
 constexpr uint32_t kMaxStages = 8;
 constexpr uint32_t kTmemColumns = 512;
-constexpr uint32_t kSpread = 4;           // powers of two that one grid covers (see above)
+constexpr uint32_t kHeldByEight = 14, kHeldByTwelve = 24;   // powers of two below the largest value that the digits hold exactly (see above)
 constexpr uint32_t kLeftWords = 128;      // rows times units of a CTA: more than its shared memory has room for digits of
-constexpr uint32_t kLeastExponent = 48;   // of a row's slice: smaller values keep the grid of 2^-79
+constexpr uint32_t kLeastExponent = 48;   // of a row's slice: the grid does not get finer than that of 2^-79
 
 __host__ __device__ inline uint32_t units_of(uint32_t k) { return (k + kUnit - 1u) / kUnit; }
 // BF16 rows: CTAs of a cluster that share a tile's K, and so the slices that are added in order: a function of K only. More of them
@@ -203,6 +205,21 @@ __device__ __forceinline__ uint32_t largest_exponent(const uint4& v) {
     const uint32_t most = __vmaxu2(__vmaxu2(v.x & 0x7FFF7FFFu, v.y & 0x7FFF7FFFu), __vmaxu2(v.z & 0x7FFF7FFFu, v.w & 0x7FFF7FFFu));
     return max(most & 0xFFFFu, most >> 16) >> 7;
 }
+// The least exponent of the eight, zeros aside (subnormal values: 0). More than 255: nothing but zeros.
+__device__ __forceinline__ uint32_t least_exponent(const uint4& v) {
+    auto less_one = [](uint32_t w) { return ((w & 0x7FFF7FFFu) + 0x7FFF7FFFu) ^ 0x80008000u; };   // both halves' magnitudes; of a zero 65535
+    const uint32_t low = __vminu2(__vminu2(less_one(v.x), less_one(v.y)), __vminu2(less_one(v.z), less_one(v.w)));
+    return (min(low & 0xFFFFu, low >> 16) + 1u) >> 7;
+}
+// What the digits of a BF16 value leave out of it. `per`: 1 / the unit of its row; more: the row has the further digits.
+__device__ __forceinline__ float not_held(uint32_t bits, float per, bool more) {
+    const float x = eb::bf16_bits_to_float(bits), unit = __uint_as_float(0x7F000000u - __float_as_uint(per));
+    const float behind = __fmaf_rn(-__fsub_rn(__fmaf_rn(x, per, 12582912.0f), 12582912.0f), unit, x);
+    // The further digits count that in units of 2^-22 / `per`; of eight digits, the last four (-2340 to 1755) are not kept.
+    const int count = (int)(__float_as_uint(__fmaf_rn(behind, __uint_as_float(__float_as_uint(per) + (22u << 23)), 12582912.0f)) - 0x4B400000u);
+    const float last = __fmaf_rn(-(float)((count + 2340) & ~4095), __uint_as_float(__float_as_uint(unit) - (22u << 23)), behind);
+    return (bits & 0x7F80u) == 0x7F80u ? x : more ? last : behind;
+}
 // Eight BF16 values with zeros in the place of those that are not finite.
 __device__ __forceinline__ uint4 finite_only(const uint4& v) {
     auto word = [](uint32_t w) {
@@ -223,23 +240,24 @@ struct Slice {
         const uint32_t at = (unit_begin + unit) * kUnit + lane * 8u;
         return row < rows && at < k ? *reinterpret_cast<const uint4*>(x + (uint64_t)row * k + at) : make_uint4(0u, 0u, 0u, 0u);
     }
-    __device__ __forceinline__ bool has_outliers(uint32_t row) const { return least[row] + kSpread < exponents[row]; }
+    __device__ __forceinline__ bool has_more(uint32_t row) const { return least[row] + kHeldByEight < exponents[row]; }
     __device__ __forceinline__ void find(uint32_t row, const uint4& v) const {
-        const uint32_t mine = largest_exponent(v);
-        const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, mine), low = __reduce_min_sync(0xFFFFFFFFu, mine == 0u ? 255u : mine);
+        const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, largest_exponent(v)), low = __reduce_min_sync(0xFFFFFFFFu, least_exponent(v));
         if (row < rows && lane == 0) {
             atomicMax(&exponents[row], most);
             atomicMin(&least[row], low);
         }
     }
+    __device__ __forceinline__ float per(uint32_t row) const { return __uint_as_float((275u - exponents[row]) << 23); }   // 1 / the row's unit
+    // Whether the digits of the row leave values out: there are some that are not finite, or too small.
+    __device__ __forceinline__ bool leaves_out(uint32_t row) const { return exponents[row] == 255u || least[row] + kHeldByTwelve < exponents[row]; }
     __device__ __forceinline__ void write(uint32_t row, uint32_t unit, const uint4& values) const {
-        const float per = __uint_as_float((275u - exponents[row]) << 23);
         uint8_t* tile = digits + unit * columns * 128u + (lane & 3u) * 4u;
-        const uint32_t passes = has_outliers(row) ? 2u : 1u;
+        const uint32_t passes = has_more(row) ? 2u : 1u;
 #pragma unroll 1
         for (uint32_t pass = 0; pass < passes; ++pass) {
             uint32_t word[8];
-            octal_digits(values, per, pass != 0u, word);
+            octal_digits(values, per(row), pass != 0u, word);
             const uint32_t column = pass == 0u ? row * kDigits : rows * kDigits + row * kMoreDigits;   // of digit 0; rows of 128 bytes, swizzled
             uint8_t* to = tile + (column >> 3) * 1024u;
             const uint32_t first = column & 7u;   // 0, or 4 for every other row's further digits
@@ -266,36 +284,83 @@ __device__ __forceinline__ void stage_again(const Slice& slice, const uint32_t o
     stagers_sync();
     for_units([&](uint32_t row, uint32_t u) {
         const uint4 values = slice.load(row, u);
-        const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, largest_exponent(values) == 255u);
+        const uint32_t pairs[4] = {values.x, values.y, values.z, values.w};
+        bool some = false;
+#pragma unroll
+        for (uint32_t i = 0; i < 8u; ++i) some = some || not_held((pairs[i >> 1] >> (16u * (i & 1u))) & 0xFFFFu, slice.per(row), slice.has_more(row)) != 0.0f;
+        const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, some);
         if (slice.lane == 0u) slice.left[row * slice.units + u] = lanes;
         slice.write(row, u, finite_only(values));
     });
     stagers_sync();   // the words are there for the draining warps
 }
 
-// What the digits of activation row m leave out of a slice (`left`: its words, one per unit), summed against one weight row in FP32 in
-// K order. The weights are read where they lie: the ring has moved on.
+// What the digits of the odd rows leave out of a slice, summed against one weight row per lane in FP32 in K order: beside[m] of every
+// odd row m. The weights are read where they lie (the ring has moved on), 32 values of K at a time: a lane finds what is left of one
+// of them and all take it from there. The loads of four such parts are in flight together: one at a time took twice as long. Taken by
+// whole warps.
 template <bool kTable>
-__device__ __forceinline__ float left_out(const Tensor& t, uint32_t row, uint32_t m, uint32_t k, uint32_t unit_begin, uint32_t units, const uint32_t* left) {
-    float sum = 0.0f;
-    if (row >= t.n) return sum;
-    const uint32_t* codes = reinterpret_cast<const uint32_t*>(t.weights) + (uint64_t)row * (k / 8u);
-    const uint8_t* scale_codes = t.scales + (uint64_t)row * (k / (kTable ? 32u : 16u));
-#pragma unroll 1
-    for (uint32_t u = 0; u < units; ++u)
-#pragma unroll 1
-        for (uint32_t lanes = left[u]; lanes != 0u; lanes &= lanes - 1u) {
-            const uint32_t eighth = (unit_begin + u) * 32u + (uint32_t)__ffs((int)lanes) - 1u;   // of K
-            const uint4 values = *reinterpret_cast<const uint4*>(t.x + (uint64_t)m * k + eighth * 8u);
-            const uint32_t pairs[4] = {values.x, values.y, values.z, values.w}, word = codes[eighth];
-            const float scale = exact::e4m3(kTable ? t.table[(scale_codes[eighth >> 2] >> ((eighth & 2u) * 2u)) & 15u] : scale_codes[eighth >> 1]);
-#pragma unroll
-            for (uint32_t i = 0; i < 8u; ++i) {
-                const uint32_t bits = (pairs[i >> 1] >> (16u * (i & 1u))) & 0xFFFFu;
-                if ((bits & 0x7F80u) == 0x7F80u) sum = __fmaf_rn(eb::bf16_bits_to_float(bits), __fmul_rn(exact::e2m1((word >> (4u * i)) & 15u), scale), sum);
+__device__ __forceinline__ void left_out(const Tensor& t, const Slice& slice, uint32_t row, uint32_t odd_rows, float (&beside)[kMaxRows]) {
+    row = min(row, t.n - 1u);
+    const uint8_t* codes = t.weights + (uint64_t)row * (slice.k / 2u);
+    const uint8_t* scale_codes = t.scales + (uint64_t)row * (slice.k / (kTable ? 32u : 16u));
+    struct Part {
+        uint32_t m, first, eighths;   // activation row (kMaxRows: there are no more), the first of its 32 values, which eighths of the 32
+    };
+    uint32_t m = 0, u = slice.units, lanes = 0u;
+    auto next = [&]() -> Part {
+        while (lanes == 0u) {
+            if (++u >= slice.units) {
+                if (odd_rows == 0u) return {kMaxRows, 0u, 0u};
+                m = (uint32_t)__ffs((int)odd_rows) - 1u;
+                odd_rows &= odd_rows - 1u;
+                u = 0u;
+                beside[m] = 0.0f;
             }
+            lanes = slice.left[m * slice.units + u];
         }
-    return sum;
+        const uint32_t shift = ((uint32_t)__ffs((int)lanes) - 1u) & ~3u, eighths = (lanes >> shift) & 15u;
+        lanes &= ~(15u << shift);
+        return {m, ((slice.unit_begin + u) * 32u + shift) * 8u, eighths};
+    };
+    constexpr int kParts = 4;
+#pragma unroll 1
+    while (true) {
+        uint32_t of[kParts], scale[kParts];
+        float rest[kParts];
+        uint4 code[kParts];
+        bool some = false;
+#pragma unroll
+        for (int j = 0; j < kParts; ++j) {
+            const Part part = next();
+            of[j] = part.m;
+            if (part.m == kMaxRows) continue;
+            some = true;
+            code[j] = *reinterpret_cast<const uint4*>(codes + part.first / 2u);
+            scale[j] = kTable ? scale_codes[part.first / 32u] : *reinterpret_cast<const uint16_t*>(scale_codes + part.first / 16u);
+            const uint32_t bits = (part.eighths >> (slice.lane >> 3)) & 1u ? t.x[(uint64_t)part.m * slice.k + part.first + slice.lane] : 0u;
+            rest[j] = not_held(bits, slice.per(part.m), slice.has_more(part.m));
+        }
+        if (!some) break;
+#pragma unroll 1
+        for (int turn = 0; turn < kParts && of[0] != kMaxRows; ++turn) {
+            if (kTable) scale[0] = t.table[scale[0] & 15u] | (uint32_t)t.table[scale[0] >> 4] << 8;
+            const uint32_t words[4] = {code[0].x, code[0].y, code[0].z, code[0].w};
+            const float blocks[2] = {exact::e4m3(scale[0] & 0xFFu), exact::e4m3(scale[0] >> 8)};
+            float sum = beside[of[0]];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+                const uint32_t code4 = words[i >> 3] >> (4 * (i & 7));
+                // sign and magnitude where an FP32 number reads them as e2m1 * 2^-126
+                const float weight = __fmul_rn(__uint_as_float((code4 & 8u) << 28 | (code4 & 7u) << 22), 8.507059173023462e37f);
+                sum = __fmaf_rn(__shfl_sync(0xFFFFFFFFu, rest[0], i), __fmul_rn(weight, blocks[i >> 4]), sum);
+            }
+            beside[of[0]] = sum;
+#pragma unroll
+            for (int j = 0; j + 1 < kParts; ++j) of[j] = of[j + 1], scale[j] = scale[j + 1], rest[j] = rest[j + 1], code[j] = code[j + 1];
+            of[kParts - 1] = kMaxRows;
+        }
+    }
 }
 
 // One lane's four words of scales (K blocks 0..3 of a unit) of a row, from its bytes in the stage.
@@ -334,9 +399,9 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(gather_empty + 2);
     uint32_t* failed = tmem_holder + 1;
     uint32_t* exponents = failed + 1;        // per row: the largest exponent of the slice
-    uint32_t* least = exponents + kMaxRows;  // per row: the least of the largest exponents of eight neighbours
+    uint32_t* least = exponents + kMaxRows;  // per row: the least exponent of the slice, zeros aside
     uint32_t* left = least + kMaxRows;       // of a row whose digits leave values out, [row][unit of the slice]: bit i: of values 8 i .. 8 i + 7 of the unit
-    auto has_outliers = [&](uint32_t row) { return least[row] + kSpread < exponents[row]; };
+    auto has_more = [&](uint32_t row) { return least[row] + kHeldByEight < exponents[row]; };   // four more digits
     const uint32_t kBoxColumns = layout.columns;
 
     if (warp == 0) {
@@ -471,7 +536,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
             if (kResident && t.x != held) {
                 held = t.x;
                 wait(staged, stagings++ & 1u);
-                const bool more = __any_sync(0xFFFFFFFFu, lane < rows && has_outliers(min(lane, rows - 1u)));
+                const bool more = __any_sync(0xFFFFFFFFu, lane < rows && has_more(min(lane, rows - 1u)));
                 instruction = instruction_of(more ? layout.n : layout.plain_n);
             }
             const uint32_t buffer = accumulator.stage;
@@ -514,6 +579,9 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
         const uint32_t divisor = max(mine, 1u), step_rows = kStagers / 32u / divisor, step_units = kStagers / 32u % divisor;
         const Task first_task = {stager / divisor, stager % divisor};
 
+        auto slice_of = [&](const uint16_t* x) {
+            return Slice{x, rows, k, unit_begin, mine, stager, lane, exponents, least, left, smem + layout.off_rows, layout.columns};
+        };
         uint32_t odd_rows = 0u;   // bit m: the digits of row m leave values of the slice out
 
         // The digits of every row of the slice, by the staging warps. Taken by all of them at the same points of the tile list; the
@@ -522,7 +590,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
             // 8 values per lane. The first kHold loads of a warp are in flight together while it finds the rows' exponents; the pass
             // that writes the digits finds the values in L1.
             constexpr uint32_t kHold = 4;
-            const Slice slice = {x, rows, k, unit_begin, mine, stager, lane, exponents, least, left, smem + layout.off_rows, layout.columns};
+            const Slice slice = slice_of(x);
             Task at = first_task;
             auto next = [&]() {
                 at.row += step_rows;
@@ -550,7 +618,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
 #pragma unroll 1
                 for (; at.row < rows; next()) slice.find(at.row, slice.load(at.row, at.unit));
                 stagers_sync();
-                odd_rows = __ballot_sync(0xFFFFFFFFu, lane < rows && exponents[lane & (kMaxRows - 1u)] == 255u);
+                odd_rows = __ballot_sync(0xFFFFFFFFu, lane < rows && slice.leaves_out(lane & (kMaxRows - 1u)));
 #pragma unroll 1
                 for (at = first_task; at.row < rows; next()) slice.write(at.row, at.unit, slice.load(at.row, at.unit));
                 if (odd_rows != 0u) stage_again(slice, odd_rows);
@@ -665,6 +733,8 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                         if (dt < width) row_scales[dt] = now.first + dt < rows ? __fmul_rn(group.row_globals[now.first + dt], now.global) : 0.0f;
                         drainers_sync();
                     }
+                    float beside[kMaxRows];   // of the odd rows: what their digits leave out, summed while the tensor core works
+                    if (kResident && odd_rows != 0u) left_out<kTable>(t, slice_of(t.x), now.tile * kTile + local, odd_rows, beside);
                     wait(&acc_full[buffer], use & 1u);
                     nvfp4n::tcgen05_fence_after();
                     const uint32_t d = tmem + lanes + buffer * acc_columns;
@@ -677,7 +747,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
 #pragma unroll
                             for (int i = 6; i >= 0; --i) sum = __fmaf_rn(sum, 0.125f, __uint_as_float(r[i]));
                             if (mine == 0u) sum = 0.0f;
-                            if (has_outliers(m)) {
+                            if (has_more(m)) {
                                 uint32_t q[4];
                                 tmem_load_4(q, d + rows * kDigits + m * kMoreDigits);
                                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -706,9 +776,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                             uint32_t r[8];
                             tmem_load_8(r, d + m * 8u);
                             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                            const float rest = left_out<kTable>(t, now.tile * kTile + local, m, k, unit_begin, mine, left + m * mine);
-                            __syncwarp();
-                            send_f32(to + m * owned * 4u, __fadd_rn(joined(m, r), rest), bar);
+                            send_f32(to + m * owned * 4u, __fadd_rn(joined(m, r), beside[m]), bar);
                         }
                     } else {
                         // eight columns of this thread's weight row: both terms' sums added

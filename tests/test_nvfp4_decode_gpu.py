@@ -54,6 +54,40 @@ def test_edges_and_outliers(dev, n, k):
             assert np.all(np.abs(got - expect) <= np.abs(expect) * 2.0 ** -8 + terms * 2.0 ** -18), (rows, n, k)
 
 
+@pytest.mark.parametrize("n,k", [(48, 384), (160, 5120)])
+@pytest.mark.parametrize("sd4", [False, True])
+def test_every_finite_value_counts(dev, n, k, sd4):
+    """Outputs whose weights are zero wherever the activations are large: what is left must count in full, however far below the
+    row's largest value it lies."""
+    rng = np.random.default_rng(n + k + sd4)
+    x = rng.standard_normal((9, k))
+    x[1, 7] = 2.0 ** 100                                          # one value that no common grid spans with the others
+    x[2] *= 2.0 ** rng.integers(-60, 60, k)                       # all over
+    x[3] *= 2.0 ** -112                                           # next to nothing
+    x[4, : k // 2] *= 2.0 ** -17                                  # two populations inside a slice
+    x[5, ::3] = 0.0
+    x[6] = np.where(np.arange(k) % 97 == 5, 2.0 ** 90, 2.0 ** -90)
+    x[7] = 0.0
+    x[8, ::50] *= 2.0 ** 14
+    x = O.bf16_bits(x.astype(np.float32))
+    values = O.bf16_to_f32(x).astype(np.float64)
+    weights = (rng.standard_normal((n, k)) * 0.02).astype(np.float32)
+    for j in range(n):                                            # weight row j sees the smallest (j + 1) / n of row j % 9
+        size = np.abs(values[j % 9])
+        weights[j, size > np.quantile(size, (j + 1) / n)] = 0.0
+    weights[0, np.argsort(np.abs(values[0]))[3:]] = 0.0           # and the first of them three values
+    blob = OC.nvfp4_quantize(weights).tobytes()
+    if sd4:
+        blob = O.nvfp4_sd4_from_plain(blob, n, k, rng)
+    dense = O.nvfp4_dense(O.nvfp4_sd4_to_plain(blob, n, k) if sd4 else blob, n, k).astype(np.float64)
+    d_w = dev.put(np.frombuffer(blob, dtype=np.uint8))
+    got_bits = run(dev, x, d_w, n, k, len(blob))
+    got, expect, terms = O.bf16_to_f32(got_bits).astype(np.float64), values @ dense.T, np.abs(values) @ np.abs(dense).T
+    assert np.all(np.abs(got - expect) <= np.abs(expect) * 2.0 ** -8 + terms * 2.0 ** -18)   # half a BF16 step and rounded FP32 sums
+    for row in range(9):
+        assert np.array_equal(run(dev, x[row:row + 1], d_w, n, k, len(blob))[0], got_bits[row]), row
+
+
 @pytest.mark.parametrize("n,k", [(64, 512), (144, 1152), (272, 5120)])
 @pytest.mark.parametrize("sd4", [False, True])
 def test_values_that_are_not_finite(dev, n, k, sd4):
