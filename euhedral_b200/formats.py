@@ -108,7 +108,6 @@ class TrellisFormat:
     EPILOGUE_BLOCK_COLUMNS = 512
     FRAGMENT_FP16, COLUMN_BF16, BLOCK_FP8 = 0, 1, 2
     MAX_GRID_ROWS = 65535
-    DECODE_ROWS = 8
 
     def __init__(self, settings: TrellisSettings):
         self.settings = settings
@@ -208,23 +207,7 @@ class _TrellisLaunch:
             KernelArguments().pointer(self.launch.input).pointer(self.suh).pointer(activations).int32(self.rows)
             .int32(self.k).int32(self.segments).int32(layout))
 
-    def one_launch(self, settings: TrellisSettings) -> bool:
-        """Decode-sized launches as one kernel with the library's own split count, in the scratch of the three-launch plan. It
-        wins where the column blocks alone leave SMs idle and K is long enough to be cut (us at one row, three launches -> one:
-        7168 x 5120 21.0 -> 17.7, 5120 x 5120 16.8 -> 13.8, 5120 x 17408 38.5 -> 31.5; at 34816 x 5120 59.6 -> 60.2 and at 1024 x
-        1024 6.1 -> 7.1 it does not). Row-exact launches keep the plan's split count, which is the same for every row count."""
-        if self.launch.row_exact or self.rows > TrellisFormat.DECODE_ROWS or self.k < 2048 or self.n // layouts.TRELLIS_BLOCK * 8 > settings.target_ctas:
-            return False
-        need = self.gpu.lib.euhedral_b200_linear_trellis_scratch_bytes(self.rows, self.k, self.n, self.segments, 0)
-        if self.launch.scratch == 0 or self.launch.scratch_bytes < need:
-            return False
-        self.gpu.linear_trellis_bf16(self.launch.input, self.words, self.suh, self.svh, self.ends, self.launch.output, self.launch.scratch,
-                                     self.launch.scratch_bytes, self.rows, self.k, self.n, self.w, self.segments)
-        return True
-
     def tensor_core(self, settings: TrellisSettings) -> None:
-        if self.one_launch(settings):
-            return
         splits = TrellisFormat.splits(self.k, self.n, settings.target_ctas)
         activations = layouts.align_up(self.segments * self.rows * self.k * 2, layouts.SCRATCH_ALIGNMENT)
         if self.rows >= settings.whole_k_rows:

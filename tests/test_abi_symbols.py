@@ -184,3 +184,37 @@ def test_operators_route_by_row_count(monkeypatch):
     fmt.linear(memory, LinearLaunch(0x5000, 0x6000, handles, 63, 256, 256, scratch=0x7000, scratch_bytes=1 << 20))
     assert "euhedral_b200_prefill_trellis_bf16" not in [name for name, _ in calls]
     assert [name for name, _ in calls].count("euhedral_cuda_linear_launch") >= 2                                      # prepass + mma
+
+
+@pytest.mark.parametrize("k,n,segments", [(2048, 14336, 1), (2560, 8320, 1), (3072, 13696, 1), (4096, 9984, 1), (8192, 5120, 3), (5120, 7168, 3), (1024, 512, 1)])
+def test_trellis_rows_share_one_k_cut(k, n, segments):
+    """The K split count fixes the order of a row's sums, so the operator passes the same one for every row count below the
+    prefill plan's, row-exact or not, in exactly the scratch that scratch_bytes names."""
+    from euhedral_b200 import gpu as G
+    from euhedral_b200.formats import LinearLaunch, TensorHandle, TrellisFormat, TrellisSettings
+    splits = []
+
+    class Recorder:
+        def euhedral_cuda_linear_launch(self, kernel, *rest):
+            if G.LINEAR_KERNELS[kernel] == "TRELLIS_MMA":
+                splits.append(rest[7][10])
+            return 0
+
+        def euhedral_b200_linear_trellis_scratch_bytes(self, *args):
+            return library.load().euhedral_b200_linear_trellis_scratch_bytes(*args)
+
+        def euhedral_b200_linear_trellis_bf16(self, *args):
+            splits.append(args[-1])
+            return 0
+
+    memory = G.CudaGpuMemory.__new__(G.CudaGpuMemory)
+    memory.lib = Recorder()
+    fmt = TrellisFormat(TrellisSettings.for_device(148))
+    handles = [TensorHandle("p", (k // 16, n // 16, 48), 0x1000, k * n * 48 // 128), TensorHandle("suh", (segments, k), 0x2000, segments * k * 2),
+               TensorHandle("svh", (n,), 0x3000, 2 * n), TensorHandle("ends", (segments,), 0x4000, 4 * segments)]
+    for rows in (1, 2, 8, 9, 17, 63):
+        for row_exact in (False, True):
+            assert fmt.row_exact(rows)
+            need = fmt.scratch_bytes(memory, rows, k, n, segments, row_exact=row_exact)
+            fmt.linear(memory, LinearLaunch(0x5000, 0x6000, handles, rows, k, n, scratch=0x7000, scratch_bytes=need, row_exact=row_exact))
+    assert len(splits) == 12 and set(splits) == {TrellisFormat.splits(k, n, 8 * 148)}

@@ -41,12 +41,12 @@ class DeviceLinear:
         shapes = [payload.shape, (len(self.ends), self.k), (self.n,), (len(self.ends),)]
         self.handles = [TensorHandle(f"t{i}", tuple(shape), t.data_ptr(), t.numel()) for i, (t, shape) in enumerate(zip(self.tensors, shapes))]
 
-    def linear(self, x_bits, **select):
+    def linear(self, x_bits, row_exact=True, **select):
         rows = x_bits.shape[0]
-        need = self.format.scratch_bytes(self.dev.gpu, rows, self.k, self.n, len(self.ends))
+        need = self.format.scratch_bytes(self.dev.gpu, rows, self.k, self.n, len(self.ends), row_exact=row_exact)
         d_x, d_y, d_s = self.dev.put(x_bits), self.dev.empty(rows * self.n * 2), self.dev.empty(need)
         launch = LinearLaunch(d_x.data_ptr(), d_y.data_ptr(), self.handles, rows, self.k, self.n, scratch=d_s.data_ptr(),
-                              scratch_bytes=need, row_exact=True)
+                              scratch_bytes=need, row_exact=row_exact)
         with self.dev.submit(**select) as gpu:
             self.format.linear(gpu, launch)
         return self.dev.get(d_y, np.uint16, (rows, self.n))
@@ -193,6 +193,23 @@ def test_rows_are_bitwise_independent(dev):
                 if r < rows:
                     assert np.array_equal(got[r], single[at]), (target, rows, r)
         assert np.array_equal(linear.linear(x[:5], pdl=True), linear.linear(x[:5]))
+
+
+# Verification of drafted tokens compares rows of a call of several with calls of one row: up to 63 rows, row-exact or not, a row has
+# the same bits in the scratch that scratch_bytes names. Shapes with few and with many column blocks, whose K is cut often.
+@pytest.mark.parametrize("n,k,segments", [(7168, 5120, 3), (14336, 2048, 1), (8320, 3072, 1), (5120, 8192, 3), (512, 1024, 2)])
+def test_a_row_has_its_bits_in_every_call(dev, n, k, segments):
+    rng = np.random.default_rng(n + k)
+    ends = [n * (i + 1) // segments // 128 * 128 for i in range(segments)]
+    payload, suh, svh = random_object(rng, k, n, 32, segments=segments)
+    linear = DeviceLinear(dev, payload, suh, svh, ends, 8 * dev.gpu.multiprocessor_count())
+    x = random_x(rng, 63, k)
+    single = {r: linear.linear(x[r:r + 1], row_exact=False, pdl=True)[0] for r in (0, 1, 6, 14, 62)}
+    for row_exact in (False, True):
+        for rows in (1, 2, 7, 8, 9, 17, 63):
+            got = linear.linear(x[:rows], row_exact=row_exact, pdl=True)
+            for r, bits in single.items():
+                assert r >= rows or np.array_equal(got[r], bits), (row_exact, rows, r)
 
 
 def test_scalar_kernel_matches_float64(dev):
