@@ -402,7 +402,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bf16_ge
             }
             nvfp4n::tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0) nvfp4n::signal_rank(&acc_empty[buffer], 0u);   // what it orders are tensor-memory reads
+            if (lane == 0) nvfp4n::signal_rank_relaxed(&acc_empty[buffer], 0u);   // what it orders are tensor-memory reads
             if (!works) continue;
             const Place at = place(item);
             const uint32_t row = (2u * at.tm + rank) * kTileM + quarter * 32u + lane, col = at.out + half * 128u;

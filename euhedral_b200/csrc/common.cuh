@@ -108,6 +108,23 @@ __device__ __forceinline__ void mbar_wait_or_fail(uint64_t* bar, uint32_t parity
     *reinterpret_cast<volatile uint32_t*>(failed) = 1u;
 }
 
+// The same for a barrier that threads of other CTAs of the cluster arrive on to pass shared memory on.
+__device__ __forceinline__ void mbar_wait_cluster_or_fail(uint64_t* bar, uint32_t parity, uint32_t* failed) {
+    for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
+        uint32_t done;
+        asm volatile(
+                "{\n.reg .pred p;\n"
+                "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                "selp.u32 %0, 1, 0, p;\n}"
+                : "=r"(done)
+                : "r"(smem_u32(bar)), "r"(parity)
+                : "memory");
+        if (done != 0u) return;
+        if ((spin & 15u) == 15u && *reinterpret_cast<volatile uint32_t*>(failed) != 0u) return;
+    }
+    *reinterpret_cast<volatile uint32_t*>(failed) = 1u;
+}
+
 // True in one lane of the (converged) warp, the same one every time. A role that one thread plays is written as a loop of the whole
 // warp with the instructions that only one thread may issue under this predicate: control flow and addresses stay uniform, so
 // that they live in uniform registers. Under `if (lane == 0)` every tcgen05.mma cost about 190 cycles to issue.

@@ -875,7 +875,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                     // Everybody has read the buffer: the exchange after the next may fill it. Nobody waits for the last two signals, so
                     // they are not sent: what a CTA is sent it waits for, and no CTA needs to outlive its own last wait.
                     drainers_sync();
-                    if (dt < split && last + 2u < exchanges) nvfp4n::signal_rank(&gather_empty[slot], dt);
+                    if (dt < split && last + 2u < exchanges) nvfp4n::signal_rank_relaxed(&gather_empty[slot], dt);
                 }
             }
         } else if (kResident) {

@@ -587,10 +587,16 @@ __device__ __forceinline__ void pair_commit(uint64_t* bar) {
             "h"((uint16_t)3)
             : "memory");
 }
-// Arrives on the barrier at this shared address in CTA `rank` without a release of ordinary memory: what it signals are completed
-// tensor-memory operations of the thread, which tcgen05.fence::before_thread_sync has ordered. (An arrive with release waits for
-// the thread's stores to be performed, about a microsecond: 420 us instead of 315 us for the GEMM of 4096 x 17408 x 5120.)
+// Arrives on the barrier at this shared address in CTA `rank`; what the thread (and those it has synchronized with) read and wrote
+// before is ordered before what follows a wait for it (eb::mbar_wait_cluster_or_fail).
 __device__ __forceinline__ void signal_rank(uint64_t* bar, uint32_t rank) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(eb::map_to_rank(eb::smem_u32(bar), rank)) : "memory");
+}
+// The same without a release of ordinary memory, for the barriers `scaled` and `acc_empty` only: what they signal are completed
+// tensor-memory operations of the thread, which tcgen05.fence::before_thread_sync has ordered. (An arrive with release waits for the
+// global stores that the epilogue's threads have in flight, about a microsecond: 420 us instead of 315 us for the GEMM of 4096 x
+// 17408 x 5120.)
+__device__ __forceinline__ void signal_rank_relaxed(uint64_t* bar, uint32_t rank) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(eb::map_to_rank(eb::smem_u32(bar), rank)) : "memory");
 }
 
@@ -732,7 +738,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kScaledThreads, 1) g
                 }
                 scales_to_tmem(reinterpret_cast<const uint4*>(smem + s * kPairStageBytes + kPairCodes) + lane,
                         tmem + (((warp & 3u) * 32u) << 16) + kTmemScales + s * kScaleColumns);
-                if (lane == 0) signal_rank(&scaled[s], 0u);
+                if (lane == 0) signal_rank_relaxed(&scaled[s], 0u);
             }
     } else {
         // Epilogue, in both CTAs, each over its own 128 rows: as in gemm_kernel.
@@ -758,7 +764,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kScaledThreads, 1) g
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0) signal_rank(acc_empty, 0u);   // what it orders are tensor-memory reads
+            if (lane == 0) signal_rank_relaxed(acc_empty, 0u);   // what it orders are tensor-memory reads
             const uint32_t row = (2u * tm + rank) * kTileM + quarter * 32u + lane;
             const float scale = row < rows ? __fmul_rn(row_globals[row], scale_w) : 0.0f;
             store_block(r, out, row, rows, n, paired ? tn * 128u + half * 64u : tn * kTileN + half * 128u, scale, paired);

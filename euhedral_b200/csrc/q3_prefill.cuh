@@ -18,6 +18,7 @@
 //   * warps 4..19: codes -> the two BF16 tiles of 64 values (128-byte swizzle), four stages
 //   * warp 0: the activation tile of a stage by TMA, half in each CTA, counted on the even CTA's barrier
 //   * warp 1 of the even CTA: eight MMAs a stage; two accumulators of up to 256 columns
+//   * warps 1 and 3 of the odd CTA: pass on to the even one that the odd half of a stage is made
 //   * warps 20..23: a thread has one output column and walks the tile's rows; in the paired region (a tile holds 64 gate rows and the
 //     64 up rows that match them) the up half meets the gate half in shared memory
 // Every wait is bounded.
@@ -87,7 +88,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) kernel(
             eb::mbar_init(&raw_empty[lane], 16);
         } else if (lane >= 8u && lane < 8u + kStages) {
             eb::mbar_init(&rows_full[lane - 8u], 1);
-            eb::mbar_init(&made[lane - 8u], 16);   // eight converting warps of both CTAs
+            eb::mbar_init(&made[lane - 8u], rank == 0u ? 9 : 8);   // eight converting warps, and word from the odd CTA
             eb::mbar_init(&empty[lane - 8u], 1);
         } else if (lane >= 16u && lane < 18u) {
             eb::mbar_init(&acc_full[lane - 16u], 1);
@@ -106,6 +107,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) kernel(
     nvfp4n::tcgen05_fence_after();
     const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *tmem_holder, 0);
     eb::pdl_launch_dependents();
+
+    // Odd CTA: tells the even one of every second stage that its terms are made. An arrive that releases memory to another CTA takes
+    // several hundred cycles: by the converting warps themselves a layer's linears took 1.4 to 1.8 times as long.
+    auto pass_on = [&](uint32_t odd) {
+        eb::Ring ring;   // of pairs of stages
+        for (uint32_t item = pair; item < items; item += pairs)
+            for (uint32_t c = 0; c < chunks; ++c) {
+                const uint32_t stage = 2u * ring.stage + odd;
+                wait(&made[stage], ring.parity);
+                if (lane == 0u) nvfp4n::signal_rank(&made[stage], 0u);
+                __syncwarp();
+                ring.advance(kStages / 2u);
+            }
+    };
 
     if (warp == 0) {
         const bool leader = eb::elect_one();
@@ -140,7 +155,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) kernel(
                 const uint32_t d = tmem + accumulator.stage * 256u;
                 for (uint32_t ks = 0; ks < stages_item; ++ks) {
                     wait(&rows_full[ring.stage], ring.parity);
-                    wait(&made[ring.stage], ring.parity);
+                    eb::mbar_wait_cluster_or_fail(&made[ring.stage], ring.parity, failed);   // half of the terms are in the other CTA
                     nvfp4n::tcgen05_fence_after();
                     const uint64_t hi = first + (uint64_t)(ring.stage * kStageBytes >> 4), lo = hi + (uint64_t)(kATile >> 4), x = lo + (uint64_t)(kATile >> 4);
                     if (leader) {
@@ -158,7 +173,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) kernel(
                 accumulator.advance(2u);
                 used = used || accumulator.stage == 0u;
             }
+        } else {
+            pass_on(0u);
         }
+    } else if (warp == 3) {
+        if (rank != 0u) pass_on(1u);
     } else if (warp == 2) {
         const bool leader = eb::elect_one();
         eb::Ring ring;
@@ -230,7 +249,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) kernel(
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // what was written is for the tensor core to read
                 __syncwarp();
-                if (lane == 0u) nvfp4n::signal_rank(&made[stage], 0u);
+                if (lane == 0u) eb::mbar_arrive(&made[stage]);
                 ring.advance(kStages / 2u);
                 first_round = first_round && ring.stage != 0u;
             }
@@ -276,7 +295,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) kernel(
             }
             nvfp4n::tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0u) nvfp4n::signal_rank(&acc_empty[accumulator.stage], 0u);
+            if (lane == 0u) nvfp4n::signal_rank_relaxed(&acc_empty[accumulator.stage], 0u);
             accumulator.advance(2u);
         }
     }
