@@ -59,6 +59,9 @@ constexpr uint32_t kCodeBytes = kTile * kUnit / 2u, kScaleBytes = kTile * kUnit 
 constexpr uint32_t kMaxStages = 8;
 constexpr uint32_t kTmemColumns = 512;
 constexpr uint32_t kHeldByEight = 14, kHeldByTwelve = 24;   // powers of two below the largest value that the digits hold exactly (see above)
+// Exchange buffers of a CTA. The word that one may be filled again reaches the other CTAs a microsecond or two after it was read;
+// with two buffers for BF16 rows the draining warps waited for it (34816 x 5120 at one row 26.4 us, now 22.1).
+__host__ __device__ constexpr uint32_t gather_slots(bool resident) { return resident ? 4u : 2u; }
 constexpr uint32_t kLeftWords = 128;      // rows times units of a CTA: more than its shared memory has room for digits of
 constexpr uint32_t kLeastExponent = 48;   // of a row's slice: the grid does not get finer than that of 2^-79
 
@@ -103,12 +106,12 @@ struct Layout {
         plain_n = resident ? (rows * kDigits + 15u) / 16u * 16u : n;   // of rows without outliers: the first eight digits come first
         width = resident ? rows : columns;                           // sums of a weight row and slice that travel together
         pitch = columns + 4u;                                        // quantized rows: floats from row to row of an exchange buffer
-        gather_bytes = resident ? kTile * width * 4u : kTile * pitch * 4u;   // one of the two exchange buffers
+        gather_bytes = resident ? kTile * width * 4u : kTile * pitch * 4u;   // one of the exchange buffers
         stage_bytes = kCodeBytes + kScaleBytes + (resident ? 0u : nvfp4n::kTerms * columns * 128u + nvfp4n::kSfaStage);
         stage_bytes = (stage_bytes + 1023u) & ~1023u;
         off_rows = stages * stage_bytes;                             // resident digits: a tile of `columns` x 128 bytes per unit
         off_gather = off_rows + (resident ? units_cta * columns * 128u : 0u);
-        off_bars = off_gather + (split > 1u ? 2u * gather_bytes : paired ? gather_bytes / 2u : 0u);
+        off_bars = off_gather + (split > 1u ? gather_slots(resident) * gather_bytes : paired ? gather_bytes / 2u : 0u);
         bytes = off_bars + 1024u + 1024u;                            // barriers, the rows' exponents and left-out values or scales; slack to align to 1024
     }
 };
@@ -391,12 +394,13 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
     const uint32_t rank = exchange ? eb::cluster_rank() : 0u, clusters = gridDim.x / split, cluster = blockIdx.x / split;
     const uint32_t run_begin = (uint32_t)((uint64_t)cluster * group.tiles / clusters), run_end = (uint32_t)((uint64_t)(cluster + 1u) * group.tiles / clusters);
     const uint32_t unit_begin = rank * units / split, unit_end = (rank + 1u) * units / split, mine = unit_end - unit_begin;
+    constexpr uint32_t kSlots = gather_slots(kResident);
     const bool paired = !kResident && group.pair_rows != 0u;
     const Layout layout(kResident, rows, (units + split - 1u) / split, stages, split, paired);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + layout.off_bars);
     uint64_t *full = bars, *empty = full + kMaxStages, *scaled = empty + kMaxStages, *acc_full = scaled + kMaxStages, *acc_empty = acc_full + 2,
-             *staged = acc_empty + 2, *gather_full = staged + 1, *gather_empty = gather_full + 2;
-    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(gather_empty + 2);
+             *staged = acc_empty + 2, *gather_full = staged + 1, *gather_empty = gather_full + kSlots, *gather_read = gather_empty + kSlots;
+    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(gather_read + kSlots);
     uint32_t* failed = tmem_holder + 1;
     uint32_t* exponents = failed + 1;        // per row: the largest exponent of the slice
     uint32_t* least = exponents + kMaxRows;  // per row: the least exponent of the slice, zeros aside
@@ -413,8 +417,11 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
             const uint32_t b = lane - 16u;
             eb::mbar_init(&acc_full[b], 1);
             eb::mbar_init(&acc_empty[b], 4);
+        } else if (lane >= 20u && lane < 20u + kSlots) {
+            const uint32_t b = lane - 20u;
             eb::mbar_init(&gather_full[b], 1);
             eb::mbar_init(&gather_empty[b], split);
+            eb::mbar_init(&gather_read[b], 4);
         } else if (lane == 18u) {
             eb::mbar_init(staged, kStagers / 32u);
             *failed = 0u;
@@ -727,7 +734,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                         stage_rows(t.x, held != nullptr);
                         held = t.x;
                     }
-                    const uint32_t buffer = buffers == 2u ? e & 1u : 0u, use = buffers == 2u ? e >> 1 : e, slot = e & 1u;
+                    const uint32_t buffer = buffers == 2u ? e & 1u : 0u, use = buffers == 2u ? e >> 1 : e, slot = e % kSlots;
                     if (!kResident && !exchange) {   // the scales of the item's activation rows
                         drainers_sync();   // those of the item before have been read
                         if (dt < width) row_scales[dt] = now.first + dt < rows ? __fmul_rn(group.row_globals[now.first + dt], now.global) : 0.0f;
@@ -738,7 +745,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                     wait(&acc_full[buffer], use & 1u);
                     nvfp4n::tcgen05_fence_after();
                     const uint32_t d = tmem + lanes + buffer * acc_columns;
-                    if (exchange && e >= 2u) wait(&gather_empty[slot], ((e >> 1) - 1u) & 1u);
+                    if (exchange && e >= kSlots) eb::mbar_wait_cluster_or_fail(&gather_empty[slot], (e / kSlots - 1u) & 1u, failed);
                     const uint32_t to = peer_gather + slot * slot_bytes, bar = peer_full + slot * 8u;
                     if constexpr (kResident) {
                         // This thread's sum of row m of the slice, from its eight digits' sums.
@@ -833,9 +840,9 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                 }
                 if (exchange && e > 0u) {
                     // The slices of the exchange before, added in order; this CTA's share of the outputs.
-                    const uint32_t last = e - 1u, slot = last & 1u;
+                    const uint32_t last = e - 1u, slot = last % kSlots;
                     if (dt == 0u) eb::mbar_arrive_expect_tx(&gather_full[slot], kResident ? slot_bytes : kTile * width * 4u);
-                    wait(&gather_full[slot], (last >> 1) & 1u);
+                    wait(&gather_full[slot], (last / kSlots) & 1u);
                     const float* from = reinterpret_cast<const float*>(smem + layout.off_gather + slot * slot_bytes);
                     const uint32_t row0 = before.tile * (paired ? 64u : kTile) + rank * outputs;
                     if constexpr (kResident) {
@@ -872,17 +879,28 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                             }
                         }
                     }
-                    // Everybody has read the buffer: the exchange after the next may fill it. Nobody waits for the last two signals, so
-                    // they are not sent: what a CTA is sent it waits for, and no CTA needs to outlive its own last wait.
-                    drainers_sync();
-                    if (dt < split && last + 2u < exchanges) nvfp4n::signal_rank_relaxed(&gather_empty[slot], dt);
+                    __syncwarp();
+                    if (lane == 0 && last + kSlots < exchanges) eb::mbar_arrive(&gather_read[slot]);   // warp 2 passes it on
                 }
             }
-        } else if (kResident) {
-            for_tiles([&](const Tensor& t, uint32_t, uint32_t, uint32_t) {
-                if (t.x != held) {
+        } else if (kResident || (warp == 2u && exchange)) {
+            // Warp 2 also tells the cluster which exchange buffers of this CTA may be filled again: the draining warps have read them. An
+            // arrive that releases memory to another CTA waits for the thread's global stores, and the draining warps have some in
+            // flight: by them, 34816 x 5120 at one row took 26.8 us instead of 21.4 without the release. Nobody waits for the last signals, so they
+            // are not sent: what a CTA is sent it waits for, and no CTA needs to outlive its own last wait.
+            const bool passes = warp == 2u && exchange;
+            const uint32_t exchanges = run_end - run_begin;
+            if (passes) eb::cluster_wait();   // the other CTAs' barriers exist
+            for_tiles([&](const Tensor& t, uint32_t, uint32_t e, uint32_t) {
+                if (kResident && t.x != held) {
                     stage_rows(t.x, held != nullptr);
                     held = t.x;
+                }
+                if (passes && e > 0u && e - 1u + kSlots < exchanges) {
+                    const uint32_t last = e - 1u;
+                    wait(&gather_read[last % kSlots], (last / kSlots) & 1u);
+                    if (lane < split) nvfp4n::signal_rank(&gather_empty[last % kSlots], lane);
+                    __syncwarp();
                 }
             });
         }
@@ -892,7 +910,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
     if (*failed != 0u) {   // a wait gave up: stay until the other CTAs of the cluster, which may still write here, are done too
         if (tid == 0) atomicOr(error, 1u);
         if (exchange) {
-            if ((warp < 8u || warp >= 12u)) eb::cluster_wait();   // the draining warps have taken this phase already
+            if (warp != 2u && (warp < 8u || warp >= 12u)) eb::cluster_wait();   // warp 2 and the draining warps have taken this phase already
             __syncwarp();
             eb::cluster_sync();
         }

@@ -19,7 +19,7 @@ def code(path):
 def test_signals_without_release_announce_tensor_memory_only(path):
     text = code(path)
     barriers = set(re.findall(r"signal_rank_relaxed\(&?(\w+)", text)) - {"uint64_t"}
-    assert barriers <= TENSOR_MEMORY | ALLOWED.get(path.name, set()), barriers
+    assert barriers <= TENSOR_MEMORY, barriers
     # one place issues the relaxed arrive; everything else goes through the two named functions
     assert text.count("mbarrier.arrive.relaxed") == (1 if path.name == "nvfp4_native.cuh" else 0)
 
@@ -31,4 +31,6 @@ def test_the_q3_terms_are_released_to_the_even_cta():
     assert native.count("mbarrier.arrive.release.cluster") == 1
 
 
-ALLOWED = {"nvfp4_decode.cuh": {"gather_empty"}}
+def test_the_exchange_buffers_are_released_after_they_were_read():
+    text = code(next(path for path in SOURCES if path.name == "nvfp4_decode.cuh"))
+    assert "signal_rank(&gather_empty[" in text and "mbar_wait_cluster_or_fail(&gather_empty[" in text
