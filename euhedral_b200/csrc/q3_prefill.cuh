@@ -14,7 +14,8 @@
 //
 // The weights are the M operand (256 rows on a CTA pair, tcgen05 cta_group::2, 128 in each CTA), the activation rows the N operand, so
 // that a call of any row count is cut into equal tiles of up to 256 rows (a multiple of 16) with next to no padding.
-//   * warp 2: raw codes of 128 values (48 bytes a row) by TMA, their two scales a row by cp.async, three slots
+//   * warp 2: raw codes of 128 values (48 bytes a row) by TMA, their two scales a row by cp.async, three slots. Tensor maps address
+//     device memory only: codes that lie elsewhere (host-mapped, managed) come by cp.async as the scales do.
 //   * warps 4..19: codes -> the two BF16 tiles of 64 values (128-byte swizzle), four stages
 //   * warp 0: the activation tile of a stage by TMA, half in each CTA, counted on the even CTA's barrier
 //   * warp 1 of the even CTA: eight MMAs a stage; two accumulators of up to 256 columns
@@ -58,10 +59,10 @@ __device__ __forceinline__ void sts_v4(uint32_t to, uint32_t a, uint32_t b, uint
 __device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 //   grid 2 x pairs, cluster 2, block kThreads, dynamic shared kSharedBytes. map_x: activations [rows][k] BF16, box 64 x tile / 2;
-//   map_w: codes [weight_rows][k * 3 / 32] 32-bit, box 12 x 64. tile: activation rows of an item. gate_rows != 0: the paired region
+//   map_w: codes [weight_rows][k * 3 / 32] 32-bit, box 12 x 64, used when `codes` (the same plane) is null. tile: activation rows of an item. gate_rows != 0: the paired region
 //   (the output has gate_rows columns), else the output has weight_rows columns.
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ CUtensorMap map_x,
-        const __grid_constant__ CUtensorMap map_w, const uint8_t* __restrict__ scales, uint16_t* __restrict__ out, uint32_t rows, uint32_t weight_rows,
+        const __grid_constant__ CUtensorMap map_w, const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales, uint16_t* __restrict__ out, uint32_t rows, uint32_t weight_rows,
         uint32_t k, uint32_t tile, uint32_t gate_rows, uint32_t* __restrict__ error) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
@@ -187,16 +188,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) kernel(
             const uint32_t low = first_column(item), high = paired ? gate_rows + low : low + 64u;   // first weight rows of the tile's halves
             const uint8_t* from[4];
             bool live[4];
+            auto weight_row = [&](uint32_t j) { return (j < 2u ? low : high - 64u) + j * 32u + lane; };
 #pragma unroll
             for (uint32_t j = 0; j < 4u; ++j) {
-                const uint32_t row = (j < 2u ? low : high - 64u) + j * 32u + lane;
-                live[j] = row < weight_rows;
-                from[j] = scales + (uint64_t)(live[j] ? row : 0u) * pitch;
+                live[j] = weight_row(j) < weight_rows;
+                from[j] = scales + (uint64_t)(live[j] ? weight_row(j) : 0u) * pitch;
             }
             for (uint32_t c = 0; c < chunks; ++c) {
                 if (!first_round) wait(&raw_empty[ring.stage], ring.parity ^ 1u);
                 uint8_t* slot = smem + kOffRaw + ring.stage * kRawBytes;
-                if (leader) {
+                if (codes != nullptr) {
+#pragma unroll 1
+                    for (uint32_t j = 0; j < 4u; ++j) {
+                        const uint8_t* row = codes + (uint64_t)(live[j] ? weight_row(j) : 0u) * (chunks * 48u) + c * 48u;
+                        for (uint32_t i = 0; i < 48u; i += 16u)
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(eb::smem_u32(slot) + (j * 32u + lane) * 48u + i), "l"(row + i),
+                                    "r"(live[j] ? 16 : 0)
+                                    : "memory");
+                    }
+                    if (leader) eb::mbar_arrive(&raw_full[ring.stage]);
+                } else if (leader) {
                     eb::mbar_arrive_expect_tx(&raw_full[ring.stage], kRawCodes);
                     eb::tma_load_2d(slot, &map_w, (int)(c * 12u), (int)low, &raw_full[ring.stage]);
                     eb::tma_load_2d(slot + kRawCodes / 2u, &map_w, (int)(c * 12u), (int)high, &raw_full[ring.stage]);
@@ -326,7 +337,8 @@ inline uint32_t tile_of(uint32_t rows, uint32_t weight_tiles, uint32_t pairs) {
     return best;
 }
 
-// x [rows][k] BF16, w a Q3G64_F16S tensor of weight_rows rows; all 16-byte aligned device memory, k % 128 == 0, weight_rows % 128 == 0.
+// x [rows][k] BF16, w a Q3G64_F16S tensor of weight_rows rows; all 16-byte aligned, k % 128 == 0, weight_rows % 128 == 0. x and out are
+// device memory, w any memory that the device can read.
 // paired: w is a gate/up object (gate rows first), the output [rows][weight_rows / 2] SwiGLU values.
 inline cudaError_t linear(const void* x, const void* w, void* out, uint32_t rows, uint32_t k, uint32_t weight_rows, bool paired, int sms, cudaStream_t stream,
         bool pdl, uint32_t* error) {
@@ -335,19 +347,23 @@ inline cudaError_t linear(const void* x, const void* w, void* out, uint32_t rows
     const q3::Geometry geo(weight_rows, k);
     const uint32_t gate_rows = paired ? weight_rows / 2u : 0u, columns = paired ? gate_rows : weight_rows, span = paired ? 128u : 256u;
     const uint32_t weight_tiles = (columns + span - 1u) / span, most = (uint32_t)sms / 2u, tile = tile_of(rows, weight_tiles, most);
+    cudaPointerAttributes attributes;
+    const bool device_memory = cudaPointerGetAttributes(&attributes, w) == cudaSuccess && attributes.type == cudaMemoryTypeDevice;
+    (void)cudaGetLastError();
     CUtensorMap map_x, map_w;
     const cuuint32_t ones[2] = {1u, 1u}, x_box[2] = {64u, tile / 2u}, w_box[2] = {12u, 64u};
     const cuuint64_t x_dims[2] = {k, rows}, x_strides[1] = {(cuuint64_t)k * 2u}, w_dims[2] = {geo.row_bytes / 4u, weight_rows}, w_strides[1] = {geo.row_bytes};
     if (encode(&map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x), x_dims, x_strides, x_box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
                     != CUDA_SUCCESS
-            || encode(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(w), w_dims, w_strides, w_box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            || (device_memory && encode(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(w), w_dims, w_strides, w_box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
-                    != CUDA_SUCCESS)
+                    != CUDA_SUCCESS))
         return cudaErrorInvalidValue;
+    if (!device_memory) map_w = map_x;
     const uint32_t items = weight_tiles * ((rows + tile - 1u) / tile);
     return eb::launch_on(stream, pdl, 1u, kernel, dim3(2u * std::min(most, items)), dim3(kThreads), kSharedBytes, map_x, map_w,
-            static_cast<const uint8_t*>(w) + geo.scale_offset, static_cast<uint16_t*>(out), rows, weight_rows, k, tile, gate_rows, error);
+            device_memory ? nullptr : static_cast<const uint8_t*>(w), static_cast<const uint8_t*>(w) + geo.scale_offset, static_cast<uint16_t*>(out), rows, weight_rows, k, tile, gate_rows, error);
 }
 
 }  // namespace q3p

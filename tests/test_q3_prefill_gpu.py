@@ -89,6 +89,36 @@ def test_gate_up_swiglu(dev):
     assert np.all(np.abs(O.bf16_to_f32(got).astype(np.float64) - expect) <= 2.0 ** -7 * np.abs(expect) + 1e-30)
 
 
+def test_weights_outside_device_memory(dev):
+    """Weights in pinned host memory are not given to a tensor map: their codes come by plain copies, the results are the same."""
+    import ctypes as C
+    rng = np.random.default_rng(61)
+    lib = dev.gpu.lib
+    k, n = 384, 384
+    blob, _ = random_tensor(rng, n, k)
+    host = lib.euhedral_cuda_host_malloc(blob.size)
+    assert host
+    try:
+        C.memmove(host, blob.ctypes.data, blob.size)
+        for rows in (33, 300):
+            x = random_x(rng, rows, k)
+            d_x, d_y, d_s = dev.put(x), dev.empty(rows * n * 2), dev.empty(lib.euhedral_cuda_q3_mx_scratch_bytes(rows, k, n))
+            with dev.submit(pdl=True) as gpu:
+                gpu.linear_q3_bf16(d_x.data_ptr(), host, d_y.data_ptr(), rows, k, n, blob.size)
+            assert np.array_equal(dev.get(d_y, np.uint16, (rows, n)), prefill(dev, x, blob, n, k)), rows
+            pairs = 256                                       # the first 256 weight rows as a gate/up object
+            part, _ = slice_rows(blob, n, k, 0, pairs)
+            C.memmove(host, part.ctypes.data, part.size)
+            with dev.submit():
+                assert lib.euhedral_cuda_q3_mx_gate_up_swiglu_bf16(d_x.data_ptr(), host, d_y.data_ptr(), d_s.data_ptr(), rows, k, pairs, part.size,
+                                                                   d_s.numel()) == 0
+            assert np.array_equal(dev.get(d_y, np.uint16, (rows, pairs // 2)), prefill(dev, x, part, pairs, k, paired=True)), rows
+            C.memmove(host, blob.ctypes.data, blob.size)
+    finally:
+        dev.torch.cuda.synchronize()
+        lib.euhedral_cuda_host_free(host)
+
+
 def test_statuses(dev):
     lib = dev.gpu.lib
     rng = np.random.default_rng(1)
