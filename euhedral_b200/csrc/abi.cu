@@ -698,8 +698,8 @@ int euhedral_cuda_linear_q3_reference_bf16(const void* input, const void* weight
 // The reference's entry points for Q3 linears of 9 rows and more (native/include/euhedral_cuda.h:173-197; its kernels run
 // block-scaled FP8 MMAs of sm_12x on two-term E4M3 activations). Here the operands are exact the other way round: every weight
 // code * f32(scale) is two BF16 terms whose sum is the weight exactly, made on their way into the tensor core's tiles (q3_prefill.cuh);
-// both multiply the unchanged BF16 activations: sums of exact products, rounded once to BF16, as the reference's route gives. The
-// scratch, which an earlier form of this route filled with the terms, is asked for and checked as before and not used.
+// both multiply the unchanged BF16 activations: sums of exact products, rounded once to BF16, as the reference's route gives.
+// Nothing is kept in the scratch. Its size is not 0 because the entry points take none (null) as an error, as the reference's do.
 constexpr uint32_t kQ3PrefillMinRows = 33;
 
 int euhedral_cuda_q3_mx_available(void) {
@@ -708,8 +708,8 @@ int euhedral_cuda_q3_mx_available(void) {
 }
 
 uint64_t euhedral_cuda_q3_mx_scratch_bytes(uint32_t rows, uint32_t width, uint32_t weight_rows) {
-    (void)rows;   // the activations are read where they are
-    return ((uint64_t)weight_rows * width * 4u + 255u) & ~(uint64_t)255u;
+    (void)rows, (void)width, (void)weight_rows;
+    return 256u;
 }
 
 // No K split on this route: the summation order is the K order whatever the tensor's rows.

@@ -130,8 +130,8 @@ def test_statuses(dev):
     d = dev.empty(1 << 20)
     p = d.data_ptr()
     assert lib.euhedral_cuda_linear_q3_mx_bf16(p, p, p, p, 40, 128, 128, blob.size - 1, 1 << 20) == -3      # not the tensor's size
-    assert lib.euhedral_cuda_linear_q3_mx_bf16(p, p, p, p, 40, 128, 128, blob.size, 1024) == -2             # scratch too small
-    assert lib.euhedral_cuda_q3_mx_scratch_bytes(9, 128, 128) == 128 * 128 * 4
+    assert lib.euhedral_cuda_linear_q3_mx_bf16(p, p, p, p, 40, 128, 128, blob.size, 128) == -2             # scratch too small
+    assert lib.euhedral_cuda_q3_mx_scratch_bytes(9, 128, 128) == 256
     small, _ = random_tensor(rng, 64, 128)
     assert lib.euhedral_cuda_linear_q3_mx_bf16(p, p, p, p, 40, 128, 64, small.size, 1 << 20) == -5          # weight rows not a multiple of 128
     previous = lib.euhedral_cuda_select_exact_numerics(1)
