@@ -66,12 +66,8 @@ constexpr uint32_t kPanel = 8u;                            // tile columns per p
 __host__ __device__ inline uint64_t align256(uint64_t v) { return (v + 255ull) & ~255ull; }
 
 // Caller scratch of one native linear.
-// Callers of at most kSkinnyRows rows are asked for room for kMaxSplits FP32 copies of the output behind it, which no kernel here
-// uses any more: the size is part of what callers were told.
-constexpr uint32_t kSkinnyRows = 64, kMaxSplits = 8;
-
 struct ActivationLayout {
-    uint64_t sfa_offset, global_offset, sfb_offset, partial_offset, bytes;
+    uint64_t sfa_offset, global_offset, sfb_offset, bytes;
     uint32_t row_tiles, k_blocks;
     __host__ __device__ ActivationLayout(uint32_t rows, uint32_t k, uint32_t out_features = 0) {
         const uint64_t kp = ((uint64_t)k + 127u) / 128u * 128u;
@@ -81,8 +77,7 @@ struct ActivationLayout {
         global_offset = align256(sfa_offset + (uint64_t)row_tiles * k_blocks * kTerms * kAtom);
         sfb_offset = align256(global_offset + 4ull * rows);
         const uint64_t n128 = ((uint64_t)out_features + 255u) / 256u * 2u;
-        partial_offset = align256(sfb_offset + n128 * k_blocks * kAtom);
-        bytes = rows <= kSkinnyRows && out_features != 0u ? partial_offset + (uint64_t)kMaxSplits * rows * out_features * 4u : partial_offset;
+        bytes = align256(sfb_offset + n128 * k_blocks * kAtom);
     }
 };
 
