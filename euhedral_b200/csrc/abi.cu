@@ -466,10 +466,6 @@ cudaError_t launch_trellis_finish(const void* partials, int splits, const void* 
 
 // Several decode linears that share K and the row count (the q, k and v projections of a layer, or gate and up) as ONE
 // launch per 8 tensors. Every output is bit for bit what the single-tensor entry point gives.
-struct Nvfp4Cut {   // for euhedral_b200_decode_plan
-    static constexpr uint32_t kPieceChunks = 3, kMaxPiece = 4;
-};
-
 enum class DecodeFormat { kQ3, kNvfp4, kNvfp4Table };
 
 template <DecodeFormat kFormat>
@@ -1180,11 +1176,11 @@ int euhedral_b200_decode_plan(int format, uint32_t rows, uint32_t in_features, u
     DecodePlan plan;
     const uint32_t tiles = out_features / 16u;
     if (format == 0) {
-        // The slices and pieces by which a register decode would cut K; the launch is nvfp4_decode.cuh's.
         nvfp4d::Plan launch;
-        plan.order = gemv::order_of<Nvfp4Cut>(in_features);
-        if (!plan.order.ok || !nvfp4d::plan_rows(rows, in_features, &launch)) return EUHEDRAL_CUDA_INVALID_ARGUMENT;
-        plan.ctas = std::min((uint32_t)sms / plan.order.split, std::max(1u, out_features / nvfp4d::kTile)) * plan.order.split;
+        if (in_features == 0 || !nvfp4d::plan_rows(rows, in_features, &launch)) return EUHEDRAL_CUDA_INVALID_ARGUMENT;
+        const uint32_t resident = nvfp4d::most_clusters(true, false, launch, sms), units = nvfp4d::units_of(in_features);
+        plan.order = {in_features / 128u, launch.split, 1u, (units + launch.split - 1u) / launch.split * (nvfp4d::kUnit / 128u), true};
+        plan.ctas = std::min(resident != 0u ? resident : (uint32_t)sms / launch.split, (out_features + nvfp4d::kTile - 1u) / nvfp4d::kTile) * launch.split;
         plan.shared = launch.shared;
     } else if (!plan_decode<q3::Format>(rows, in_features, tiles, tiles, sms, &plan)) {
         return EUHEDRAL_CUDA_INVALID_ARGUMENT;

@@ -1032,6 +1032,12 @@ inline cudaError_t fill_tensor(Tensor* t, const Item& item, uint32_t k, bool tab
     return cudaSuccess;
 }
 
+// Clusters that the current device holds at once, at most the SMs' number of CTAs. 0: none, or there is no device.
+inline uint32_t most_clusters(bool resident, bool table, const Plan& p, int sms) {
+    const uint32_t most = (uint32_t)sms / p.split;
+    return p.split == 1u ? most : std::min(most, eb::resident_clusters(reinterpret_cast<const void*>(kernel_of(resident, table)), kThreads, p.shared, p.split));
+}
+
 inline cudaError_t launch(bool resident, bool table, Group* group, const Plan& p, int sms, cudaStream_t stream, bool pdl, uint32_t* error) {
     group->stages = p.stages;
     group->split = p.split;
@@ -1039,8 +1045,7 @@ inline cudaError_t launch(bool resident, bool table, Group* group, const Plan& p
     group->buffers = p.buffers;
     group->scale_row_bytes = group->k / (table ? 32u : 16u);
     const Kernel kernel = kernel_of(resident, table);
-    uint32_t most = (uint32_t)sms / p.split;
-    if (p.split > 1u) most = std::min(most, eb::resident_clusters(reinterpret_cast<const void*>(kernel), kThreads, p.shared, p.split));
+    const uint32_t most = most_clusters(resident, table, p, sms);
     if (most == 0u) return cudaErrorInvalidConfiguration;
     const uint32_t clusters = std::min(most, group->tiles);
     return eb::launch_on(stream, pdl, p.split, kernel, dim3(clusters * p.split), dim3(kThreads), p.shared, *group, error);

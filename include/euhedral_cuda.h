@@ -110,11 +110,10 @@ EUHEDRAL_CUDA_EXPORT int euhedral_cuda_linear_launch(int32_t kernel, uint32_t gr
  * (bit 0 NVFP4 GEMV, bit 1 Q3 GEMV, bit 2 trellis GEMM, bit 3 NVFP4 prefill GEMM, bit 4 the BF16 GEMM of the Q3 and trellis
  * prefill). Synchronizes the device. */
 EUHEDRAL_CUDA_EXPORT int euhedral_b200_take_device_error(uint32_t* word);
-/* How a decode GEMV of this shape runs. k_slices (cluster size), pieces (warps that share a 16-row tile's slice) and
- * piece_chunks (128-value chunks of the widest piece) depend on the format and in_features only and fix the summation
- * order; ctas and shared_bytes are the launch for `rows` activation rows. format: 0 NVFP4, 1 Q3. For NVFP4, whose kernel lets
- * the tensor core sum its slices, k_slices, pieces and piece_chunks are the cut of a decode through registers and say nothing
- * about the launch. Returns 0, or -1 for a shape the decode kernels do not take. */
+/* How a decode GEMV of this shape runs. k_slices (cluster size), pieces of a slice (Q3: warps that share a 16-row tile; NVFP4: 1,
+ * the tensor core sums a slice in one run) and piece_chunks (128-value chunks of the widest piece) depend on the format and
+ * in_features only and fix the summation order; ctas and shared_bytes are the launch for `rows` activation rows. format: 0 NVFP4
+ * (up to 16 rows a launch), 1 Q3 (up to 8). Returns 0, or -1 for a shape the decode kernels do not take. */
 EUHEDRAL_CUDA_EXPORT int euhedral_b200_decode_plan(int format, uint32_t rows, uint32_t in_features, uint32_t out_features,
         uint32_t* k_slices, uint32_t* pieces, uint32_t* piece_chunks, uint32_t* ctas, uint32_t* shared_bytes);
 

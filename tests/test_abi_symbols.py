@@ -58,14 +58,13 @@ def test_decode_plans_depend_on_k_only_for_the_summation_order():
     for n in (128, 640, 1024, 5120, 17408):
         for rows in (1, 5, 8):
             for fmt in ("nvfp4", "q3"):
-                if (fmt, rows) == ("nvfp4", 8):
-                    continue   # 8 rows of K = 5120 do not fit beside the NVFP4 rings: such a call runs as two groups of 4
                 plan = library.decode_plan(fmt, rows, 5120, n)
                 plans.setdefault(fmt, set()).add((plan["k_slices"], plan["pieces"], plan["piece_chunks"]))
                 assert plan["ctas"] % plan["k_slices"] == 0 and 1 <= plan["ctas"] <= 148
                 assert plan["shared_bytes"] <= 227 * 1024
     assert all(len(v) == 1 for v in plans.values())      # a row's K order is the same whatever the shard's N and the row count
-    assert library.decode_plan("nvfp4", 1, 17408, 5120)["k_slices"] == 4
+    assert library.decode_plan("nvfp4", 1, 17408, 5120)["k_slices"] == 8
+    assert library.decode_plan("nvfp4", 16, 5120, 17408)["k_slices"] == 4
     assert library.decode_plan("q3", 3, 5120, 17408)["k_slices"] == 1
     with pytest.raises(ValueError):
         library.decode_plan("nvfp4", 1, 100, 16)
@@ -104,7 +103,11 @@ def test_decode_plans_stay_launchable_and_cut_k_by_k_alone():
                 assert plan["k_slices"] in (1, 2, 4, 8) and plan["pieces"] in (1, 2, 4, 8, 16)
                 chunks = k // 128
                 assert plan["pieces"] * plan["piece_chunks"] * plan["k_slices"] >= chunks
-                assert plan["piece_chunks"] <= (4 if fmt == "nvfp4" else 5)
+                if fmt == "q3":
+                    assert plan["piece_chunks"] <= 5
+                else:   # whole units of 256 values, as even as they go; the last may be half
+                    assert plan["pieces"] == 1 and plan["piece_chunks"] == 2 * -(-(-(-chunks // 2)) // plan["k_slices"])
+                    assert plan["ctas"] <= plan["k_slices"] * -(-n // 128)
                 assert plan["shared_bytes"] <= 227 * 1024
                 cut = (plan["k_slices"], plan["pieces"], plan["piece_chunks"])
                 assert cuts.setdefault((fmt, k), cut) == cut
