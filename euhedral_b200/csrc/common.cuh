@@ -50,9 +50,6 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_at(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     uint32_t done;
     asm volatile(
@@ -178,15 +175,6 @@ __device__ __forceinline__ void tma_load_2d_at(uint32_t dst, const CUtensorMap* 
 }
 
 // ---- cp.async (LDGSTS) for pieces too small or too misaligned for a bulk copy ------------------------------------
-__device__ __forceinline__ void cp_async_4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_8(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 // Waits until at most N of this thread's most recent groups are still in flight.
@@ -196,21 +184,12 @@ __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.w
 __device__ __forceinline__ void cp_async_4_to(uint32_t dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async_8_to(uint32_t dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
-}
 
 // ---- shared-memory loads by 32-bit shared address plus a compile-time byte offset (folded into the instruction) -------
 template <int OFFSET>
 __device__ __forceinline__ uint32_t lds_u32(uint32_t address) {
     uint32_t v;
     asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(address), "n"(OFFSET));
-    return v;
-}
-template <int OFFSET>
-__device__ __forceinline__ uint32_t lds_u16(uint32_t address) {
-    uint16_t v;
-    asm volatile("ld.shared.u16 %0, [%1+%2];" : "=h"(v) : "r"(address), "n"(OFFSET));
     return v;
 }
 template <int OFFSET>
@@ -238,11 +217,6 @@ __device__ __forceinline__ uint32_t cluster_rank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
-__device__ __forceinline__ uint32_t cluster_size() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-    return r;
-}
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync() {
@@ -254,23 +228,6 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t local, uint32_t rank) {
     uint32_t remote;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
     return remote;
-}
-// Global loads of weight bytes. Streamed bytes are read once and bypass L1; small pieces that neighbouring chunks share
-// (scales, overlapping code words) keep the default L1 policy.
-__device__ __forceinline__ uint4 ldg_stream_v4(const void* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ uint32_t ldg_u32(const void* p) {
-    uint32_t v;
-    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ uint32_t ldg_u16(const void* p) {
-    uint16_t v;
-    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
-    return v;
 }
 
 __device__ __forceinline__ void st_cluster_f32(uint32_t address, float value) {
@@ -344,7 +301,6 @@ __device__ __forceinline__ void static_for(Body&& body) {
     }
 }
 constexpr int kLutAndXor = 0x6A;     // (a & b) ^ c
-constexpr int kLutAndOr = 0xEA;      // (a & b) | c
 constexpr int kLutSelect = 0xE4;     // (a & c) | (b & ~c)
 
 __device__ __forceinline__ uint32_t bf16x2_mul(uint32_t a, uint32_t b) {

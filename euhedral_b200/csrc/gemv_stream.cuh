@@ -1,4 +1,4 @@
-// The decode GEMV skeleton shared by the NVFP4 and Q3 formats on sm_100a: y[M, N] = x[M, K] . W^T for 1 to 8 BF16
+// The decode GEMV skeleton of the Q3 format on sm_100a: y[M, N] = x[M, K] . W^T for 1 to 8 BF16
 // activation rows, for ONE weight tensor or for a GROUP of tensors that share K and the row count (the q, k, v
 // projections of a layer, or gate and up), all in one persistent launch. The format (byte geometry, activation staging,
 // register decode) is a policy class.
@@ -38,10 +38,8 @@
 //   kErrorBit                       bit of the device error word for a wait that gave up
 //   extra_bytes(chunks)             extra shared bytes next to the activation slice
 //   stage(...)                      CTA-wide staging of the activation slice in the decode's pairing
-//   lane_scale_offset(q)            byte offset of lane q's scales within a chunk's scale bytes
-//   State                           accumulators: tensor(w, geo) at the start of every tensor; chunk<I, W>(codes, scales, x) consumes chunk I of a piece whose box rows
+//   State                           accumulators: chunk<I, W>(codes, scales, x) consumes chunk I of a piece whose box rows
 //                                   are W chunks wide, given the lane's shared addresses; result(out); reset()
-//   Finish(w, geo)                  apply(sum) = the value to round to BF16
 #pragma once
 
 #include "common.cuh"
@@ -175,13 +173,8 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) kernel(const __grid_constan
     const uint32_t slice = slice_end - slice_begin;
     const Layout<F> layout(order, rows, warps, depth, group.span);
     const uint32_t smem_a = eb::smem_u32(smem);
-    // Always true; without the test the compiler gives the loop 126 registers instead of 124 and a layer at one row takes 59.9 us, not 59.2.
-    if (warp < warps) {
-        if (lane == 0) {
-            for (uint32_t s = 0; s < depth; ++s) eb::mbar_init(reinterpret_cast<uint64_t*>(smem + layout.off_bars) + warp * depth + s, 1);
-        }
-    }
-    if (lane == 0) eb::mbar_fence_init();
+    if (lane < depth) eb::mbar_init(reinterpret_cast<uint64_t*>(smem + layout.off_bars) + warp * depth + lane, 1);
+    eb::mbar_fence_init();
     __syncwarp();
     if (split > 1u) eb::cluster_arrive();   // every CTA of the cluster has started before its shared memory is written to
 
@@ -199,7 +192,6 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) kernel(const __grid_constan
     };
     // With K slices: every rank adds the slice sums of the tiles it owns, in rank order. Taken by every thread of the cluster.
     auto join_slices = [&](const Tensor& t, uint32_t first_tile, uint32_t segment_begin, uint32_t segment_end) {
-        const typename F::Finish finish(t.w, typename F::Geometry(t.n, group.k));
         eb::cluster_sync();
         const uint32_t count = segment_end - segment_begin;
         const uint32_t owned = count > rank ? (count - rank + split - 1u) / split : 0u;
@@ -209,7 +201,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) kernel(const __grid_constan
                 const uint32_t from = smem_a + layout.off_gather + local * split * kPartial + rest * 4u;
                 float sum = ld_shared_f(from);
                 for (uint32_t s = 1; s < split; ++s) sum = __fadd_rn(sum, ld_shared_f(from + s * kPartial));
-                t.y[(uint64_t)column * t.n + (segment_begin - first_tile + local * split + rank) * 16u + row] = eb::float_to_bf16_bits(finish.apply(sum));
+                t.y[(uint64_t)column * t.n + (segment_begin - first_tile + local * split + rank) * 16u + row] = eb::float_to_bf16_bits(sum);
             }
         }
         eb::cluster_sync();   // the gather buffers are free for the next tensor
@@ -217,13 +209,13 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) kernel(const __grid_constan
 
     // Adds the T piece sums of a tile in piece order and rounds to BF16 (one slice) or hands the slice sum to the tile's
     // owner rank. The tile's 16 x rows outputs are dealt to the calling threads: `e` from `begin` in steps of `step`.
-    auto add_pieces = [&](const Tensor& t, const typename F::Finish& finish, uint32_t pieces, uint32_t row0, uint32_t local, uint32_t begin, uint32_t step) {
+    auto add_pieces = [&](const Tensor& t, uint32_t pieces, uint32_t row0, uint32_t local, uint32_t begin, uint32_t step) {
         for (uint32_t e = begin; e < 16u * rows; e += step) {
             const uint32_t column = e >> 4, row = e & 15u, at = (row * 8u + column) * 4u;
             float sum = ld_shared_f(pieces + at);
             for (uint32_t j = 1; j < team_size; ++j) sum = __fadd_rn(sum, ld_shared_f(pieces + j * kPartial + at));
             if (split == 1u) {
-                t.y[(uint64_t)column * t.n + row0 + row] = eb::float_to_bf16_bits(finish.apply(sum));
+                t.y[(uint64_t)column * t.n + row0 + row] = eb::float_to_bf16_bits(sum);
             } else {
                 // Tile i of the segment is summed by rank i % S: its gather buffer is [i / S][source rank][row][column].
                 const uint32_t owner = local % split;
@@ -265,10 +257,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) kernel(const __grid_constan
                 const typename F::Geometry geo(t.n, group.k);
                 const uint8_t* from = t.w + geo.scale_offset + (uint64_t)(row + (lane & 15u)) * geo.scale_row_bytes + (uint64_t)piece_begin * F::kScaleBytes;
                 const uint32_t into = to + layout.code_bytes + (lane & 15u) * F::kScaleBox;
-                for (uint32_t c = lane >> 4; c < piece_end - piece_begin; c += 2u) {
-                    if (F::kScaleBytes == 8u) eb::cp_async_8_to(into + c * 8u, from + c * 8u);
-                    else eb::cp_async_4_to(into + c * 4u, from + c * 4u);
-                }
+                for (uint32_t c = lane >> 4; c < piece_end - piece_begin; c += 2u) eb::cp_async_4_to(into + c * 4u, from + c * 4u);
             }
             ask_tile += teams;
             if (++ask_slot == depth) ask_slot = 0;
@@ -285,7 +274,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) kernel(const __grid_constan
     // Lane constants. Lane (g, q) decodes rows g and g + 8 of a tile; its activations are those of row min(g, rows - 1).
     const uint32_t x_lane = eb::pinned(smem_a + (g < rows ? g : rows - 1u) * layout.stride_x + q * 16u + (piece_begin - slice_begin) * 256u);
     const uint32_t code_lane = eb::pinned(g * (uint32_t)P * F::kCodeBytes);
-    const uint32_t scale_lane = eb::pinned(layout.code_bytes + g * F::kScaleBox + scale_rem + F::lane_scale_offset(q));
+    const uint32_t scale_lane = eb::pinned(layout.code_bytes + g * F::kScaleBox + scale_rem);
     const uint32_t extra_lane = smem_a + layout.off_extra + (piece_begin - slice_begin) * (F::extra_bytes(2) - F::extra_bytes(1));
     // This lane's place in its team's two sum buffers: [buffer][member][row of the tile][activation row]; lane (g, q) holds
     // rows g, g + 8 for columns 2q, 2q + 1.
@@ -298,8 +287,6 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) kernel(const __grid_constan
         const uint32_t segment_begin = max(run_begin, first_tile), segment_end = min(run_end, t.tile_end);
         if (segment_begin < segment_end) {   // uniform over the cluster
             stage(t);
-            const typename F::Finish finish(t.w, typename F::Geometry(t.n, group.k));
-            state.tensor(t.w, typename F::Geometry(t.n, group.k));   // what the decode keeps per tensor (a scale table, if the format has one)
             for (; use_tile < segment_end; use_tile += teams, ++turn) {
                 if (!kTmaScales) {
                     if (depth == 2u) eb::cp_async_wait_group<1>();
@@ -324,7 +311,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) kernel(const __grid_constan
                 // The team meets on its named barrier; its threads share the tile's outputs. Two buffers: a warp that runs
                 // ahead writes the other one, and passes the next barrier only after every teammate has finished here.
                 if (team_size > 1u) team_sync(team, team_size * 32u);
-                add_pieces(t, finish, smem_a + layout.off_partials + (team * 2u + buffer) * team_size * kPartial, (use_tile - first_tile) * 16u,
+                add_pieces(t, smem_a + layout.off_partials + (team * 2u + buffer) * team_size * kPartial, (use_tile - first_tile) * 16u,
                         use_tile - segment_begin, tid - team * team_size * 32u, team_size * 32u);
             }
             if (split > 1u) join_slices(t, first_tile, segment_begin, segment_end);

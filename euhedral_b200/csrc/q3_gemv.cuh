@@ -98,7 +98,6 @@ struct Format {
     // float [chunk][group][lane q][4]: minus the biased sum of the group's activations of rows 2q and 2q+1, twice over
     // (x, y, x, y), which is the accumulator quad lane q starts a group with.
     __host__ __device__ static constexpr uint32_t extra_bytes(uint32_t chunks) { return chunks * 128u; }
-    __device__ static uint32_t lane_scale_offset(uint32_t) { return 0; }
 
     // One unit = 16 consecutive activations of one row, (row, chunk, group, quarter): stored in the decode's pairing for
     // the lane quartet that reads it. The four quarters of a group sit in four neighbouring lanes, which add their
@@ -169,7 +168,6 @@ struct Format {
             : bias_lane(eb::pinned(extra + q * 16u)), first_word(eb::pinned(((q >> 1) * 3u + (q & 1u) * 2u) * 4u)),
               second_word(eb::pinned(((q >> 1) * 3u + 1u) * 4u)), select_low(eb::pinned((q & 1u) ? 0x1076u : 0x3210u)),
               select_high(eb::pinned((q & 1u) ? 0x3232u : 0x7654u)) {}
-        __device__ __forceinline__ void tensor(const uint8_t*, const Geometry&) {}   // nothing is kept per tensor
         // codes: shared address of row g of the piece's code box (rows are W chunks wide, row g + 8 eight rows further);
         // scales: of the two FP16 scales of row g and the piece's first chunk (row g + 8: 8 * kScaleBox further);
         // x: of the lane's activations of the piece's first chunk.
@@ -216,11 +214,6 @@ struct Format {
 #pragma unroll
             for (int i = 0; i < 4; ++i) acc[i] = 0.0f;
         }
-    };
-
-    struct Finish {
-        __device__ Finish(const uint8_t*, const Geometry&) {}
-        __device__ __forceinline__ float apply(float sum) const { return sum; }
     };
 };
 
