@@ -185,16 +185,14 @@ def test_model_shapes_at_4096_rows(dev, n, k):
     assert (got[sample] == run(dev, x[sample], blob, n, k)).mean() > 0.97
 
 
-def test_cta_pairs_give_the_single_cta_bits(dev):
-    lib = dev.gpu.lib
+def test_bits_do_not_depend_on_the_row_tile(dev):
+    """A call is cut into equal tiles of activation rows whose height depends on the row count: 512 rows in tiles of 256, and the
+    same rows in calls with tiles of 48, 144, 112, 128 and 176 rows, give the same bits, plain and paired."""
     rng = np.random.default_rng(52)
-    rows, k, n = 700, 384, 768
+    rows, k, n = 512, 256, 37 * 256
     blob, _ = random_tensor(rng, n, k)
     x = random_x(rng, rows, k)
-    pairs, pairs_swiglu = prefill(dev, x, blob, n, k), prefill(dev, x, blob, n, k, paired=True)
-    lib.euhedral_b200_select_bf16_pairs(0)
-    try:
-        assert np.array_equal(prefill(dev, x, blob, n, k), pairs)
-        assert np.array_equal(prefill(dev, x, blob, n, k, paired=True), pairs_swiglu)
-    finally:
-        lib.euhedral_b200_select_bf16_pairs(1)
+    for paired in (False, True):
+        whole = prefill(dev, x, blob, n, k, paired=paired)
+        for first, count in ((0, 33), (100, 130), (312, 200), (256, 256), (11, 350)):
+            assert np.array_equal(prefill(dev, x[first:first + count], blob, n, k, paired=paired), whole[first:first + count]), (paired, first, count)
