@@ -21,11 +21,14 @@
 // Bound: HBM, with about 5 us of launch, staging and exchange around the stream. Per 128 rows x 64 values the weights are 4.6 KB =
 // 200 cycles of an SM's share of the bandwidth; an MMA takes about 110 of them, whatever its columns up to 64. The decode
 // through registers and mma.sync that this replaces was bound by its instruction issue at 0.4 of the bandwidth. Measured, NVFP4,
-// back to back with programmatic dependent launch, before -> now (us at 1 / 5 rows): 34816 x 5120 32.8 / 34.7 -> 20.6 / 24.4 (4.87
-// TB/s at one row); 17408 x 5120 19.2 / 21.1 -> 13.4 / 16.8; 5120 x 17408 22.1 / 25.1 -> 13.4 / 17.1; 5120 x 5120 10.0 / 11.6 -> 8.8 /
-// 11.1. Tensors of a few MB, where the fixed part is not hidden, lose 1.4 to 1.7 us (1024 x 5120: 4.7 / 6.7 -> 6.1 / 8.5): a
-// choice by the number of rows of the weights would give shards and group members other bits than the whole. The native route's few rows: a layer's four fused
-// linears at 40 rows 176 -> 98 us, quantizers included.
+// replayed back to back with programmatic dependent launch, before -> now (us at 1 / 5 / 8 rows): 34816 x 5120 33.6 / 35.7 / 68.3 -> 21.0 /
+// 23.8 / 25.8 (4.8 TB/s at one row); 17408 x 5120 19.6 / 21.5 / 41.0 -> 13.3 / 15.6 / 17.1; 5120 x 17408 22.3 / 25.4 / 46.5 -> 13.7 / 17.4 / 21.2;
+// 5120 x 5120 9.6 / 11.5 / 21.7 -> 8.4 / 10.5 / 11.4. Tensors of a few MB, where the fixed part is not hidden, lose about 1 us up to 5
+// rows (1024 x 5120: 4.1 / 6.2 / 11.0 -> 5.3 / 7.2 / 8.2): a choice by the number of rows of the weights would give shards and group
+// members other bits than the whole. The native route's few rows: a layer's four fused linears at 40 rows 176 -> 90 us, quantizers included.
+// The fixed part is a chain of short pieces of code that every launch fetches anew, so what is rarely needed stands after the loops,
+// a loop runs one copy of its body over values held in registers, and an item's fields are copied before they are needed: together
+// with the digits by table (octal_digits) 1024 x 5120 at 1 / 5 / 8 rows went from 6.0 / 8.6 / 9.8 to 5.3 / 7.2 / 8.2 us.
 // Instructions that one thread issues for the tensor core sit in a loop of the whole warp under an elected predicate (eb::elect_one):
 // 757 -> 453 cycles per unit of 256 values.
 //
@@ -167,40 +170,35 @@ __device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t
 }
 
 // Eight values as eight octal digits each, transposed: word t holds digit t (the highest first) of the eight values as E2M1 codes,
-// value i in nibble i. The values are counted in units of 1 / `per`; `more`: what that count cuts off, in units of 2^-22 / `per`.
-__device__ __forceinline__ void octal_digits(const uint4& v, float per, bool more, uint32_t (&word)[8]) {
+// value i in nibble i. The values are counted in units of 1 / `per`; kMore: what that count cuts off, in units of 2^-22 / `per`.
+template <bool kMore>
+__device__ __forceinline__ void octal_digits(const uint4& v, float per, uint32_t (&word)[8]) {
     const uint32_t pairs[4] = {v.x, v.y, v.z, v.w};
-    const float unit = __uint_as_float(0x7F000000u - __float_as_uint(per)), count = more ? __uint_as_float(__float_as_uint(per) + (22u << 23)) : per;
-    uint32_t a[8];
+    const float unit = __uint_as_float(0x7F000000u - __float_as_uint(per)), count = kMore ? __uint_as_float(__float_as_uint(per) + (22u << 23)) : per;
+    uint32_t low[4], high[4];   // of a pair of neighbouring values, digits 0 to 3 and 4 to 7 (0: the lowest), a byte each
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         float x = (i & 1) ? __uint_as_float(pairs[i >> 1] & 0xFFFF0000u) : __uint_as_float(pairs[i >> 1] << 16);
-        if (more) x = __fmaf_rn(-__fsub_rn(__fmaf_rn(x, per, 12582912.0f), 12582912.0f), unit, x);   // exact
+        if (kMore) x = __fmaf_rn(-__fsub_rn(__fmaf_rn(x, per, 12582912.0f), 12582912.0f), unit, x);   // exact
         // 1.5 * 2^23 + the integer, then + 4 in every octal digit: each digit less 4 is the signed digit
-        const uint32_t n = __float_as_uint(__fmaf_rn(x, count, 12582912.0f)) - 0x4B400000u + 9586980u;
-        uint32_t s = (n & 0x00000FFFu) | ((n << 4) & 0x0FFF0000u);   // 24 bits of octal digits to eight nibbles
-        s = (s & 0x003F003Fu) | ((s << 2) & 0x3F003F00u);
-        s = (s & 0x07070707u) | ((s << 1) & 0x70707070u);
-        const uint32_t negative = (~s >> 2) & 0x11111111u;            // digits 0..3 are -4..-1
-        a[i] = ((s & 0x33333333u) ^ (negative * 3u)) + negative * 9u; // sign and magnitude: E2M1 counts 0, 1, 2, 3, 4 halves
+        uint32_t s = __float_as_uint(__fmaf_rn(x, count, 12582912.0f)) - 0x4B400000u + 9586980u;
+        s += (s & 0x00FFF000u) * 15u;   // 24 bits of octal digits to eight nibbles
+        s += (s & 0x0FC00FC0u) * 3u;
+        s += s & 0x38383838u;
+        // Each nibble selects its E2M1 code from eight bytes: -4 to -1 and 0 to 3 halves, of odd values in the byte's upper half.
+        const uint32_t below = (i & 1) ? 0x90A0B0C0u : 0x090A0B0Cu, above = (i & 1) ? 0x30201000u : 0x03020100u;
+        const uint32_t four = __byte_perm(below, above, s), next = __byte_perm(below, above, s >> 16);
+        low[i >> 1] = (i & 1) ? low[i >> 1] | four : four;
+        high[i >> 1] = (i & 1) ? high[i >> 1] | next : next;
     }
-    // 8 x 8 nibbles across the words: halves, bytes, nibbles
-    uint32_t low[4], high[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        low[i] = __byte_perm(a[i], a[i + 4], 0x5410);
-        high[i] = __byte_perm(a[i], a[i + 4], 0x7632);
-    }
-    auto finish = [&](const uint32_t (&c)[4], int first) {   // c: nibbles first .. first + 3 of every value
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t even = __byte_perm(c[0], c[2], h ? 0x7351 : 0x6240), odd = __byte_perm(c[1], c[3], h ? 0x7351 : 0x6240);
-            word[7 - (first + 2 * h)] = (even & 0x0F0F0F0Fu) | ((odd << 4) & 0xF0F0F0F0u);
-            word[7 - (first + 2 * h + 1)] = ((even >> 4) & 0x0F0F0F0Fu) | (odd & 0xF0F0F0F0u);
-        }
+    auto transposed = [&](const uint32_t (&c)[4], uint32_t* highest) {   // 4 x 4 bytes; the highest digit first
+        const uint32_t a = __byte_perm(c[0], c[1], 0x5140), b = __byte_perm(c[2], c[3], 0x5140);
+        const uint32_t d = __byte_perm(c[0], c[1], 0x7362), e = __byte_perm(c[2], c[3], 0x7362);
+        highest[3] = __byte_perm(a, b, 0x5410), highest[2] = __byte_perm(a, b, 0x7632);
+        highest[1] = __byte_perm(d, e, 0x5410), highest[0] = __byte_perm(d, e, 0x7632);
     };
-    finish(low, 0);
-    finish(high, 4);
+    transposed(high, word);
+    transposed(low, word + 4);
 }
 
 // The largest exponent of eight BF16 values. 0: nothing but zeros (or subnormal values); 255: not all of them are finite.
@@ -255,19 +253,19 @@ struct Slice {
     // Whether the digits of the row leave values out: there are some that are not finite, or too small.
     __device__ __forceinline__ bool leaves_out(uint32_t row) const { return exponents[row] == 255u || least[row] + kHeldByTwelve < exponents[row]; }
     __device__ __forceinline__ void write(uint32_t row, uint32_t unit, const uint4& values) const {
-        uint8_t* tile = digits + unit * columns * 128u + (lane & 3u) * 4u;
-        const uint32_t passes = has_more(row) ? 2u : 1u;
-#pragma unroll 1
-        for (uint32_t pass = 0; pass < passes; ++pass) {
-            uint32_t word[8];
-            octal_digits(values, per(row), pass != 0u, word);
-            const uint32_t column = pass == 0u ? row * kDigits : rows * kDigits + row * kMoreDigits;   // of digit 0; rows of 128 bytes, swizzled
-            uint8_t* to = tile + (column >> 3) * 1024u;
-            const uint32_t first = column & 7u;   // 0, or 4 for every other row's further digits
+        write_digits<false>(row * kDigits, row, unit, values);
+        if (has_more(row)) write_digits<true>(rows * kDigits + row * kMoreDigits, row, unit, values);
+    }
+    // `column`: of digit 0; rows of 128 bytes, swizzled.
+    template <bool kMore>
+    __device__ __forceinline__ void write_digits(uint32_t column, uint32_t row, uint32_t unit, const uint4& values) const {
+        uint32_t word[8];
+        octal_digits<kMore>(values, per(row), word);
+        uint8_t* to = digits + unit * columns * 128u + (column >> 3) * 1024u + (lane & 3u) * 4u;
+        const uint32_t first = kMore ? column & 7u : 0u;   // 4 for every other row's further digits
 #pragma unroll
-            for (uint32_t t = 0; t < 8u; ++t)
-                if (t < kMoreDigits || pass == 0u) *reinterpret_cast<uint32_t*>(to + (first + t) * 128u + (((lane >> 2) ^ (first + t)) << 4)) = word[t];
-        }
+        for (uint32_t t = 0; t < (kMore ? kMoreDigits : kDigits); ++t)
+            *reinterpret_cast<uint32_t*>(to + (first + t) * 128u + (((lane >> 2) ^ (first + t)) << 4)) = word[t];
     }
 };
 
@@ -590,6 +588,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
             return Slice{x, rows, k, unit_begin, mine, stager, lane, exponents, least, left, smem + layout.off_rows, layout.columns};
         };
         uint32_t odd_rows = 0u;   // bit m: the digits of row m leave values of the slice out
+        uint32_t more_rows = 0u;  // or there are further ones
 
         // The digits of every row of the slice, by the staging warps. Taken by all of them at the same points of the tile list; the
         // draining warps come when every MMA that reads the digits held before is done.
@@ -609,26 +608,35 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
             };
             if (mine != 0u) {
                 uint4 v[kHold];
-                uint32_t row[kHold];
 #pragma unroll
-                for (uint32_t i = 0; i < kHold; ++i, next()) {
-                    v[i] = slice.load(at.row, at.unit);
-                    row[i] = at.row;
-                }
+                for (uint32_t i = 0; i < kHold; ++i, next()) v[i] = slice.load(at.row, at.unit);
+                // Task i in v[0] when its turn comes: one copy of the code for all of them.
+                auto turn = [&](const uint4& done) { v[0] = v[1], v[1] = v[2], v[2] = v[3], v[3] = done; };
                 if (again) {
                     stagers_sync();
                     if (stager == 0u && lane < rows) exponents[lane] = kLeastExponent, least[lane] = 255u;
                     stagers_sync();
                 }
-#pragma unroll
-                for (uint32_t i = 0; i < kHold; ++i) slice.find(row[i], v[i]);
+                uint32_t i = 0;
 #pragma unroll 1
-                for (; at.row < rows; next()) slice.find(at.row, slice.load(at.row, at.unit));
+                for (at = first_task; at.row < rows; next(), ++i) {
+                    const uint4 values = i < kHold ? v[0] : slice.load(at.row, at.unit);
+                    slice.find(at.row, values);
+                    turn(values);
+                }
+                const bool held = i <= kHold;
+#pragma unroll 1
+                for (; i < kHold; ++i) turn(v[0]);
                 stagers_sync();
                 odd_rows = __ballot_sync(0xFFFFFFFFu, lane < rows && slice.leaves_out(lane & (kMaxRows - 1u)));
 #pragma unroll 1
-                for (at = first_task; at.row < rows; next()) slice.write(at.row, at.unit, slice.load(at.row, at.unit));
+                for (at = first_task; at.row < rows; next()) {
+                    const uint4 values = held ? v[0] : slice.load(at.row, at.unit);
+                    slice.write(at.row, at.unit, values);
+                    turn(values);
+                }
                 if (odd_rows != 0u) stage_again(slice, odd_rows);
+                more_rows = odd_rows | __ballot_sync(0xFFFFFFFFu, lane < rows && has_more(lane & (kMaxRows - 1u)));
             }
             fence_async_proxy();
             __syncwarp();
@@ -704,15 +712,16 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                     + (kResident ? rank * width * owned + place : (rank * owned + place) * layout.pitch) * 4u;
             const uint32_t peer_full = exchange ? eb::map_to_rank(eb::smem_u32(gather_full), owner) : 0u;
             const uint32_t exchanges = run_end - run_begin;                     // one per item
-            const uint32_t outputs = paired ? half_owned : owned;               // output rows of a tile that this CTA writes
+            const uint32_t outputs = paired ? half_owned : owned;               // output rows of a tile that this CTA writes: a power of two
+            const uint32_t outputs_log = 31u - (uint32_t)__clz((int)outputs);
             const uint32_t out_stride = paired ? group.pair_rows : group.tensor[0].n;   // (quantized rows)
             float* row_scales = reinterpret_cast<float*>(exponents);            // quantized rows: of the item's activation rows
             // The item of exchange e, and the one whose slices are added while it is on its way.
             struct Place {
-                const Tensor* t;
-                uint32_t tile, first;   // the item's tile and first activation row
+                uint16_t* y;
+                uint32_t n, tile, first;   // the item's tile and first activation row
                 float global;
-            } now = {nullptr, 0u, 0u, 0.0f}, before = now;
+            } now = {nullptr, 0u, 0u, 0u, 0.0f}, before = now;   // by value: read through a pointer, they arrive late
             uint32_t ti = 0, tile_first = 0;
             // bf16(silu(gate) * up) of two sums: the reference's expression (native/src/nvfp4_native/native.cuh:390-413)
             auto swiglu = [](float gate_sum, float up_sum) {
@@ -726,7 +735,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                     if (kResident)
                         while (item >= group.tensor[ti].tile_end) tile_first = group.tensor[ti++].tile_end;
                     const Tensor& t = group.tensor[ti];
-                    now.t = &t;
+                    now.y = t.y, now.n = t.n;
                     now.tile = kResident ? item - tile_first : item / group.row_groups;
                     now.first = kResident ? 0u : item % group.row_groups * kMaxColumns;
                     now.global = *t.global;   // requested before the wait for the sums
@@ -748,42 +757,36 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                     if (exchange && e >= kSlots) eb::mbar_wait_cluster_or_fail(&gather_empty[slot], (e / kSlots - 1u) & 1u, failed);
                     const uint32_t to = peer_gather + slot * slot_bytes, bar = peer_full + slot * 8u;
                     if constexpr (kResident) {
-                        // This thread's sum of row m of the slice, from its eight digits' sums.
-                        auto joined = [&](uint32_t m, const uint32_t* r) {
+                        // This thread's sum of a row of the slice from the sums of its eight digits, in units of half the largest value's.
+                        auto joined = [&](const uint32_t* r) {
                             float sum = __uint_as_float(r[7]);
 #pragma unroll
                             for (int i = 6; i >= 0; --i) sum = __fmaf_rn(sum, 0.125f, __uint_as_float(r[i]));
-                            if (mine == 0u) sum = 0.0f;
-                            if (has_more(m)) {
-                                uint32_t q[4];
-                                tmem_load_4(q, d + rows * kDigits + m * kMoreDigits);
-                                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                                float rest = __uint_as_float(q[3]);
-#pragma unroll
-                                for (int i = 2; i >= 0; --i) rest = __fmaf_rn(rest, 0.125f, __uint_as_float(q[i]));
-                                if (mine != 0u) sum = __fmaf_rn(rest, 2.384185791015625e-07f, sum);   // 2^-22
-                            }
-                            return __fmul_rn(__fadd_rn(sum, sum), __uint_as_float(exponents[m] << 23));
+                            return mine == 0u ? 0.0f : sum;
                         };
+                        auto scaled_up = [&](uint32_t m, float sum) { return __fmul_rn(__fadd_rn(sum, sum), __uint_as_float(exponents[m] << 23)); };
 #pragma unroll 1
                         for (uint32_t m = 0; m < rows; m += 2u) {   // two rows at a time (the columns of an odd last one's neighbour exist)
                             uint32_t r[16];
                             tmem_load_16(r, d + m * 8u);
                             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                            for (uint32_t h = 0; h < 2u; ++h)
-                                if (m + h < rows) {
-                                    const float value = joined(m + h, r + 8u * h);
-                                    if (((odd_rows >> (m + h)) & 1u) == 0u) send_f32(to + (m + h) * owned * 4u, value, bar);
-                                }
+                            const float one = scaled_up(m, joined(r)), two = scaled_up(min(m + 1u, kMaxRows - 1u), joined(r + 8));
+                            if (((more_rows >> m) & 1u) == 0u) send_f32(to + m * owned * 4u, one, bar);
+                            if (m + 1u < rows && ((more_rows >> m) & 2u) == 0u) send_f32(to + (m + 1u) * owned * 4u, two, bar);
                         }
 #pragma unroll 1
-                        for (uint32_t odd = odd_rows; odd != 0u; odd &= odd - 1u) {   // with what their digits leave out
-                            const uint32_t m = (uint32_t)__ffs((int)odd) - 1u;
-                            uint32_t r[8];
+                        for (uint32_t more = more_rows; more != 0u; more &= more - 1u) {   // rows with further digits, or values that those leave out
+                            const uint32_t m = (uint32_t)__ffs((int)more) - 1u;
+                            uint32_t r[8], q[4];
                             tmem_load_8(r, d + m * 8u);
+                            tmem_load_4(q, d + rows * kDigits + m * kMoreDigits);
                             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                            send_f32(to + m * owned * 4u, __fadd_rn(joined(m, r), beside[m]), bar);
+                            float sum = joined(r), rest = __uint_as_float(q[3]);
+#pragma unroll
+                            for (int i = 2; i >= 0; --i) rest = __fmaf_rn(rest, 0.125f, __uint_as_float(q[i]));
+                            if (mine != 0u && has_more(m)) sum = __fmaf_rn(rest, 2.384185791015625e-07f, sum);   // 2^-22
+                            const float value = scaled_up(m, sum);
+                            send_f32(to + m * owned * 4u, (odd_rows >> m) & 1u ? __fadd_rn(value, beside[m]) : value, bar);
                         }
                     } else {
                         // eight columns of this thread's weight row: both terms' sums added
@@ -848,11 +851,11 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                     if constexpr (kResident) {
 #pragma unroll 1
                         for (uint32_t o = dt; o < outputs * width; o += 128u) {
-                            const uint32_t row = o % outputs, i = o / outputs, at = row0 + row;
+                            const uint32_t row = o & (outputs - 1u), i = o >> outputs_log, at = row0 + row;
                             const float* p = from + i * owned + row;
                             float sum = p[0];
                             for (uint32_t q = 1; q < split; ++q) sum = __fadd_rn(sum, p[q * width * owned]);
-                            if (at < before.t->n) before.t->y[(uint64_t)i * before.t->n + at] = (uint16_t)eb::bf16_pair(__fmul_rn(sum, before.global), 0.0f);   // keeps a NaN one
+                            if (at < before.n) before.y[(uint64_t)i * before.n + at] = (uint16_t)eb::bf16_pair(__fmul_rn(sum, before.global), 0.0f);   // keeps a NaN one
                         }
                     } else {
                         const uint32_t quads = width / 4u;
@@ -867,7 +870,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                         };
 #pragma unroll 2
                         for (uint32_t o = dt; o < outputs * quads; o += 128u) {   // four columns of a row; neighbouring threads neighbouring rows
-                            const uint32_t row = o % outputs, quad = o / outputs, at = row0 + row;
+                            const uint32_t row = o & (outputs - 1u), quad = o >> outputs_log, at = row0 + row;
                             const float4 sum = total(row, quad), up = paired ? total(half_owned + row, quad) : sum;
                             const float sums[4] = {sum.x, sum.y, sum.z, sum.w}, ups[4] = {up.x, up.y, up.z, up.w};
 #pragma unroll
@@ -875,7 +878,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                                 const uint32_t column = before.first + 4u * quad + i;
                                 if (column >= rows || at >= out_stride) continue;
                                 const float scale = __fmul_rn(group.row_globals[column], before.global), value = __fmul_rn(sums[i], scale);
-                                before.t->y[(uint64_t)column * out_stride + at] = paired ? swiglu(value, __fmul_rn(ups[i], scale)) : eb::float_to_bf16_bits(value);
+                                before.y[(uint64_t)column * out_stride + at] = paired ? swiglu(value, __fmul_rn(ups[i], scale)) : eb::float_to_bf16_bits(value);
                             }
                         }
                     }
