@@ -319,15 +319,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) kernel(
 
 inline cudaError_t initialize() { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSharedBytes); }
 
-// Activation rows of an item: the fewest waves of pairs times what a stage of an item costs, the longer of its MMAs (4 cycles a row)
-// and of what else a stage takes (about 800 cycles measured with few rows: a stage's activations are requested when the stage four
-// before it is done), and a little for every item's epilogue.
+// Activation rows of an item: the fewest waves of pairs times what a stage of 64 values of K costs, and a little for every item's
+// epilogue. A stage measured 466 / 545 / 589 / 645 ns at 48 / 128 / 160 / 208 rows (the difference of K = 10240 and 5120 on 18,944 weight
+// rows), in which shared memory moves 32 KB of terms in and out and the activations in once and out twice; at 256 rows, where the
+// MMAs take 1024 cycles, 709 ns in a call of 4096 rows under the power cap.
 inline uint32_t tile_of(uint32_t rows, uint32_t weight_tiles, uint32_t pairs) {
     uint32_t best = 256u;
     uint64_t best_cost = ~0ull;
     for (uint32_t count = (rows + 255u) / 256u; count <= (rows + 31u) / 32u; ++count) {
         const uint32_t tile = ((rows + count - 1u) / count + 15u) / 16u * 16u, tiles = (rows + tile - 1u) / tile;
-        const uint64_t cost = (((uint64_t)weight_tiles * tiles + pairs - 1u) / pairs) * (std::max(4u * tile, 800u) + 40u);
+        const uint64_t cost = (((uint64_t)weight_tiles * tiles + pairs - 1u) / pairs) * (std::max(44000u + 85u * tile, 310u * tile) + 2000u);   // 1/100 ns
         if (cost < best_cost) {
             best_cost = cost;
             best = tile;

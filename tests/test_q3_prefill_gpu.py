@@ -187,7 +187,7 @@ def test_model_shapes_at_4096_rows(dev, n, k):
 
 def test_bits_do_not_depend_on_the_row_tile(dev):
     """A call is cut into equal tiles of activation rows whose height depends on the row count: 512 rows in tiles of 256, and the
-    same rows in calls with tiles of 48, 144, 112, 128 and 176 rows, give the same bits, plain and paired."""
+    same rows in calls with tiles of 32, 80, 112, 128 and 176 rows, give the same bits, plain and paired."""
     rng = np.random.default_rng(52)
     rows, k, n = 512, 256, 37 * 256
     blob, _ = random_tensor(rng, n, k)
