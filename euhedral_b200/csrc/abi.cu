@@ -716,9 +716,11 @@ static int q3_prefill(const void* input, const void* weights, void* output, void
     int status = q3_validate(input, weights, output, rows, in_features, weight_rows, weights_byte_size);
     if (status != EUHEDRAL_CUDA_SUCCESS) return status;
     if (scratch == nullptr) return EUHEDRAL_CUDA_INVALID_ARGUMENT;
-    // the reference declines the route under exact numerics and row-exact execution (the bits are not the decode kernels');
-    // here it also declines up to 32 rows, which the decode kernels take as groups of 8 several times faster than the
-    // expansion of the whole tensor costs (gate at 32 rows: 90 us against 160)
+    // The reference declines the route under exact numerics and row-exact execution (the bits are not the decode kernels'). Here it also
+    // declines up to 32 rows, as many as the decode entry point takes, as groups of 8. There a layer's linears cost the same both ways:
+    // query_key_value 6144, o 4096, gate_up 28672 (wide 4096) and down 4096 x 14336 take 36 + 30 + 92 + 69 us in four groups, 33 + 32 + 71 +
+    // 98 here; at 24 rows, three groups, 28 + 23 + 69 + 52 against the same 234 us. Single tensors cross elsewhere (gate_up at 17
+    // rows, down past 32), but one row count for all keeps the bits of a layer's rows on one route.
     if (rows <= kQ3PrefillMinRows - 1u || in_features % 128u != 0 || weight_rows % (paired ? 256u : 128u) != 0 || g_exact.load() || t_row_exact
             || (((uintptr_t)input | (uintptr_t)weights | (uintptr_t)output) & 15u) != 0 || ((uintptr_t)scratch & 255u) != 0)
         return EUHEDRAL_CUDA_ROUTE_UNAVAILABLE;
