@@ -19,7 +19,7 @@
 //   * warps 4..19: codes -> the two BF16 tiles of 64 values (128-byte swizzle), four stages
 //   * warp 0: the activation tile of a stage by TMA, half in each CTA, counted on the even CTA's barrier
 //   * warp 1 of the even CTA: eight MMAs a stage; two accumulators of up to 256 columns
-//   * warps 1 and 3 of the odd CTA: pass on to the even one that the odd half of a stage is made
+//   * warps 1, 3, 24 and 25 of the odd CTA: pass on to the even one that the odd half of a stage is made
 //   * warps 20..23: a thread has one output column and walks the tile's rows; in the paired region (a tile holds 64 gate rows and the
 //     64 up rows that match them) the up half meets the gate half in shared memory
 // Every wait is bounded.
@@ -32,7 +32,7 @@
 
 namespace q3p {
 
-constexpr uint32_t kThreads = 768, kStages = 4, kRawSlots = 3;
+constexpr uint32_t kThreads = 832, kStages = 4, kRawSlots = 3;
 constexpr uint32_t kATile = 128u * 128u, kBTile = 128u * 128u, kStageBytes = 2u * kATile + kBTile;   // hi, lo, half of the activation tile
 constexpr uint32_t kRawCodes = 128u * 48u, kRawBytes = kRawCodes + 128u * 4u;
 constexpr uint32_t kOffRaw = kStages * kStageBytes, kOffUp = kOffRaw + kRawSlots * kRawBytes, kUpPitch = 17u;
@@ -109,18 +109,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) kernel(
     const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *tmem_holder, 0);
     eb::pdl_launch_dependents();
 
-    // Odd CTA: tells the even one of every second stage that its terms are made. An arrive that releases memory to another CTA takes
-    // several hundred cycles: by the converting warps themselves a layer's linears took 1.4 to 1.8 times as long.
-    auto pass_on = [&](uint32_t odd) {
-        eb::Ring ring;   // of pairs of stages
-        for (uint32_t item = pair; item < items; item += pairs)
-            for (uint32_t c = 0; c < chunks; ++c) {
-                const uint32_t stage = 2u * ring.stage + odd;
-                wait(&made[stage], ring.parity);
-                if (lane == 0u) nvfp4n::signal_rank(&made[stage], 0u);
-                __syncwarp();
-                ring.advance(kStages / 2u);
-            }
+    // Odd CTA: tells the even one whenever the terms of this stage are made. An arrive that releases memory to another CTA takes a
+    // microsecond or more: by the converting warps themselves a layer's linears took 1.4 to 1.8 times as long, by one warp for every two
+    // stages 4096 x 14336 at 600 rows took 123 us, by one for each 120 (107 without the release).
+    auto pass_on = [&](uint32_t stage) {
+        const uint32_t total = (items - pair + pairs - 1u) / pairs * stages_item;   // stages of all items
+        uint32_t parity = 0u;
+        for (uint32_t i = stage; i < total; i += kStages, parity ^= 1u) {
+            wait(&made[stage], parity);
+            if (lane == 0u) nvfp4n::signal_rank(&made[stage], 0u);
+            __syncwarp();
+        }
     };
 
     if (warp == 0) {
@@ -177,8 +176,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) kernel(
         } else {
             pass_on(0u);
         }
-    } else if (warp == 3) {
-        if (rank != 0u) pass_on(1u);
+    } else if (warp == 3 || warp >= 24u) {
+        if (rank != 0u) pass_on(warp == 3u ? 1u : warp - 22u);
     } else if (warp == 2) {
         const bool leader = eb::elect_one();
         eb::Ring ring;
