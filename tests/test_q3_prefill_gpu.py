@@ -50,6 +50,23 @@ def test_against_float64(dev, rows, k, n):
     assert np.all(np.abs(O.bf16_to_f32(got).astype(np.float64) - exact) <= 2.0 ** -8 * np.abs(exact) + 1e-5 * scale)
 
 
+@pytest.mark.parametrize("k", [5120, 17408])
+def test_long_sums_against_float64(dev, k):
+    """The share of outputs with the bits of the rounded float64 result falls with K: an output passes through K / 8 accumulations of
+    the tensor core (two terms, 16 values each), each of which loses up to 2^-24 of the sum, against BF16 steps of 2^-8 of it at
+    least. Two such losses (either side of a step) give 1 - K 2^-18 as the least share; 99.7 and 98.9 % were measured."""
+    from oracle import oracle_c as OC
+    rng = np.random.default_rng(k)
+    n, rows = 256, 64
+    blob = OC.q3_quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32))
+    x = random_x(rng, rows, k)
+    got, exact = prefill(dev, x, blob, n, k), O.linear_f64(x, OC.q3_dense(blob, n, k))
+    rounded = O.bf16_bits(exact.astype(np.float32))
+    assert (got == rounded).mean() >= 1.0 - k * 2.0 ** -18
+    bound = 2.0 ** -8 * np.abs(exact) + k / 8 * 2.0 ** -24 * np.abs(exact).max(axis=1, keepdims=True)
+    assert np.all(np.abs(O.bf16_to_f32(got).astype(np.float64) - exact) <= bound)
+
+
 def test_rows_do_not_depend_on_their_neighbours(dev):
     rng = np.random.default_rng(3)
     k, n = 512, 256
