@@ -608,8 +608,8 @@ def measure_trellis_prefill(bench: Bench, rows, steps, warmup):
 
 
 def measure_q3_prefill(bench: Bench, rows, steps, warmup):
-    """Q3 prefill of the layer at `rows` tokens through the reference's Q3 MX entry points (two exact BF16 terms per weight
-    written to the scratch, one tcgen05 BF16 GEMM over both): TFLOP/s of 2 M N K; the GEMM issues twice that."""
+    """Q3 prefill of the layer at `rows` tokens through the reference's Q3 MX entry points (two exact BF16 terms per weight, made
+    on their way into one tcgen05 BF16 GEMM): TFLOP/s of 2 M N K; the GEMM issues twice that."""
     torch, gpu, lib = bench.torch, bench.gpu, bench.lib
     tensors, flops, xs = [], 0, {}
     for index, (name, n, k) in enumerate(LAYER):
@@ -634,7 +634,7 @@ def measure_q3_prefill(bench: Bench, rows, steps, warmup):
               "roofline": {"bound": "tensor", "achieved": 2 * tflops, "algorithmic": tflops, "peak": peak, "unit": "TFLOP/s",
                            "frac": 2 * tflops / peak if peak else None, "peak_kind": f"of {bench.peaks['kind']} (cuBLAS BF16 burst)",
                            "frac_of_sustained": 2 * tflops / bench.peaks["bf16_sustained"] if bench.peaks["bf16_sustained"] else None,
-                           "note": "achieved = issued FLOP (two BF16 terms per weight); algorithmic = 2 M N K; the expansion of the codes runs before the GEMM and counts as time"}}
+                           "note": "achieved = issued FLOP (two BF16 terms per weight); algorithmic = 2 M N K; the codes become operands inside the GEMM"}}
     del tensors, xs, y, scratch
     torch.cuda.empty_cache()
     return result

@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(kThreads, 1) bf16_gemm_kernel(const __grid_con
 // A last wave with fewer tiles than half of the pairs runs them as halves of 128 columns: 5120 columns at 2048 rows are 160 tiles on
 // 74 pairs, 2 waves and 12 tiles, which took a third whole wave. The segments of a trellis object share one launch for the same
 // reason (query_key_value at 2048 rows: 160 + 32 + 32 tiles were 3 + 1 + 1 waves). A trellis layer of 512 / 1024 / 2048 rows, with
-// its rotate and decode side by side: 702 / 975 / 1630 -> 598 / 892 / 1568 us.
+// its rotate and decode side by side (w = 64): 703 / 985 / 1518 -> 580 / 872 / 1426 us.
 constexpr uint32_t kPairStages = 6;
 constexpr uint32_t kPairStageBytes = kATile + 128u * 128u;
 constexpr uint32_t kPairShared = kPairStages * kPairStageBytes + 256u + 1024u;

@@ -23,9 +23,8 @@
 // order with the MMAs (16 copies of about 37 cycles beside 8 MMAs of 135 per stage) and wants the weights' scales re-laid-out by
 // a launch of its own; the registers' way runs beside the MMAs and reads the tensor's plane. What then limited the single-CTA
 // kernel was the epilogue's 16-byte stores (every sector written in halves) and shared-memory bandwidth (12 KB read per MMA
-// and 9 KB filled per 135 cycles at 128 bytes a cycle; the pairs read 8 and fill 7). 4096 x 17408 x 5120 under ncu, in SM
-// cycles: tcgen05.cp 478k; tcgen05.st 428k; with 32-byte stores 379k, on pairs 350k (tensor pipe 86 % active; the clock falls
-// to 1.4 GHz: the rest is power). Back to back: 300 us before, 262 to 277 us now.
+// and 9 KB filled per 135 cycles at 128 bytes a cycle; the pairs read 8 and fill 7). 4096 x 17408 x 5120, activations quantized
+// before, back to back under the power cap: 245 to 276 us on pairs, 261 to 299 on single CTAs (the clock moves between runs).
 // Tiles are walked in panels of eight tile columns with the row index fastest, so that CTAs running together share
 // weight tiles and re-read activation tiles from L2. Every CTA issues its own loads.
 #pragma once
@@ -783,9 +782,9 @@ inline cudaError_t initialize() {
     return e != cudaSuccess ? e : cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairShared);
 }
 
-// Fewer rows than this run on single CTAs. The pairs are 2 to 6 % faster from 1024 rows on (1024 x 5120 x 17408: 171 against 176
-// us, 4096 x 17408 x 5120: 318 against 337 in turn), equal within 1 % at 512 to 1024; with fewer rows their 256-row tiles
-// leave more of the last wave empty.
+// Fewer rows than this run on single CTAs. us on pairs / single CTAs, in turn, rows x 17408 x 5120 and rows x 5120 x 17408: 256 rows
+// 20.4 / 20.3 and 46.0 / 47.9, 384 rows 33.2 / 34.5 and 49.2 / 48.4, 512 rows 33.5 / 35.4 and 49.1 / 50.0, 1024 rows 66.4 / 71.0 and
+// 92.2 / 99.5, 4096 rows 260 / 281 and 277 / 298: from 512 rows on both shapes are faster on pairs, below that one of them is not.
 constexpr uint32_t kPairRows = 512;
 
 template <typename... Params, typename... Args>

@@ -6,8 +6,10 @@
 // activations; products are exact in FP32, an output is one FP32 sum in K order (64 values of hi terms, the same 64 of lo terms),
 // rounded once to BF16. Nothing in that order depends on the rows of a call or of the tensor.
 //
-// Bound: tensor pipe, 4 M N K FLOP. A separate launch that wrote both terms to memory (4 bytes a weight), which this replaces,
-// took most of a call of few rows (a layer at 40 / 600 / 4096 rows: 741 / 984 / 3925 us before, 253 / 569 / 3255 now). Here the terms of a weight are made once per tile of up to 256 activation rows, beside the MMAs:
+// Bound: shared memory (profiles/q3_prefill_kernel_600_rows.md), then the tensor pipe, 4 M N K FLOP. A separate launch that wrote both terms to memory (4 bytes a weight), which this replaces,
+// took most of a call of few rows (a layer's four fused linears, 5120 wide, at 40 / 300 / 600 / 1024 / 4096 rows: 745 / 853 / 1093 / 1467 / 4332 us before,
+// 284 / 430 / 662 / 1083 / 3997 now, 250 / 383 / 634 / 1010 / 3843 without the release at cluster scope that passes the odd CTA's word on).
+// Here the terms of a weight are made once per tile of up to 256 activation rows, beside the MMAs:
 // 2.6 instructions a code (16-bit windows of the code stream, so that two neighbouring codes land in the two halves of a
 // BF16 pair: one mask, one packed FMA, two packed multiplies), 190 issue slots per 64 values of K where the MMAs of a full tile take
 // 1024 cycles.
