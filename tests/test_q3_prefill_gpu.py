@@ -106,6 +106,28 @@ def test_gate_up_swiglu(dev):
     assert np.all(np.abs(O.bf16_to_f32(got).astype(np.float64) - expect) <= 2.0 ** -7 * np.abs(expect) + 1e-30)
 
 
+def test_captured_calls(dev):
+    """Calls recorded into a CUDA graph, the first ones on their weights among them, give the bits of the direct call when replayed."""
+    torch, lib = dev.torch, dev.gpu.lib
+    rng = np.random.default_rng(62)
+    rows, k, n = 70, 256, 384
+    blobs = [random_tensor(rng, n, k)[0] for _ in range(2)]
+    x = random_x(rng, rows, k)
+    expect = [prefill(dev, x, blob, n, k) for blob in blobs]
+    d_x, d_s = dev.put(x), dev.empty(256)
+    d_w, d_y = [dev.put(blob) for blob in blobs], [dev.empty(rows * n * 2) for _ in blobs]
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream), dev.gpu.submit(stream.cuda_stream, pdl=True):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            for w, y, blob in zip(d_w, d_y, blobs):
+                assert lib.euhedral_cuda_linear_q3_mx_bf16(d_x.data_ptr(), w.data_ptr(), y.data_ptr(), d_s.data_ptr(), rows, k, n, blob.size, 256) == 0
+        graph.replay()
+    for y, bits in zip(d_y, expect):
+        assert np.array_equal(dev.get(y, np.uint16, (rows, n)), bits)
+
+
 def test_weights_outside_device_memory(dev):
     """Weights in pinned host memory are not given to a tensor map: their codes come by plain copies, the results are the same."""
     import ctypes as C
