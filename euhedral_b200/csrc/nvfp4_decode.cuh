@@ -66,7 +66,8 @@ constexpr uint32_t kTmemColumns = 512;
 constexpr uint32_t kHeldByEight = 14, kHeldByTwelve = 24;   // powers of two below the largest value that the digits hold exactly (see above)
 // Exchange buffers of a CTA. The word that one may be filled again reaches the other CTAs a microsecond or two after it was read;
 // with two buffers for BF16 rows the draining warps waited for it (34816 x 5120 at one row 26.4 us, with four 22.1).
-__host__ __device__ constexpr uint32_t gather_slots(bool resident) { return resident ? 4u : 2u; }
+// Two remain for quantized rows, whose buffers are large and whose calls exchange few tiles, and where four leave no room for the digits.
+constexpr uint32_t kMostSlots = 4, kFewSlots = 2;
 constexpr uint32_t kLeftWords = 128;      // rows times units of a CTA: more than its shared memory has room for digits of
 constexpr uint32_t kLeastExponent = 48;   // of a row's slice: the grid does not get finer than that of 2^-79
 
@@ -92,6 +93,7 @@ struct alignas(64) Group {
     uint32_t split;            // CTAs of a cluster, each with a slice of K; 1 (quantized rows only): no cluster, no exchange
     uint32_t tmem_columns;     // allocated: a power of two
     uint32_t buffers;          // accumulators of consecutive items: 2, or 1 where tensor memory is short
+    uint32_t slots;            // exchange buffers
     uint32_t row_groups;       // quantized rows: groups of kMaxColumns; an item of the launch is a tile and a group
     uint32_t pair_rows;        // the paired region: gate rows of the tensor (0: a plain linear)
     const uint8_t* atoms;      // quantized rows: their block scales (nvfp4n::ActivationLayout)
@@ -105,7 +107,7 @@ struct alignas(64) Group {
 //   bring their two terms as columns of their own.
 struct Layout {
     uint32_t columns, n, plain_n, width, pitch, stage_bytes, off_rows, off_gather, gather_bytes, off_bars, bytes;
-    __host__ __device__ Layout(bool resident, uint32_t rows, uint32_t units_cta, uint32_t stages, uint32_t split, bool paired) {
+    __host__ __device__ Layout(bool resident, uint32_t rows, uint32_t units_cta, uint32_t stages, uint32_t split, bool paired, uint32_t slots) {
         columns = resident ? (rows * (kDigits + kMoreDigits) + 15u) / 16u * 16u : rows >= kMaxColumns ? kMaxColumns : (rows + 7u) / 8u * 8u;
         n = resident ? columns : nvfp4n::kTerms * columns;
         plain_n = resident ? (rows * kDigits + 15u) / 16u * 16u : n;   // of rows without outliers: the first eight digits come first
@@ -116,7 +118,7 @@ struct Layout {
         stage_bytes = (stage_bytes + 1023u) & ~1023u;
         off_rows = stages * stage_bytes;                             // resident digits: a tile of `columns` x 128 bytes per unit
         off_gather = off_rows + (resident ? units_cta * columns * 128u : 0u);
-        off_bars = off_gather + (split > 1u ? gather_slots(resident) * gather_bytes : paired ? gather_bytes / 2u : 0u);
+        off_bars = off_gather + (split > 1u ? slots * gather_bytes : paired ? gather_bytes / 2u : 0u);
         bytes = off_bars + 1024u + 1024u;                            // barriers, the rows' exponents and left-out values or scales; slack to align to 1024
     }
 };
@@ -394,13 +396,13 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
     const uint32_t rank = exchange ? eb::cluster_rank() : 0u, clusters = gridDim.x / split, cluster = blockIdx.x / split;
     const uint32_t run_begin = (uint32_t)((uint64_t)cluster * group.tiles / clusters), run_end = (uint32_t)((uint64_t)(cluster + 1u) * group.tiles / clusters);
     const uint32_t unit_begin = rank * units / split, unit_end = (rank + 1u) * units / split, mine = unit_end - unit_begin;
-    constexpr uint32_t kSlots = gather_slots(kResident);
+    const uint32_t slots = group.slots, slots_log = slots >> 1;   // 4 or 2
     const bool paired = !kResident && group.pair_rows != 0u;
-    const Layout layout(kResident, rows, (units + split - 1u) / split, stages, split, paired);
+    const Layout layout(kResident, rows, (units + split - 1u) / split, stages, split, paired, slots);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + layout.off_bars);
     uint64_t *full = bars, *empty = full + kMaxStages, *scaled = empty + kMaxStages, *acc_full = scaled + kMaxStages, *acc_empty = acc_full + 2,
-             *staged = acc_empty + 2, *gather_full = staged + 1, *gather_empty = gather_full + kSlots, *gather_read = gather_empty + kSlots;
-    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(gather_read + kSlots);
+             *staged = acc_empty + 2, *gather_full = staged + 1, *gather_empty = gather_full + kMostSlots, *gather_read = gather_empty + kMostSlots;
+    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(gather_read + kMostSlots);
     uint32_t* failed = tmem_holder + 1;
     uint32_t* exponents = failed + 1;        // per row: the largest exponent of the slice
     uint32_t* least = exponents + kMaxRows;  // per row: the least exponent of the slice, zeros aside
@@ -417,7 +419,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
             const uint32_t b = lane - 16u;
             eb::mbar_init(&acc_full[b], 1);
             eb::mbar_init(&acc_empty[b], 4);
-        } else if (lane >= 20u && lane < 20u + kSlots) {
+        } else if (lane >= 20u && lane < 20u + slots) {
             const uint32_t b = lane - 20u;
             eb::mbar_init(&gather_full[b], 1);
             eb::mbar_init(&gather_empty[b], split);
@@ -745,7 +747,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                         stage_rows(t.x, held != nullptr);
                         held = t.x;
                     }
-                    const uint32_t buffer = buffers == 2u ? e & 1u : 0u, use = buffers == 2u ? e >> 1 : e, slot = e % kSlots;
+                    const uint32_t buffer = buffers == 2u ? e & 1u : 0u, use = buffers == 2u ? e >> 1 : e, slot = e & (slots - 1u);
                     if (!kResident && !exchange) {   // the scales of the item's activation rows
                         drainers_sync();   // those of the item before have been read
                         if (dt < width) row_scales[dt] = now.first + dt < rows ? __fmul_rn(group.row_globals[now.first + dt], now.global) : 0.0f;
@@ -756,7 +758,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                     wait(&acc_full[buffer], use & 1u);
                     nvfp4n::tcgen05_fence_after();
                     const uint32_t d = tmem + lanes + buffer * acc_columns;
-                    if (exchange && e >= kSlots) eb::mbar_wait_cluster_or_fail(&gather_empty[slot], (e / kSlots - 1u) & 1u, failed);
+                    if (exchange && e >= slots) eb::mbar_wait_cluster_or_fail(&gather_empty[slot], ((e >> slots_log) - 1u) & 1u, failed);
                     const uint32_t to = peer_gather + slot * slot_bytes, bar = peer_full + slot * 8u;
                     if constexpr (kResident) {
                         // This thread's sum of a row of the slice from the sums of its eight digits, in units of half the largest value's.
@@ -845,9 +847,9 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                 }
                 if (exchange && e > 0u) {
                     // The slices of the exchange before, added in order; this CTA's share of the outputs.
-                    const uint32_t last = e - 1u, slot = last % kSlots;
+                    const uint32_t last = e - 1u, slot = last & (slots - 1u);
                     if (dt == 0u) eb::mbar_arrive_expect_tx(&gather_full[slot], kResident ? slot_bytes : kTile * width * 4u);
-                    wait(&gather_full[slot], (last / kSlots) & 1u);
+                    wait(&gather_full[slot], (last >> slots_log) & 1u);
                     const float* from = reinterpret_cast<const float*>(smem + layout.off_gather + slot * slot_bytes);
                     const uint32_t row0 = before.tile * (paired ? 64u : kTile) + rank * outputs;
                     if constexpr (kResident) {
@@ -885,7 +887,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                         }
                     }
                     __syncwarp();
-                    if (lane == 0 && last + kSlots < exchanges) eb::mbar_arrive(&gather_read[slot]);   // warp 2 passes it on
+                    if (lane == 0 && last + slots < exchanges) eb::mbar_arrive(&gather_read[slot]);   // warp 2 passes it on
                 }
             }
         } else if (kResident || (warp == 2u && exchange)) {
@@ -901,10 +903,10 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                     stage_rows(t.x, held != nullptr);
                     held = t.x;
                 }
-                if (passes && e > 0u && e - 1u + kSlots < exchanges) {
+                if (passes && e > 0u && e - 1u + slots < exchanges) {
                     const uint32_t last = e - 1u;
-                    wait(&gather_read[last % kSlots], (last / kSlots) & 1u);
-                    if (lane < split) nvfp4n::signal_rank(&gather_empty[last % kSlots], lane);
+                    wait(&gather_read[last & (slots - 1u)], (last >> slots_log) & 1u);
+                    if (lane < split) nvfp4n::signal_rank(&gather_empty[last & (slots - 1u)], lane);
                     __syncwarp();
                 }
             });
@@ -941,7 +943,7 @@ inline cudaError_t initialize() {
 }
 
 struct Plan {
-    uint32_t split, stages, shared, tmem, buffers;
+    uint32_t split, stages, shared, tmem, buffers, slots;
 };
 
 // Whether a launch of `rows` rows over clusters of `split` fits, and how deep its ring is: as many stages as an SM's shared and tensor
@@ -950,15 +952,16 @@ struct Plan {
 inline bool plan(bool resident, uint32_t rows, uint32_t k, uint32_t split, bool paired, Plan* out) {
     const uint32_t units = units_of(k), units_cta = (units + split - 1u) / split;
     if (rows == 0u || (resident && (rows > kMaxRows || rows * units_cta > kLeftWords))) return false;
-    for (uint32_t stages = kMaxStages; stages >= 3u; --stages)
-        for (uint32_t buffers = 2; buffers >= 1u; --buffers) {
-            const Layout layout(resident, rows, units_cta, stages, split, paired);
-            const uint32_t columns = buffers * layout.n + stages * (resident ? 16u : 32u) + (resident ? 16u : 0u);
-            if (layout.bytes <= kSharedLimit && columns <= kTmemColumns) {
-                *out = {split, stages, layout.bytes, columns <= 128u ? 128u : columns <= 256u ? 256u : 512u, buffers};
-                return true;
+    for (uint32_t slots = resident ? kMostSlots : kFewSlots; slots >= kFewSlots; slots >>= 1)
+        for (uint32_t stages = kMaxStages; stages >= 3u; --stages)
+            for (uint32_t buffers = 2; buffers >= 1u; --buffers) {
+                const Layout layout(resident, rows, units_cta, stages, split, paired, slots);
+                const uint32_t columns = buffers * layout.n + stages * (resident ? 16u : 32u) + (resident ? 16u : 0u);
+                if (layout.bytes <= kSharedLimit && columns <= kTmemColumns) {
+                    *out = {split, stages, layout.bytes, columns <= 128u ? 128u : columns <= 256u ? 256u : 512u, buffers, slots};
+                    return true;
+                }
             }
-        }
     return false;
 }
 
@@ -1048,6 +1051,7 @@ inline cudaError_t launch(bool resident, bool table, Group* group, const Plan& p
     group->split = p.split;
     group->tmem_columns = p.tmem;
     group->buffers = p.buffers;
+    group->slots = p.slots;
     group->scale_row_bytes = group->k / (table ? 32u : 16u);
     const Kernel kernel = kernel_of(resident, table);
     const uint32_t most = most_clusters(resident, table, p, sms);
@@ -1091,7 +1095,7 @@ inline cudaError_t decode(const Item* items, uint32_t count, uint32_t rows, uint
 }
 
 // Columns of an item for quantized rows.
-inline uint32_t columns_of(uint32_t rows) { return Layout(false, rows, 1u, 1u, 1u, false).columns; }
+inline uint32_t columns_of(uint32_t rows) { return Layout(false, rows, 1u, 1u, 1u, false, kFewSlots).columns; }
 
 // Whether this kernel takes a native call of `rows` quantized rows rather than the large GEMM (nvfp4_native.cuh), by what each keeps
 // an SM busy with: per unit of K the GEMM spends about 1080 cycles on an output tile of 128 rows x 256 columns and leaves the SMs

@@ -113,6 +113,13 @@ def test_decode_plans_stay_launchable_and_cut_k_by_k_alone():
                 assert cuts.setdefault((fmt, k), cut) == cut
 
 
+def test_nvfp4_decode_takes_the_longest_rows():
+    """One row of K = 174080 is the most whose digits and buffers fit an SM's shared memory; longer ones run on the scalar kernel."""
+    assert library.decode_plan("nvfp4", 1, 174080, 16)["shared_bytes"] <= 227 * 1024
+    with pytest.raises(ValueError):
+        library.decode_plan("nvfp4", 1, 174080 + 128, 16)
+
+
 def test_prefill_entry_points_validate_without_a_device():
     lib = library.load()
     # sizes are pure arithmetic

@@ -54,6 +54,19 @@ def test_edges_and_outliers(dev, n, k):
             assert np.all(np.abs(got - expect) <= np.abs(expect) * 2.0 ** -8 + terms * 2.0 ** -18), (rows, n, k)
 
 
+def test_few_and_many_exchange_buffers(dev):
+    """16 rows of K = 5376 leave room for two exchange buffers beside the digits, one row for four: several tiles per cluster, so that
+    both sets are used again, give a row the same bits."""
+    from euhedral_b200 import synthetic
+    n, k = 18944, 5376                                            # four tiles of 128 rows for each of 37 clusters
+    d_w = synthetic.nvfp4_tensor(synthetic.gaussian(n, k, 5, 0.02, device="cuda"))
+    x = random_x(np.random.default_rng(6), 16, k)
+    for _ in range(3):
+        got = run(dev, x, d_w, n, k, d_w.numel())
+        for row in (0, 7, 15):
+            assert np.array_equal(run(dev, x[row:row + 1], d_w, n, k, d_w.numel())[0], got[row]), row
+
+
 @pytest.mark.parametrize("n,k", [(48, 384), (160, 5120)])
 @pytest.mark.parametrize("sd4", [False, True])
 def test_every_finite_value_counts(dev, n, k, sd4):
