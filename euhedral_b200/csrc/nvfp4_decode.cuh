@@ -9,8 +9,8 @@
 //     slice. Every value counts in full. Eight digits hold a BF16 value exactly down to 2^-14 of the power of two of the slice's largest;
 //     where a row has smaller ones, four more columns hold the next four digits, down to 2^-24; what is smaller still (or is below
 //     2^-103 whatever the largest, or not finite) is left out of the digits, and the draining warps add its products in FP32 from the
-//     weights in memory (about 1 us a tile and 32 values: 34816 x 5120 at 5 rows 24 us, 52 where one value in 97 is 2^12 times larger,
-//     1060 where the values spread evenly over 40 powers of two). So an infinity gives every output what IEEE arithmetic gives it. The choice is a row's and slice's own and
+//     weights in memory (about 0.5 us a tile and 32 values: 34816 x 5120 at 5 rows 24 us, 36 where four values of a row are 1000 times
+//     larger, 731 where the values spread evenly over 40 powers of two). So an infinity gives every output what IEEE arithmetic gives it. The choice is a row's and slice's own and
 //     changes no bit of the rows beside it. Of 1280 normally distributed values, one slice in eight takes more digits, one in ten
 //     thousand leaves a value out.
 //   * two NVFP4 terms per row, quantized into the scratch before (the native route): a row is one column, both terms accumulate
@@ -273,21 +273,26 @@ struct Slice {
     }
 };
 
-// The rows of a mask, whose digits leave values out, once more: their exponents over the other values, their digits, and the words that
-// say where the values left out are. Taken by every staging warp when all digits have been written.
+// For the rows of a mask, whose digits leave values out: the words that say where those are. Rows with values that are not finite first
+// get their exponents over the others, and their digits again. Taken by every staging warp when all digits have been written.
 __device__ __forceinline__ void stage_again(const Slice& slice, const uint32_t odd_rows) {
-    auto for_units = [&](auto&& body) {
+    auto for_units = [&](uint32_t mask, auto&& body) {
 #pragma unroll 1
-        for (uint32_t odd = odd_rows; odd != 0u; odd &= odd - 1u)
+        for (; mask != 0u; mask &= mask - 1u)
 #pragma unroll 1
-            for (uint32_t u = slice.stager; u < slice.units; u += kStagers / 32u) body((uint32_t)__ffs((int)odd) - 1u, u);
+            for (uint32_t u = slice.stager; u < slice.units; u += kStagers / 32u) body((uint32_t)__ffs((int)mask) - 1u, u);
     };
-    stagers_sync();   // nobody needs the exponents that led here any more
-    if (slice.stager == 0u && ((odd_rows >> slice.lane) & 1u)) slice.exponents[slice.lane] = kLeastExponent, slice.least[slice.lane] = 255u;
-    stagers_sync();
-    for_units([&](uint32_t row, uint32_t u) { slice.find(row, finite_only(slice.load(row, u))); });
-    stagers_sync();
-    for_units([&](uint32_t row, uint32_t u) {
+    const bool mine = ((odd_rows >> slice.lane) & 1u) && slice.exponents[slice.lane & (kMaxRows - 1u)] == 255u;
+    const uint32_t again = __ballot_sync(0xFFFFFFFFu, mine);
+    if (again != 0u) {
+        stagers_sync();   // nobody needs the exponents that led here any more
+        if (slice.stager == 0u && mine) slice.exponents[slice.lane] = kLeastExponent, slice.least[slice.lane] = 255u;
+        stagers_sync();
+        for_units(again, [&](uint32_t row, uint32_t u) { slice.find(row, finite_only(slice.load(row, u))); });
+        stagers_sync();
+        for_units(again, [&](uint32_t row, uint32_t u) { slice.write(row, u, finite_only(slice.load(row, u))); });
+    }
+    for_units(odd_rows, [&](uint32_t row, uint32_t u) {
         const uint4 values = slice.load(row, u);
         const uint32_t pairs[4] = {values.x, values.y, values.z, values.w};
         bool some = false;
@@ -295,76 +300,79 @@ __device__ __forceinline__ void stage_again(const Slice& slice, const uint32_t o
         for (uint32_t i = 0; i < 8u; ++i) some = some || not_held((pairs[i >> 1] >> (16u * (i & 1u))) & 0xFFFFu, slice.per(row), slice.has_more(row)) != 0.0f;
         const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, some);
         if (slice.lane == 0u) slice.left[row * slice.units + u] = lanes;
-        slice.write(row, u, finite_only(values));
     });
     stagers_sync();   // the words are there for the draining warps
 }
 
 // What the digits of the odd rows leave out of a slice, summed against one weight row per lane in FP32 in K order: beside[m] of every
 // odd row m. The weights are read where they lie (the ring has moved on), 32 values of K at a time: a lane finds what is left of one
-// of them and all take it from there. The loads of four such parts are in flight together: one at a time took twice as long. Taken by
+// of them and all take it from there. The loads of a part are in flight while the part before it is summed. Taken by
 // whole warps.
 template <bool kTable>
 __device__ __forceinline__ void left_out(const Tensor& t, const Slice& slice, uint32_t row, uint32_t odd_rows, float (&beside)[kMaxRows]) {
     row = min(row, t.n - 1u);
-    const uint8_t* codes = t.weights + (uint64_t)row * (slice.k / 2u);
-    const uint8_t* scale_codes = t.scales + (uint64_t)row * (slice.k / (kTable ? 32u : 16u));
+    const uint32_t code_pitch = slice.k / 2u, scale_pitch = slice.k / (kTable ? 32u : 16u);
+    const uint8_t* codes = t.weights + (uint64_t)row * code_pitch;
+    const uint8_t* scale_codes = t.scales + (uint64_t)row * scale_pitch;
     struct Part {
-        uint32_t m, first, eighths;   // activation row (kMaxRows: there are no more), the first of its 32 values, which eighths of the 32
-    };
-    uint32_t m = 0, u = slice.units, lanes = 0u;
-    auto next = [&]() -> Part {
-        while (lanes == 0u) {
-            if (++u >= slice.units) {
-                if (odd_rows == 0u) return {kMaxRows, 0u, 0u};
-                m = (uint32_t)__ffs((int)odd_rows) - 1u;
-                odd_rows &= odd_rows - 1u;
-                u = 0u;
-                beside[m] = 0.0f;
-            }
-            lanes = slice.left[m * slice.units + u];
-        }
-        const uint32_t shift = ((uint32_t)__ffs((int)lanes) - 1u) & ~3u, eighths = (lanes >> shift) & 15u;
-        lanes &= ~(15u << shift);
-        return {m, ((slice.unit_begin + u) * 32u + shift) * 8u, eighths};
-    };
-    constexpr int kParts = 4;
+        uint32_t m, scale, value;   // activation row (kMaxRows: there are no more), the weight row's scale codes, the lane's value
+        uint4 code;
+    } now = {kMaxRows, 0u, 0u, make_uint4(0u, 0u, 0u, 0u)}, ahead = now;
+    const uint16_t* x = t.x;
+    const uint8_t* table = t.table;
+    uint32_t m = 0u, base = slice.units, word = 0u, units = 0u, u = 0u, lanes = 0u;   // a lane looks at every 32nd unit's word
+    float sum = 0.0f;
 #pragma unroll 1
     while (true) {
-        uint32_t of[kParts], scale[kParts];
-        float rest[kParts];
-        uint4 code[kParts];
-        bool some = false;
-#pragma unroll
-        for (int j = 0; j < kParts; ++j) {
-            const Part part = next();
-            of[j] = part.m;
-            if (part.m == kMaxRows) continue;
-            some = true;
-            code[j] = *reinterpret_cast<const uint4*>(codes + part.first / 2u);
-            scale[j] = kTable ? scale_codes[part.first / 32u] : *reinterpret_cast<const uint16_t*>(scale_codes + part.first / 16u);
-            const uint32_t bits = (part.eighths >> (slice.lane >> 3)) & 1u ? t.x[(uint64_t)part.m * slice.k + part.first + slice.lane] : 0u;
-            rest[j] = not_held(bits, slice.per(part.m), slice.has_more(part.m));
-        }
-        if (!some) break;
+        ahead.m = kMaxRows;
 #pragma unroll 1
-        for (int turn = 0; turn < kParts && of[0] != kMaxRows; ++turn) {
-            if (kTable) scale[0] = t.table[scale[0] & 15u] | (uint32_t)t.table[scale[0] >> 4] << 8;
-            const uint32_t words[4] = {code[0].x, code[0].y, code[0].z, code[0].w};
-            const float blocks[2] = {exact::e4m3(scale[0] & 0xFFu), exact::e4m3(scale[0] >> 8)};
-            float sum = beside[of[0]];
+        while (lanes == 0u) {
+            if (units != 0u) {
+                const uint32_t at = (uint32_t)__ffs((int)units) - 1u;
+                units &= units - 1u;
+                u = base + at;
+                lanes = __shfl_sync(0xFFFFFFFFu, word, (int)at);
+                break;
+            }
+            base += 32u;
+            if (base >= slice.units) {
+                if (odd_rows == 0u) break;
+                m = (uint32_t)__ffs((int)odd_rows) - 1u;
+                odd_rows &= odd_rows - 1u;
+                base = 0u;
+                beside[m] = 0.0f;
+            }
+            word = base + slice.lane < slice.units ? slice.left[m * slice.units + base + slice.lane] : 0u;
+            units = __ballot_sync(0xFFFFFFFFu, word != 0u);
+        }
+        if (lanes != 0u) {
+            const uint32_t shift = ((uint32_t)__ffs((int)lanes) - 1u) & ~3u, eighths = (lanes >> shift) & 15u;
+            lanes &= ~(15u << shift);
+            const uint32_t first = ((slice.unit_begin + u) * 32u + shift) * 8u;   // of its 32 values
+            ahead.m = m;
+            ahead.code = *reinterpret_cast<const uint4*>(codes + first / 2u);
+            ahead.scale = kTable ? scale_codes[first / 32u] : *reinterpret_cast<const uint16_t*>(scale_codes + first / 16u);
+            ahead.value = (eighths >> (slice.lane >> 3)) & 1u ? x[(uint64_t)m * slice.k + first + slice.lane] : 0u;
+        }
+        if (now.m != kMaxRows) {
+            const uint32_t scale = kTable ? table[now.scale & 15u] | (uint32_t)table[now.scale >> 4] << 8 : now.scale;
+            const float rest = not_held(now.value, slice.per(now.m), slice.has_more(now.m));
+            const uint32_t words[4] = {now.code.x, now.code.y, now.code.z, now.code.w};
+            const float blocks[2] = {exact::e4m3(scale & 0xFFu), exact::e4m3(scale >> 8)};
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
                 const uint32_t code4 = words[i >> 3] >> (4 * (i & 7));
                 // sign and magnitude where an FP32 number reads them as e2m1 * 2^-126
                 const float weight = __fmul_rn(__uint_as_float((code4 & 8u) << 28 | (code4 & 7u) << 22), 8.507059173023462e37f);
-                sum = __fmaf_rn(__shfl_sync(0xFFFFFFFFu, rest[0], i), __fmul_rn(weight, blocks[i >> 4]), sum);
+                sum = __fmaf_rn(__shfl_sync(0xFFFFFFFFu, rest, i), __fmul_rn(weight, blocks[i >> 4]), sum);
             }
-            beside[of[0]] = sum;
-#pragma unroll
-            for (int j = 0; j + 1 < kParts; ++j) of[j] = of[j + 1], scale[j] = scale[j + 1], rest[j] = rest[j + 1], code[j] = code[j + 1];
-            of[kParts - 1] = kMaxRows;
+            if (ahead.m != now.m) {   // the row's last part
+                beside[now.m] = sum;
+                sum = 0.0f;
+            }
         }
+        if (ahead.m == kMaxRows) break;
+        now = ahead;
     }
 }
 

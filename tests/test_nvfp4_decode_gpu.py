@@ -67,7 +67,7 @@ def test_few_and_many_exchange_buffers(dev):
             assert np.array_equal(run(dev, x[row:row + 1], d_w, n, k, d_w.numel())[0], got[row]), row
 
 
-@pytest.mark.parametrize("n,k", [(48, 384), (160, 5120)])
+@pytest.mark.parametrize("n,k", [(48, 384), (160, 5120), (32, 69632)])     # the last: more than 32 units of K in a CTA
 @pytest.mark.parametrize("sd4", [False, True])
 def test_every_finite_value_counts(dev, n, k, sd4):
     """Outputs whose weights are zero wherever the activations are large: what is left must count in full, however far below the
