@@ -857,7 +857,7 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(const __grid_constant__ Gr
                     // The slices of the exchange before, added in order; this CTA's share of the outputs.
                     const uint32_t last = e - 1u, slot = last & (slots - 1u);
                     if (dt == 0u) eb::mbar_arrive_expect_tx(&gather_full[slot], kResident ? slot_bytes : kTile * width * 4u);
-                    wait(&gather_full[slot], (last >> slots_log) & 1u);
+                    eb::mbar_wait_cluster_or_fail(&gather_full[slot], (last >> slots_log) & 1u, failed);   // st.async of all CTAs of the cluster
                     const float* from = reinterpret_cast<const float*>(smem + layout.off_gather + slot * slot_bytes);
                     const uint32_t row0 = before.tile * (paired ? 64u : kTile) + rank * outputs;
                     if constexpr (kResident) {

@@ -34,3 +34,4 @@ def test_the_q3_terms_are_released_to_the_even_cta():
 def test_the_exchange_buffers_are_released_after_they_were_read():
     text = code(next(path for path in SOURCES if path.name == "nvfp4_decode.cuh"))
     assert "signal_rank(&gather_empty[" in text and "mbar_wait_cluster_or_fail(&gather_empty[" in text
+    assert "mbar_wait_cluster_or_fail(&gather_full[" in text   # what the other CTAs' st.async wrote
