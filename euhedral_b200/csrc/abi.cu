@@ -84,9 +84,10 @@ void initialize_device(int device, DeviceState* state) {
     if (e == cudaSuccess) e = cudaGetSymbolAddress(reinterpret_cast<void**>(&state->static_scratch), g_static_scratch);
     if (e == cudaSuccess) e = allow_gemv<q3::Format>();
     if (e == cudaSuccess) e = allow_big_smem(exact::trellis_linear);
-#define EB_ALLOW_ENCODER(KA, HALF) if (e == cudaSuccess) e = allow_big_smem(trellis_encode::viterbi_kernel<KA, HALF>);
-    EB_ALLOW_ENCODER(2, false) EB_ALLOW_ENCODER(2, true) EB_ALLOW_ENCODER(3, false) EB_ALLOW_ENCODER(3, true)
-    EB_ALLOW_ENCODER(4, false) EB_ALLOW_ENCODER(5, false) EB_ALLOW_ENCODER(6, false)
+#define EB_ALLOW_ENCODER(...) if (e == cudaSuccess) e = allow_big_smem(trellis_encode::__VA_ARGS__);
+    EB_ALLOW_ENCODER(register_kernel<2, false>) EB_ALLOW_ENCODER(register_kernel<2, true>) EB_ALLOW_ENCODER(register_kernel<3, false>)
+    EB_ALLOW_ENCODER(register_kernel<3, true>) EB_ALLOW_ENCODER(register_kernel<4, false>) EB_ALLOW_ENCODER(viterbi_kernel<5>)
+    EB_ALLOW_ENCODER(viterbi_kernel<6>)
 #undef EB_ALLOW_ENCODER
 #define EB_ALLOW(W) if (e == cudaSuccess) e = allow_trellis_width<W>();
     EB_TRELLIS_WIDTHS(EB_ALLOW)
@@ -1114,13 +1115,10 @@ int euhedral_b200_prefill_trellis_bf16(const void* input, const void* words, con
 
 // The converter's tile encoder: 256-weight tiles (FP32, kernel element order) -> the 16-bit state of every position, for
 // the rates the format stores tiles at (tile_words = 16 x bits per weight: 32, 40, 48, 56, 64, 80, 96). The scratch holds
-// one history slab per group of a resident CTA (one CTA per SM, one or two groups that encode side by side).
-static uint32_t encoder_ctas(uint32_t count, uint32_t ka, int sms) {
-    const uint32_t groups = (uint32_t)trellis_encode::groups_of((int)ka);
-    return std::max(1u, std::min((count + groups - 1u) / groups, (uint32_t)sms));
-}
+// a slab of history per tile in flight (one CTA per SM, two tiles each).
+static uint32_t encoder_ctas(uint32_t count, int sms) { return std::min(count, (uint32_t)sms); }
 static uint64_t encoder_scratch(uint32_t count, uint32_t ka, int sms) {
-    return (uint64_t)encoder_ctas(count, ka, sms) * (uint64_t)trellis_encode::groups_of((int)ka) * trellis_encode::history_bytes((int)ka);
+    return std::min((uint64_t)std::max(1u, count), (uint64_t)sms * trellis_encode::kGroups) * trellis_encode::history_bytes((int)ka);
 }
 
 uint64_t euhedral_b200_trellis_encode_scratch_bytes(uint32_t count, uint32_t tile_words) {
@@ -1142,22 +1140,22 @@ int euhedral_b200_trellis_encode_tiles(const void* tiles, uint32_t count, uint32
     DeviceState* state = nullptr;
     const int status = bind(&state);
     if (status != EUHEDRAL_CUDA_SUCCESS) return status;
-    const uint32_t ctas = encoder_ctas(count, ka, state->sms);
     if (encoder_scratch(count, ka, state->sms) > scratch_bytes) return EUHEDRAL_CUDA_SIZE_OVERFLOW;
-    const size_t shared = trellis_encode::shared_bytes((int)ka);
-    auto run = [&](auto kernel) {
-        return launch(kOrdered, kernel, dim3(ctas), dim3(trellis_encode::kThreads), shared, 1u, static_cast<const float*>(tiles), count,
+    auto run = [&](auto kernel, int threads, uint32_t shared) {
+        return launch(kOrdered, kernel, dim3(encoder_ctas(count, state->sms)), dim3(threads), shared, 1u, static_cast<const float*>(tiles), count,
                 static_cast<uint16_t*>(states), static_cast<float*>(decoded), static_cast<uint8_t*>(scratch));
     };
+    auto registers = [&](auto kernel) { return run(kernel, trellis_encode::kRegisterThreads, trellis_encode::register_shared_bytes((int)ka)); };
+    auto shared = [&](auto kernel) { return run(kernel, trellis_encode::kThreads, trellis_encode::shared_bytes((int)ka)); };
     cudaError_t e = cudaErrorInvalidValue;
     switch (tile_words) {
-        case 32: e = run(trellis_encode::viterbi_kernel<2, false>); break;
-        case 40: e = run(trellis_encode::viterbi_kernel<2, true>); break;
-        case 48: e = run(trellis_encode::viterbi_kernel<3, false>); break;
-        case 56: e = run(trellis_encode::viterbi_kernel<3, true>); break;
-        case 64: e = run(trellis_encode::viterbi_kernel<4, false>); break;
-        case 80: e = run(trellis_encode::viterbi_kernel<5, false>); break;
-        case 96: e = run(trellis_encode::viterbi_kernel<6, false>); break;
+        case 32: e = registers(trellis_encode::register_kernel<2, false>); break;
+        case 40: e = registers(trellis_encode::register_kernel<2, true>); break;
+        case 48: e = registers(trellis_encode::register_kernel<3, false>); break;
+        case 56: e = registers(trellis_encode::register_kernel<3, true>); break;
+        case 64: e = registers(trellis_encode::register_kernel<4, false>); break;
+        case 80: e = shared(trellis_encode::viterbi_kernel<5>); break;
+        case 96: e = shared(trellis_encode::viterbi_kernel<6>); break;
     }
     if (e == cudaSuccess && words != nullptr) {
         const uint64_t total = (uint64_t)count * (tile_words / 2u);

@@ -61,6 +61,25 @@ def test_more_tiles_than_ctas_against_the_cpu_restatement(dev, w, ka, mask):
     assert np.array_equal(again, states[count - 8:])
 
 
+@pytest.mark.parametrize("w,ka,mask", RATES)
+@pytest.mark.parametrize("extra", [0, 1, 2])
+def test_tiles_in_flight_against_the_cpu_restatement(dev, w, ka, mask, extra):
+    """One tile alone, as many as CTAs and a few more (a CTA with one tile beside CTAs with two): the states of the whole tiles, tiles of
+    equal weights (every cost ties), weights beyond FP16 (infinite costs) and no weight at all among them."""
+    rng = np.random.default_rng(100 * w + extra)
+    count = [1, dev.gpu.multiprocessor_count() + 2, 2 * dev.gpu.multiprocessor_count() + 3][extra]
+    tiles = rng.standard_normal((count, 256)).astype(np.float32)
+    if count > 1:
+        tiles[1] = 0.25
+        tiles[-1, 100:140] = 1e6
+        tiles[-2] = 0.0
+        tiles[-3, 5] = -70000.0
+    states = encode(dev, tiles, w)
+    for part in (slice(0, 4), slice(-4, None)):
+        expect, _ = OC.trellis_encode_tiles(tiles[part], ka, mask)
+        assert np.array_equal(states[part], expect)
+
+
 def test_status_codes(dev):
     lib = dev.gpu.lib
     tiles = dev.put(np.zeros((2, 256), dtype=np.float32))
