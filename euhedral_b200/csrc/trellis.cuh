@@ -86,18 +86,27 @@ __device__ __forceinline__ void finish128(float (&v)[4], const uint16_t* __restr
 }
 
 // One warp: partials[i * stride + 4 lane ..] of splits i = 0 .. splits - 1 added in that order (read past L1: other SMs
-// wrote them), then finish128.
+// wrote them), then finish128. The loads of kPartialsAhead splits are in flight together: one by one they cost a trip to L2 each, and
+// a finish launch of 20 splits took 7.4 us.
+constexpr int kPartialsAhead = 16;
 __device__ __forceinline__ void add_and_finish128(const float* __restrict__ partials, size_t stride, int splits,
         const uint16_t* __restrict__ svh, uint16_t* __restrict__ out, int lane) {
-    float4 sum = __ldcg(reinterpret_cast<const float4*>(partials) + lane);
-    for (int i = 1; i < splits; ++i) {
-        const float4 part = __ldcg(reinterpret_cast<const float4*>(partials + (size_t)i * stride) + lane);
-        sum.x = __fadd_rn(sum.x, part.x);
-        sum.y = __fadd_rn(sum.y, part.y);
-        sum.z = __fadd_rn(sum.z, part.z);
-        sum.w = __fadd_rn(sum.w, part.w);
+    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int first = 0; first < splits; first += kPartialsAhead) {
+        float4 part[kPartialsAhead];
+#pragma unroll
+        for (int i = 0; i < kPartialsAhead; ++i)
+            if (first + i < splits) part[i] = __ldcg(reinterpret_cast<const float4*>(partials + (size_t)(first + i) * stride) + lane);
+#pragma unroll
+        for (int i = 0; i < kPartialsAhead; ++i) {
+            if (first + i >= splits) break;
+            const bool start = first + i == 0;   // not 0 + the first: a sum of -0 stays one
+            v[0] = start ? part[i].x : __fadd_rn(v[0], part[i].x);
+            v[1] = start ? part[i].y : __fadd_rn(v[1], part[i].y);
+            v[2] = start ? part[i].z : __fadd_rn(v[2], part[i].z);
+            v[3] = start ? part[i].w : __fadd_rn(v[3], part[i].w);
+        }
     }
-    float v[4] = {sum.x, sum.y, sum.z, sum.w};
     finish128(v, svh, out, lane);
 }
 
