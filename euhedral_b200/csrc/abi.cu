@@ -949,9 +949,10 @@ int euhedral_b200_take_device_error(uint32_t* word) {
 
 uint64_t euhedral_b200_static_scratch_bytes(void) { return kStaticScratchBytes; }
 
-// A whole trellis linear as ONE launch. The scratch holds what the K splits exchange: a flag per (column block, split),
-// then the FP32 partials of every split; nothing of it needs clearing (a call's flags carry a tag of its own) and nothing
-// is allocated or freed. With one split the scratch is not touched.
+// A whole trellis linear as one call. With a split count of its own (one wave) it is ONE launch: the scratch holds what the K splits
+// exchange, a flag per (column block, split), then the FP32 partials of every split; nothing of it needs clearing (a call's flags
+// carry a tag of its own). With the caller's count (a host's plan: several waves, where a CTA that waits for flags holds up the
+// next) a second launch adds the splits, and no flags are kept. With one split the scratch is not touched.
 static std::atomic<unsigned long long> g_trellis_tag{0x9E3779B97F4A7C15ull ^ (unsigned long long)(uintptr_t)&g_trellis_tag};
 
 // The split count of a one-launch trellis linear when the caller leaves it open: the one that needs the fewest tile rows
@@ -974,6 +975,10 @@ static uint32_t trellis_default_splits(uint32_t rows, uint32_t in_features, uint
     return best;
 }
 
+// Most rows whose rotation is made inside the linear's launch: every CTA repeats it for its columns, which up to 8 rows costs less than
+// the launch of its own (a layer at one row 129.9 -> 126.4 us; 8320 x 4224 at 17 rows 33.7, repeated 37.6).
+constexpr uint32_t kMostFusedRows = 8;
+
 static uint64_t trellis_flag_bytes(uint32_t out_features, uint32_t splits) {
     return splits > 1u ? ((uint64_t)(out_features / 128u) * splits * 8u + 255u) & ~255ull : 0u;
 }
@@ -995,8 +1000,9 @@ static int trellis_linear(unsigned char* scratch, uint64_t scratch_bytes, const 
     }
     // splits == 0: the count that keeps the SMs' resident CTA slots busiest (trellis_default_splits). (The reference's host
     // aims at 8 blocks per SM, core/.../artifact/format/TrellisFormat.java:369-376; a caller that wants that count passes it.)
+    const bool planned = splits > 1u;   // by the caller
     if (splits == 0u) splits = trellis_default_splits(rows, in_features, out_features, tile_words, state->sms);
-    const uint64_t flags = trellis_flag_bytes(out_features, splits);
+    const uint64_t flags = planned ? 0u : trellis_flag_bytes(out_features, splits);
     const uint64_t partials = splits > 1u ? (uint64_t)splits * rows * out_features * 4u : 0u;
     if (rows > 65535u || segments > 65535u || splits > 65535u || flags + partials > scratch_bytes || ((uintptr_t)scratch & 15u) != 0)
         return EUHEDRAL_CUDA_SIZE_OVERFLOW;
@@ -1006,17 +1012,29 @@ static int trellis_linear(unsigned char* scratch, uint64_t scratch_bytes, const 
     job.ends = static_cast<const int*>(segment_ends);
     job.svh = static_cast<const uint16_t*>(svh);
     job.out = static_cast<uint16_t*>(output);
+    cudaError_t e = cudaSuccess;
     if (splits > 1u) {
-        job.flags = reinterpret_cast<unsigned long long*>(scratch);
         job.partials = reinterpret_cast<float*>(scratch + flags);
-        job.tag = g_trellis_tag.fetch_add(0x9E3779B97F4A7C15ull, std::memory_order_relaxed);
+        if (!planned) {
+            job.flags = reinterpret_cast<unsigned long long*>(scratch);
+            job.tag = g_trellis_tag.fetch_add(0x9E3779B97F4A7C15ull, std::memory_order_relaxed);
+        } else if (rows > kMostFusedRows) {
+            const uint64_t activations = ((uint64_t)segments * rows * in_features * 2u + 255u) & ~255ull;
+            if (activations + partials <= scratch_bytes) {
+                job.activations = reinterpret_cast<const uint16_t*>(scratch);
+                job.partials = reinterpret_cast<float*>(scratch + activations);
+                e = launch_trellis_rotate(input, suh, scratch, (int)rows, (int)in_features, (int)segments, 0);
+            }
+        }
     }
     job.rows = (int)rows;
     job.k = (int)in_features;
     job.n = (int)out_features;
     job.splits = (int)splits;
     job.s = (int)segments;
-    return finish(launch_trellis_linear_width((int)tile_words, static_cast<const uint16_t*>(words), job, state->error_word));
+    if (e == cudaSuccess) e = launch_trellis_linear_width((int)tile_words, static_cast<const uint16_t*>(words), job, state->error_word);
+    if (e == cudaSuccess && planned) e = launch_trellis_finish(job.partials, (int)splits, svh, output, (int)rows, (int)out_features);
+    return finish(e);
 }
 
 // The scratch is the library's own static device array instead of caller memory.

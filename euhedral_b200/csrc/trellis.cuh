@@ -19,7 +19,8 @@
 //     the tensor core (two m16n8k32 u8 MMAs against a 0/1 selector, accumulator preset to the FP16 bit pattern 0x6400),
 //     which also hands each lane the values in the order of its FP16 A fragment; the 16 k of a tile reach the FP16 MMA in
 //     a fixed permutation that the activations in shared memory follow.
-//   * The K splits meet without a second launch and without a counter that would need clearing: a CTA stores its FP32
+//   * The K splits of a host's plan, several waves of CTAs, are added by a finish launch. Those of the count that a call picks itself
+//     (one wave) meet without a second launch and without a counter that would need clearing: a CTA stores its FP32
 //     partials, publishes a flag holding this call's tag, and reads the flags of its column block; whoever sees all of
 //     them set adds the partials in split order, rotates, scales and writes BF16, then unsets the flags (a launch replayed
 //     from a CUDA graph carries the same tag again). Two CTAs that finish together may both do that; they write the same bits.

@@ -215,15 +215,15 @@ class _TrellisLaunch:
         partials = 0 if splits == 1 else splits * self.rows * self.n * 4
         self._require_scratch(activations + partials)
         scratch = self.launch.scratch
+        if splits > 1:
+            # The three launches below as one call of the library: queued one by one from here they take the host 27 us.
+            self.gpu.linear_trellis_bf16(self.launch.input, self.words, self.suh, self.svh, self.ends, self.launch.output, scratch,
+                                         activations + partials, self.rows, self.k, self.n, self.w, self.segments, splits)
+            return
         self.prepass(scratch, TrellisFormat.FRAGMENT_FP16)
         self.gpu.launch_table_kernel(
             "TRELLIS_MMA", self.n // layouts.TRELLIS_BLOCK, splits, 1, 256, 1, 1, 0,
             KernelArguments().pointer(scratch).pointer(self.words).pointer(self.ends).pointer(self.svh)
             .pointer(scratch + activations).pointer(self.launch.output).int32(self.rows).int32(self.k).int32(self.n)
             .int32(self.w).int32(splits).int32(self.segments))
-        if splits == 1:
-            return
-        self.gpu.launch_table_kernel(
-            "TRELLIS_EPILOGUE", -(-self.n // TrellisFormat.EPILOGUE_BLOCK_COLUMNS), self.rows, 1, 128, 1, 1, 0,
-            KernelArguments().pointer(scratch + activations).int32(splits).pointer(self.svh).pointer(self.launch.output)
-            .int32(self.rows).int32(self.n))
+

@@ -171,6 +171,35 @@ def test_one_call_linear_is_bitwise_the_table_launches(dev):
         assert lib.euhedral_b200_linear_trellis_bf16(d_x.data_ptr(), t[0], t[1], t[2], t[3], d_y.data_ptr(), d_s.data_ptr(), 1024, 2, k, n, w, 2, 0) == -2
 
 
+@pytest.mark.parametrize("k,n,w,ends,target", [(2048, 512, 48, [256, 512], 140), (1408, 384, 64, [384], 64), (4224, 256, 56, [128, 256], 8), (1024, 640, 128, [640], 1)])
+@pytest.mark.parametrize("rows", [1, 8, 9, 16, 17, 24, 25, 32, 33, 48, 49, 63])
+def test_operator_is_bitwise_the_table_launches(dev, k, n, w, ends, target, rows):
+    """What the operator queues as one call against the plan's launches through the kernel table, on both sides of every group of eight
+    rows that a launch holds; in the operator's scratch and in one that has room for the partial sums only."""
+    rng = np.random.default_rng(1000 * rows + k)
+    payload, suh, svh = random_object(rng, k, n, w, segments=len(ends))
+    linear = DeviceLinear(dev, payload, suh, svh, ends, target)
+    x = random_x(rng, rows, k)
+    splits = TrellisFormat.splits(k, n, target)
+    words, d_suh, d_svh, d_ends = [t.data_ptr() for t in linear.tensors]
+    d_x, d_act, d_part, d_y = dev.put(x), dev.empty(len(ends) * rows * k * 2), dev.empty(max(splits * rows * n * 4, 16)), dev.empty(rows * n * 2)
+    with dev.submit(pdl=True) as gpu:
+        gpu.launch_table_kernel("TRELLIS_PREPASS", (k + 511) // 512, rows, len(ends), 128, 1, 1, 0,
+                                KernelArguments().pointer(d_x.data_ptr()).pointer(d_suh).pointer(d_act.data_ptr()).int32(rows).int32(k).int32(len(ends)).int32(0))
+        gpu.launch_table_kernel("TRELLIS_MMA", n // 128, splits, 1, 256, 1, 1, 0,
+                                KernelArguments().pointer(d_act.data_ptr()).pointer(words).pointer(d_ends).pointer(d_svh).pointer(d_part.data_ptr())
+                                .pointer(d_y.data_ptr()).int32(rows).int32(k).int32(n).int32(w).int32(splits).int32(len(ends)))
+        if splits > 1:
+            gpu.launch_table_kernel("TRELLIS_EPILOGUE", (n + 511) // 512, rows, 1, 128, 1, 1, 0,
+                                    KernelArguments().pointer(d_part.data_ptr()).int32(splits).pointer(d_svh).pointer(d_y.data_ptr()).int32(rows).int32(n))
+    expect = dev.get(d_y, np.uint16, (rows, n))
+    assert np.array_equal(linear.linear(x), expect)
+    with dev.submit(pdl=True) as gpu:
+        gpu.linear_trellis_bf16(d_x.data_ptr(), words, d_suh, d_svh, d_ends, d_y.data_ptr(), d_part.data_ptr(), splits * rows * n * 4, rows, k, n, w,
+                                len(ends), splits)
+    assert np.array_equal(dev.get(d_y, np.uint16, (rows, n)), expect)
+
+
 def test_golden_linear_fixture(dev, golden):
     g = golden("trellis")
     linear = DeviceLinear(dev, g["linear_payload"], g["linear_suh"], g["linear_svh"], [256], 140)
