@@ -65,6 +65,8 @@ cudaError_t allow_big_smem(K kernel) {
 template <int W>
 cudaError_t allow_trellis_width() {
     cudaError_t e = allow_big_smem(trellis::linear_kernel<W, 1>);
+    if (e == cudaSuccess) e = allow_big_smem(trellis::linear_kernel<W, 2>);
+    if (e == cudaSuccess) e = allow_big_smem(trellis::linear_kernel<W, 3>);
     if (e == cudaSuccess) e = allow_big_smem(trellis::linear_kernel<W, 4>);
     return e;
 }
@@ -396,9 +398,13 @@ cudaError_t launch_trellis_linear(const uint16_t* words, const trellis::Job& job
     if (map == nullptr) return cudaErrorNotSupported;
     const dim3 grid((unsigned)(job.n / 128), (unsigned)job.splits), block(trellis::kThreads);
     const size_t stages = (size_t)trellis::kStages * trellis::kStageTiles * 16u * W;
-    if (job.rows <= 8)
-        return launch(kOverlappable, trellis::linear_kernel<W, 1>, grid, block, stages + trellis::act_bytes(1), 1u, *map, job, error);
-    return launch(kOverlappable, trellis::linear_kernel<W, 4>, grid, block, stages + trellis::act_bytes(4), 1u, *map, job, error);
+    auto run = [&](auto kernel, int groups) { return launch(kOverlappable, kernel, grid, block, stages + trellis::act_bytes(groups), 1u, *map, job, error); };
+    switch (trellis::groups_of(job.rows)) {
+        case 1: return run(trellis::linear_kernel<W, 1>, 1);
+        case 2: return run(trellis::linear_kernel<W, 2>, 2);
+        case 3: return run(trellis::linear_kernel<W, 3>, 3);
+        default: return run(trellis::linear_kernel<W, 4>, 4);
+    }
 }
 
 cudaError_t launch_trellis_linear_width(int w, const uint16_t* words, const trellis::Job& job, uint32_t* error) {
@@ -959,9 +965,9 @@ static std::atomic<unsigned long long> g_trellis_tag{0x9E3779B97F4A7C15ull ^ (un
 // per SM slot in sequence - waves of resident CTAs times the tile rows of a split, plus a few tile rows' worth of rotate,
 // flag exchange and in-order sum for every split - among splits of 20 tile rows or more.
 static uint32_t trellis_default_splits(uint32_t rows, uint32_t in_features, uint32_t out_features, uint32_t tile_words, int sms) {
-    const uint32_t groups = rows <= 8u ? 1u : 4u;
+    const uint32_t groups = (uint32_t)trellis::groups_of((int)rows);
     const uint32_t shared = (uint32_t)trellis::kStages * trellis::kStageTiles * 16u * tile_words + trellis::act_bytes((int)groups) + 1024u + 128u;
-    const uint32_t per_sm = std::max(1u, std::min(groups == 1u ? (uint32_t)trellis::kResident : 2u, (uint32_t)kGemvSmem / shared));
+    const uint32_t per_sm = std::max(1u, std::min((uint32_t)trellis::kResident, (uint32_t)kGemvSmem / shared));
     const uint32_t resident = per_sm * (uint32_t)sms, blocks = out_features / 128u, tiles = in_features / 16u;
     uint32_t best = 1u, best_cost = 0xFFFFFFFFu;
     for (uint32_t splits = 1u; splits <= std::max(1u, tiles / 20u); ++splits) {

@@ -38,14 +38,22 @@ namespace trellis {
 
 constexpr int kStageTiles = 16;                       // tile rows (k16 steps) per streaming stage
 constexpr int kStages = 3;
-constexpr int kResident = 3;                          // CTAs of up to 8 rows an SM holds (72 registers a thread)
+constexpr int kResident = 3;                          // CTAs an SM holds (72 registers a thread; shared memory up to 64-word tiles)
 constexpr int kUnroll = 8;                            // tiles decoded per trip of the inner loop
 constexpr int kChunkLimit = 512;                      // most tile rows whose activations are in shared memory at once
 constexpr int kDecodeWarps = 8;                       // one per tile column of the CTA's 128 output columns
 constexpr int kThreads = 32 * (kDecodeWarps + 1);     // and the warp that requests the payload
 // Shared memory for the activations of a chunk: the live rows only, each chunk * 32 + 32 bytes long (32 modulo 128: the
-// 8 rows x 4 quads of one load tile the banks). 8 rows get 64 tile rows, 5 rows 96, one row 512; 32 rows get 32.
-__host__ __device__ constexpr uint32_t act_bytes(int groups) { return groups == 1 ? 8u * (64u * 32u + 32u) : 32u * (32u * 32u + 32u); }
+// 8 rows x 4 quads of one load tile the banks). 8 rows get 64 tile rows, 5 rows 96, one row 512; 32 rows get 24.
+// Groups of 8 rows are held as 1 to 4, the fewest that take the same number of passes over the payload as four do: with four for every
+// count from 9 on, and 2 CTAs an SM, 17408 x 5120 at 12 / 16 / 20 / 24 rows took 58 / 64 / 67 / 72 us, now 47 / 50 / 56 / 61.
+__host__ __device__ constexpr uint32_t act_bytes(int groups) {
+    return groups == 1 ? 8u * (64u * 32u + 32u) : groups == 2 ? 16u * (48u * 32u + 32u) : groups == 3 ? 24u * (32u * 32u + 32u) : 32u * (24u * 32u + 32u);
+}
+__host__ __device__ constexpr int groups_of(int rows) {
+    const int all = (rows + 7) / 8, passes = (all + 3) / 4;
+    return (all + passes - 1) / passes;
+}
 __host__ __device__ inline int chunk_tiles(int groups, int live) {
     const int fit = (int)((act_bytes(groups) / (uint32_t)live - 32u) / 32u) & ~7;
     return fit < kChunkLimit ? fit : kChunkLimit;
@@ -414,7 +422,7 @@ __device__ __forceinline__ void decoders_sync() { asm volatile("bar.sync 1, %0;"
 // P = groups of 8 activation rows held at once (rows beyond 8 P take another pass over the payload).
 //   grid (n / 128, splits), block kThreads, dynamic shared kStages * kStageTiles * 16 W + act_bytes(P) bytes.
 template <int W, int P>
-__global__ void __launch_bounds__(kThreads, P == 1 ? kResident : 2) linear_kernel(const __grid_constant__ CUtensorMap payload_map,
+__global__ void __launch_bounds__(kThreads, kResident) linear_kernel(const __grid_constant__ CUtensorMap payload_map,
         const __grid_constant__ Job job, uint32_t* __restrict__ error) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr uint32_t kTileBytes = 2u * W, kTileRowBytes = 8u * kTileBytes, kStageBytes = kStageTiles * kTileRowBytes;
