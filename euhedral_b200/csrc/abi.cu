@@ -446,13 +446,14 @@ cudaError_t launch_trellis_rotate(const void* x, const void* suh, void* act, int
             static_cast<const uint16_t*>(x), static_cast<const uint16_t*>(suh), static_cast<uint16_t*>(act), rows, k, s, layout);
 }
 
-cudaError_t launch_trellis_decode_bf16(const void* words, void* out, int k, int n, int w, bool beside) {
-    const uint64_t tiles = (uint64_t)(k / 16) * (uint64_t)(n / 16);
+cudaError_t launch_trellis_decode_bf16(const void* words, void* out, int k, int n, int w, bool beside, int sms) {
+    const uint64_t units = (uint64_t)((k / 16 + trellis::kBatch - 1) / trellis::kBatch) * (uint64_t)(n / 16);
+    const dim3 grid((unsigned)std::min<uint64_t>((units + 7) / 8, (uint64_t)sms * trellis::kDecodeResident));
     switch (w) {
 #define EB_CASE(W) \
         case W: \
-            return launch(kOverlappable, trellis::decode_bf16_kernel<W>, dim3((unsigned)((tiles + 8 * trellis::kBatch - 1) / (8 * trellis::kBatch))), dim3(256), 0, 1u, \
-                    static_cast<const uint16_t*>(words), static_cast<uint16_t*>(out), k, n, beside ? 1 : 0);
+            return launch(kOverlappable, trellis::decode_bf16_kernel<W>, grid, dim3(256), 0, 1u, static_cast<const uint16_t*>(words), static_cast<uint16_t*>(out), \
+                    k, n, beside ? 1 : 0);
         EB_TRELLIS_WIDTHS(EB_CASE)
 #undef EB_CASE
         default: return cudaErrorInvalidValue;
@@ -917,7 +918,7 @@ int euhedral_cuda_linear_launch(int32_t kernel, uint32_t grid_x, uint32_t grid_y
                 return EUHEDRAL_CUDA_INVALID_ARGUMENT;   // 4-byte loads of the ring words, 16-byte stores of eight values
             const uint64_t tiles = (uint64_t)(k / 16) * (uint64_t)(n / 16);
             if (tiles > 2147483647ull) return EUHEDRAL_CUDA_SIZE_OVERFLOW;
-            return finish(launch_trellis_decode_bf16(reinterpret_cast<const void*>(a[0]), reinterpret_cast<void*>(a[1]), k, n, w, false));
+            return finish(launch_trellis_decode_bf16(reinterpret_cast<const void*>(a[0]), reinterpret_cast<void*>(a[1]), k, n, w, false, state->sms));
         }
         case 6: {   // epilogue_bf16(rotated, ends, s, svh, out, rows, n)
             const int s = (int)a[2], rows = (int)a[5], n = (int)a[6];
@@ -1122,7 +1123,7 @@ int euhedral_b200_prefill_trellis_bf16(const void* input, const void* words, con
     uint8_t* activations = static_cast<uint8_t*>(scratch);
     uint8_t* decoded = activations + align_scratch((uint64_t)segments * rows * k * 2u);
     cudaError_t e = launch_trellis_rotate(input, suh, activations, (int)rows, (int)k, (int)segments, 1);
-    if (e == cudaSuccess) e = launch_trellis_decode_bf16(words, decoded, (int)k, (int)n, (int)tile_words, true);
+    if (e == cudaSuccess) e = launch_trellis_decode_bf16(words, decoded, (int)k, (int)n, (int)tile_words, true, state->sms);
     const bool pdl = t_pdl != 0 && t_stream != nullptr;
     // the GEMM takes up to kMaxSegments segments a launch
     start = 0;

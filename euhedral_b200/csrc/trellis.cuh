@@ -58,7 +58,8 @@ __host__ __device__ inline int chunk_tiles(int groups, int live) {
     const int fit = (int)((act_bytes(groups) / (uint32_t)live - 32u) / 32u) & ~7;
     return fit < kChunkLimit ? fit : kChunkLimit;
 }
-constexpr int kBatch = 4;                             // tiles a warp of the BF16 decode takes side by side
+constexpr int kDecodeResident = 3;                    // CTAs of the BF16 decode an SM holds: 4 and 5 leave too few registers (106 and 107 us)
+constexpr int kBatch = 4;                             // tiles along k that a warp of the BF16 decode takes at a time
 constexpr uint32_t kWaitFailed = 4u;                  // error bit: a stage did not arrive (or was never freed)
 
 // ---- pieces shared by the one-kernel linear and the table entries -------------------------------------------------------
@@ -324,80 +325,97 @@ struct Lane {
 #pragma unroll
         for (int i = 0; i < kWords; ++i) u[i] = eb::lds_u32<OFFSET>(tile + at[i]);
         align(u);
+        uint32_t packed[4];
+        sums(u, select, packed);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const __half2 v = value(packed[i]);
+            a[i] = *reinterpret_cast<const uint32_t*>(&v);
+        }
+    }
+
+    // The byte sums of the lane's eight products over 0x6400, in pairs: what lane q's columns 2q and 2q + 1 of the selector take, for
+    // positions 0, 1 (row g, then g + 8: positions 4, 5) and 2, 3 (6, 7).
+    __device__ __forceinline__ static void sums(const uint32_t (&u)[kWords + 1], const uint32_t (&take)[2], uint32_t (&packed)[4]) {
         constexpr uint32_t kHash = 0x83DCD12Du;
         const uint32_t p0 = state<0>(u) * kHash, p1 = state<1>(u) * kHash, p2 = state<2>(u) * kHash, p3 = state<3>(u) * kHash;
         const uint32_t p4 = state<4>(u) * kHash, p5 = state<5>(u) * kHash, p6 = state<6>(u) * kHash, p7 = state<7>(u) * kHash;
         // Positions 0..3 are tile row g (k = 2q, 2q+1, 2q+8, 2q+9), 4..7 the same k of row g + 8.
         uint32_t low[4], high[4];
-        eb::mma_u8_16832_from(low, p0, p4, p1, p5, select[0], select[1], 0x6400u);    // k = 2q' and 2q'+1 of every lane q'
-        eb::mma_u8_16832_from(high, p2, p6, p3, p7, select[0], select[1], 0x6400u);   // k = 2q'+8 and 2q'+9
-        const __half2 slope = __half2half2(__ushort_as_half((unsigned short)0x1EEE)), offset = __half2half2(__ushort_as_half((unsigned short)0xC931));
+        eb::mma_u8_16832_from(low, p0, p4, p1, p5, take[0], take[1], 0x6400u);    // k = 2q' and 2q'+1 of every lane q'
+        eb::mma_u8_16832_from(high, p2, p6, p3, p7, take[0], take[1], 0x6400u);   // k = 2q'+8 and 2q'+9
         // half of them by each of the two pipes that can
-        const uint32_t packed[4] = {__byte_perm(low[0], low[1], 0x5410), __byte_perm(low[2], low[3], 0x5410), pair_by_multiplying(high[0], high[1]),
-                pair_by_multiplying(high[2], high[3])};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const __half2 value = __hfma2(*reinterpret_cast<const __half2*>(&packed[i]), slope, offset);
-            a[i] = *reinterpret_cast<const uint32_t*>(&value);
-        }
+        packed[0] = __byte_perm(low[0], low[1], 0x5410), packed[1] = __byte_perm(low[2], low[3], 0x5410);
+        packed[2] = pair_by_multiplying(high[0], high[1]), packed[3] = pair_by_multiplying(high[2], high[3]);
+    }
+    // The codebook's values of two sums.
+    __device__ __forceinline__ static __half2 value(uint32_t packed) {
+        return __hfma2(*reinterpret_cast<const __half2*>(&packed), __half2half2(__ushort_as_half((unsigned short)0x1EEE)),
+                __half2half2(__ushort_as_half((unsigned short)0xC931)));
     }
 };
 
-// Payload -> BF16 rotated weight [n][k] (row-major weights of a BF16 linear). A warp takes kBatch tiles side by side: a lane
-// reads its ring words of all of them from global memory first, then takes its eight states of each as the linear does and
-// stores 16 contiguous bytes of one weight row (the quad's pairs regrouped through shared memory).
+// Payload -> BF16 rotated weight [n][k] (row-major weights of a BF16 linear). A warp takes units of four tiles that follow one
+// another along k, so that each of the 16 weight rows gets a whole line of 128 bytes: a lane decodes its eight states of each tile (the
+// byte sums by the tensor core as in the linear, with a selector that hands them back to the lane), and the pairs meet in shared
+// memory. The warps stay for all units; the ring words of the next
+// unit are on their way while one is decoded. Bound: writing the weight (34816 x 5120 at 4 bits: 446 MB in 95 us, 0.72 of a plain
+// copy); with one batch of tiles a warp, 32-byte pieces of rows and the byte sums on the integer pipe latency bound it, 137 us.
 // `beside`: the launch in front of this one neither writes what this one reads nor reads what it writes (the prefill's rotate), so
 // both may run at a time.
-//   grid ceil((k / 16) * (n / 16) / (8 kBatch)), block 256.
+//   grid: any, block 256.
 template <int W>
-__global__ void __launch_bounds__(256) decode_bf16_kernel(const uint16_t* __restrict__ words, uint16_t* __restrict__ out, int k, int n,
+__global__ void __launch_bounds__(256, kDecodeResident) decode_bf16_kernel(const uint16_t* __restrict__ words, uint16_t* __restrict__ out, int k, int n,
         int beside) {
     using L = Lane<W>;
     const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-    constexpr int kExchangePitch = 40;   // words of an exchange row: 32 lanes + 8, so that a quarter warp's 16-byte loads tile the banks
-    __shared__ __align__(16) uint32_t exchange_rows[8][4 * kExchangePitch];
+    constexpr uint32_t kPitch = 36;   // words of an exchange row: 128 bytes + 16, so that the lanes' stores tile the banks
+    __shared__ __align__(16) uint32_t exchange_rows[8][16 * kPitch];
     uint32_t* exchange = exchange_rows[threadIdx.x >> 5];
-    const uint32_t first = (blockIdx.x * 8u + (threadIdx.x >> 5)) * (uint32_t)kBatch, tiles = (uint32_t)(k >> 4) * (uint32_t)(n >> 4);   // < 2^31
+    const uint32_t across = (uint32_t)n >> 4, down = (uint32_t)k >> 4, units = (down + kBatch - 1u) / kBatch * across, step = gridDim.x * 8u;   // < 2^31 tiles
     eb::pdl_launch_dependents();
     if (beside == 0) eb::pdl_wait();
-    if (first >= tiles) {
-        eb::pdl_wait();
-        return;
-    }
     L me;
     me.init(lane);
-    uint32_t u[kBatch][L::kWords + 1];
+    const uint32_t own[2] = {g == 2 * q ? 0x01010101u : 0u, g == 2 * q + 1 ? 0x01010101u : 0u};
+    uint32_t ahead[kBatch][L::kWords];
+    auto load = [&](uint32_t unit) {
+        const uint32_t along = unit / across;
 #pragma unroll
-    for (int t = 0; t < kBatch; ++t) {
-        const uint32_t tile = first + t < tiles ? first + t : tiles - 1u;
-        const uint8_t* ring = reinterpret_cast<const uint8_t*>(words + (size_t)tile * W);
+        for (int t = 0; t < kBatch; ++t) {
+            const uint8_t* ring = reinterpret_cast<const uint8_t*>(words + ((size_t)min(along * kBatch + t, down - 1u) * across + (unit - along * across)) * W);
 #pragma unroll
-        for (int i = 0; i < L::kWords; ++i) u[t][i] = __ldg(reinterpret_cast<const uint32_t*>(ring + me.at[i]));
-    }
-#pragma unroll
-    for (int t = 0; t < kBatch; ++t) {
-        const uint32_t tile = first + t;
-        if (tile >= tiles) break;
-        const int ti = (int)(tile / (uint32_t)(n >> 4)), tj = (int)(tile % (uint32_t)(n >> 4));
-        me.align(u[t]);
-        const uint32_t state[8] = {L::template state<0>(u[t]), L::template state<1>(u[t]), L::template state<2>(u[t]), L::template state<3>(u[t]),
-                L::template state<4>(u[t]), L::template state<5>(u[t]), L::template state<6>(u[t]), L::template state<7>(u[t])};
-        uint32_t pair[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint32_t values = value_pair(state[2 * j], state[2 * j + 1]);   // two FP16 codebook values
-            const float2 wide = __half22float2(*reinterpret_cast<const __half2*>(&values));
-            pair[j] = eb::bf16_pair(wide.x, wide.y);
+            for (int i = 0; i < L::kWords; ++i) ahead[t][i] = __ldg(reinterpret_cast<const uint32_t*>(ring + me.at[i]));
         }
-        // positions 0..3 are tile row g at k = 2q, 2q+1, 2q+8, 2q+9; positions 4..7 the same k of row g + 8. The four lanes of a
-        // quad trade their pairs through shared memory so that each stores 16 contiguous bytes: lane q gets pair q of all
-        // four, i.e. k 0..7 (q = 0) or 8..15 (q = 1) of row g, or the same of row g + 8 (q = 2, 3).
-        __syncwarp();   // the tile before has been read out of the exchange rows
+    };
+    uint32_t unit = blockIdx.x * 8u + (threadIdx.x >> 5);
+    if (unit < units) load(unit);
+    for (; unit < units; unit += step) {
+        uint32_t now[kBatch][L::kWords + 1];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) exchange[j * kExchangePitch + lane] = pair[j];
+        for (int t = 0; t < kBatch; ++t)
+#pragma unroll
+            for (int i = 0; i < L::kWords; ++i) now[t][i] = ahead[t][i];
+        if (unit + step < units) load(unit + step);
+        __syncwarp();   // the unit before has been read out of the exchange rows
+#pragma unroll
+        for (int t = 0; t < kBatch; ++t) {
+            me.align(now[t]);
+            uint32_t packed[4];   // row g at k = 2q, 2q+1; row g + 8; row g at k = 2q+8, 2q+9; row g + 8
+            L::sums(now[t], own, packed);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const __half2 value = L::value(packed[j]);
+                const float2 wide = __half22float2(value);
+                exchange[(g + 8 * (j & 1)) * kPitch + 8 * t + 4 * (j >> 1) + q] = eb::bf16_pair(wide.x, wide.y);
+            }
+        }
         __syncwarp();
-        const uint4 mine = *reinterpret_cast<const uint4*>(exchange + q * kExchangePitch + 4 * g);
-        *reinterpret_cast<uint4*>(out + (size_t)(tj * 16 + g + 8 * (q >> 1)) * k + ti * 16 + 8 * (q & 1)) = mine;
+        const uint32_t along = unit / across, row = (uint32_t)lane >> 3, piece = (uint32_t)lane & 7u;
+        uint16_t* to = out + (size_t)((unit - along * across) * 16u + row) * (uint32_t)k + along * 64u + piece * 8u;
+#pragma unroll
+        for (uint32_t i = 0; i < 16u; i += 4u)
+            if (along * 64u + piece * 8u < (uint32_t)k) *reinterpret_cast<uint4*>(to + (size_t)i * (uint32_t)k) = *reinterpret_cast<const uint4*>(exchange + (row + i) * kPitch + piece * 4u);
     }
     eb::pdl_wait();   // the launch behind waits for this one: when it runs, the one in front has ended too
 }

@@ -171,6 +171,21 @@ def test_one_call_linear_is_bitwise_the_table_launches(dev):
         assert lib.euhedral_b200_linear_trellis_bf16(d_x.data_ptr(), t[0], t[1], t[2], t[3], d_y.data_ptr(), d_s.data_ptr(), 1024, 2, k, n, w, 2, 0) == -2
 
 
+@pytest.mark.parametrize("k,n", [(16, 16), (48, 32), (80, 4112), (64, 16), (1040, 272), (4096, 2064)])
+@pytest.mark.parametrize("w", [24, 64, 128])
+def test_decode_bf16_of_odd_sizes(dev, w, k, n):
+    """Fewer tiles along k than a warp takes at a time, a last unit that is not whole, more units than warps."""
+    rng = np.random.default_rng(k * n + w)
+    payload = rng.integers(0, 65536, (k // 16, n // 16, w), dtype=np.uint16)
+    d_words, d_out = dev.put(payload.astype("<i2")), dev.put(np.full(n * k + 64, 0x1234, dtype=np.uint16))
+    with dev.submit() as gpu:
+        gpu.launch_table_kernel("TRELLIS_DECODE_BF16", (k // 16) * (n // 16), 1, 1, 256, 1, 1, 0,
+                                KernelArguments().pointer(d_words.data_ptr()).pointer(d_out.data_ptr()).int32(k).int32(n).int32(w))
+    got = dev.get(d_out, np.uint16, (n * k + 64,))
+    assert np.array_equal(got[:n * k].reshape(n, k), O.bf16_bits(O.trellis_rotated_weight(payload).astype(np.float32).T))
+    assert np.all(got[n * k:] == 0x1234)
+
+
 @pytest.mark.parametrize("k,n,w,ends,target", [(2048, 512, 48, [256, 512], 140), (1408, 384, 64, [384], 64), (4224, 256, 56, [128, 256], 8), (1024, 640, 128, [640], 1)])
 @pytest.mark.parametrize("rows", [1, 8, 9, 16, 17, 24, 25, 32, 33, 48, 49, 63])
 def test_operator_is_bitwise_the_table_launches(dev, k, n, w, ends, target, rows):
