@@ -133,30 +133,35 @@ cudaError_t launch(Overlap overlap, void (*kernel)(Params...), dim3 grid, dim3 b
 // clusters of `split`), and the shared-memory request.
 struct DecodePlan {
     gemv::Order order;
-    uint32_t warps, depth, ctas, span, shared;
+    uint32_t warps, depth, ctas, span, shared, box;   // box: chunks of a ring slot
     bool tma_scales;
 };
 
 template <class F>
 using GemvKernel = void (*)(const gemv::Group, uint32_t*);
 
+// Chunks of a ring slot that holds a part of a piece: the rows of 1 and 3 chunks keep the shared-memory loads free of bank conflicts.
+constexpr int part_box(int piece) { return piece >= 4 ? 3 : piece; }
+
 template <class F, int P>
-GemvKernel<F> gemv_kernel_from(uint32_t piece, bool tma_scales) {
+GemvKernel<F> gemv_kernel_from(uint32_t piece, uint32_t box, bool tma_scales) {
     if constexpr (P > (int)F::kMaxPiece) {
         return nullptr;
     } else {
-        if (piece == (uint32_t)P) return tma_scales ? gemv::kernel<F, P, true> : gemv::kernel<F, P, false>;
-        return gemv_kernel_from<F, P + 1>(piece, tma_scales);
+        if (piece == (uint32_t)P && box == piece) return tma_scales ? gemv::kernel<F, P, P, true> : gemv::kernel<F, P, P, false>;
+        if (piece == (uint32_t)P) return tma_scales ? gemv::kernel<F, P, part_box(P), true> : gemv::kernel<F, P, part_box(P), false>;
+        return gemv_kernel_from<F, P + 1>(piece, box, tma_scales);
     }
 }
 template <class F>
-GemvKernel<F> gemv_kernel(uint32_t piece, bool tma_scales) { return gemv_kernel_from<F, 1>(piece, tma_scales); }
+GemvKernel<F> gemv_kernel(uint32_t piece, uint32_t box, bool tma_scales) { return gemv_kernel_from<F, 1>(piece, box, tma_scales); }
 
 template <class F>
 cudaError_t allow_gemv() {
     cudaError_t e = cudaSuccess;
     for (uint32_t piece = 1; piece <= F::kMaxPiece && e == cudaSuccess; ++piece)
-        for (int tma = 0; tma < 2 && e == cudaSuccess; ++tma) e = cudaFuncSetAttribute(gemv_kernel<F>(piece, tma != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvSmem);
+        for (int i = 0; i < 4 && e == cudaSuccess; ++i)
+            e = cudaFuncSetAttribute(gemv_kernel<F>(piece, i & 2 ? piece : (uint32_t)part_box((int)piece), (i & 1) != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvSmem);
     return e;
 }
 
@@ -175,10 +180,12 @@ bool plan_decode(uint32_t rows, uint32_t k, uint32_t tiles, uint32_t widest, int
     if (!order.ok) return false;
     plan->order = order;
     plan->tma_scales = typename F::Geometry(16, k).scale_row_bytes % 16u == 0;
-    const GemvKernel<F> kernel = gemv_kernel<F>(order.piece, plan->tma_scales);
-    if (kernel == nullptr) return false;
+    // As many warps as there can be; then slots of whole pieces before slots of parts, deeper rings before shallower ones.
     for (uint32_t warps = gemv::kMaxWarps; warps >= order.team; warps >>= 1) {
-        for (uint32_t depth = 3; depth >= 2; --depth) {
+        for (uint32_t choice = 0; choice < 4u; ++choice) {
+            const uint32_t box = choice < 2u ? order.piece : (uint32_t)part_box((int)order.piece), depth = 3u - (choice & 1u);
+            const GemvKernel<F> kernel = gemv_kernel<F>(order.piece, box, plan->tma_scales);
+            if (kernel == nullptr) return false;
             // The gather buffer grows with a cluster's share of the tallest tensor, which depends on the cluster count,
             // which can depend on the shared-memory request: settle in two rounds.
             uint32_t clusters = std::min<uint32_t>(std::max(1u, (uint32_t)sms / order.split), tiles);
@@ -186,7 +193,7 @@ bool plan_decode(uint32_t rows, uint32_t k, uint32_t tiles, uint32_t widest, int
             bool fits = true;
             for (int round = 0; round < 2 && fits; ++round) {
                 span = std::min(widest, (tiles + clusters - 1u) / clusters + 1u);
-                shared = gemv::Layout<F>(order, rows, warps, depth, span).bytes;
+                shared = gemv::Layout<F>(order, rows, warps, depth, span, box).bytes;
                 if (shared > (uint32_t)kGemvSmem) {
                     fits = false;
                     break;
@@ -201,6 +208,7 @@ bool plan_decode(uint32_t rows, uint32_t k, uint32_t tiles, uint32_t widest, int
             if (!fits) continue;
             plan->warps = warps;
             plan->depth = depth;
+            plan->box = box;
             plan->ctas = clusters * order.split;
             plan->span = span;
             plan->shared = shared;
@@ -220,7 +228,7 @@ template <class F>
 const gemv::Tensor* cached_tensor(const void* w, uint32_t n, uint32_t k, const DecodePlan& plan, bool* device_memory) {
     struct Cached {
         const void* weights;
-        uint32_t n, k, format, piece;
+        uint32_t n, k, format, box;
         int device;
         bool tma_scales, device_memory;
         gemv::Tensor tensor;
@@ -230,18 +238,18 @@ const gemv::Tensor* cached_tensor(const void* w, uint32_t n, uint32_t k, const D
     int device = 0;
     (void)cudaGetDevice(&device);
     Cached& slot = cache[(uint32_t)(((uintptr_t)w >> 8) * 0x9E3779B1u >> 16) % kCached];
-    if (slot.weights != w || slot.n != n || slot.k != k || slot.format != F::kErrorBit || slot.piece != plan.order.piece
+    if (slot.weights != w || slot.n != n || slot.k != k || slot.format != F::kErrorBit || slot.box != plan.box
             || slot.tma_scales != plan.tma_scales || slot.device != device) {
         cudaPointerAttributes attributes;
         bool plain = cudaPointerGetAttributes(&attributes, w) == cudaSuccess && attributes.type == cudaMemoryTypeDevice;
         (void)cudaGetLastError();
         slot.weights = nullptr;
-        if (plain && !gemv::encode_tensor<F>(&slot.tensor, w, n, k, plan.order, plan.tma_scales)) return nullptr;
+        if (plain && !gemv::encode_tensor<F>(&slot.tensor, w, n, k, plan.box, plan.tma_scales)) return nullptr;
         slot.weights = w;
         slot.n = n;
         slot.k = k;
         slot.format = F::kErrorBit;
-        slot.piece = plan.order.piece;
+        slot.box = plan.box;
         slot.tma_scales = plan.tma_scales;
         slot.device = device;
         slot.device_memory = plain;
@@ -290,7 +298,7 @@ cudaError_t launch_gemv(const DecodeItem* items, uint32_t count, uint32_t rows, 
     group.tiles = tiles;
     group.depth = plan.depth;
     group.span = plan.span;
-    return launch(kOverlappable, gemv_kernel<F>(plan.order.piece, plan.tma_scales), dim3(plan.ctas), dim3(32u * plan.warps), plan.shared,
+    return launch(kOverlappable, gemv_kernel<F>(plan.order.piece, plan.box, plan.tma_scales), dim3(plan.ctas), dim3(32u * plan.warps), plan.shared,
             plan.order.split, group, error);
 }
 

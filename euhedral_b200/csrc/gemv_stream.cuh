@@ -12,6 +12,9 @@
 // Execution:
 //   * One CTA per SM (a cluster of S CTAs when S > 1, rank r staging and streaming slice r only). The 16-row tiles of
 //     all tensors of the group form one list, cut evenly over the CTAs (clusters): a CTA walks a contiguous run of it.
+//   * A slot holds a whole piece where sixteen warps' rings of them fit beside the activations, else the larger part of one (three
+//     chunks): eight warps with whole pieces, what 7 and 8 rows of K = 5120 had before, leave the decode waiting (34816 x 5120 at 8 rows
+//     31.1 us, with sixteen warps and slots of parts 28.3; 24 rows 92.1 and 83.9).
 //   * A CTA's warps form teams of T; team member j owns piece j of every tile its team takes. A warp streams its pieces
 //     through a private ring of 2 or 3 shared-memory slots. A slot is filled by two tiled TMA copies signalled on one
 //     mbarrier: the piece's code bytes through a tensor map of the code plane - always a box of 16 rows x P chunks, so a
@@ -38,8 +41,8 @@
 //   kErrorBit                       bit of the device error word for a wait that gave up
 //   extra_bytes(chunks)             extra shared bytes next to the activation slice
 //   stage(...)                      CTA-wide staging of the activation slice in the decode's pairing
-//   State                           accumulators: chunk<I, W>(codes, scales, x) consumes chunk I of a piece whose box rows
-//                                   are W chunks wide, given the lane's shared addresses; result(out); reset()
+//   State                           accumulators: chunk<I, J, W>(codes, scales, x) consumes chunk I of a piece, chunk J of a slot whose
+//                                   box rows are W chunks wide, given the lane's shared addresses; result(out); reset()
 #pragma once
 
 #include "common.cuh"
@@ -73,7 +76,7 @@ __host__ __device__ inline Order order_of(uint32_t k) {
 
 // One tensor of a group.
 struct alignas(64) Tensor {
-    CUtensorMap codes;         // box: 16 rows x `piece` chunks
+    CUtensorMap codes;         // box: 16 rows x the chunks of a ring slot
     CUtensorMap scales;        // box: 16 rows x F::kScaleBox bytes
     const uint16_t* x;
     const uint8_t* w;
@@ -92,7 +95,8 @@ struct alignas(64) Group {
 template <class F>
 struct Layout {
     uint32_t stride_x, off_extra, off_partials, off_gather, off_slots, off_bars, slot_bytes, code_bytes, bytes;
-    __host__ __device__ Layout(const Order& o, uint32_t rows, uint32_t warps, uint32_t depth, uint32_t span) {
+    // box: chunks of a ring slot.
+    __host__ __device__ Layout(const Order& o, uint32_t rows, uint32_t warps, uint32_t depth, uint32_t span, uint32_t box) {
         const uint32_t widest = (o.chunks + o.split - 1u) / o.split;
         stride_x = widest * 256u + 64u;   // 64 modulo 128: the rows a quarter-warp reads fall in distinct banks
         off_extra = rows * stride_x;
@@ -100,23 +104,23 @@ struct Layout {
         off_gather = off_partials + warps * 2u * kPartial;
         const uint32_t owned = o.split > 1u ? (span + o.split - 1u) / o.split + 1u : 0u;
         off_slots = (off_gather + owned * o.split * kPartial + 127u) & ~127u;
-        code_bytes = 16u * o.piece * F::kCodeBytes;
+        code_bytes = 16u * box * F::kCodeBytes;
         slot_bytes = code_bytes + 16u * F::kScaleBox;
         off_bars = off_slots + warps * depth * slot_bytes;
         bytes = off_bars + warps * depth * 8u;
     }
 };
 
-// The tensor maps of one weight tensor. Codes: 32-bit elements [n rows][row_bytes / 4], boxes of 16 rows x `piece` chunks.
+// The tensor maps of one weight tensor. Codes: 32-bit elements [n rows][row_bytes / 4], boxes of 16 rows x `chunks` chunks.
 // Scales: bytes [n rows][scale_row_bytes], boxes of 16 rows x kScaleBox bytes (only when the pitch is a multiple of 16).
 template <class F>
-inline bool encode_tensor(Tensor* t, const void* weights, uint32_t n, uint32_t k, const Order& o, bool tma_scales) {
+inline bool encode_tensor(Tensor* t, const void* weights, uint32_t n, uint32_t k, uint32_t chunks, bool tma_scales) {
     const eb::EncodeTiled encode = eb::encoder();
     if (encode == nullptr) return false;
     const typename F::Geometry geo(n, k);
     const cuuint32_t ones[2] = {1u, 1u};
     const cuuint64_t dims[2] = {geo.row_bytes / 4u, n}, strides[1] = {geo.row_bytes};
-    const cuuint32_t box[2] = {o.piece * F::kCodeBytes / 4u, 16u};
+    const cuuint32_t box[2] = {chunks * F::kCodeBytes / 4u, 16u};
     if (encode(&t->codes, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(weights), dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
             != CUDA_SUCCESS)
@@ -145,18 +149,20 @@ __device__ __forceinline__ float ld_shared_f(uint32_t address) {
     return v;
 }
 
-// Decodes one piece of PC chunks from a filled slot into the lane's four sums.
-template <class F, int P, int PC>
-__device__ __forceinline__ void decode_piece(typename F::template State<P>& state, uint32_t codes, uint32_t scales, uint32_t x, float (&acc)[4]) {
-    state.reset();
+// Decodes chunks FIRST to FIRST + PC - 1 of a piece, the first PC of a filled slot whose rows are B chunks wide, on top of the lane's
+// sums so far.
+template <class F, int P, int B, int FIRST, int PC>
+__device__ __forceinline__ void decode_chunks(typename F::template State<P>& state, uint32_t codes, uint32_t scales, uint32_t x, float (&acc)[4]) {
+    if (FIRST == 0) state.reset();
     eb::static_for<PC>([&](auto index) {
         constexpr int I = decltype(index)::value;
-        state.template chunk<I, P>(codes, scales, x);   // the box rows are always P chunks wide
+        state.template chunk<FIRST + I, I, B>(codes, scales, x);
     });
     state.result(acc);
 }
 
-template <class F, int P, bool kTmaScales>
+//   P: chunks of the widest piece; B: of a ring slot, P or (pieces in two parts) between P / 2 and P.
+template <class F, int P, int B, bool kTmaScales>
 __global__ void __launch_bounds__(32 * kMaxWarps, 1) kernel(const __grid_constant__ Group group, uint32_t* __restrict__ error) {
     extern __shared__ __align__(128) uint8_t smem[];
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, g = lane >> 2, q = lane & 3u;
@@ -171,7 +177,8 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) kernel(const __grid_constan
     const uint32_t run_begin = (uint32_t)((uint64_t)cluster * group.tiles / clusters), run_end = (uint32_t)((uint64_t)(cluster + 1u) * group.tiles / clusters);
     const uint32_t slice_begin = (uint32_t)((uint64_t)rank * order.chunks / split), slice_end = (uint32_t)((uint64_t)(rank + 1u) * order.chunks / split);
     const uint32_t slice = slice_end - slice_begin;
-    const Layout<F> layout(order, rows, warps, depth, group.span);
+    const Layout<F> layout(order, rows, warps, depth, group.span, B == P ? order.piece : (uint32_t)B);   // (the constant costs 1 %)
+    constexpr uint32_t kParts = B < P ? 2u : 1u;   // slots of a piece
     const uint32_t smem_a = eb::smem_u32(smem);
     if (lane < depth) eb::mbar_init(reinterpret_cast<uint64_t*>(smem + layout.off_bars) + warp * depth + lane, 1);
     eb::mbar_fence_init();
@@ -232,13 +239,14 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) kernel(const __grid_constan
     const uint32_t bars_a = smem_a + layout.off_bars + warp * depth * 8u;
     // Where a piece's bytes sit in the planes: the code box starts at the piece; the scale box starts on the 16-byte
     // boundary at or before the piece's scales.
-    const uint32_t code_x = piece_begin * (F::kCodeBytes / 4u);
-    const uint32_t scale_byte = piece_begin * F::kScaleBytes, scale_x = scale_byte & ~15u;
+    const uint32_t code_x = piece_begin * (F::kCodeBytes / 4u), scale_byte = piece_begin * F::kScaleBytes, scale_x = scale_byte & ~15u;
     const uint32_t scale_rem = kTmaScales ? scale_byte - scale_x : 0u;
-    const uint32_t fill_bytes = 16u * (uint32_t)P * F::kCodeBytes + (kTmaScales ? 16u * F::kScaleBox : 0u);
+    const uint32_t next_scale_x = (scale_byte + (uint32_t)B * F::kScaleBytes) & ~15u;   // of a second part
+    const uint32_t next_scale_rem = kTmaScales ? scale_byte + (uint32_t)B * F::kScaleBytes - next_scale_x : 0u;
+    const uint32_t fill_bytes = 16u * (uint32_t)B * F::kCodeBytes + (kTmaScales ? 16u * F::kScaleBox : 0u);
 
     // The team's tiles: run_begin + team, + teams, ... Two cursors walk them: `ask` requests, `use` decodes.
-    uint32_t ask_tile = run_begin + team, ask_slot = 0, ask_tensor = 0, ask_first = 0, ask_end = group.tensor[0].tile_end;
+    uint32_t ask_tile = run_begin + team, ask_part = 0, ask_slot = 0, ask_tensor = 0, ask_first = 0, ask_end = group.tensor[0].tile_end;
     auto request = [&]() {
         if (ask_tile < run_end) {
             while (ask_tile >= ask_end) {   // the next tensor of the group
@@ -249,17 +257,24 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) kernel(const __grid_constan
             const uint32_t row = (ask_tile - ask_first) * 16u;
             const uint32_t to = slots_a + ask_slot * layout.slot_bytes, bar = bars_a + ask_slot * 8u;
             if (lane == 0) {
-                eb::tma_load_2d_expect(to, &t.codes, (int)code_x, (int)row, bar, fill_bytes);
-                if (kTmaScales) eb::tma_load_2d_at(to + layout.code_bytes, &t.scales, (int)scale_x, (int)row, bar);
+                const uint32_t codes_at = kParts == 1u ? code_x : code_x + ask_part * ((uint32_t)B * F::kCodeBytes / 4u);
+                eb::tma_load_2d_expect(to, &t.codes, (int)codes_at, (int)row, bar, fill_bytes);
+                if (kTmaScales) eb::tma_load_2d_at(to + layout.code_bytes, &t.scales, (int)(kParts == 1u || ask_part == 0u ? scale_x : next_scale_x), (int)row, bar);
             }
             if (!kTmaScales) {
                 // lane l copies row l % 16, every other chunk's scales
                 const typename F::Geometry geo(t.n, group.k);
-                const uint8_t* from = t.w + geo.scale_offset + (uint64_t)(row + (lane & 15u)) * geo.scale_row_bytes + (uint64_t)piece_begin * F::kScaleBytes;
+                const uint32_t first = kParts == 1u ? 0u : ask_part * (uint32_t)B, here = kParts == 1u ? piece_end - piece_begin : min((uint32_t)B, piece_end - piece_begin - first);
+                const uint8_t* from = t.w + geo.scale_offset + (uint64_t)(row + (lane & 15u)) * geo.scale_row_bytes + (uint64_t)(piece_begin + first) * F::kScaleBytes;
                 const uint32_t into = to + layout.code_bytes + (lane & 15u) * F::kScaleBox;
-                for (uint32_t c = lane >> 4; c < piece_end - piece_begin; c += 2u) eb::cp_async_4_to(into + c * 4u, from + c * 4u);
+                for (uint32_t c = lane >> 4; c < here; c += 2u) eb::cp_async_4_to(into + c * 4u, from + c * 4u);
             }
-            ask_tile += teams;
+            if (kParts == 1u) {
+                ask_tile += teams;
+            } else if (++ask_part == kParts) {
+                ask_part = 0;
+                ask_tile += teams;
+            }
             if (++ask_slot == depth) ask_slot = 0;
         }
         if (!kTmaScales) eb::cp_async_commit();
@@ -273,7 +288,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) kernel(const __grid_constan
 
     // Lane constants. Lane (g, q) decodes rows g and g + 8 of a tile; its activations are those of row min(g, rows - 1).
     const uint32_t x_lane = eb::pinned(smem_a + (g < rows ? g : rows - 1u) * layout.stride_x + q * 16u + (piece_begin - slice_begin) * 256u);
-    const uint32_t code_lane = eb::pinned(g * (uint32_t)P * F::kCodeBytes);
+    const uint32_t code_lane = eb::pinned(g * (uint32_t)B * F::kCodeBytes);
     const uint32_t scale_lane = eb::pinned(layout.code_bytes + g * F::kScaleBox + scale_rem);
     const uint32_t extra_lane = smem_a + layout.off_extra + (piece_begin - slice_begin) * (F::extra_bytes(2) - F::extra_bytes(1));
     // This lane's place in its team's two sum buffers: [buffer][member][row of the tile][activation row]; lane (g, q) holds
@@ -296,8 +311,27 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) kernel(const __grid_constan
                 if (complete) complete = eb::mbar_wait_at(bars_a + use_slot * 8u, parity);   // after one wait gave up, no further wait is taken
                 const uint32_t slot = slots_a + use_slot * layout.slot_bytes;
                 float acc[4];
-                if (P == 1 || wide) decode_piece<F, P, P>(state, slot + code_lane, slot + scale_lane, x_lane, acc);
-                else decode_piece<F, P, (P > 1 ? P - 1 : 1)>(state, slot + code_lane, slot + scale_lane, x_lane, acc);
+                if constexpr (B == P) {
+                    if (P == 1 || wide) decode_chunks<F, P, B, 0, P>(state, slot + code_lane, slot + scale_lane, x_lane, acc);
+                    else decode_chunks<F, P, B, 0, (P > 1 ? P - 1 : 1)>(state, slot + code_lane, slot + scale_lane, x_lane, acc);
+                } else {
+                    decode_chunks<F, P, B, 0, B>(state, slot + code_lane, slot + scale_lane, x_lane, acc);
+                    __syncwarp();   // every lane is done with the slot
+                    request();
+                    if (++use_slot == depth) {
+                        use_slot = 0;
+                        parity ^= 1u;
+                    }
+                    if (!kTmaScales) {
+                        if (depth == 2u) eb::cp_async_wait_group<1>();
+                        else eb::cp_async_wait_group<2>();
+                        __syncwarp();
+                    }
+                    if (complete) complete = eb::mbar_wait_at(bars_a + use_slot * 8u, parity);
+                    const uint32_t second = slots_a + use_slot * layout.slot_bytes, scales = second + scale_lane + next_scale_rem - scale_rem;
+                    if (wide) decode_chunks<F, P, B, B, P - B>(state, second + code_lane, scales, x_lane, acc);
+                    else decode_chunks<F, P, B, B, P - B - 1>(state, second + code_lane, scales, x_lane, acc);
+                }
                 const uint32_t buffer = turn & 1u;
                 const uint32_t mine = sum_lane + buffer * team_size * kPartial;
                 st_shared_f2(mine, acc[0], acc[1]);

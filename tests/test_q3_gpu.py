@@ -164,6 +164,19 @@ def test_launch_geometries(dev, n, k):
 
 
 
+# Rings whose slots hold parts of pieces (the rows leave no room for whole ones), against one-row calls, whose slots hold whole pieces: a
+# piece of five chunks and of four, even and odd cuts, one slice and several, scale planes that TMA takes and that it does not.
+@pytest.mark.parametrize("n,k", [(48, 5120), (272, 4224), (4800, 4736), (64, 6016), (32, 8192), (336, 12416), (16, 17408)])
+@pytest.mark.parametrize("rows", [6, 7, 8, 24])
+def test_rows_in_parted_rings_equal_one_row_calls(dev, n, k, rows):
+    rng = np.random.default_rng(n + k + rows)
+    blob, _ = random_tensor(rng, n, k)
+    x = random_x(rng, rows, k)
+    got = run(dev, x, blob, n, k)
+    for r in {0, rows // 2, rows - 1}:
+        assert np.array_equal(run(dev, x[r:r + 1], blob, n, k)[0], got[r]), r
+
+
 def test_every_fp16_scale_pattern(dev):
     """The FP16 group scale reaches the sum as its exact FP32 value for every finite bit pattern, subnormals and both
     zeros included (the reference pins its conversion over all 65,536 patterns, native/tests/test_q3_conversion.py:18-41;
