@@ -105,7 +105,9 @@ __device__ __forceinline__ void register_step(const uint32_t (&values)[1 << kHig
 
 // Walks back over two positions from `node` after the odd position `position` (taken by a whole warp). kept: the costs before the even
 // position in front of it, or null where that is the pass's first, entered at `pinned`. Returns the two states, the even position's in
-// the upper half. On equal costs the lowest predecessor wins, of the odd position before the even one's, as the search is defined.
+// the upper half. On equal costs the lowest predecessor wins, of the odd position before the even one's, as the search is defined. A NaN
+// cost is less than none: behind a NaN weight all costs of a position are NaN or infinite, and the lowest predecessors win. They do here,
+// where all are one or the other; only at a pass's first position does one path with the weight's NaN stand beside infinite ones.
 template <int KA, int KB>
 __device__ __forceinline__ uint32_t two_back(const __half* __restrict__ kept, const __half* weights, int position, uint32_t node, int pinned, int lane) {
     constexpr int kLanes = 32 >> KA, kEach = (1 << KB) > kLanes ? (1 << KB) / kLanes : 1;   // lanes of an odd predecessor; paths of a lane
@@ -124,7 +126,7 @@ __device__ __forceinline__ uint32_t two_back(const __half* __restrict__ kept, co
         const __half e = __hsub(__ushort_as_half(trellis::value_bits(state)), w_even);
         uint32_t cost;
         if (kept != nullptr) cost = __half_as_ushort(__hfma(e, e, before[m]));
-        else cost = pinned >= 0 && (int)(state >> KA) != pinned ? kInfinity : __half_as_ushort(__hmul(e, e));
+        else cost = pinned >= 0 && (int)(state >> KA) != pinned ? kInfinity : min((uint32_t)__half_as_ushort(__hmul(e, e)), kInfinity);   // NaN: no less
         if (even < 1u << KB) least = min(least, cost << 16 | even);
     }
 #pragma unroll

@@ -80,6 +80,22 @@ def test_tiles_in_flight_against_the_cpu_restatement(dev, w, ka, mask, extra):
         assert np.array_equal(states[part], expect)
 
 
+@pytest.mark.parametrize("w,ka,mask", RATES)
+def test_weights_that_are_not_numbers_against_the_cpu_restatement(dev, w, ka, mask):
+    """A NaN weight's costs win no comparison: its position and those behind it take the lowest predecessors. At either end of each pass,
+    at even and odd positions, NaN of both signs, beside an infinite weight, in a whole tile."""
+    rng = np.random.default_rng(w)
+    at = [0, 1, 2, 3, 126, 127, 128, 129, 254, 255]
+    tiles = rng.standard_normal((len(at) + 4, 256)).astype(np.float32)
+    tiles[np.arange(len(at)), at] = np.nan
+    tiles[len(at), 0], tiles[len(at), 128] = -np.nan, np.nan
+    tiles[len(at) + 1, 0], tiles[len(at) + 1, 1] = np.nan, -np.inf
+    tiles[len(at) + 2, 0], tiles[len(at) + 2, 2] = np.inf, np.nan
+    tiles[len(at) + 3] = np.nan
+    expect, _ = OC.trellis_encode_tiles(tiles, ka, mask)
+    assert np.array_equal(encode(dev, tiles, w), expect)
+
+
 def test_status_codes(dev):
     lib = dev.gpu.lib
     tiles = dev.put(np.zeros((2, 256), dtype=np.float32))
