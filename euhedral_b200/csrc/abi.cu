@@ -1174,12 +1174,15 @@ int euhedral_b200_trellis_encode_tiles(const void* tiles, uint32_t count, uint32
     const int status = bind(&state);
     if (status != EUHEDRAL_CUDA_SUCCESS) return status;
     if (encoder_scratch(count, ka, state->sms) > scratch_bytes) return EUHEDRAL_CUDA_SIZE_OVERFLOW;
-    auto run = [&](auto kernel, int threads, uint32_t shared) {
+    auto run = [&](auto kernel, int threads, uint32_t shared, uintptr_t slabs) {
         return launch(kOrdered, kernel, dim3(encoder_ctas(count, state->sms)), dim3(threads), shared, 1u, static_cast<const float*>(tiles), count,
-                static_cast<uint16_t*>(states), static_cast<float*>(decoded), static_cast<uint8_t*>(scratch));
+                static_cast<uint16_t*>(states), static_cast<float*>(decoded), reinterpret_cast<uint8_t*>(slabs));
     };
-    auto registers = [&](auto kernel) { return run(kernel, trellis_encode::kRegisterThreads, trellis_encode::register_shared_bytes((int)ka)); };
-    auto shared = [&](auto kernel) { return run(kernel, trellis_encode::kThreads, trellis_encode::shared_bytes((int)ka)); };
+    // The register kernel stores 16 bytes of costs at a time; the last row of a slab, which it leaves alone, has room to round any scratch up.
+    auto registers = [&](auto kernel) {
+        return run(kernel, trellis_encode::kRegisterThreads, trellis_encode::register_shared_bytes((int)ka), ((uintptr_t)scratch + 15u) & ~(uintptr_t)15u);
+    };
+    auto shared = [&](auto kernel) { return run(kernel, trellis_encode::kThreads, trellis_encode::shared_bytes((int)ka), (uintptr_t)scratch); };
     cudaError_t e = cudaErrorInvalidValue;
     switch (tile_words) {
         case 32: e = registers(trellis_encode::register_kernel<2, false>); break;

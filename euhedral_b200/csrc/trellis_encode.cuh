@@ -141,7 +141,7 @@ __device__ __forceinline__ uint32_t two_back(const __half* __restrict__ kept, co
 __device__ __forceinline__ uint32_t reverse5(uint32_t v) { return __brev(v) >> 27; }
 
 // tiles f32 [count][256] -> states u16 [count][256] (and, when asked for, their codebook values as f32). slabs: history_bytes(KA) bytes
-// per tile in flight, at most count of them.
+// per tile in flight, at most count of them, on a 16-byte boundary; the last row of the last one (2 (65536 >> KA) bytes) is not touched.
 //   grid: at most count CTAs (CTA b takes tiles b, b + gridDim.x, ...; two at a time), block kRegisterThreads, dynamic shared
 //   register_shared_bytes(KA).
 template <int KA, bool kHalfStep>
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kRegisterThreads, 1) register_kernel(const flo
                     if (i == 0) register_step<KA, KB, true>(values, row_odd, row_even, nullptr, __low2half(w), pinned, t);
                     else register_step<KA, KB, false>(values, row_odd, row_even, nullptr, __low2half(w), pinned, t);
                     searchers_sync();
-                    const bool keeps = second != 0u || i >= 126;   // what the way back reads
+                    const bool keeps = i < 254 && (second != 0u || i >= 126);   // what the way back reads: never a slab's last row
                     register_step<KB, KA, false>(values, row_even, row_odd, keeps ? slab + (size_t)(i >> 1) * kMost : nullptr, __high2half(w), pinned, t);
                     searchers_sync();
                 }

@@ -22,14 +22,16 @@ def dev():
     device.release()
 
 
-def encode(dev, tiles, w):
+def encode(dev, tiles, w, need=None, offset=0):
     lib = dev.gpu.lib
     count = tiles.shape[0]
-    need = lib.euhedral_b200_trellis_encode_scratch_bytes(count, w)
-    d_t, d_s, d_h = dev.put(np.ascontiguousarray(tiles, dtype=np.float32)), dev.empty(count * 512), dev.empty(need)
+    need = need or lib.euhedral_b200_trellis_encode_scratch_bytes(count, w)
+    d_t, d_s, d_h = dev.put(np.ascontiguousarray(tiles, dtype=np.float32)), dev.empty(count * 512), dev.empty(offset + need + 64)
     d_v, d_w = dev.empty(count * 1024), dev.empty(count * w * 2)
     with dev.submit():
-        assert lib.euhedral_b200_trellis_encode_tiles(d_t.data_ptr(), count, w, d_s.data_ptr(), d_v.data_ptr(), d_w.data_ptr(), d_h.data_ptr(), need) == 0
+        assert lib.euhedral_b200_trellis_encode_tiles(d_t.data_ptr(), count, w, d_s.data_ptr(), d_v.data_ptr(), d_w.data_ptr(), d_h.data_ptr() + offset, need) == 0
+    guard = dev.get(d_h[offset + need:], np.uint8, (64,))
+    assert np.all(guard == 0xA5) and np.all(dev.get(d_h, np.uint8, (offset,)) == 0xA5)   # nothing beyond the scratch
     encode.decoded, encode.words = dev.get(d_v, np.float32, (count, 256)), dev.get(d_w, np.int16, (count, w))
     return dev.get(d_s, np.uint16, (count, 256))
 
@@ -94,6 +96,16 @@ def test_weights_that_are_not_numbers_against_the_cpu_restatement(dev, w, ka, ma
     tiles[len(at) + 3] = np.nan
     expect, _ = OC.trellis_encode_tiles(tiles, ka, mask)
     assert np.array_equal(encode(dev, tiles, w), expect)
+
+
+@pytest.mark.parametrize("w,ka,mask", RATES)
+@pytest.mark.parametrize("offset", [4, 8, 12])
+def test_scratch_at_any_multiple_of_four(dev, w, ka, mask, offset):
+    """The scratch need not lie on the boundary of the kernels' widest stores; what is used of it stays inside."""
+    rng = np.random.default_rng(w + offset)
+    tiles = rng.standard_normal((3, 256)).astype(np.float32)
+    expect, _ = OC.trellis_encode_tiles(tiles, ka, mask)
+    assert np.array_equal(encode(dev, tiles, w, offset=offset), expect)
 
 
 def test_status_codes(dev):
