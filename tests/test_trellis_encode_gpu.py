@@ -108,6 +108,24 @@ def test_scratch_at_any_multiple_of_four(dev, w, ka, mask, offset):
     assert np.array_equal(encode(dev, tiles, w, offset=offset), expect)
 
 
+@pytest.mark.parametrize("w,ka,mask", [(32, 2, 0), (40, 2, 0xAAAA)])
+@pytest.mark.parametrize("count", [1, 2, 150, 299])
+def test_two_bits_in_a_slab_an_sm(dev, w, ka, mask, count):
+    """At 2 and 2.5 bits a scratch of one slab of 4 MB for each SM will do (a tile in flight), also at an odd address; less is refused."""
+    rng = np.random.default_rng(w + count)
+    tiles = rng.standard_normal((count, 256)).astype(np.float32)
+    least = min(count, dev.gpu.multiprocessor_count()) << 22
+    expect = encode(dev, tiles, w)
+    assert np.array_equal(encode(dev, tiles, w, need=least), expect)
+    assert np.array_equal(encode(dev, tiles, w, need=least, offset=8), expect)
+    assert np.array_equal(encode(dev, tiles, w, need=least + 100), expect)
+    ends = np.r_[0:1, count - 1:count]
+    assert np.array_equal(expect[ends], OC.trellis_encode_tiles(tiles[ends], ka, mask)[0])
+    d_t, d_s, d_h = dev.put(tiles), dev.empty(count * 512), dev.empty(least)
+    with dev.submit():
+        assert dev.gpu.lib.euhedral_b200_trellis_encode_tiles(d_t.data_ptr(), count, w, d_s.data_ptr(), 0, 0, d_h.data_ptr(), least - 1) == library.SIZE_OVERFLOW
+
+
 def test_status_codes(dev):
     lib = dev.gpu.lib
     tiles = dev.put(np.zeros((2, 256), dtype=np.float32))
