@@ -51,8 +51,40 @@ class DeviceLinear:
             self.format.linear(gpu, launch)
         return self.dev.get(d_y, np.uint16, (rows, self.n))
 
+    def table_launches(self, x_bits, splits, **select):
+        """The plan's launches through the kernel table, one by one: what every other way to a linear has to give, bit for bit."""
+        rows, segments = x_bits.shape[0], len(self.ends)
+        words, suh, svh, ends = [t.data_ptr() for t in self.tensors]
+        d_x, d_act, d_y = self.dev.put(x_bits), self.dev.empty(segments * rows * self.k * 2), self.dev.empty(rows * self.n * 2)
+        d_part = self.dev.empty(splits * rows * self.n * 4)
+        with self.dev.submit(**select) as gpu:
+            gpu.launch_table_kernel("TRELLIS_PREPASS", (self.k + 511) // 512, rows, segments, 128, 1, 1, 0,
+                                    KernelArguments().pointer(d_x.data_ptr()).pointer(suh).pointer(d_act.data_ptr()).int32(rows).int32(self.k)
+                                    .int32(segments).int32(0))
+            gpu.launch_table_kernel("TRELLIS_MMA", self.n // 128, splits, 1, 256, 1, 1, 0,
+                                    KernelArguments().pointer(d_act.data_ptr()).pointer(words).pointer(ends).pointer(svh).pointer(d_part.data_ptr())
+                                    .pointer(d_y.data_ptr()).int32(rows).int32(self.k).int32(self.n).int32(self.w).int32(splits).int32(segments))
+            if splits > 1:
+                gpu.launch_table_kernel("TRELLIS_EPILOGUE", (self.n + 511) // 512, rows, 1, 128, 1, 1, 0,
+                                        KernelArguments().pointer(d_part.data_ptr()).int32(splits).pointer(svh).pointer(d_y.data_ptr()).int32(rows)
+                                        .int32(self.n))
+        return self.dev.get(d_y, np.uint16, (rows, self.n))
+
+    def one_launch(self, x_bits, **select):
+        """The linear with a split count of its own (splits = 0): (output, that count, read off the flags that the launch leaves)."""
+        rows = x_bits.shape[0]
+        need = self.dev.gpu.lib.euhedral_b200_linear_trellis_scratch_bytes(rows, self.k, self.n, len(self.ends), 0)
+        d_x, d_y, d_s = self.dev.put(x_bits), self.dev.empty(rows * self.n * 2), self.dev.empty(max(need, 256), fill=0xA5)
+        with self.dev.submit(**select) as gpu:
+            gpu.linear_trellis_bf16(d_x.data_ptr(), *[t.data_ptr() for t in self.tensors[:3]], self.tensors[3].data_ptr(), d_y.data_ptr(),
+                                    d_s.data_ptr(), need, rows, self.k, self.n, self.w, len(self.ends), 0)
+        flags = self.dev.get(d_s, np.uint64, (max(need, 256) // 8,))
+        joined = int(np.count_nonzero(flags == flags[0])) if flags[0] != 0xA5A5A5A5A5A5A5A5 else 0   # every block's flags end as one value
+        assert joined % (self.n // 128) == 0
+        return self.dev.get(d_y, np.uint16, (rows, self.n)), max(1, joined // (self.n // 128))
+
     def one_call(self, x_bits, splits, **select):
-        """The same linear as ONE launch (euhedral_b200_linear_trellis_bf16) with the split count given."""
+        """The same linear as one call (euhedral_b200_linear_trellis_bf16) with the split count given."""
         rows = x_bits.shape[0]
         need = self.dev.gpu.lib.euhedral_b200_linear_trellis_scratch_bytes(rows, self.k, self.n, len(self.ends), splits)
         d_x, d_y, d_s = self.dev.put(x_bits), self.dev.empty(rows * self.n * 2), self.dev.empty(max(need, 256), fill=0xA5)
@@ -116,7 +148,8 @@ def test_tensor_core_route_matches_float64(dev, w, target):
         got = linear.linear(x)
         assert within_kernel_tolerance(got, expect), (w, target, rows)
         if rows in (5, 13):
-            assert np.array_equal(linear.one_call(x, splits), got), (w, target, rows)   # one launch: the same bits
+            assert np.array_equal(linear.one_call(x, splits), got), (w, target, rows)
+            assert np.array_equal(linear.table_launches(x, splits), got), (w, target, rows)
 
 
 # The layer's projection shapes (N x K) at the model's stored widths, one and two segments, through the operator's own
@@ -137,12 +170,12 @@ def test_layer_shapes(dev, n, k, w):
         expect = OC.trellis_linear(x, payload, suh, svh, ends).astype(np.float64)
         got = linear.linear(x)
         assert within_kernel_tolerance(got, expect), (n, k, w, rows)
-        assert np.array_equal(linear.one_call(x, splits, pdl=True), got), (n, k, w, rows)   # one launch, the same bits
+        assert np.array_equal(linear.one_call(x, splits, pdl=True), got), (n, k, w, rows)
+        assert np.array_equal(linear.table_launches(x, splits, pdl=True), got), (n, k, w, rows)
 
 
 def test_one_call_linear_is_bitwise_the_table_launches(dev):
-    """The one-launch linear (activations rotated inside the kernel, splits joined by whoever finishes last) against the
-    three table launches a host plans one by one."""
+    """The one-call linear and the operator's against the three table launches a host plans one by one."""
     rng = np.random.default_rng(44)
     k, n, w = 2048, 512, 48
     payload, suh, svh = random_object(rng, k, n, w, segments=2)
@@ -151,8 +184,9 @@ def test_one_call_linear_is_bitwise_the_table_launches(dev):
     for target, rows in ((8, 3), (140, 5), (140, 1), (1, 7), (1, 20), (30, 13), (64, 40)):
         table = DeviceLinear(dev, payload, suh, svh, ends, target)
         x = random_x(rng, rows, k)
-        expect = table.linear(x)
         splits = TrellisFormat.splits(k, n, target)
+        expect = table.table_launches(x, splits)
+        assert np.array_equal(table.linear(x), expect), (target, rows)
         assert np.array_equal(table.one_call(x, splits), expect), (target, rows)
         need = lib.euhedral_b200_linear_trellis_scratch_bytes(rows, k, n, 2, splits)
         # a flag per block and split, then the partials; nothing with one split
@@ -196,23 +230,30 @@ def test_operator_is_bitwise_the_table_launches(dev, k, n, w, ends, target, rows
     linear = DeviceLinear(dev, payload, suh, svh, ends, target)
     x = random_x(rng, rows, k)
     splits = TrellisFormat.splits(k, n, target)
+    expect = linear.table_launches(x, splits, pdl=True)
     words, d_suh, d_svh, d_ends = [t.data_ptr() for t in linear.tensors]
-    d_x, d_act, d_part, d_y = dev.put(x), dev.empty(len(ends) * rows * k * 2), dev.empty(max(splits * rows * n * 4, 16)), dev.empty(rows * n * 2)
-    with dev.submit(pdl=True) as gpu:
-        gpu.launch_table_kernel("TRELLIS_PREPASS", (k + 511) // 512, rows, len(ends), 128, 1, 1, 0,
-                                KernelArguments().pointer(d_x.data_ptr()).pointer(d_suh).pointer(d_act.data_ptr()).int32(rows).int32(k).int32(len(ends)).int32(0))
-        gpu.launch_table_kernel("TRELLIS_MMA", n // 128, splits, 1, 256, 1, 1, 0,
-                                KernelArguments().pointer(d_act.data_ptr()).pointer(words).pointer(d_ends).pointer(d_svh).pointer(d_part.data_ptr())
-                                .pointer(d_y.data_ptr()).int32(rows).int32(k).int32(n).int32(w).int32(splits).int32(len(ends)))
-        if splits > 1:
-            gpu.launch_table_kernel("TRELLIS_EPILOGUE", (n + 511) // 512, rows, 1, 128, 1, 1, 0,
-                                    KernelArguments().pointer(d_part.data_ptr()).int32(splits).pointer(d_svh).pointer(d_y.data_ptr()).int32(rows).int32(n))
-    expect = dev.get(d_y, np.uint16, (rows, n))
+    d_x, d_part, d_y = dev.put(x), dev.empty(max(splits * rows * n * 4, 16)), dev.empty(rows * n * 2)
     assert np.array_equal(linear.linear(x), expect)
     with dev.submit(pdl=True) as gpu:
         gpu.linear_trellis_bf16(d_x.data_ptr(), words, d_suh, d_svh, d_ends, d_y.data_ptr(), d_part.data_ptr(), splits * rows * n * 4, rows, k, n, w,
                                 len(ends), splits)
     assert np.array_equal(dev.get(d_y, np.uint16, (rows, n)), expect)
+
+
+# The launch that picks its split count itself and whose CTAs join the splits by flags, on both sides of every group of eight rows, against
+# the plan's launches at the count that the flags show. One and several segments, whole and half-step widths.
+@pytest.mark.parametrize("k,n,w,ends", [(2048, 512, 48, [256, 512]), (1408, 384, 64, [384]), (4224, 256, 56, [128, 256]), (5120, 1024, 96, [1024])])
+@pytest.mark.parametrize("rows", [1, 8, 9, 16, 17, 25, 32, 33, 40, 63])
+def test_joined_launch_is_bitwise_the_table_launches(dev, k, n, w, ends, rows):
+    rng = np.random.default_rng(1000 * rows + k)
+    payload, suh, svh = random_object(rng, k, n, w, segments=len(ends))
+    linear = DeviceLinear(dev, payload, suh, svh, ends, 140)
+    x = random_x(rng, rows, k)
+    got, splits = linear.one_launch(x, pdl=True)
+    assert splits > 1
+    assert np.array_equal(got, linear.table_launches(x, splits))
+    again, same = linear.one_launch(x)
+    assert same == splits and np.array_equal(again, got)
 
 
 def test_golden_linear_fixture(dev, golden):
@@ -307,6 +348,41 @@ def test_table_abi(dev):
     with pytest.raises(GpuMemoryException) as unavailable:
         dev.gpu.launch_table_kernel("TRELLIS_MMA_ROWS", 1, 1, 1, 256, 1, 1, 0, KernelArguments())
     assert unavailable.value.status == -5
+
+
+@pytest.mark.parametrize("rows", [5, 20, 40])
+@pytest.mark.parametrize("splits", [0, 9])
+def test_one_call_linear_replayed_from_a_graph(dev, rows, splits):
+    """A captured launch that joins its splits (splits = 0) carries the same flag tag on every replay: each replay must still wait for its
+    own partial sums (the CTA that finishes a column block unsets the block's flags). A named count beside it."""
+    torch = dev.torch
+    rng = np.random.default_rng(45 + rows)
+    k, n, w = 2048, 512, 48
+    payload, suh, svh = random_object(rng, k, n, w)
+    linear = DeviceLinear(dev, payload, suh, svh, [n], 140)
+    lib = dev.gpu.lib
+    need = lib.euhedral_b200_linear_trellis_scratch_bytes(rows, k, n, 1, splits)
+    xs = [random_x(rng, rows, k) for _ in range(4)]
+    count = splits or linear.one_launch(xs[0])[1]
+    assert count > 1
+    d_x, d_y, d_s = dev.put(xs[0]), dev.empty(rows * n * 2), dev.empty(need)
+    t = [h.data_ptr() for h in linear.tensors]
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream), dev.gpu.submit(stream.cuda_stream, pdl=True):
+        args = (d_x.data_ptr(), t[0], t[1], t[2], t[3], d_y.data_ptr(), d_s.data_ptr(), need, rows, k, n, w, 1, splits)
+        assert lib.euhedral_b200_linear_trellis_bf16(*args) == 0          # warm: plans and maps are made before the capture
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            assert lib.euhedral_b200_linear_trellis_bf16(*args) == 0
+    for x in xs + xs[:1]:
+        d_x.copy_(torch.from_numpy(x.view(np.uint8).reshape(-1).copy()))
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        got = dev.get(d_y, np.uint16, (rows, n))
+        d_y.fill_(0xA5)
+        assert np.array_equal(got, linear.table_launches(x, count))
 
 
 def test_one_launch_linear_replayed_from_a_graph(dev):
