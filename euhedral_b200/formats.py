@@ -105,7 +105,6 @@ class TrellisFormat:
     [payload int16 [k/16, n/16, w], suh f16 [s, k], svh f16 [n], segments i32 [s]]."""
 
     PREPASS_BLOCK_COLUMNS = 512
-    EPILOGUE_BLOCK_COLUMNS = 512
     FRAGMENT_FP16, COLUMN_BF16, BLOCK_FP8 = 0, 1, 2
     MAX_GRID_ROWS = 65535
 
@@ -216,7 +215,8 @@ class _TrellisLaunch:
         self._require_scratch(activations + partials)
         scratch = self.launch.scratch
         if splits > 1:
-            # The three launches below as one call of the library: queued one by one from here they take the host 27 us.
+            # The plan's launches (rotation, GEMM, the sum of the splits) as one call of the library: queued one by one from here, as the two
+            # of a single split are below, they took the host 27 us.
             self.gpu.linear_trellis_bf16(self.launch.input, self.words, self.suh, self.svh, self.ends, self.launch.output, scratch,
                                          activations + partials, self.rows, self.k, self.n, self.w, self.segments, splits)
             return

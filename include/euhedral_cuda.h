@@ -134,8 +134,8 @@ EUHEDRAL_CUDA_EXPORT int euhedral_b200_linear_group_nvfp4_bf16(uint32_t count, c
 /* No counterpart in the reference. A whole trellis linear for callers that cannot provide scratch because they cannot
  * allocate device memory at the point of the call: a host that only holds the weight and activation addresses it was
  * given, a plugin running inside somebody else's memory plan, or a step that runs after the process's allocator has
- * been frozen. The scratch (the FP32 partial sums of the splits) lives in a static
- * device array inside the library, euhedral_b200_static_scratch_bytes() bytes (8 MiB) on every device that loads the
+ * been frozen. The scratch (the FP32 partial sums of the splits; from 9 rows on, where they fit too, the rotated activations) lives
+ * in a static device array inside the library, euhedral_b200_static_scratch_bytes() bytes (8 MiB) on every device that loads the
  * library, held until the process exits. The call allocates and frees nothing.
  *   input BF16 [rows][in_features]; words the payload [in/16][out/16][tile_words]; suh FP16 [segments][in]; svh FP16 [out];
  *   segment_ends int32 [segments]; output BF16 [rows][out]; splits = the K splits (1: nothing is exchanged).
@@ -143,7 +143,7 @@ EUHEDRAL_CUDA_EXPORT int euhedral_b200_linear_group_nvfp4_bf16(uint32_t count, c
  * (use euhedral_b200_linear_trellis_bf16 with caller scratch). Same results, bit for bit, as the three table launches.
  * The first call on a device looks the array's device address up; make that call before any stream capture.
  * Every call uses the same array and leaves its last contents there: calls that overlap on the GPU (two streams, or
- * two threads) race on it. Nothing in it needs clearing between calls - a flag counts only when it holds the call's own tag. */
+ * two threads) race on it. Nothing in it needs clearing between calls. */
 EUHEDRAL_CUDA_EXPORT uint64_t euhedral_b200_static_scratch_bytes(void);
 EUHEDRAL_CUDA_EXPORT int euhedral_b200_linear_trellis_bf16_static(const void* input, const void* words, const void* suh,
         const void* svh, const void* segment_ends, void* output, uint32_t rows, uint32_t in_features, uint32_t out_features,

@@ -3,7 +3,7 @@
 import numpy as np
 import pytest
 
-from euhedral_b200 import library, sharding
+from euhedral_b200 import layouts, library, sharding
 from oracle import oracle_c as OC
 from oracle import oracle_np as O
 from tests.gpu_util import Device, max_relative_error, random_x
@@ -164,8 +164,27 @@ def test_launch_geometries(dev, n, k):
 
 
 
-# Rings whose slots hold parts of pieces (the rows leave no room for whole ones), against one-row calls, whose slots hold whole pieces: a
-# piece of five chunks and of four, even and odd cuts, one slice and several, scale planes that TMA takes and that it does not.
+def slot_chunks(rows, k, n):
+    """(chunks of a ring slot, of a piece) of the decode launch: the one choice of warps, slot and depth whose shared memory is the plan's."""
+    plan = library.decode_plan("q3", rows, k, n)
+    split, team, piece = plan["k_slices"], plan["pieces"], plan["piece_chunks"]
+    tiles, widest = n // 16, -(-(k // 128) // split)
+    span = min(tiles, -(-tiles // (plan["ctas"] // split)) + 1)
+    owned = -(-span // split) + 1 if split > 1 else 0
+    found = set()
+    for warps in (16, 8, 4, 2, 1):
+        for box in {piece, min(piece, 3)}:
+            for depth in (3, 2):
+                partials = layouts.align_up(rows * (widest * 256 + 64) + widest * 128, 128)
+                slots = layouts.align_up(partials + warps * 1024 + owned * split * 512, 128)
+                if warps >= team and slots + warps * depth * (16 * box * 48 + 16 * 48 + 8) == plan["shared_bytes"]:
+                    found.add(box)
+    assert len(found) == 1
+    return found.pop(), piece
+
+
+# Against one-row calls, whose slots hold whole pieces, at the row counts where the rows leave no room for whole ones at some K: even and
+# odd cuts, one slice and several, scale planes that TMA takes and that it does not.
 @pytest.mark.parametrize("n,k", [(48, 5120), (272, 4224), (4800, 4736), (64, 6016), (32, 8192), (336, 12416), (16, 17408)])
 @pytest.mark.parametrize("rows", [6, 7, 8, 24])
 def test_rows_in_parted_rings_equal_one_row_calls(dev, n, k, rows):
@@ -175,6 +194,53 @@ def test_rows_in_parted_rings_equal_one_row_calls(dev, n, k, rows):
     got = run(dev, x, blob, n, k)
     for r in {0, rows // 2, rows - 1}:
         assert np.array_equal(run(dev, x[r:r + 1], blob, n, k)[0], got[r]), r
+
+
+# Slots of parts, of pieces of five chunks and of four. Among those of four are pieces of three, whose second slot brings nothing that is
+# decoded. Scale planes that TMA takes (K a multiple of 512) and that it does not.
+@pytest.mark.parametrize("rows,n,k,piece", [(8, 48, 5120, 5), (7, 4800, 5120, 5), (8, 4800, 4736, 5), (8, 32768, 16384, 4), (8, 32768, 14336, 4),
+                                            (8, 32768, 14080, 4), (7, 32768, 16000, 4), (8, 24576, 16000, 4)])
+def test_slots_of_parts_equal_one_row_calls(dev, rows, n, k, piece):
+    assert slot_chunks(rows, k, n) == (3, piece)
+    assert slot_chunks(1, k, n) == (piece, piece)
+    rng = np.random.default_rng(n + k + rows)
+    size, scales = layouts.q3_byte_size(n, k), layouts.q3_scale_offset(n, k)
+    blob = rng.integers(0, 256, size, dtype=np.uint8)
+    blob[scales:scales + n * k // 32].view(np.float16)[:] = (rng.standard_normal(n * k // 64, dtype=np.float32) * 0.01).astype(np.float16)
+    x = random_x(rng, rows, k)
+    d_x, d_w, d_y = dev.put(x), dev.put(blob), dev.empty(rows * n * 2)
+    with dev.submit() as gpu:
+        gpu.linear_q3_bf16(d_x.data_ptr(), d_w.data_ptr(), d_y.data_ptr(), rows, k, n, size)
+    got = dev.get(d_y, np.uint16, (rows, n))
+    for r in (0, rows // 2, rows - 1):
+        with dev.submit() as gpu:
+            gpu.linear_q3_bf16(d_x.data_ptr() + r * k * 2, d_w.data_ptr(), d_y.data_ptr(), 1, k, n, size)
+        assert np.array_equal(dev.get(d_y, np.uint16, (1, n))[0], got[r]), r
+    dev.release()   # some of the weights are large
+
+
+# Calls of one row, of eight and of nine (eight and one) on the same weight want maps of both kinds of slots, as members of a group too.
+@pytest.mark.parametrize("k", [5120, 4736])
+def test_a_weight_called_with_changing_row_counts(dev, k):
+    rng = np.random.default_rng(k)
+    shapes = [1024, 512, 48]
+    blobs = [random_tensor(rng, n, k)[0] for n in shapes]
+    weights = [dev.put(blob) for blob in blobs]
+    x = random_x(rng, 9, k)
+    d_x, d_y = dev.put(x), [dev.empty(9 * n * 2) for n in shapes]
+    single = [np.concatenate([run(dev, x[r:r + 1], blob, n, k) for r in range(9)]) for n, blob in zip(shapes, blobs)]
+    assert slot_chunks(8, k, sum(shapes))[0] == 3 and slot_chunks(1, k, sum(shapes))[0] == 5
+    for rows in (1, 8, 9, 1, 7, 2, 8):
+        if rows <= 8:
+            with dev.submit() as gpu:
+                assert gpu.linear_group_bf16("q3", [d_x.data_ptr()] * 3, [w.data_ptr() for w in weights], [y.data_ptr() for y in d_y], rows, k, shapes,
+                                             [b.size for b in blobs]) is not False
+            for n, y, expect in zip(shapes, d_y, single):
+                assert np.array_equal(dev.get(y, np.uint16, (rows, n)), expect[:rows]), (rows, n)
+        for n, w, blob, y, expect in zip(shapes, weights, blobs, d_y, single):
+            with dev.submit() as gpu:
+                gpu.linear_q3_bf16(d_x.data_ptr(), w.data_ptr(), y.data_ptr(), rows, k, n, blob.size)
+            assert np.array_equal(dev.get(y, np.uint16, (rows, n)), expect[:rows]), (rows, n)
 
 
 def test_every_fp16_scale_pattern(dev):
