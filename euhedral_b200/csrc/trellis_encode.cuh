@@ -19,7 +19,8 @@
 // Bound: packed FP16 arithmetic, which one of the two FMA pipes does at two cycles an instruction: a subtraction and a fused
 // multiply-add per pair of states, 1024 cycles a position and tile. The kernel for more bits (viterbi_kernel) reads the values from
 // shared memory for each position and selects winners with logic instructions, seven instructions per pair; 2 to 4 bits ran on it
-// before. 1024 x 1024 weights at 3 bits (4096 tiles and 1800 of the scale's search): 25.4 -> 17.1 ms.
+// before. 4096 tiles at 2 / 2.5 / 3 / 3.5 / 4 bits 22.1 / 23.7 / 15.6 / 16.1 / 16.8 -> 9.9 / 10.2 / 10.1 / 10.1 / 10.2 ms (2 and 2.5 bits with one
+// tile in flight 14.2 and 14.4); 1024 x 1024 weights at 3 bits (4096 tiles and 1800 of the scale's search): 25.4 -> 17.1 ms.
 //
 // 5 and 6 bits (viterbi_kernel; a thread's states there would not share predecessors in registers): one CTA per SM, 1024 threads,
 // persistent over the tile list. The CTA first writes the codebook value of every state to shared memory (128 KB of FP16) - a
