@@ -54,6 +54,12 @@ __host__ __device__ constexpr int groups_of(int rows) {
     const int all = (rows + 7) / 8, passes = (all + 3) / 4;
     return (all + passes - 1) / passes;
 }
+// CTAs of a launch that an SM is to hold: three, but two where four groups' kernel has shared memory for no more (from 72-word tiles on):
+// it then has 96 registers instead of 72, and 34816 x 5120 at 4.5 and 6 bits and 32 rows took 141 and 148 us instead of 147 and 157. The
+// kernels of one to three groups fit 72, and were up to 5 % slower with 96.
+__host__ __device__ constexpr int resident(int w, int groups) {
+    return groups == 4 && (kStages * kStageTiles * 16 * w + (int)act_bytes(groups) + 1024 + 128) * kResident > 233472 ? 2 : kResident;
+}
 __host__ __device__ inline int chunk_tiles(int groups, int live) {
     const int fit = (int)((act_bytes(groups) / (uint32_t)live - 32u) / 32u) & ~7;
     return fit < kChunkLimit ? fit : kChunkLimit;
@@ -440,7 +446,7 @@ __device__ __forceinline__ void decoders_sync() { asm volatile("bar.sync 1, %0;"
 // P = groups of 8 activation rows held at once (rows beyond 8 P take another pass over the payload).
 //   grid (n / 128, splits), block kThreads, dynamic shared kStages * kStageTiles * 16 W + act_bytes(P) bytes.
 template <int W, int P>
-__global__ void __launch_bounds__(kThreads, kResident) linear_kernel(const __grid_constant__ CUtensorMap payload_map,
+__global__ void __launch_bounds__(kThreads, resident(W, P)) linear_kernel(const __grid_constant__ CUtensorMap payload_map,
         const __grid_constant__ Job job, uint32_t* __restrict__ error) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr uint32_t kTileBytes = 2u * W, kTileRowBytes = 8u * kTileBytes, kStageBytes = kStageTiles * kTileRowBytes;
