@@ -488,7 +488,7 @@ def measure_per_shape(bench: Bench, steps_floor=40):
                     table[f"{fmt}:{alias}:{rows}"] = [round(us, 2), round(gbs, 1), round(gbs / bench.peaks["hbm"], 4)]
             del tensors, first
             torch.cuda.empty_cache()
-    return {"columns": ["us per launch", "GB/s", "fraction of HBM peak"], "note": "key = format:shape:M; trellis at 48 words per tile",
+    return {"columns": ["us per launch", "GB/s", "fraction of HBM peak"], "note": "key = format:shape:M; trellis at 48 words per tile, as one launch with a split count of its own (the operator's planned count is a launch more)",
             "rows": table}
 
 

@@ -971,10 +971,13 @@ int euhedral_b200_take_device_error(uint32_t* word) {
 
 uint64_t euhedral_b200_static_scratch_bytes(void) { return kStaticScratchBytes; }
 
-// A whole trellis linear as one call. With a split count of its own (one wave) it is ONE launch: the scratch holds what the K splits
-// exchange, a flag per (column block, split), then the FP32 partials of every split; nothing of it needs clearing (a call's flags
-// carry a tag of its own). With the caller's count (a host's plan: several waves, where a CTA that waits for flags holds up the
-// next) a second launch adds the splits, and no flags are kept. With one split the scratch is not touched.
+// A whole trellis linear as one call. A second launch adds the K splits, whose FP32 partials are in the scratch; on the device that is
+// faster than a join in the linear's own launch, by flags, fences and whichever CTA of a column block ends last: 1024 x 5120 in 16 splits
+// at 1 / 24 / 40 rows 7.6 / 13.9 / 21.2 us against 9.9 / 17.4 / 29.1, 17408 x 5120 in 3 splits 29 / 56 / 98 against 32 / 91 / 150. But it is
+// one launch more for the host, which small linears of a few rows are bound by when they are queued one by one (128 x 1024 at one row 7.6
+// against 10.1 us). So a call of up to 8 rows that leaves the count open (splits = 0: one wave) stays ONE launch: the scratch then holds a
+// flag per (column block, split) in front of the partials; nothing of it needs clearing (a call's flags carry a tag of its own). A caller
+// that names one split need not bring a scratch.
 static std::atomic<unsigned long long> g_trellis_tag{0x9E3779B97F4A7C15ull ^ (unsigned long long)(uintptr_t)&g_trellis_tag};
 
 // The split count of a one-launch trellis linear when the caller leaves it open: the one that needs the fewest tile rows
@@ -1022,9 +1025,9 @@ static int trellis_linear(unsigned char* scratch, uint64_t scratch_bytes, const 
     }
     // splits == 0: the count that keeps the SMs' resident CTA slots busiest (trellis_default_splits). (The reference's host
     // aims at 8 blocks per SM, core/.../artifact/format/TrellisFormat.java:369-376; a caller that wants that count passes it.)
-    const bool planned = splits > 1u;   // by the caller
-    if (splits == 0u) splits = trellis_default_splits(rows, in_features, out_features, tile_words, state->sms);
-    const uint64_t flags = planned ? 0u : trellis_flag_bytes(out_features, splits);
+    const bool open = splits == 0u, joined = open && rows <= kMostFusedRows;   // joined: in the linear's launch
+    if (open) splits = trellis_default_splits(rows, in_features, out_features, tile_words, state->sms);
+    const uint64_t flags = joined ? trellis_flag_bytes(out_features, splits) : 0u;
     const uint64_t partials = splits > 1u ? (uint64_t)splits * rows * out_features * 4u : 0u;
     if (rows > 65535u || segments > 65535u || splits > 65535u || flags + partials > scratch_bytes || ((uintptr_t)scratch & 15u) != 0)
         return EUHEDRAL_CUDA_SIZE_OVERFLOW;
@@ -1035,18 +1038,16 @@ static int trellis_linear(unsigned char* scratch, uint64_t scratch_bytes, const 
     job.svh = static_cast<const uint16_t*>(svh);
     job.out = static_cast<uint16_t*>(output);
     cudaError_t e = cudaSuccess;
-    if (splits > 1u) {
-        job.partials = reinterpret_cast<float*>(scratch + flags);
-        if (!planned) {
-            job.flags = reinterpret_cast<unsigned long long*>(scratch);
-            job.tag = g_trellis_tag.fetch_add(0x9E3779B97F4A7C15ull, std::memory_order_relaxed);
-        } else if (rows > kMostFusedRows) {
-            const uint64_t activations = ((uint64_t)segments * rows * in_features * 2u + 255u) & ~255ull;
-            if (activations + partials <= scratch_bytes) {
-                job.activations = reinterpret_cast<const uint16_t*>(scratch);
-                job.partials = reinterpret_cast<float*>(scratch + activations);
-                e = launch_trellis_rotate(input, suh, scratch, (int)rows, (int)in_features, (int)segments, 0);
-            }
+    if (splits > 1u) job.partials = reinterpret_cast<float*>(scratch + flags);
+    if (joined) {
+        job.flags = reinterpret_cast<unsigned long long*>(scratch);
+        job.tag = g_trellis_tag.fetch_add(0x9E3779B97F4A7C15ull, std::memory_order_relaxed);
+    } else if (rows > kMostFusedRows && (open || splits > 1u)) {
+        const uint64_t activations = ((uint64_t)segments * rows * in_features * 2u + 255u) & ~255ull;
+        if (activations + partials <= scratch_bytes) {
+            job.activations = reinterpret_cast<const uint16_t*>(scratch);
+            job.partials = reinterpret_cast<float*>(scratch + activations);
+            e = launch_trellis_rotate(input, suh, scratch, (int)rows, (int)in_features, (int)segments, 0);
         }
     }
     job.rows = (int)rows;
@@ -1055,7 +1056,7 @@ static int trellis_linear(unsigned char* scratch, uint64_t scratch_bytes, const 
     job.splits = (int)splits;
     job.s = (int)segments;
     if (e == cudaSuccess) e = launch_trellis_linear_width((int)tile_words, static_cast<const uint16_t*>(words), job, state->error_word);
-    if (e == cudaSuccess && planned) e = launch_trellis_finish(job.partials, (int)splits, svh, output, (int)rows, (int)out_features);
+    if (e == cudaSuccess && splits > 1u && !joined) e = launch_trellis_finish(job.partials, (int)splits, svh, output, (int)rows, (int)out_features);
     return finish(e);
 }
 
@@ -1067,6 +1068,7 @@ int euhedral_b200_linear_trellis_bf16_static(const void* input, const void* word
     return trellis_linear(nullptr, 0, input, words, suh, svh, segment_ends, output, rows, in_features, out_features, tile_words, segments, splits);
 }
 
+// Flags and partial sums, which is what callers have sized by; the room for rotated activations, from 9 rows on, is theirs to add.
 uint64_t euhedral_b200_linear_trellis_scratch_bytes(uint32_t rows, uint32_t in_features, uint32_t out_features, uint32_t segments, uint32_t splits) {
     (void)segments;
     const uint32_t most = splits != 0u ? splits : std::max(1u, in_features / 256u);

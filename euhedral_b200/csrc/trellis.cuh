@@ -19,8 +19,8 @@
 //     the tensor core (two m16n8k32 u8 MMAs against a 0/1 selector, accumulator preset to the FP16 bit pattern 0x6400),
 //     which also hands each lane the values in the order of its FP16 A fragment; the 16 k of a tile reach the FP16 MMA in
 //     a fixed permutation that the activations in shared memory follow.
-//   * The K splits of a host's plan, several waves of CTAs, are added by a finish launch. Those of the count that a call picks itself
-//     (one wave) meet without a second launch and without a counter that would need clearing: a CTA stores its FP32
+//   * The K splits are added by a finish launch. Up to 8 rows, those of the count that a call picks itself (one wave)
+//     meet without a second launch and without a counter that would need clearing: a CTA stores its FP32
 //     partials, publishes a flag holding this call's tag, and reads the flags of its column block; whoever sees all of
 //     them set adds the partials in split order, rotates, scales and writes BF16, then unsets the flags (a launch replayed
 //     from a CUDA graph carries the same tag again). Two CTAs that finish together may both do that; they write the same bits.
@@ -64,6 +64,7 @@ __host__ __device__ inline int chunk_tiles(int groups, int live) {
     const int fit = (int)((act_bytes(groups) / (uint32_t)live - 32u) / 32u) & ~7;
     return fit < kChunkLimit ? fit : kChunkLimit;
 }
+constexpr int kCopyAhead = 2;                         // pairs of rotated blocks a warp has on their way from the scratch (3 and 4: 1 and 4 % slower)
 constexpr int kDecodeResident = 3;                    // CTAs of the BF16 decode an SM holds: 4 and 5 leave too few registers (106 and 107 us)
 constexpr int kBatch = 4;                             // tiles along k that a warp of the BF16 decode takes at a time
 constexpr uint32_t kWaitFailed = 4u;                  // error bit: a stage did not arrive (or was never freed)
@@ -102,19 +103,21 @@ __device__ __forceinline__ void finish128(float (&v)[4], const uint16_t* __restr
 }
 
 // One warp: partials[i * stride + 4 lane ..] of splits i = 0 .. splits - 1 added in that order (read past L1: other SMs
-// wrote them), then finish128. The loads of kPartialsAhead splits are in flight together: one by one they cost a trip to L2 each, and
-// a finish launch of 20 splits took 7.4 us.
-constexpr int kPartialsAhead = 16;
+// wrote them), then finish128. The loads of AHEAD splits are in flight together: one by one they cost a trip to L2 each, and
+// a finish launch of 20 splits took 7.4 us. In the linear's own tail, where 72 registers are all there is, 16 loads
+// spill, each spilled one a trip of its own: 3 to 6 % of a linear of one row, and half of one of 32 rows, which the tail no longer adds.
+constexpr int kFinishAhead = 16, kJoinAhead = 12;
+template <int AHEAD>
 __device__ __forceinline__ void add_and_finish128(const float* __restrict__ partials, size_t stride, int splits,
         const uint16_t* __restrict__ svh, uint16_t* __restrict__ out, int lane) {
     float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    for (int first = 0; first < splits; first += kPartialsAhead) {
-        float4 part[kPartialsAhead];
+    for (int first = 0; first < splits; first += AHEAD) {
+        float4 part[AHEAD];
 #pragma unroll
-        for (int i = 0; i < kPartialsAhead; ++i)
+        for (int i = 0; i < AHEAD; ++i)
             if (first + i < splits) part[i] = __ldcg(reinterpret_cast<const float4*>(partials + (size_t)(first + i) * stride) + lane);
 #pragma unroll
-        for (int i = 0; i < kPartialsAhead; ++i) {
+        for (int i = 0; i < AHEAD; ++i) {
             if (first + i >= splits) break;
             const bool start = first + i == 0;   // not 0 + the first: a sum of -0 stays one
             v[0] = start ? part[i].x : __fadd_rn(v[0], part[i].x);
@@ -228,7 +231,7 @@ __global__ void __launch_bounds__(256) finish_kernel(const float* __restrict__ p
     eb::pdl_wait();
     if (task >= (long long)rows * blocks) return;
     const size_t at = (size_t)(task / blocks) * n + (size_t)(task % blocks) * 128;
-    add_and_finish128(partials + at, (size_t)rows * n, splits, svh + (size_t)(task % blocks) * 128, out + at, lane);
+    add_and_finish128<kFinishAhead>(partials + at, (size_t)rows * n, splits, svh + (size_t)(task % blocks) * 128, out + at, lane);
 }
 
 // rotated bf16: the product of segment g starts at element rows * start_g with row stride width_g (start_g, width_g from the
@@ -427,7 +430,7 @@ __global__ void __launch_bounds__(256, kDecodeResident) decode_bf16_kernel(const
 }
 
 // What a launch of the linear works on. `activations` (the scratch's fragment-order FP16 [s][rows][k], written by a
-// rotate launch) or, when it is null, x and suh. `flags` null: the partials of a split K are left for a finish launch.
+// rotate launch) or, when it is null, x and suh. `flags` null, as it always is above 8 rows: the partials of a split K are left for a finish launch.
 struct Job {
     const uint16_t* activations;
     const uint16_t* x;
@@ -513,26 +516,56 @@ __global__ void __launch_bounds__(kThreads, resident(W, P)) linear_kernel(const 
             const int c1 = min(last, (c0 / chunk + 1) * chunk);
             const int block0 = c0 >> 3, blocks = ((c1 + 7) >> 3) - block0;
             decoders_sync();   // nobody reads the chunk before any more
-            for (int task = warp; task < live * blocks; task += kDecodeWarps) {
-                const int r = task % live, block = block0 + task / live;
-                uint8_t* to = act + r * stride + (block - block0) * 256 + (lane >> 2) * 32;   // this lane's group of 16 k
-                const int a = lane & 3;
-                if (job.activations == nullptr) {
-                    float v[4];
-                    rotate128(job.x + (size_t)(row_base + r) * k + (size_t)block * 128, job.suh + (size_t)seg * k + (size_t)block * 128, lane, v);
-                    // the lane's k are 4a .. 4a+3 of its group: (4a, 4a+2) are neighbours in the order above, (4a+1, 4a+3) 8 further
-                    uint32_t* pair = reinterpret_cast<uint32_t*>(to) + 2 * (a & 1) + (a >> 1);
-                    pair[0] = half_pair(v[0], v[2]);
-                    pair[4] = half_pair(v[1], v[3]);
-                } else {
-                    // the scratch holds k = 2a, 2a+1, 2a+8, 2a+9 of the group at 4a
-                    const uint2 from = *reinterpret_cast<const uint2*>(
-                            job.activations + ((size_t)seg * rows + row_base + r) * k + (size_t)block * 128 + 4 * lane);
-                    uint16_t* half = reinterpret_cast<uint16_t*>(to) + 4 * (a >> 1) + (a & 1);
-                    half[0] = (uint16_t)(from.x & 0xFFFFu);
-                    half[8] = (uint16_t)(from.x >> 16);
-                    half[2] = (uint16_t)(from.y & 0xFFFFu);
-                    half[10] = (uint16_t)(from.y >> 16);
+            if (P > 1 && job.activations != nullptr) {
+                // Half a warp a block, 16 bytes a lane, in two 8-byte stores. One block a warp at a time, in eight 2-byte stores a lane, each load
+                // was waited for by itself: 34816 x 5120 at 3 bits and 12 / 17 / 24 / 32 / 63 rows 78 / 93 / 101 / 128 / 250
+                // us, now 74 / 91 / 94 / 117 / 229.
+                const int tasks = live * blocks, half_warp = lane >> 4, piece = lane & 15;
+                int r = (2 * warp + half_warp) % live, at = (2 * warp + half_warp) / live;   // of the lane's next block
+                auto next = [live](int& row, int& block) {
+                    for (row += 2 * kDecodeWarps; row >= live; ++block) row -= live;
+                };
+                for (int first_task = 2 * warp; first_task < tasks; first_task += kCopyAhead * 2 * kDecodeWarps) {
+                    uint2 from[kCopyAhead][2];
+                    int row = r, block = at;
+#pragma unroll
+                    for (int i = 0; i < kCopyAhead; ++i, next(row, block))
+                        if (first_task + half_warp + i * 2 * kDecodeWarps < tasks) {
+                            const uint2* eight = reinterpret_cast<const uint2*>(
+                                    job.activations + ((size_t)seg * rows + row_base + row) * k + (size_t)(block0 + block) * 128) + 2 * piece;
+                            from[i][0] = eight[0], from[i][1] = eight[1];
+                        }
+#pragma unroll
+                    for (int i = 0; i < kCopyAhead; ++i, next(r, at))
+                        if (first_task + half_warp + i * 2 * kDecodeWarps < tasks) {
+                            // the scratch holds k = 2a, 2a+1, 2a+8, 2a+9 of a group of 16 at 4a; the lane has those of a = 2h and 2h + 1
+                            uint2* to = reinterpret_cast<uint2*>(act + r * stride + at * 256 + (piece >> 1) * 32 + (piece & 1) * 8);
+                            to[0] = make_uint2(__byte_perm(from[i][0].x, from[i][1].x, 0x5410), __byte_perm(from[i][0].y, from[i][1].y, 0x5410));
+                            to[2] = make_uint2(__byte_perm(from[i][0].x, from[i][1].x, 0x7632), __byte_perm(from[i][0].y, from[i][1].y, 0x7632));
+                        }
+                }
+            } else {
+                for (int task = warp; task < live * blocks; task += kDecodeWarps) {
+                    const int r = task % live, block = block0 + task / live;
+                    uint8_t* to = act + r * stride + (block - block0) * 256 + (lane >> 2) * 32;   // this lane's group of 16 k
+                    const int a = lane & 3;
+                    if (job.activations == nullptr) {
+                        float v[4];
+                        rotate128(job.x + (size_t)(row_base + r) * k + (size_t)block * 128, job.suh + (size_t)seg * k + (size_t)block * 128, lane, v);
+                        // the lane's k are 4a .. 4a+3 of its group: (4a, 4a+2) are neighbours in the order above, (4a+1, 4a+3) 8 further
+                        uint32_t* pair = reinterpret_cast<uint32_t*>(to) + 2 * (a & 1) + (a >> 1);
+                        pair[0] = half_pair(v[0], v[2]);
+                        pair[4] = half_pair(v[1], v[3]);
+                    } else {
+                        // the scratch holds k = 2a, 2a+1, 2a+8, 2a+9 of the group at 4a
+                        const uint2 from = *reinterpret_cast<const uint2*>(
+                                job.activations + ((size_t)seg * rows + row_base + r) * k + (size_t)block * 128 + 4 * lane);
+                        uint16_t* half = reinterpret_cast<uint16_t*>(to) + 4 * (a >> 1) + (a & 1);
+                        half[0] = (uint16_t)(from.x & 0xFFFFu);
+                        half[8] = (uint16_t)(from.x >> 16);
+                        half[2] = (uint16_t)(from.y & 0xFFFFu);
+                        half[10] = (uint16_t)(from.y >> 16);
+                    }
                 }
             }
             decoders_sync();
@@ -607,7 +640,7 @@ __global__ void __launch_bounds__(kThreads, resident(W, P)) linear_kernel(const 
         }
     }
 
-    if (splits > 1 && job.flags != nullptr) {
+    if (P == 1 && splits > 1 && job.flags != nullptr) {   // the only kernel that is asked for it
         decoders_sync();   // every thread's partials are stored; the fence of thread 0 below orders them before the flag
         if (warp == 0) {
             volatile unsigned long long* flags = job.flags + (size_t)blockIdx.x * splits;
@@ -626,7 +659,7 @@ __global__ void __launch_bounds__(kThreads, resident(W, P)) linear_kernel(const 
         decoders_sync();
         if (last_arrival != 0) {
             for (int row = warp; row < rows; row += kDecodeWarps)
-                add_and_finish128(job.partials + (size_t)row * n + column0, (size_t)rows * n, splits, job.svh + column0,
+                add_and_finish128<kJoinAhead>(job.partials + (size_t)row * n + column0, (size_t)rows * n, splits, job.svh + column0,
                         job.out + (size_t)row * n + column0, lane);
             // The block is done: its flags stop carrying the tag, so that the same launch replayed from a CUDA graph (same
             // tag) starts from flags that are not set. A CTA that reads them only now sees them unset and leaves the block

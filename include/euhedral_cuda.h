@@ -167,14 +167,15 @@ EUHEDRAL_CUDA_EXPORT void euhedral_b200_select_native_pairs(int enabled);
 
 /* No counterpart in the reference, whose Java host plans a trellis linear as three launches through the kernel table
  * (core/.../artifact/format/TrellisFormat.java:484-567). Here the whole linear is ONE call. splits = 0 takes this device's
- * one-wave split count and one launch: the activations are rotated inside the kernel, and the CTA that finishes a column block
- * last adds the K splits in split order, rotates, scales and writes BF16. A count that the caller names runs as the plan's
- * launches without the host's way between them: up to 8 rows, or in a scratch that has no room for the rotated activations in
- * front of the partial sums (align256(segments*rows*in*2) bytes), the rotation is part of the linear's launch. Caller scratch of at
+ * one-wave split count. Up to 8 rows that is one launch: the activations are rotated inside the kernel, and the CTA that finishes a
+ * column block last adds the K splits in split order, rotates, scales and writes BF16. Else, and with a count that the caller names, it is
+ * the plan's launches without the host's way between them: up to 8 rows, or in a scratch that has no room for the rotated activations
+ * in front of the partial sums (align256(segments*rows*in*2) bytes), the rotation is part of the linear's launch. Caller scratch of at
  * least euhedral_b200_linear_trellis_scratch_bytes(...) bytes (16-byte aligned, contents arbitrary, 0 bytes with one split): a
- * 64-bit flag per column block and split (splits = 0), then the FP32 partial sums of the splits; a named count needs the partial
- * sums only. With the reference host's count (TrellisFormat.java:369-376) the result is bit for bit that of the three table launches; an N-shard passes the split count of the whole tensor so that
- * it reproduces the whole tensor's bits. Arguments otherwise as euhedral_b200_linear_trellis_bf16_static. */
+ * 64-bit flag per column block and split (the one launch), then the FP32 partial sums of the splits; the other calls need the partial
+ * sums only, and from 9 rows on are faster with the room for the rotated activations added. With the reference host's count
+ * (TrellisFormat.java:369-376) the result is bit for bit that of the three table launches; an N-shard passes the split count of the whole
+ * tensor so that it reproduces the whole tensor's bits. Arguments otherwise as euhedral_b200_linear_trellis_bf16_static. */
 EUHEDRAL_CUDA_EXPORT uint64_t euhedral_b200_linear_trellis_scratch_bytes(uint32_t rows, uint32_t in_features,
         uint32_t out_features, uint32_t segments, uint32_t splits);
 EUHEDRAL_CUDA_EXPORT int euhedral_b200_linear_trellis_bf16(const void* input, const void* words, const void* suh,

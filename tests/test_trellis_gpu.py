@@ -70,18 +70,26 @@ class DeviceLinear:
                                         .int32(self.n))
         return self.dev.get(d_y, np.uint16, (rows, self.n))
 
-    def one_launch(self, x_bits, **select):
-        """The linear with a split count of its own (splits = 0): (output, that count, read off the flags that the launch leaves)."""
-        rows = x_bits.shape[0]
-        need = self.dev.gpu.lib.euhedral_b200_linear_trellis_scratch_bytes(rows, self.k, self.n, len(self.ends), 0)
+    def own_count(self, x_bits, room=0, **select):
+        """The linear with a split count of its own (splits = 0): (output, that count). Up to 8 rows it is read off the flags that the
+        launch leaves, of more rows, in a scratch with room for the rotated activations, off the length of what is written."""
+        rows, lib = x_bits.shape[0], self.dev.gpu.lib
+        activations = layouts.align_up(len(self.ends) * rows * self.k * 2, 256) if rows > 8 and room else 0
+        need = lib.euhedral_b200_linear_trellis_scratch_bytes(rows, self.k, self.n, len(self.ends), 0) + activations
         d_x, d_y, d_s = self.dev.put(x_bits), self.dev.empty(rows * self.n * 2), self.dev.empty(max(need, 256), fill=0xA5)
         with self.dev.submit(**select) as gpu:
             gpu.linear_trellis_bf16(d_x.data_ptr(), *[t.data_ptr() for t in self.tensors[:3]], self.tensors[3].data_ptr(), d_y.data_ptr(),
                                     d_s.data_ptr(), need, rows, self.k, self.n, self.w, len(self.ends), 0)
-        flags = self.dev.get(d_s, np.uint64, (max(need, 256) // 8,))
-        joined = int(np.count_nonzero(flags == flags[0])) if flags[0] != 0xA5A5A5A5A5A5A5A5 else 0   # every block's flags end as one value
-        assert joined % (self.n // 128) == 0
-        return self.dev.get(d_y, np.uint16, (rows, self.n)), max(1, joined // (self.n // 128))
+        left = self.dev.get(d_s, np.uint64, (max(need, 256) // 8,))
+        count = 1
+        if rows <= 8 and left[0] != 0xA5A5A5A5A5A5A5A5:
+            blocks = self.n // 128
+            joined = int(np.count_nonzero(left == left[0]))   # every block's flags end as one value
+            assert joined % blocks == 0
+            count = joined // blocks
+        elif rows > 8:
+            count = -(-(8 * int(np.flatnonzero(left != 0xA5A5A5A5A5A5A5A5)[-1]) + 8 - activations) // (rows * self.n * 4))
+        return self.dev.get(d_y, np.uint16, (rows, self.n)), count
 
     def one_call(self, x_bits, splits, **select):
         """The same linear as one call (euhedral_b200_linear_trellis_bf16) with the split count given."""
@@ -240,20 +248,21 @@ def test_operator_is_bitwise_the_table_launches(dev, k, n, w, ends, target, rows
     assert np.array_equal(dev.get(d_y, np.uint16, (rows, n)), expect)
 
 
-# The launch that picks its split count itself and whose CTAs join the splits by flags, on both sides of every group of eight rows, against
-# the plan's launches at the count that the flags show. One and several segments, whole and half-step widths.
+# The call that picks its split count itself (up to 8 rows one launch whose CTAs join the splits by flags) against the plan's launches at
+# that count, on both sides of every group of eight rows, with and without room for the rotated activations. One and several segments,
+# whole and half-step widths.
 @pytest.mark.parametrize("k,n,w,ends", [(2048, 512, 48, [256, 512]), (1408, 384, 64, [384]), (4224, 256, 56, [128, 256]), (5120, 1024, 96, [1024])])
-@pytest.mark.parametrize("rows", [1, 8, 9, 16, 17, 25, 32, 33, 40, 63])
-def test_joined_launch_is_bitwise_the_table_launches(dev, k, n, w, ends, rows):
+@pytest.mark.parametrize("rows", [1, 5, 8, 9, 16, 17, 24, 25, 32, 33, 40, 63, 97])
+def test_own_split_count_is_bitwise_the_table_launches(dev, k, n, w, ends, rows):
     rng = np.random.default_rng(1000 * rows + k)
     payload, suh, svh = random_object(rng, k, n, w, segments=len(ends))
     linear = DeviceLinear(dev, payload, suh, svh, ends, 140)
     x = random_x(rng, rows, k)
-    got, splits = linear.one_launch(x, pdl=True)
+    got, splits = linear.own_count(x, room=1, pdl=True)
     assert splits > 1
     assert np.array_equal(got, linear.table_launches(x, splits))
-    again, same = linear.one_launch(x)
-    assert same == splits and np.array_equal(again, got)
+    again, _ = linear.own_count(x)
+    assert np.array_equal(again, got)
 
 
 def test_golden_linear_fixture(dev, golden):
@@ -353,8 +362,9 @@ def test_table_abi(dev):
 @pytest.mark.parametrize("rows", [5, 20, 40])
 @pytest.mark.parametrize("splits", [0, 9])
 def test_one_call_linear_replayed_from_a_graph(dev, rows, splits):
-    """A captured launch that joins its splits (splits = 0) carries the same flag tag on every replay: each replay must still wait for its
-    own partial sums (the CTA that finishes a column block unsets the block's flags). A named count beside it."""
+    """A captured launch that joins its splits (splits = 0, up to 8 rows) carries the same flag tag on every replay: each replay must
+    still wait for its own partial sums (the CTA that finishes a column block unsets the block's flags). More rows and a named count
+    beside it."""
     torch = dev.torch
     rng = np.random.default_rng(45 + rows)
     k, n, w = 2048, 512, 48
@@ -363,7 +373,7 @@ def test_one_call_linear_replayed_from_a_graph(dev, rows, splits):
     lib = dev.gpu.lib
     need = lib.euhedral_b200_linear_trellis_scratch_bytes(rows, k, n, 1, splits)
     xs = [random_x(rng, rows, k) for _ in range(4)]
-    count = splits or linear.one_launch(xs[0])[1]
+    count = splits or linear.own_count(xs[0], room=1)[1]
     assert count > 1
     d_x, d_y, d_s = dev.put(xs[0]), dev.empty(rows * n * 2), dev.empty(need)
     t = [h.data_ptr() for h in linear.tensors]
@@ -386,8 +396,7 @@ def test_one_call_linear_replayed_from_a_graph(dev, rows, splits):
 
 
 def test_one_launch_linear_replayed_from_a_graph(dev):
-    """A captured one-launch linear carries the same flag tag on every replay: each replay must still wait for its own
-    partial sums (the CTA that finishes a column block unsets the block's flags)."""
+    """A captured linear with a named split count, replayed with changing inputs, against calls of its own."""
     torch = dev.torch
     rng = np.random.default_rng(45)
     k, n, w, rows = 2048, 512, 48, 5
