@@ -1162,9 +1162,10 @@ static uint32_t encoder_ctas(uint32_t count, int sms) { return std::min(count, (
 static uint64_t encoder_scratch(uint32_t count, uint32_t ka, int sms) {
     return std::min((uint64_t)std::max(1u, count), (uint64_t)sms * trellis_encode::kGroups) * trellis_encode::history_bytes((int)ka);
 }
-// The least that is taken. At 2 and 2.5 bits a slab has 4 MB and two a CTA make 1.2 GB: half of that will do, with one tile in flight.
+// The least that is taken. At 2 and 2.5 bits a slab has 4 MB and two an SM make 1.2 GB: half of that will do, with half as many CTAs.
 static uint64_t encoder_least_scratch(uint32_t count, uint32_t ka, int sms) {
-    return ka == 2u ? (uint64_t)encoder_ctas(count, sms) * trellis_encode::history_bytes((int)ka) : encoder_scratch(count, ka, sms);
+    const uint64_t all = encoder_scratch(count, ka, sms), half = (uint64_t)std::max(encoder_ctas(count, sms), 2u) * trellis_encode::history_bytes((int)ka);
+    return ka == 2u ? std::min(all, half) : all;
 }
 
 uint64_t euhedral_b200_trellis_encode_scratch_bytes(uint32_t count, uint32_t tile_words) {
@@ -1187,14 +1188,16 @@ int euhedral_b200_trellis_encode_tiles(const void* tiles, uint32_t count, uint32
     const int status = bind(&state);
     if (status != EUHEDRAL_CUDA_SUCCESS) return status;
     if (encoder_least_scratch(count, ka, state->sms) > scratch_bytes) return EUHEDRAL_CUDA_SIZE_OVERFLOW;
-    auto run = [&](auto kernel, int threads, uint32_t shared, uintptr_t slabs, auto... more) {
-        return launch(kOrdered, kernel, dim3(encoder_ctas(count, state->sms)), dim3(threads), shared, 1u, static_cast<const float*>(tiles), count,
-                static_cast<uint16_t*>(states), static_cast<float*>(decoded), reinterpret_cast<uint8_t*>(slabs), more...);
+    // CTA b uses slabs b and, if it has a second tile, b + CTAs: with fewer slabs than the tiles in flight need, as many CTAs as have two each
+    const uint32_t ctas = scratch_bytes >= encoder_scratch(count, ka, state->sms)
+            ? encoder_ctas(count, state->sms) : (uint32_t)(scratch_bytes / trellis_encode::history_bytes((int)ka) / trellis_encode::kGroups);
+    auto run = [&](auto kernel, int threads, uint32_t shared, uintptr_t slabs) {
+        return launch(kOrdered, kernel, dim3(ctas), dim3(threads), shared, 1u, static_cast<const float*>(tiles), count,
+                static_cast<uint16_t*>(states), static_cast<float*>(decoded), reinterpret_cast<uint8_t*>(slabs));
     };
     // The register kernel stores 16 bytes of costs at a time; the last row of a slab, which it leaves alone, has room to round any scratch up.
-    const uint32_t beside = scratch_bytes >= encoder_scratch(count, ka, state->sms) ? 1u : 0u;
     auto registers = [&](auto kernel) {
-        return run(kernel, trellis_encode::kRegisterThreads, trellis_encode::register_shared_bytes((int)ka), ((uintptr_t)scratch + 15u) & ~(uintptr_t)15u, beside);
+        return run(kernel, trellis_encode::kRegisterThreads, trellis_encode::register_shared_bytes((int)ka), ((uintptr_t)scratch + 15u) & ~(uintptr_t)15u);
     };
     auto shared = [&](auto kernel) { return run(kernel, trellis_encode::kThreads, trellis_encode::shared_bytes((int)ka), (uintptr_t)scratch); };
     cudaError_t e = cudaErrorInvalidValue;

@@ -19,8 +19,8 @@
 // Bound: packed FP16 arithmetic, which one of the two FMA pipes does at two cycles an instruction: a subtraction and a fused
 // multiply-add per pair of states, 1024 cycles a position and tile. The kernel for more bits (viterbi_kernel) reads the values from
 // shared memory for each position and selects winners with logic instructions, seven instructions per pair; 2 to 4 bits ran on it
-// before. 4096 tiles at 2 / 2.5 / 3 / 3.5 / 4 bits 22.1 / 23.7 / 15.6 / 16.1 / 16.8 -> 9.9 / 10.2 / 10.1 / 10.1 / 10.2 ms (2 and 2.5 bits with one
-// tile in flight 14.2 and 14.4); 1024 x 1024 weights at 3 bits (4096 tiles and 1800 of the scale's search): 25.4 -> 17.1 ms.
+// before. 4096 tiles at 2 / 2.5 / 3 / 3.5 / 4 bits 22.1 / 23.7 / 15.6 / 16.1 / 16.8 -> 9.9 / 10.2 / 10.1 / 10.1 / 10.2 ms (2 and 2.5 bits in half the
+// scratch 19.4 and 20.3); 1024 x 1024 weights at 3 bits (4096 tiles and 1800 of the scale's search): 25.4 -> 17.1 ms.
 //
 // 5 and 6 bits (viterbi_kernel; a thread's states there would not share predecessors in registers): one CTA per SM, 1024 threads,
 // persistent over the tile list. The CTA first writes the codebook value of every state to shared memory (128 KB of FP16) - a
@@ -143,11 +143,11 @@ __device__ __forceinline__ uint32_t reverse5(uint32_t v) { return __brev(v) >> 2
 
 // tiles f32 [count][256] -> states u16 [count][256] (and, when asked for, their codebook values as f32). slabs: history_bytes(KA) bytes
 // per tile in flight, at most count of them, on a 16-byte boundary; the last row of the last one (2 (65536 >> KA) bytes) is not touched.
-// beside: 1: a CTA has two tiles in flight; 0: one, whose ways back are waited for, for slabs that have no room for two.
-//   grid: at most count CTAs (CTA b takes tiles b, b + gridDim.x, ...), block kRegisterThreads, dynamic shared register_shared_bytes(KA).
+//   grid: at most count CTAs (CTA b takes tiles b, b + gridDim.x, ...; two at a time), block kRegisterThreads, dynamic shared
+//   register_shared_bytes(KA).
 template <int KA, bool kHalfStep>
 __global__ void __launch_bounds__(kRegisterThreads, 1) register_kernel(const float* __restrict__ tiles, uint32_t count, uint16_t* __restrict__ states,
-        float* __restrict__ decoded, uint8_t* __restrict__ slabs, uint32_t beside) {
+        float* __restrict__ decoded, uint8_t* __restrict__ slabs) {
     extern __shared__ __align__(16) uint8_t smem[];
     constexpr int kMost = 65536 >> KA, KB = kHalfStep ? KA + 1 : KA;   // an even position brings KA bits, an odd one KB
     __shared__ __align__(4) __half weights[kGroups][256];
@@ -155,11 +155,10 @@ __global__ void __launch_bounds__(kRegisterThreads, 1) register_kernel(const flo
     __shared__ int entered[kGroups];   // the node that a tile's second pass enters position 0 from
     const int t = threadIdx.x, lane = t & 31;
     // Pass n: of the CTA's tiles 2 (n / 4) and 2 (n / 4) + 1 in turn; n / 2 odd: the second pass. A CTA's last tile may be without a
-    // partner, whose passes are then empty. One tile in flight: of tile n / 2; n odd: the second pass.
-    const uint32_t mine = (count - blockIdx.x + gridDim.x - 1u) / gridDim.x, passes = (mine + beside) >> beside << (beside + 1u);
-    auto slot_of = [&](uint32_t n) { return n & beside; };
-    auto tile_of = [&](uint32_t n) { return blockIdx.x + (uint64_t)((n >> (beside + 1u) << beside) + slot_of(n)) * gridDim.x; };
-    auto slab_of = [&](uint32_t n) { return reinterpret_cast<__half*>(slabs + (blockIdx.x + (uint64_t)slot_of(n) * gridDim.x) * history_bytes(KA)); };
+    // partner, whose passes are then empty.
+    const uint32_t mine = (count - blockIdx.x + gridDim.x - 1u) / gridDim.x, passes = (mine + 1u) / 2u * 4u;
+    auto tile_of = [&](uint32_t n) { return blockIdx.x + (uint64_t)((n >> 2) * 2u + (n & 1u)) * gridDim.x; };
+    auto slab_of = [&](uint32_t n) { return reinterpret_cast<__half*>(slabs + (blockIdx.x + (uint64_t)(n & 1u) * gridDim.x) * history_bytes(KA)); };
 
     if (t < kSearchers) {
         uint32_t values[1 << kHigh][4];
@@ -173,8 +172,8 @@ __global__ void __launch_bounds__(kRegisterThreads, 1) register_kernel(const flo
         __half *row_even = reinterpret_cast<__half*>(smem), *row_odd = row_even + kMost;   // costs after an even and an odd position
 #pragma unroll 1
         for (uint32_t n = 0; n < passes; ++n) {
-            const uint32_t slot = slot_of(n), second = (n >> beside) & 1u;
-            if (n > beside) meet(4u + slot);   // the way back of the slot's pass before has been walked: its slab, weights and result
+            const uint32_t slot = n & 1u, second = (n >> 1) & 1u;
+            if (n >= 2u) meet(4u + slot);   // the way back of pass n - 2 has been walked: its slab, weights and result
             if (tile_of(n) < count) {
                 if (second == 0u && t < 256) weights[slot][t] = __float2half_rn(tiles[tile_of(n) * 256u + (uint32_t)t]);
                 searchers_sync();
@@ -204,12 +203,12 @@ __global__ void __launch_bounds__(kRegisterThreads, 1) register_kernel(const flo
             }
             announce(2u + slot);
         }
-        // the last ways back end on barriers that every thread must have come to
-        for (uint32_t slot = 0; slot <= beside; ++slot) meet(4u + slot);
+        // the ways back of the last two passes end on barriers that every thread must have come to
+        for (uint32_t n = passes; n < passes + 2u; ++n) meet(4u + (n & 1u));
     } else {
 #pragma unroll 1
         for (uint32_t n = 0; n < passes; ++n) {
-            const uint32_t slot = slot_of(n), second = (n >> beside) & 1u;
+            const uint32_t slot = n & 1u, second = (n >> 1) & 1u;
             meet(2u + slot);
             const uint64_t tile = tile_of(n);
             if (tile < count) {

@@ -235,7 +235,7 @@ EUHEDRAL_CUDA_EXPORT int euhedral_b200_linear_bf16(const void* input, const void
  * of 32, 40, 48, 56, 64, 80, 96 (else -5). decoded (may be null): the states' codebook values, float [count][256]. words
  * (may be null): the packed payload, int16 [count][tile_words], as the linears read it. scratch: at least
  * euhedral_b200_trellis_encode_scratch_bytes(count, tile_words) bytes of device memory (-2 if smaller), at any multiple of 4: room for two tiles in flight on each SM. At 32 and 40 words that is 8 MiB an SM, 1.24 GB on 148; half of
- * it, 4 MiB for each of min(count, SMs), is taken there too, with one tile in flight (4096 tiles 14.2 ms instead of 10.1). */
+ * it, 4 MiB for each of min(count, SMs), is taken there too, at half the speed. */
 EUHEDRAL_CUDA_EXPORT uint64_t euhedral_b200_trellis_encode_scratch_bytes(uint32_t count, uint32_t tile_words);
 EUHEDRAL_CUDA_EXPORT int euhedral_b200_trellis_encode_tiles(const void* tiles, uint32_t count, uint32_t tile_words, void* states,
         void* decoded, void* words, void* scratch, uint64_t scratch_bytes);

@@ -111,7 +111,7 @@ def test_scratch_at_any_multiple_of_four(dev, w, ka, mask, offset):
 @pytest.mark.parametrize("w,ka,mask", [(32, 2, 0), (40, 2, 0xAAAA)])
 @pytest.mark.parametrize("count", [1, 2, 150, 299])
 def test_two_bits_in_a_slab_an_sm(dev, w, ka, mask, count):
-    """At 2 and 2.5 bits a scratch of one slab of 4 MB for each SM will do (a tile in flight), also at an odd address; less is refused."""
+    """At 2 and 2.5 bits a scratch of one slab of 4 MB for each SM will do (half as many CTAs), also at an odd address; less is refused."""
     rng = np.random.default_rng(w + count)
     tiles = rng.standard_normal((count, 256)).astype(np.float32)
     least = min(count, dev.gpu.multiprocessor_count()) << 22
