@@ -980,9 +980,9 @@ uint64_t euhedral_b200_static_scratch_bytes(void) { return kStaticScratchBytes; 
 // that names one split need not bring a scratch.
 static std::atomic<unsigned long long> g_trellis_tag{0x9E3779B97F4A7C15ull ^ (unsigned long long)(uintptr_t)&g_trellis_tag};
 
-// The split count of a one-launch trellis linear when the caller leaves it open: the one that needs the fewest tile rows
+// The split count of a trellis linear when the caller leaves it open: the one that needs the fewest tile rows
 // per SM slot in sequence - waves of resident CTAs times the tile rows of a split, plus a few tile rows' worth of rotate,
-// flag exchange and in-order sum for every split - among splits of 20 tile rows or more.
+// exchange and in-order sum for every split - among splits of 20 tile rows or more.
 static uint32_t trellis_default_splits(uint32_t rows, uint32_t in_features, uint32_t out_features, uint32_t tile_words, int sms) {
     const uint32_t groups = (uint32_t)trellis::groups_of((int)rows);
     const uint32_t shared = (uint32_t)trellis::kStages * trellis::kStageTiles * 16u * tile_words + trellis::act_bytes((int)groups) + 1024u + 128u;

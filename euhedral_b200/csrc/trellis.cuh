@@ -8,7 +8,7 @@
 //   entry 5 "decode":   the rotated weight as BF16 [n][k]
 // and the scratch layout between them (activations, then FP32 partials [split][row][n]).
 //
-// How it runs here: ONE kernel does a whole linear. A CTA owns 128 output columns and one K split.
+// How it runs here: ONE kernel does a linear but for the sum of its K splits. A CTA owns 128 output columns and one K split.
 //   * Warp 8 only requests payload: one tiled TMA copy per stage (16 tile rows x the CTA's 8 tiles), a ring of stages
 //     with a full and an empty mbarrier each, so the eight decoding warps drift apart by up to a ring instead of meeting
 //     at a CTA barrier every stage.

@@ -241,8 +241,8 @@ class CudaGpuMemory:
     def linear_trellis_bf16(self, input: int, words: int, suh: int, svh: int, ends: int, output: int, scratch: int, scratch_bytes: int,
                             rows: int, in_features: int, out_features: int, tile_words: int, segments: int, splits: int = 0) -> None:
         """A whole trellis linear as one call. No counterpart in the reference, whose host queues three table launches; same
-        bits for the same split count. splits = 0: the device's one-wave default, as one launch (activations rotated and K
-        splits joined inside the kernel)."""
+        bits for the same split count. splits = 0: the device's one-wave default, up to 8 rows as one launch (activations rotated
+        and K splits joined inside the kernel)."""
         self._check("trellis linear", self.lib.euhedral_b200_linear_trellis_bf16(
             input, words, suh, svh, ends, output, scratch, scratch_bytes, rows, in_features, out_features, tile_words, segments, splits))
 

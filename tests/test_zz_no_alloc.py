@@ -1,6 +1,6 @@
 """The trellis linear that brings its own scratch (a static device array inside the library), for callers that cannot
-allocate device memory when they call: two calls in a row through the C ABI must equal, bit for bit, the regular
-three-launch route with caller scratch. Collected last on purpose."""
+allocate device memory when they call: two calls in a row through the C ABI must equal, bit for bit, the plan's
+launches through the kernel table with caller scratch. Collected last on purpose."""
 
 import numpy as np
 import pytest
@@ -28,7 +28,7 @@ def test_static_scratch_linear_matches_caller_scratch_twice():
         d_words, d_suh, d_svh, d_ends = regular.tensors
         for call, rows in enumerate((5, 8)):        # two calls in a row share the array; the second reuses its bytes
             x = random_x(rng, rows, k)
-            expect = regular.linear(x)
+            expect = regular.table_launches(x, splits)
             d_x, d_y = dev.put(x), dev.empty(rows * n * 2)
             with dev.submit():
                 status = lib.euhedral_b200_linear_trellis_bf16_static(d_x.data_ptr(), d_words.data_ptr(), d_suh.data_ptr(), d_svh.data_ptr(),
@@ -42,7 +42,7 @@ def test_static_scratch_linear_matches_caller_scratch_twice():
         with dev.submit():
             assert lib.euhedral_b200_linear_trellis_bf16_static(d_x.data_ptr(), d_words.data_ptr(), d_suh.data_ptr(), d_svh.data_ptr(),
                                                                 d_ends.data_ptr(), d_y.data_ptr(), 3, k, n, w, 2, 1) == 0
-        assert np.array_equal(dev.get(d_y, np.uint16, (3, n)), one.linear(x))
+        assert np.array_equal(dev.get(d_y, np.uint16, (3, n)), one.table_launches(x, 1))
         # too large for the static array: refused before anything is launched
         assert lib.euhedral_b200_linear_trellis_bf16_static(d_x.data_ptr(), d_words.data_ptr(), d_suh.data_ptr(), d_svh.data_ptr(),
                                                             d_ends.data_ptr(), d_y.data_ptr(), 4096, k, n, w, 2, splits) == library.SIZE_OVERFLOW
